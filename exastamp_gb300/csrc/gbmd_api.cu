@@ -122,7 +122,30 @@ static void invalidate_list(gbmd_context* c) {
   drop_graph(c);
 }
 
-static void set_rlist(gbmd_context* c, double rcut_max) {
+// The FP64 re-test bands of the current potential for the current list radius.
+static int set_bands(gbmd_context* c) {
+  const double reach = c->rlist + c->list_buffer;
+  auto band = [&](double rc, float& lo, float& hi) {
+    const double w = band_rel(reach, rc);
+    lo = (float)(rc * rc * (1.0 - w));
+    hi = (float)(rc * rc * (1.0 + w));
+  };
+  if (c->pot == GBMD_POT_LJ || c->pot == GBMD_POT_LJ_MULTI) {
+    const int nt = c->lj.ntypes;
+    for (int q = 0; q < nt * nt; ++q) band(c->lj.p[q].rc, c->lj.p[q].rc2lo, c->lj.p[q].rc2hi);
+    if (c->pot == GBMD_POT_LJ_MULTI)
+      GBMD_CUDA(c, cudaMemcpyAsync(c->lj_tab_d, c->lj.p, sizeof(LJPair) * nt * nt, cudaMemcpyHostToDevice, c->stream));
+  } else if (c->pot == GBMD_POT_EAM_ALLOY) {
+    band(c->eam.rcut, c->eam.rc2lo, c->eam.rc2hi);
+  } else if (c->pot == GBMD_POT_EAM_JOHNSON) {
+    band(c->ej.rcut, c->ej.rc2lo, c->ej.rc2hi);
+  } else if (c->pot == GBMD_POT_EAM_SUTTON_CHEN) {
+    band(c->esc.rcut, c->esc.rc2lo, c->esc.rc2hi);
+  }
+  return GBMD_OK;
+}
+
+static int set_rlist(gbmd_context* c, double rcut_max) {
   const double R = rcut_max + c->skin;
   if (R != c->rlist) {
     c->rlist = R;
@@ -130,6 +153,7 @@ static void set_rlist(gbmd_context* c, double rcut_max) {
     c->maxnb = c->maxnb_out = 0;
   }
   invalidate_list(c);
+  return set_bands(c);
 }
 
 static double pot_rcut_max(const gbmd_context* c) {
@@ -757,8 +781,6 @@ static LJPair make_pair(double eps, double sig, double rc) {
   p.eps4f = (float)(4.0 * eps);
   p.ecutf = (float)p.ecut;
   p.rc2f = (float)p.rc2;
-  p.rc2lo = (float)(p.rc2 * (1.0 - 0x1p-12));
-  p.rc2hi = (float)(p.rc2 * (1.0 + 0x1p-12));
   return p;
 }
 
@@ -769,8 +791,7 @@ int gbmd_set_lj(gbmd_context* c, double epsilon, double sigma, double rcut) {
   c->lj.p[0] = make_pair(epsilon, sigma, rcut);
   c->lj.rcut_max = rcut;
   c->lj.rcut_max2 = rcut * rcut;
-  set_rlist(c, rcut);
-  return GBMD_OK;
+  return set_rlist(c, rcut);
 }
 
 int gbmd_set_lj_multi(gbmd_context* c, int ntypes, const double* eps, const double* sig, const double* rc,
@@ -793,9 +814,7 @@ int gbmd_set_lj_multi(gbmd_context* c, int ntypes, const double* eps, const doub
   c->lj.rcut_max = rmax;
   c->lj.rcut_max2 = rmax * rmax;
   if (!c->lj_tab_d) GBMD_CUDA(c, cudaMalloc(&c->lj_tab_d, sizeof(LJPair) * GBMD_MAX_TYPES * GBMD_MAX_TYPES));
-  GBMD_CUDA(c, cudaMemcpy(c->lj_tab_d, c->lj.p, sizeof(LJPair) * ntypes * ntypes, cudaMemcpyHostToDevice));
-  set_rlist(c, rmax);
-  return GBMD_OK;
+  return set_rlist(c, rmax);
 }
 
 int gbmd_set_eam_alloy(gbmd_context* c, int nel, int nrho, double drho, int nr, double dr, const double* frho,
@@ -886,12 +905,9 @@ int gbmd_set_eam_alloy(gbmd_context* c, int nel, int nrho, double drho, int nr, 
   E.rdrhof = (float)E.rdrho;
   E.rhomaxf = (float)E.rhomax;
   E.rc2f = (float)E.rcut2;
-  E.rc2lo = (float)(E.rcut2 * (1.0 - 0x1p-12));
-  E.rc2hi = (float)(E.rcut2 * (1.0 + 0x1p-12));
   c->eam_fix_ok = false;
   c->pot = GBMD_POT_EAM_ALLOY;
-  set_rlist(c, rcut);
-  return GBMD_OK;
+  return set_rlist(c, rcut);
 }
 
 int gbmd_load_setfl(gbmd_context* c, const char* path, double rcut, double conv_z2r, double conv_frho) {
@@ -945,13 +961,10 @@ int gbmd_set_eam_johnson(gbmd_context* c, const double params[19], double rcut) 
   P.Bf = (float)P.B;
   P.kappaf = (float)P.kappa;
   P.lambdaf = (float)P.lambda;
-  P.rc2lo = (float)(P.rcut2 * (1.0 - 0x1p-12));
-  P.rc2hi = (float)(P.rcut2 * (1.0 + 0x1p-12));
   c->ej = P;
   c->pot = GBMD_POT_EAM_JOHNSON;
   c->energy_step = -1, c->forces_valid_step = c->rho_valid_step = -1;
-  set_rlist(c, rcut);
-  return GBMD_OK;
+  return set_rlist(c, rcut);
 }
 
 // sutton_chen_force parameters (sutton_chen.h L30-37), see gbmd_johnson.cu
@@ -973,13 +986,10 @@ int gbmd_set_eam_sutton_chen(gbmd_context* c, const double params[5], double rcu
   P.a0f = (float)P.a0;
   P.nf = (float)P.n;
   P.mf = (float)P.m;
-  P.rc2lo = (float)(P.rcut2 * (1.0 - 0x1p-12));
-  P.rc2hi = (float)(P.rcut2 * (1.0 + 0x1p-12));
   c->esc = P;
   c->pot = GBMD_POT_EAM_SUTTON_CHEN;
   c->energy_step = -1, c->forces_valid_step = c->rho_valid_step = -1;
-  set_rlist(c, rcut);
-  return GBMD_OK;
+  return set_rlist(c, rcut);
 }
 
 int gbmd_set_precision(gbmd_context* c, int precision) {
@@ -1089,14 +1099,15 @@ int gbmd_get_launch_ex(const gbmd_context* c, int* tpa, int* vec, int* block) {
 int gbmd_set_skin(gbmd_context* c, double skin) {
   if (!c || !(skin >= 0.0)) return GBMD_ERR_INVALID;
   c->skin = skin;
-  set_rlist(c, pot_rcut_max(c));
-  return GBMD_OK;
+  return set_rlist(c, pot_rcut_max(c));
 }
 
 int gbmd_set_list_buffer(gbmd_context* c, double buffer) {
   if (!c || !(buffer >= 0.0) || !std::isfinite(buffer)) return GBMD_ERR_INVALID;
   if (buffer == c->list_buffer) return GBMD_OK;
   c->list_buffer = buffer;
+  const int rc = set_bands(c);
+  if (rc) return rc;
   c->grid_valid = false;  // cells of at least the outer radius
   c->maxnb = c->maxnb_out = 0;
   invalidate_list(c);

@@ -100,6 +100,20 @@ struct Grid {
   int64_t ncells;
 };
 
+// Relative half-width of the band around rc^2 inside which a pair's FP32 d2
+// may fall on the wrong side, so that it is re-tested in FP64.  With cells of
+// edge h < 2 reach (reach = the radius the cells are built for) and
+// home-cell-relative coordinates of at most 2 h, the coordinates' rounding
+// (2^-24 each of 2 h), that of their difference and of the shift add up to
+// 8.5 x 2^-24 h an axis, sqrt(3) of it in d, twice that relative to rc in d2:
+// 2^-18.1 reach / rc.  2^-16 leaves four times that, for atoms that drift on
+// between rebuilds.  The width decides only how many pairs take the FP64 test
+// (Cu, 2^-12: one row of four entries in 14 of a warp; now one in 200).
+inline double band_rel(double reach, double rc) {
+  const double w = 0x1p-16 * (reach > rc ? reach / rc : 1.0);
+  return w < 0.5 ? w : 0.5;
+}
+
 struct StepParams {
   double dt, dth, dt2h;     // dt, dt/2, dt*dt/2
   int64_t step;             // step index (for error records)

@@ -21,7 +21,7 @@
 // kernels evaluate the same functions in FP32 on the cell-relative
 // coordinates of the main mixed path, with compensated sums, FP64 embedding
 // and FP64 state.  Pair membership (r <= rcut) is exact in both: FP64
-// directly, mixed through the FP32 screen and the FP64 re-test of the 2^-12
+// directly, mixed through the FP32 screen and the FP64 re-test of the
 // band.
 #include <cmath>
 

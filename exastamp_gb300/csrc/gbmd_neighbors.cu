@@ -6,7 +6,7 @@
 // src/debug/atom_neighbors_stats.cpp L169-228: every (i, j, image n) with
 // d2 <= (rcut_max + skin)^2, d2 computed in FP64 from ((x_j + n*L) - x_i)
 // without contraction.  Candidates are screened in FP32 on home-cell-relative
-// coordinates; only those within 2^-12 of the radius are re-tested in FP64,
+// coordinates; only those within band_rel of the radius are re-tested in FP64,
 // so the list is bit-identical to an all-FP64 build.
 //
 // Kernels (per rebuild):
@@ -325,7 +325,7 @@ __global__ void k_posf(int64_t n, const double* __restrict__ x, const double* __
   }
 }
 
-// FP64 re-test of a candidate whose FP32 d2 fell within 2^-12 of R^2.  Out of
+// FP64 re-test of a candidate whose FP32 d2 fell within the band around R^2.  Out of
 // line so the compiler cannot predicate it into every iteration of the
 // candidate loop (it runs for ~1e-4 of the candidates).
 __device__ __noinline__ bool exact_within(const double* __restrict__ x, const double* __restrict__ y,
@@ -481,7 +481,7 @@ __device__ __forceinline__ int build_walk(const BuildCell& B, const float4* __re
         const float d2f = fmaf(dx, dx, fmaf(dy, dy, __fmul_rn(dz, dz)));
         // an atom never pairs with itself: its images sit at least one box
         // edge >= R away, so k == i only ever matters in the home cell.
-        // Keep d2 <= R^2 (1 + 2^-12); flag the atom when d2 >= R^2 (1 - 2^-12).
+        // Keep d2 <= R2hi; flag the atom when d2 >= R2lo.
         const int k = (int)(w & GBMD_IDX_MASK);
         const bool in = hv && (HALF ? k > i : k != i) && d2f <= R2hi;
         unc |= in && d2f >= R2lo;
@@ -529,8 +529,8 @@ __device__ __forceinline__ int build_walk(const BuildCell& B, const float4* __re
 // (stencil code, then cell order) -- straight to the atoms' list rows.  Cells
 // of at most 16 atoms use the 16-atom grouping (two candidates per step),
 // fuller cells the 32-atom one.  The walk keeps every candidate with FP32
-// d2 <= R^2 (1 + 2^-12) and flags the atom when one lies above
-// R^2 (1 - 2^-12); flagged atoms (a few per cent) rescan their row, re-test
+// d2 <= R2hi and flags the atom when one lies above R2lo (the band of
+// band_rel); flagged atoms (below one per cent) rescan their row, re-test
 // those entries in FP64 and compact, so the walk has no call and no
 // divergent branch.
 template <bool LOOP, bool HALF>
@@ -617,8 +617,9 @@ void launch_posf(gbmd_context* c, const int* gate) {
 static int build_list(gbmd_context* c, const int* gate) {
   const double R = c->rlist;
   const double R2 = R * R;
-  const float R2lo = (float)(R2 * (1.0 - 0x1p-12));
-  const float R2hi = (float)(R2 * (1.0 + 0x1p-12));
+  // cells are at least R wide here: the band of reach = R
+  const float R2lo = (float)(R2 * (1.0 - band_rel(R, R)));
+  const float R2hi = (float)(R2 * (1.0 + band_rel(R, R)));
   const int64_t npad = ((c->n + 31) / 32) * 32;
   const int W = list_width(c);
   const int64_t stride = npad * W;
@@ -837,7 +838,7 @@ __global__ void k_save_outer(int64_t n, const double* __restrict__ r, double* __
 
 // One thread per atom: the entries of its outer row within R now, in order.
 // The FP32 distance of the cell-relative copies (the builder's expression)
-// decides outside the band R^2 (1 -+ 2^-12); band entries are re-tested in
+// decides outside the band [R2lo, R2hi]; band entries are re-tested in
 // FP64 with the pair-set rounding.  A row never grows, so the list has the
 // outer list's capacity.  V4 (rows interleaved in groups of a multiple of 4
 // entries): the row is read 4 entries per 16-byte load with the next load in
@@ -963,8 +964,9 @@ static int filter_list(gbmd_context* c, const int* gate) {
   }
   c->maxnb = c->maxnb_out;
   const double R2 = c->rlist * c->rlist;
-  const float R2lo = (float)(R2 * (1.0 - 0x1p-12));
-  const float R2hi = (float)(R2 * (1.0 + 0x1p-12));
+  const double band = band_rel(c->rlist + c->list_buffer, c->rlist);
+  const float R2lo = (float)(R2 * (1.0 - band));
+  const float R2hi = (float)(R2 * (1.0 + band));
   FilterArgs A;
   A.n = c->n;
   A.pf = c->POSF();

@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(256) k_lj_loss_grad(PairArgs A, LJAdjArgs P) {
   double ge = 0., gs = 0.;
   const uint32_t* row = A.nbr + (size_t)i * A.W;
   for (int k = 0; k < nn; ++k) {
-    const uint32_t ent = __ldg(row + (size_t)(k >> A.wsh) * A.stride + (k & (A.W - 1)));
+    const uint32_t ent = __ldg(row + list_slot(A, k));
     const uint32_t j = ent & GBMD_IDX_MASK, code = ent >> GBMD_IDX_BITS;
     const double4_32a pj = A.posd[j];
     double Sx, Sy, Sz, dx, dy, dz;
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(128) k_lj_multi_loss_grad(PairArgs A, const LJ
   const double dE = A.ep[i] - P->et[i];
   const uint32_t* row = A.nbr + (size_t)i * A.W;
   for (int k = 0; k < nn; ++k) {
-    const uint32_t ent = __ldg(row + (size_t)(k >> A.wsh) * A.stride + (k & (A.W - 1)));
+    const uint32_t ent = __ldg(row + list_slot(A, k));
     const uint32_t j = ent & GBMD_IDX_MASK, code = ent >> GBMD_IDX_BITS;
     const double4_32a pj = A.posd[j];
     double Sx, Sy, Sz, dx, dy, dz;

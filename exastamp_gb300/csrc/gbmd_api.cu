@@ -1015,8 +1015,10 @@ int gbmd_set_launch_ex(gbmd_context* c, int tpa, int vec, int block) {
     c->vec = vec;
     const int W = list_width(c);
     if (c->maxnb > 0) c->maxnb = ((c->maxnb + W - 1) / W) * W;
+    if (c->maxnb_out > 0) c->maxnb_out = ((c->maxnb_out + W - 1) / W) * W;
     invalidate_list(c);
   }
+  c->launch_set = true;
   c->block = block;
   if (c->block_rho % tpa) c->block_rho = 0;  // follow `block` until set again
   drop_graph(c);
@@ -1030,14 +1032,12 @@ int gbmd_set_launch(gbmd_context* c, int tpa, int block) {
 
 int gbmd_get_launch(const gbmd_context* c, int* tpa, int* block) {
   if (!c) return GBMD_ERR_INVALID;
-  if (tpa) *tpa = c->tpa;
-  if (block) *block = c->block;
-  return GBMD_OK;
+  return gbmd_get_launch_ex(c, tpa, nullptr, block);
 }
 
 int gbmd_set_density_block(gbmd_context* c, int block) {
   if (!c) return GBMD_ERR_INVALID;
-  if (block != 0 && (block < 32 || block > 256 || block % 32 || block % c->tpa))
+  if (block != 0 && (block < 32 || block > 256 || block % 32 || (c->launch_set && block % c->tpa)))
     return set_error(c, GBMD_ERR_INVALID, "density block must be 0 or a multiple of 32 in [32,256]");
   c->block_rho = block;
   drop_graph(c);
@@ -1046,7 +1046,7 @@ int gbmd_set_density_block(gbmd_context* c, int block) {
 
 int gbmd_get_density_block(const gbmd_context* c, int* block) {
   if (!c || !block) return GBMD_ERR_INVALID;
-  *block = c->block_rho ? c->block_rho : c->block;
+  *block = c->block_rho ? c->block_rho : (c->launch_set ? c->block : 256);
   return GBMD_OK;
 }
 
@@ -1057,6 +1057,7 @@ int gbmd_set_neighbor_staging(gbmd_context* c, int enable) {
     return set_error(c, GBMD_ERR_CUDA, "cannot raise the shared-memory limit of the staged kernels");
   if (c->staged != (enable != 0)) {
     c->staged = enable != 0;
+    if (!c->launch_set) invalidate_list(c);  // staging needs the one-lane layout
     drop_graph(c);
   }
   return GBMD_OK;
@@ -1090,9 +1091,11 @@ int gbmd_get_neighbor_staging(const gbmd_context* c, int* enabled) {
 
 int gbmd_get_launch_ex(const gbmd_context* c, int* tpa, int* vec, int* block) {
   if (!c) return GBMD_ERR_INVALID;
-  if (tpa) *tpa = c->tpa;
-  if (vec) *vec = c->vec;
-  if (block) *block = c->block;
+  // the launch the caller set, or the nominal default: what choose_launch
+  // picked for the atoms at hand is not a setting to be saved and set again
+  if (tpa) *tpa = c->launch_set ? c->tpa : 1;
+  if (vec) *vec = c->launch_set ? c->vec : 4;
+  if (block) *block = c->launch_set ? c->block : 256;
   return GBMD_OK;
 }
 

@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(256) k_lj(PairArgs A, LJSingle P, const LJPair
     ti = (int)pi.w;
     const uint32_t* row = A.nbr + (size_t)i * A.W;
     for (int k = lane; k < nn; k += T) {
-      const uint32_t ent = __ldg(row + (size_t)(k >> A.wsh) * A.stride + (k & (A.W - 1)));
+      const uint32_t ent = __ldg(row + list_slot(A, k));
       const uint32_t j = ent & GBMD_IDX_MASK, code = ent >> GBMD_IDX_BITS;
       const double4_32a pj = A.posd[j];
       double Sx, Sy, Sz, dx, dy, dz;
@@ -128,7 +128,7 @@ __global__ void __launch_bounds__(256) k_eam_rho(PairArgs A, EamDev E, double* _
     const int ti = (int)pi.w;
     const uint32_t* row = A.nbr + (size_t)i * A.W;
     for (int k = lane; k < nn; k += T) {
-      const uint32_t ent = __ldg(row + (size_t)(k >> A.wsh) * A.stride + (k & (A.W - 1)));
+      const uint32_t ent = __ldg(row + list_slot(A, k));
       const uint32_t j = ent & GBMD_IDX_MASK, code = ent >> GBMD_IDX_BITS;
       const double4_32a pj = A.posd[j];
       double Sx, Sy, Sz, dx, dy, dz;
@@ -185,7 +185,7 @@ __global__ void __launch_bounds__(256) k_eam_force(PairArgs A, EamDev E, const d
     const int ti = (int)pi.w;
     const uint32_t* row = A.nbr + (size_t)i * A.W;
     for (int k = lane; k < nn; k += T) {
-      const uint32_t ent = __ldg(row + (size_t)(k >> A.wsh) * A.stride + (k & (A.W - 1)));
+      const uint32_t ent = __ldg(row + list_slot(A, k));
       const uint32_t j = ent & GBMD_IDX_MASK, code = ent >> GBMD_IDX_BITS;
       const double4_32a pj = A.posd[j];
       double Sx, Sy, Sz, dx, dy, dz;
@@ -241,8 +241,8 @@ PairArgs make_args(gbmd_context* c, const ForceFlags& f) {
   A.i0 = f.i0;
   A.n = f.i1 >= 0 ? f.i1 : c->n;
   A.W = list_width(c);
-  A.wsh = 0;
-  while ((1 << A.wsh) < A.W) ++A.wsh;
+  A.wsh = log2_of(A.W);
+  A.tsh = log2_of(c->tpa);
   A.stride = c->npad * A.W;
   A.nbr = c->nbr;
   A.nnb = c->nnb;

@@ -9,7 +9,7 @@
 //   posd (double4_32a): FP64 absolute position, w = type bits (FP64 path gathers)
 //   nbr (u32): full neighbour list entries j | code<<26, code = (dx+1)|(dy+1)<<2|(dz+1)<<4
 //              the stencil offset of j's cell; laid out for T lanes per atom as
-//              nbr[(k/T)*(npad*T) + i*T + k%T]
+//              nbr[(k/W)*(npad*W) + i*W + list_word(k%W)], W = T * entries per load
 //   nnb (i32): neighbours per atom
 #pragma once
 #include <cuda_runtime.h>
@@ -203,8 +203,9 @@ struct gbmd_context {
   int32_t* nnb = nullptr;
   int64_t nbr_cap = 0;          // entries allocated
   int maxnb = 0;                // per-atom capacity (multiple of tpa * vec)
-  int tpa = 1;                  // lanes per atom (autotuned; default = the GB300 optimum)
-  int vec = 4;                  // list entries per lane per load (1 or 4, mixed kernels; autotuned)
+  bool launch_set = false;      // the caller chose the launch (set_launch*): tpa, vec, block are its choice
+  int tpa = 1;                  // lanes per atom of the list's layout (choose_launch, or the caller's)
+  int vec = 4;                  // list entries per lane per load (1 or 4, mixed kernels)
   bool staged = false;          // 1 lane x 4 entries: neighbour positions from shared memory
   bool fused_trigger = false;   // run_nve with the displacement trigger: kernels that move atoms test them
   bool first_half_done = false; // gbmd_run_nve_host pushed the first half while reading the state in
@@ -212,7 +213,7 @@ struct gbmd_context {
   long long* h3acc = nullptr;   // Newton-3 fixed-point accumulators, 10 planes of cap: f (3), ep, virial (6)
   double eam_fix_bound[4] = {1.0, 1.0, 1.0, 1.0};  // Newton-3 eam_alloy bounds: rho, force, energy, virial
   bool eam_fix_ok = false;      // eam_fix_bound is that of the current tables
-  int block = 256;              // threads per block of the pair / force kernels (autotuned)
+  int block = 256;              // threads per block of the pair / force kernels
   int block_rho = 128;          // threads per block of the EAM density kernels (autotuned; 0 = block)
   double skin = 0.0, rlist = 0.0;
   bool list_valid = false;
@@ -338,6 +339,9 @@ void free_outer(gbmd_context* c);
 // (the stream must be capturing; body issues on c->stream)
 int capture_if(gbmd_context* c, const int* gate, int (*body)(gbmd_context*, const int*));
 void launch_posf(gbmd_context* c, const int* gate = nullptr);
+// lanes per atom and block size for the atoms and potential at hand, unless
+// the caller set them; called where a fresh list is laid out
+void choose_launch(gbmd_context* c);
 // blocks for a rebuild-chain kernel over `items` (per_block per block): all
 // of them ungated, at most per_sm per SM when gated (grid-stride kernels)
 unsigned chain_blocks(const gbmd_context* c, int64_t items, int per_block, const int* gate, int per_sm);
@@ -479,6 +483,22 @@ __device__ __forceinline__ double exact_d2(double xi, double yi, double zi, doub
 // nbr[r * npad * W + i * W + ...].
 inline int list_width(const gbmd_context* c) { return c->tpa * c->vec; }
 
-__device__ __forceinline__ size_t nbr_slot(int64_t i, int k, int T, int64_t stride) {
-  return (size_t)(k / T) * (size_t)stride + (size_t)i * T + (k % T);
+inline int log2_of(int p2) {
+  int s = 0;
+  while ((1 << s) < p2) ++s;
+  return s;
+}
+
+// A list row's word that holds entry p (0 <= p < W = 2^wsh): lane p % T reads
+// it as the (p / T)-th of its V = W / T adjacent words, T = 2^tsh.
+__host__ __device__ __forceinline__ int list_word(int p, int wsh, int tsh) {
+  return ((p & ((1 << tsh) - 1)) << (wsh - tsh)) | (p >> tsh);
+}
+
+// (double)x in integer instructions (exact; the FP64 pipe, where the
+// conversion runs, takes 16 SM cycles an instruction).
+__device__ __forceinline__ double widen(float x) {
+  const uint32_t b = __float_as_uint(x), m = b & 0x7fffffffu;
+  if (m - 0x00800000u >= 0x7f000000u) return (double)x;  // zero, subnormal, infinity, NaN
+  return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + 0x38000000u)), (int)(b << 29));
 }

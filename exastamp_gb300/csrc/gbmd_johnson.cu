@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(256) k_ej_rho(PairArgs A, typename Fn::Params 
   if (live) pi = A.posd[i];
   const uint32_t* row = A.nbr + (size_t)i * A.W;
   for (int k = lane; k < nn; k += T) {
-    const uint32_t ent = __ldg(row + (size_t)(k >> A.wsh) * A.stride + (k & (A.W - 1)));
+    const uint32_t ent = __ldg(row + list_slot(A, k));
     const uint32_t j = ent & GBMD_IDX_MASK, code = ent >> GBMD_IDX_BITS;
     const double4_32a pj = A.posd[j];
     double Sx, Sy, Sz, dx, dy, dz;
@@ -212,7 +212,7 @@ __global__ void __launch_bounds__(256) k_ej_force(PairArgs A, typename Fn::Param
   const int ti = (int)pi.w;
   const uint32_t* row = A.nbr + (size_t)i * A.W;
   for (int k = lane; k < nn; k += T) {
-    const uint32_t ent = __ldg(row + (size_t)(k >> A.wsh) * A.stride + (k & (A.W - 1)));
+    const uint32_t ent = __ldg(row + list_slot(A, k));
     const uint32_t j = ent & GBMD_IDX_MASK, code = ent >> GBMD_IDX_BITS;
     const double4_32a pj = A.posd[j];
     double Sx, Sy, Sz, dx, dy, dz;
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(256) k_ej_rho_mixed(PairArgs A, typename Fn::P
   float rho = 0.f, crho = 0.f;
   const uint32_t* row = A.nbr + (size_t)i * A.W;
   for (int k = lane; k < nn; k += T) {
-    const uint32_t ent = __ldcs(row + (size_t)(k >> A.wsh) * A.stride + (k & (A.W - 1)));
+    const uint32_t ent = __ldcs(row + list_slot(A, k));
     const float4 pj = __ldg(&A.posf[ent & GBMD_IDX_MASK]);
     const EjGeom G = ej_geom(A, P, ent, pj, pi, i, cp);
     const float r = G.d2 * rsqrtf(G.d2);
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(256) k_ej_force_mixed(PairArgs A, typename Fn:
   float v[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f}, cv[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   const uint32_t* row = A.nbr + (size_t)i * A.W;
   for (int k = lane; k < nn; k += T) {
-    const uint32_t ent = __ldcs(row + (size_t)(k >> A.wsh) * A.stride + (k & (A.W - 1)));
+    const uint32_t ent = __ldcs(row + list_slot(A, k));
     const uint32_t j = ent & GBMD_IDX_MASK;
     const float4 pj = __ldg(&A.posf[j]);
     const float fpj = __ldg(&fpf[j]);

@@ -26,38 +26,6 @@
 
 namespace gbmd {
 
-struct GeomF {
-  float dx, dy, dz, d2;
-};
-
-// Exact FP64 cutoff test of a pair whose FP32 d2 fell in the ambiguous band:
-// d2 <= rc2 and, for per-pair cutoffs, sqrt(d2) <= rc_pair (the reference's
-// two-stage test).  Kept out of line: it runs for ~1e-4 of the pairs.
-__device__ __noinline__ bool exact_inside(const double4_32a* __restrict__ posd, int64_t i, uint32_t j,
-                                          uint32_t code, int cp, const Grid g, double rc2, double rc_pair) {
-  int cx, cy, cz;
-  unpack_cell(cp, cx, cy, cz);
-  double Sx, Sy, Sz, a, b, c;
-  image_shift(g, cx, cy, cz, code, Sx, Sy, Sz);
-  const double4_32a di = posd[i], dj = posd[j];
-  const double d2 = exact_d2(di.x, di.y, di.z, dj.x, dj.y, dj.z, Sx, Sy, Sz, a, b, c);
-  if (!(d2 <= rc2)) return false;
-  return rc_pair <= 0.0 || sqrt(d2) <= rc_pair;
-}
-
-// {0,1,2} -> -1.f, 0.f, +1.f exactly (small integer through the 2^23 mantissa
-// trick); the separation shift is then one FMA per axis.
-__device__ __forceinline__ float unit_of(uint32_t b) { return __int_as_float(0x4B000000u | b) - 8388609.0f; }
-
-__device__ __forceinline__ GeomF geom_f(uint32_t ent, const float4& pj, const float4& pi, const Grid& g) {
-  GeomF r;
-  r.dx = fmaf(unit_of((ent >> 26) & 3u), g.hf[0], pj.x - pi.x);
-  r.dy = fmaf(unit_of((ent >> 28) & 3u), g.hf[1], pj.y - pi.y);
-  r.dz = fmaf(unit_of(ent >> 30), g.hf[2], pj.z - pi.z);
-  r.d2 = fmaf(r.dx, r.dx, fmaf(r.dy, r.dy, r.dz * r.dz));
-  return r;
-}
-
 // Two list entries at once in packed FP32 (sm_100 float2 arithmetic: one
 // instruction per pair of lanes' worth of FADD / FMUL / FFMA).  Each half is
 // geom_f of its entry, operation for operation: (p_j - p_i) is p_j + (-p_i),
@@ -103,22 +71,28 @@ __device__ __forceinline__ void vir9(const float* v, double* o) {
   o[6] = v[4]; o[7] = v[5]; o[8] = v[2];
 }
 
-// The V list entries of lane `lane` in row r of atom i, read with one load
-// that bypasses L1 (each entry is used once per kernel).  Entries at or
-// beyond nn are replaced by a harmless stand-in: j = i seen through the +x
-// stencil offset, a separation of one cell edge (>= rcut + skin), which no
-// cutoff test accepts.
+// Atom i's list as the T lanes of its group read it: entry k = r*T*V + q*T +
+// lane is lane `lane`'s q-th of row r (see list_word), so that one gather of
+// the group touches T consecutive entries, which lie in the same one or two
+// cells and mostly in the same 128-byte lines.  A warp's position gather
+// touches 16.5 lines with one lane per atom, 12.0 with two and 8.7 with four
+// (Cu crystal, counted), and the L1 takes about a cycle for each.  A row's V
+// entries are one load that bypasses L1 (each entry is used once per kernel).
+// Entries at or beyond nn, in the last row only, are replaced by a harmless
+// stand-in: j = i seen through the +x stencil offset, a separation of one
+// cell edge (>= rcut + skin), which no cutoff test accepts.
 template <int T, int V>
 struct ListRows {
   static constexpr int W = T * V;
   const uint32_t* p;  // nbr + i*W + lane*V
   int64_t stride;
-  int nrow, k0, nn;
+  int nrow, nfull, rem, lane, nn;
   uint32_t standin;
-  __device__ __forceinline__ ListRows(const uint32_t* nbr, int64_t i, int lane, int64_t stride_, int nn_)
-      : p(nbr + (size_t)i * W + lane * V), stride(stride_), nn(nn_) {
-    k0 = lane * V;
-    nrow = nn > k0 ? (nn - k0 + W - 1) / W : 0;
+  __device__ __forceinline__ ListRows(const uint32_t* nbr, int64_t i, int lane_, int64_t stride_, int nn_)
+      : p(nbr + (size_t)i * W + lane_ * V), stride(stride_), lane(lane_), nn(nn_) {
+    nrow = (nn + W - 1) / W;
+    nfull = nn / W;
+    rem = nn - nfull * W;
     standin = (uint32_t)i | ((2u | (1u << 2) | (1u << 4)) << GBMD_IDX_BITS);
   }
   __device__ __forceinline__ void load(int r, uint32_t (&e)[V]) const {
@@ -133,8 +107,49 @@ struct ListRows {
       for (int v = 0; v < V; ++v) e[v] = __ldcs(q + v);
     }
   }
-  __device__ __forceinline__ bool valid(int r, int v) const { return r * W + k0 + v < nn; }
+  __device__ __forceinline__ bool valid(int r, int q) const { return r * W + q * T + lane < nn; }
+  __device__ __forceinline__ bool in_tail(int q) const { return q * T + lane < rem; }
 };
+
+// body(entries, valid): every row of L in order, N = V entries of a full row
+// or N = V / 2 (at least one) of the last, partial one, which stops after
+// the half that holds its last entry.
+template <int N>
+struct RowPart {
+  uint32_t e[N];
+  bool ok[N];
+};
+
+template <int T, int V, class Body>
+__device__ __forceinline__ void for_rows(const ListRows<T, V>& L, Body body) {
+  constexpr int H = V >= 2 ? V / 2 : 1;
+  uint32_t ent[V], nxt[V];
+  if (L.nrow > 0) L.load(0, ent);
+  for (int r = 0; r < L.nfull; ++r) {
+    if (r + 1 < L.nrow) L.load(r + 1, nxt);
+    RowPart<V> P;
+#pragma unroll
+    for (int q = 0; q < V; ++q) {
+      P.e[q] = ent[q];
+      P.ok[q] = true;
+    }
+    body(P);
+#pragma unroll
+    for (int q = 0; q < V; ++q) ent[q] = nxt[q];
+  }
+#pragma unroll
+  for (int h = 0; h < V; h += H) {
+    if (L.rem > h * T) {
+      RowPart<H> P;
+#pragma unroll
+      for (int q = 0; q < H; ++q) {
+        P.ok[q] = L.in_tail(h + q);
+        P.e[q] = P.ok[q] ? ent[h + q] : L.standin;
+      }
+      body(P);
+    }
+  }
+}
 
 // ---------------------------------------------------------------------------
 // Neighbour-position sources.  GlobalFetch gathers position j from the
@@ -254,31 +269,29 @@ __device__ __forceinline__ void lj_load_table(LJTabSmem& t, const LJPair* __rest
   __syncthreads();
 }
 
+// One atom's pair sums, reduced over its T lanes (v: virial xx yy zz xy xz yz).
+struct PairSums {
+  float f[3], e, v[6];
+};
+
 template <int T, int V, bool EV, bool MULTI, class Fetch>
-__device__ __forceinline__ void lj_atom(const PairArgs& A, const LJF& P, const LJTabSmem& tab, int ntypes,
-                                        double rcmax2, int64_t i, int lane, bool live, const Fetch& fetch) {
+__device__ __forceinline__ PairSums lj_atom(const PairArgs& A, const LJF& P, const LJTabSmem& tab, int ntypes,
+                                            double rcmax2, int64_t i, int lane, bool live, const Fetch& fetch) {
   const int nn = live ? min(A.nnb[i], A.maxnb) : 0;
   const float4 pi = live ? A.posf[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-  const int cp = live ? A.cellpack[i] : 0;
   const int ti = __float_as_int(pi.w);
   float fx = 0.f, fy = 0.f, fz = 0.f, cfx = 0.f, cfy = 0.f, cfz = 0.f, e = 0.f, ce = 0.f;
   float v[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   const ListRows<T, V> L(A.nbr, i, lane, A.stride, nn);
-  uint32_t ent[V], nxt[V];
-  if (L.nrow > 0) L.load(0, ent);
-  for (int r = 0; r < L.nrow; ++r) {
-    if (r + 1 < L.nrow) L.load(r + 1, nxt);
-    float4 pj[V];
+  for_rows(L, [&](const auto& R) {
+    constexpr int N = sizeof(R.e) / sizeof(R.e[0]);
+    float4 pj[N];
 #pragma unroll
-    for (int q = 0; q < V; ++q) {
-      if (!L.valid(r, q)) ent[q] = L.standin;
-      pj[q] = fetch(ent[q], ent[q] & GBMD_IDX_MASK);
-    }
+    for (int q = 0; q < N; ++q) pj[q] = fetch(R.e[q], R.e[q] & GBMD_IDX_MASK);
     float rx = 0.f, ry = 0.f, rz = 0.f, re = 0.f;
 #pragma unroll
-    for (int q = 0; q < V; ++q) {
-      const uint32_t j = ent[q] & GBMD_IDX_MASK;
-      const GeomF G = geom_f(ent[q], pj[q], pi, A.g);
+    for (int q = 0; q < N; ++q) {
+      const GeomF G = geom_f(R.e[q], pj[q], pi, A.g);
       float sig2, eps24, eps4, ecut, rlo, rhi;
       int pid = 0;
       if (MULTI) {
@@ -290,9 +303,9 @@ __device__ __forceinline__ void lj_atom(const PairArgs& A, const LJF& P, const L
         sig2 = P.sig2; eps24 = P.eps24; eps4 = P.eps4; ecut = P.ecut; rlo = P.rc2lo; rhi = P.rc2hi;
       }
       bool in = G.d2 < rlo;
-      if (!in && G.d2 <= rhi && L.valid(r, q))  // rare: the FP64 per-pair cutoff only here
-        in = exact_inside(A.posd, i, j, ent[q] >> GBMD_IDX_BITS, cp, A.g, MULTI ? rcmax2 : P.rc2,
-                          MULTI ? tab.r[pid] : 0.0);
+      if (!in && G.d2 <= rhi && R.ok[q])  // rare: the FP64 per-pair cutoff only here
+        in = exact_inside(A.posd, i, R.e[q] & GBMD_IDX_MASK, R.e[q] >> GBMD_IDX_BITS, A.cellpack[i], A.g,
+                          MULTI ? rcmax2 : P.rc2, MULTI ? tab.r[pid] : 0.0);
       // hardware reciprocal (within 1 ulp): the pair term's error budget is
       // ~1e-7 relative against a 1e-5 force tolerance
       float r2i;
@@ -319,36 +332,100 @@ __device__ __forceinline__ void lj_atom(const PairArgs& A, const LJF& P, const L
     kahan_add(fy, cfy, ry);
     kahan_add(fz, cfz, rz);
     if (EV) kahan_add(e, ce, re);
-#pragma unroll
-    for (int q = 0; q < V; ++q) ent[q] = nxt[q];
-  }
+  });
   group_reduce_kahan<T>(fx, cfx);
   group_reduce_kahan<T>(fy, cfy);
   group_reduce_kahan<T>(fz, cfz);
+  PairSums S;
+  S.f[0] = fx - cfx;
+  S.f[1] = fy - cfy;
+  S.f[2] = fz - cfz;
+  S.e = 0.f;
   if (EV) {
     group_reduce_kahan<T>(e, ce);
     reduce6(v, T);
+    S.e = e - ce;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) S.v[q] = v[q];
   }
-  if (live && lane == 0) {
-    const float im = A.inv_massf[ti];
-    double o[9];
-    if (EV) vir9(v, o);
-    atom_epilogue<true>(A, i, ti, 0., 0., 0., (fx - cfx) * im, (fy - cfy) * im, (fz - cfz) * im,
-                        EV ? (double)(e - ce) : 0.0, EV ? o : nullptr);
+  return S;
+}
+
+// Epilogue of one atom from its pair sums; emb: its embedding energy.  The
+// virial row is written here too, 72 bytes apart from lane to lane: for the
+// kernels whose blocks have no common loop (block_epilogue is the other).
+template <bool EV>
+__device__ __forceinline__ void atom_finish(const PairArgs& A, int64_t i, const PairSums& S, float emb) {
+  const int ti = __float_as_int(A.posf[i].w);
+  const float im = A.inv_massf[ti];
+  double o[9];
+  if (EV) vir9(S.v, o);
+  atom_epilogue<true>(A, i, ti, 0., 0., 0., S.f[0] * im, S.f[1] * im, S.f[2] * im,
+                      EV ? (double)emb + (double)S.e : 0.0, EV ? o : nullptr);
+}
+
+// Epilogue of a block's atoms i0 .. i0 + blockDim / T, whose sums the groups'
+// first lanes hold.  They pass through shared memory to the block's first
+// blockDim / T threads, so that the per-atom work (the FP64 Verlet halves,
+// the stores) runs on full warps: on each group's first lane alone it would
+// issue T times as many FP64 instructions, 16 SM cycles each.  The virial rows (9 doubles per atom) go through shared
+// memory so that the block writes them contiguously; a lane writing its own
+// row touches 32 sectors per store, nine times.
+template <int T, bool EV>
+__device__ __forceinline__ void block_epilogue(const PairArgs& A, int64_t i0, const PairSums& S,
+                                               const float* __restrict__ epf) {
+  constexpr int NV = EV ? 10 : 3;
+  constexpr bool SHARED = T > 1 || EV;
+  __shared__ float sums[SHARED ? NV : 1][SHARED ? 256 / T : 1];
+  const int nat = (int)blockDim.x / T;
+  PairSums R = S;
+  if (SHARED) {
+    const int a = (int)threadIdx.x / T;
+    if (threadIdx.x % T == 0) {
+#pragma unroll
+      for (int q = 0; q < 3; ++q) sums[q][a] = S.f[q];
+      if (EV) {
+        sums[3][a] = S.e;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) sums[4 + q][a] = S.v[q];
+      }
+    }
+    __syncthreads();
+    if (EV && A.want_virial) {
+      const int m = (int)min((int64_t)nat, A.n - i0) * 9;
+      for (int k = threadIdx.x; k < m; k += blockDim.x) {
+        const int q = k % 9;  // row-major 3x3 from xx yy zz xy xz yz
+        A.vir[9 * i0 + k] = widen(sums[4 + ((0x254513430u >> (4 * q)) & 15)][k / 9]);
+      }
+    }
+    if ((int)threadIdx.x >= nat) return;
+    if (T > 1) {
+#pragma unroll
+      for (int q = 0; q < 3; ++q) R.f[q] = sums[q][threadIdx.x];
+      if (EV) R.e = sums[3][threadIdx.x];
+    }
   }
+  const int64_t i = i0 + threadIdx.x;
+  if (i >= A.n) return;
+  const int ti = __float_as_int(A.posf[i].w);
+  const float im = A.inv_massf[ti];
+  atom_epilogue<true>(A, i, ti, 0., 0., 0., R.f[0] * im, R.f[1] * im, R.f[2] * im,
+                      EV ? (epf ? (double)epf[i] : 0.0) + (double)R.e : 0.0, nullptr);
 }
 
 // PIECE: the launch covers atoms [A.i0, A.n) only (a separate instantiation:
 // the offset costs registers that the full-range kernel, at the 64-register
 // cap, would spill).
 template <int T, int V, bool EV, bool MULTI, bool PIECE>
-__global__ void __launch_bounds__(256, 4) k_lj_mixed(PairArgs A, LJF P, const LJPair* __restrict__ tab, int ntypes,
+__global__ void __launch_bounds__(256, EV ? 3 : 4) k_lj_mixed(PairArgs A, LJF P, const LJPair* __restrict__ tab, int ntypes,
                                                   double rcmax2) {
   __shared__ LJTabSmem t;
   if (MULTI) lj_load_table(t, tab, ntypes);
   const int64_t gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t i = PIECE ? A.i0 + gt / T : gt / T;
-  lj_atom<T, V, EV, MULTI>(A, P, t, ntypes, rcmax2, i, (int)(gt % T), i < A.n, GlobalFetch{A.posf});
+  const PairSums S =
+      lj_atom<T, V, EV, MULTI>(A, P, t, ntypes, rcmax2, i, (int)(gt % T), i < A.n, GlobalFetch{A.posf});
+  block_epilogue<T, EV>(A, (PIECE ? A.i0 : 0) + blockIdx.x * (int64_t)(blockDim.x / T), S, nullptr);
 }
 
 // One lane per atom, 4 entries per load, neighbour positions from the
@@ -365,8 +442,9 @@ __global__ void __launch_bounds__(256) k_lj_staged(PairArgs A, LJF P, const LJPa
   int64_t a0, a1;
   const bool ok = stage_cells(A.g, cstart, A.posf, K, cap, staged_pos, rows, sh, a0, a1);
   for (int64_t i = a0 + threadIdx.x; i < a1; i += blockDim.x) {
-    if (ok) lj_atom<1, 4, EV, MULTI>(A, P, t, ntypes, rcmax2, i, 0, true, StagedFetch{staged_pos, rows});
-    else lj_atom<1, 4, EV, MULTI>(A, P, t, ntypes, rcmax2, i, 0, true, GlobalFetch{A.posf});
+    const PairSums S = ok ? lj_atom<1, 4, EV, MULTI>(A, P, t, ntypes, rcmax2, i, 0, true, StagedFetch{staged_pos, rows})
+                          : lj_atom<1, 4, EV, MULTI>(A, P, t, ntypes, rcmax2, i, 0, true, GlobalFetch{A.posf});
+    atom_finish<EV>(A, i, S, 0.f);
   }
 }
 
@@ -388,45 +466,37 @@ __device__ __forceinline__ float spline_der(const float4& c, float q, float rd) 
   return fmaf(fmaf(3.f * c.x, q, 2.f * c.y), q, c.z) * rd;
 }
 
-// Density + embedding.  SINGLE (one element): also writes pfp[i] = (position,
-// F'(rho_i)) so the force pass gathers both in one 16 B load.
-template <int T, int V, bool EV, bool SINGLE, class Fetch>
-__device__ __forceinline__ void eam_rho_atom(const PairArgs& A, const EamDev& E, float* __restrict__ fpf,
-                                             float* __restrict__ epf, float4* __restrict__ pfp, int64_t i,
-                                             int lane, bool live, const Fetch& fetch) {
+// Density of atom i, reduced over its T lanes.
+template <int T, int V, bool SINGLE, class Fetch>
+__device__ __forceinline__ float eam_rho_atom(const PairArgs& A, const EamDev& E, int64_t i, int lane, bool live,
+                                              const Fetch& fetch) {
   const int nn = live ? min(A.nnb[i], A.maxnb) : 0;
   const float4 pi = live ? A.posf[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-  const int cp = live ? A.cellpack[i] : 0;
-  const int ti = SINGLE ? 0 : __float_as_int(pi.w);
   const int nr = E.nr, nr1 = E.nr + 1;
   const float rdr = E.rdrf;
   float rho = 0.f, crho = 0.f;
   const PairFrame PF(pi, A.g);
   const ListRows<T, V> L(A.nbr, i, lane, A.stride, nn);
-  uint32_t ent[V], nxt[V];
-  if (L.nrow > 0) L.load(0, ent);
-  for (int r = 0; r < L.nrow; ++r) {
-    if (r + 1 < L.nrow) L.load(r + 1, nxt);
-    float4 pj[V];
+  for_rows(L, [&](const auto& R) {
+    constexpr int N = sizeof(R.e) / sizeof(R.e[0]);
+    float4 pj[N];
 #pragma unroll
-    for (int q = 0; q < V; ++q) {
-      if (!L.valid(r, q)) ent[q] = L.standin;
-      pj[q] = fetch(ent[q], ent[q] & GBMD_IDX_MASK);
-    }
+    for (int q = 0; q < N; ++q) pj[q] = fetch(R.e[q], R.e[q] & GBMD_IDX_MASK);
+    auto retest = [&](int q) {
+      return exact_inside(A.posd, i, R.e[q] & GBMD_IDX_MASK, R.e[q] >> GBMD_IDX_BITS, A.cellpack[i], A.g, E.rcut2,
+                          0.0);
+    };
     float rr = 0.f;
-    if constexpr (V == 4) {
+    if constexpr (N % 2 == 0) {
       // entries (0, 1) and (2, 3) in packed FP32; the rows' partial sums
       // stay packed until the row is added to the compensated sum
       float2 rr2 = f2(0.f, 0.f);
 #pragma unroll
-      for (int q = 0; q < V; q += 2) {
-        const GeomF2 G = PF.geom(ent[q], ent[q + 1], pj[q], pj[q + 1]);
+      for (int q = 0; q < N; q += 2) {
+        const GeomF2 G = PF.geom(R.e[q], R.e[q + 1], pj[q], pj[q + 1]);
         bool ina = G.d2.x < E.rc2lo, inb = G.d2.y < E.rc2lo;
-        if (!ina && G.d2.x <= E.rc2hi && L.valid(r, q))
-          ina = exact_inside(A.posd, i, ent[q] & GBMD_IDX_MASK, ent[q] >> GBMD_IDX_BITS, cp, A.g, E.rcut2, 0.0);
-        if (!inb && G.d2.y <= E.rc2hi && L.valid(r, q + 1))
-          inb = exact_inside(A.posd, i, ent[q + 1] & GBMD_IDX_MASK, ent[q + 1] >> GBMD_IDX_BITS, cp, A.g, E.rcut2,
-                             0.0);
+        if (!ina && G.d2.x <= E.rc2hi && R.ok[q]) ina = retest(q);
+        if (!inb && G.d2.y <= E.rc2hi && R.ok[q + 1]) inb = retest(q + 1);
         const float2 rd = __fmul2_rn(G.d2, f2(rsqrtf(G.d2.x), rsqrtf(G.d2.y)));
         const float2 tt = __ffma2_rn(rd, f2(rdr, rdr), f2(1.0f, 1.0f));
         const int ma = min((int)tt.x, nr - 1), mb = min((int)tt.y, nr - 1);
@@ -441,12 +511,10 @@ __device__ __forceinline__ void eam_rho_atom(const PairArgs& A, const EamDev& E,
       rr = rr2.x + rr2.y;
     } else {
 #pragma unroll
-      for (int q = 0; q < V; ++q) {
-        const uint32_t j = ent[q] & GBMD_IDX_MASK;
-        const GeomF G = geom_f(ent[q], pj[q], pi, A.g);
+      for (int q = 0; q < N; ++q) {
+        const GeomF G = geom_f(R.e[q], pj[q], pi, A.g);
         bool in = G.d2 < E.rc2lo;
-        if (!in && G.d2 <= E.rc2hi && L.valid(r, q))
-          in = exact_inside(A.posd, i, j, ent[q] >> GBMD_IDX_BITS, cp, A.g, E.rcut2, 0.0);
+        if (!in && G.d2 <= E.rc2hi && R.ok[q]) in = retest(q);
         const float rd = G.d2 * rsqrtf(G.d2);
         float t;
         const int m = knot_f(rd, rdr, nr, t);
@@ -455,27 +523,33 @@ __device__ __forceinline__ void eam_rho_atom(const PairArgs& A, const EamDev& E,
       }
     }
     kahan_add(rho, crho, rr);
-#pragma unroll
-    for (int q = 0; q < V; ++q) ent[q] = nxt[q];
-  }
+  });
   group_reduce_kahan<T>(rho, crho);
-  if (live && lane == 0) {
-    // Rho2EmbOp / eam_alloy_fEmbed: F'(rho) (and F(rho) on energy steps),
-    // linear continuation above rhomax
-    const float R = rho - crho;
-    float q = fmaf(R, E.rdrhof, 1.0f);
-    int m = (int)q;
-    m = max(1, min(m, E.nrho - 1));
-    q = fminf(q - (float)m, 1.0f);
-    const float4 c = __ldg(&E.frho4[(SINGLE ? 0 : ti * (E.nrho + 1)) + m]);
-    const float fp = spline_der(c, q, E.rdrhof);
-    fpf[i] = fp;
-    if (SINGLE) pfp[i] = make_float4(pi.x, pi.y, pi.z, fp);
-    if (EV) {
-      float phi = spline_val(c, q);
-      if (R > E.rhomaxf) phi = fmaf(fp, R - E.rhomaxf, phi);
-      epf[i] = phi;
-    }
+  return rho - crho;
+}
+
+// Rho2EmbOp / eam_alloy_fEmbed of one atom: F'(rho) (and F(rho) on energy
+// steps), linear continuation above rhomax.  SINGLE (one element): also
+// writes pfp[i] = (position, F'(rho_i)) so the force pass gathers both in one
+// 16 B load.
+template <bool EV, bool SINGLE>
+__device__ __forceinline__ void eam_embed(const PairArgs& A, const EamDev& E, int64_t i, float R,
+                                          float* __restrict__ fpf, float* __restrict__ epf,
+                                          float4* __restrict__ pfp) {
+  const float4 pi = A.posf[i];
+  const int ti = SINGLE ? 0 : __float_as_int(pi.w);
+  float q = fmaf(R, E.rdrhof, 1.0f);
+  int m = (int)q;
+  m = max(1, min(m, E.nrho - 1));
+  q = fminf(q - (float)m, 1.0f);
+  const float4 c = __ldg(&E.frho4[(SINGLE ? 0 : ti * (E.nrho + 1)) + m]);
+  const float fp = spline_der(c, q, E.rdrhof);
+  fpf[i] = fp;
+  if (SINGLE) pfp[i] = make_float4(pi.x, pi.y, pi.z, fp);
+  if (EV) {
+    float phi = spline_val(c, q);
+    if (R > E.rhomaxf) phi = fmaf(fp, R - E.rhomaxf, phi);
+    epf[i] = phi;
   }
 }
 
@@ -483,8 +557,19 @@ template <int T, int V, bool EV, bool SINGLE, bool PIECE>
 __global__ void __launch_bounds__(256) k_eam_rho_mixed(PairArgs A, EamDev E, float* __restrict__ fpf,
                                                        float* __restrict__ epf, float4* __restrict__ pfp) {
   const int64_t gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t i = PIECE ? A.i0 + gt / T : gt / T;
-  eam_rho_atom<T, V, EV, SINGLE>(A, E, fpf, epf, pfp, i, (int)(gt % T), i < A.n, GlobalFetch{A.posf});
+  int64_t i = PIECE ? A.i0 + gt / T : gt / T;
+  float R = eam_rho_atom<T, V, SINGLE>(A, E, i, (int)(gt % T), i < A.n, GlobalFetch{A.posf});
+  if (T > 1) {
+    // the embedding of the block's atoms on its first blockDim / T threads
+    __shared__ float rho[T > 1 ? 256 / T : 1];
+    const int nat = (int)blockDim.x / T;
+    if (threadIdx.x % T == 0) rho[threadIdx.x / T] = R;
+    __syncthreads();
+    if ((int)threadIdx.x >= nat) return;
+    R = rho[threadIdx.x];
+    i = (PIECE ? A.i0 : 0) + blockIdx.x * (int64_t)nat + threadIdx.x;
+  }
+  if (i < A.n) eam_embed<EV, SINGLE>(A, E, i, R, fpf, epf, pfp);
 }
 
 template <bool EV>
@@ -497,8 +582,9 @@ __global__ void __launch_bounds__(256) k_eam_rho_staged(PairArgs A, EamDev E, fl
   int64_t a0, a1;
   const bool ok = stage_cells(A.g, cstart, A.posf, K, cap, staged_pos, rows, sh, a0, a1);
   for (int64_t i = a0 + threadIdx.x; i < a1; i += blockDim.x) {
-    if (ok) eam_rho_atom<1, 4, EV, true>(A, E, fpf, epf, pfp, i, 0, true, StagedFetch{staged_pos, rows});
-    else eam_rho_atom<1, 4, EV, true>(A, E, fpf, epf, pfp, i, 0, true, GlobalFetch{A.posf});
+    const float R = ok ? eam_rho_atom<1, 4, true>(A, E, i, 0, true, StagedFetch{staged_pos, rows})
+                       : eam_rho_atom<1, 4, true>(A, E, i, 0, true, GlobalFetch{A.posf});
+    eam_embed<EV, true>(A, E, i, R, fpf, epf, pfp);
   }
 }
 
@@ -515,16 +601,14 @@ __device__ __forceinline__ int z2r_index_d(int a, int b) {
   return irow * (irow + 1) / 2 + icol;
 }
 
-// Force pass: f_i = sum_j u_ij (F'_i rho_j'(r) + F'_j rho_i'(r) + phi'(r)),
-// then force_to_accel and the fused Verlet halves.  SINGLE reads (position,
-// F'_j) through `fetch` from pfp; otherwise position (type in w) and fpf.
+// Force pass: f_i = sum_j u_ij (F'_i rho_j'(r) + F'_j rho_i'(r) + phi'(r)).
+// SINGLE reads (position, F'_j) through `fetch` from pfp; otherwise position
+// (type in w) and fpf.
 template <int T, int V, bool EV, bool SINGLE, class Fetch>
-__device__ __forceinline__ void eam_force_atom(const PairArgs& A, const EamDev& E, const float* __restrict__ fpf,
-                                               const float* __restrict__ epf, int64_t i, int lane, bool live,
-                                               const Fetch& fetch) {
+__device__ __forceinline__ PairSums eam_force_atom(const PairArgs& A, const EamDev& E, const float* __restrict__ fpf,
+                                                   int64_t i, int lane, bool live, const Fetch& fetch) {
   const int nn = live ? min(A.nnb[i], A.maxnb) : 0;
   const float4 pi = live ? A.posf[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-  const int cp = live ? A.cellpack[i] : 0;
   const float fpi = live ? fpf[i] : 0.f;
   const int ti = SINGLE ? 0 : __float_as_int(pi.w);
   const int nr = E.nr, nr1 = E.nr + 1;
@@ -532,27 +616,24 @@ __device__ __forceinline__ void eam_force_atom(const PairArgs& A, const EamDev& 
   float fx = 0.f, fy = 0.f, fz = 0.f, cfx = 0.f, cfy = 0.f, cfz = 0.f, e = 0.f, ce = 0.f;
   float v[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   const ListRows<T, V> L(A.nbr, i, lane, A.stride, nn);
-  uint32_t ent[V], nxt[V];
-  if (L.nrow > 0) L.load(0, ent);
-  for (int r = 0; r < L.nrow; ++r) {
-    if (r + 1 < L.nrow) L.load(r + 1, nxt);
-    float4 pj[V];
-    float fpj[V];
+  for_rows(L, [&](const auto& R) {
+    constexpr int N = sizeof(R.e) / sizeof(R.e[0]);
+    float4 pj[N];
+    float fpj[N];
 #pragma unroll
-    for (int q = 0; q < V; ++q) {
-      if (!L.valid(r, q)) ent[q] = L.standin;
-      const uint32_t j = ent[q] & GBMD_IDX_MASK;
-      pj[q] = fetch(ent[q], j);
+    for (int q = 0; q < N; ++q) {
+      const uint32_t j = R.e[q] & GBMD_IDX_MASK;
+      pj[q] = fetch(R.e[q], j);
       fpj[q] = SINGLE ? pj[q].w : __ldg(&fpf[j]);
     }
     float rx = 0.f, ry = 0.f, rz = 0.f, re = 0.f;
 #pragma unroll
-    for (int q = 0; q < V; ++q) {
-      const uint32_t j = ent[q] & GBMD_IDX_MASK;
-      const GeomF G = geom_f(ent[q], pj[q], pi, A.g);
+    for (int q = 0; q < N; ++q) {
+      const GeomF G = geom_f(R.e[q], pj[q], pi, A.g);
       bool in = G.d2 < E.rc2lo;
-      if (!in && G.d2 <= E.rc2hi && L.valid(r, q))
-        in = exact_inside(A.posd, i, j, ent[q] >> GBMD_IDX_BITS, cp, A.g, E.rcut2, 0.0);
+      if (!in && G.d2 <= E.rc2hi && R.ok[q])
+        in = exact_inside(A.posd, i, R.e[q] & GBMD_IDX_MASK, R.e[q] >> GBMD_IDX_BITS, A.cellpack[i], A.g, E.rcut2,
+                          0.0);
       const float rs = rsqrtf(G.d2);
       const float rd = G.d2 * rs;
       float t;
@@ -598,34 +679,34 @@ __device__ __forceinline__ void eam_force_atom(const PairArgs& A, const EamDev& 
     kahan_add(fy, cfy, ry);
     kahan_add(fz, cfz, rz);
     if (EV) kahan_add(e, ce, re);
-#pragma unroll
-    for (int q = 0; q < V; ++q) ent[q] = nxt[q];
-  }
+  });
   group_reduce_kahan<T>(fx, cfx);
   group_reduce_kahan<T>(fy, cfy);
   group_reduce_kahan<T>(fz, cfz);
+  PairSums S;
+  S.f[0] = fx - cfx;
+  S.f[1] = fy - cfy;
+  S.f[2] = fz - cfz;
+  S.e = 0.f;
   if (EV) {
     group_reduce_kahan<T>(e, ce);
     reduce6(v, T);
+    S.e = e - ce;
+#pragma unroll
+    for (int q = 0; q < 6; ++q) S.v[q] = v[q];
   }
-  if (live && lane == 0) {
-    const float im = A.inv_massf[ti];
-    double o[9];
-    if (EV) vir9(v, o);
-    const double epv = EV ? (double)epf[i] + (double)(e - ce) : 0.0;
-    atom_epilogue<true>(A, i, ti, 0., 0., 0., (fx - cfx) * im, (fy - cfy) * im, (fz - cfz) * im, epv,
-                        EV ? o : nullptr);
-  }
+  return S;
 }
 
 template <int T, int V, bool EV, bool SINGLE, bool PIECE>
-__global__ void __launch_bounds__(256, 4) k_eam_force_mixed(PairArgs A, EamDev E, const float* __restrict__ fpf,
+__global__ void __launch_bounds__(256, EV ? 3 : 4) k_eam_force_mixed(PairArgs A, EamDev E, const float* __restrict__ fpf,
                                                          const float* __restrict__ epf,
                                                          const float4* __restrict__ pfp) {
   const int64_t gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   const int64_t i = PIECE ? A.i0 + gt / T : gt / T;
-  eam_force_atom<T, V, EV, SINGLE>(A, E, fpf, epf, i, (int)(gt % T), i < A.n,
-                                   GlobalFetch{SINGLE ? pfp : A.posf});
+  const PairSums S = eam_force_atom<T, V, EV, SINGLE>(A, E, fpf, i, (int)(gt % T), i < A.n,
+                                                      GlobalFetch{SINGLE ? pfp : A.posf});
+  block_epilogue<T, EV>(A, (PIECE ? A.i0 : 0) + blockIdx.x * (int64_t)(blockDim.x / T), S, epf);
 }
 
 template <bool EV>
@@ -639,8 +720,9 @@ __global__ void __launch_bounds__(256) k_eam_force_staged(PairArgs A, EamDev E, 
   int64_t a0, a1;
   const bool ok = stage_cells(A.g, cstart, pfp, K, cap, staged_pos, rows, sh, a0, a1);
   for (int64_t i = a0 + threadIdx.x; i < a1; i += blockDim.x) {
-    if (ok) eam_force_atom<1, 4, EV, true>(A, E, fpf, epf, i, 0, true, StagedFetch{staged_pos, rows});
-    else eam_force_atom<1, 4, EV, true>(A, E, fpf, epf, i, 0, true, GlobalFetch{pfp});
+    const PairSums S = ok ? eam_force_atom<1, 4, EV, true>(A, E, fpf, i, 0, true, StagedFetch{staged_pos, rows})
+                          : eam_force_atom<1, 4, EV, true>(A, E, fpf, i, 0, true, GlobalFetch{pfp});
+    atom_finish<EV>(A, i, S, EV ? epf[i] : 0.f);
   }
 }
 
@@ -1208,6 +1290,8 @@ static int launch_mixed_shape(gbmd_context* c, const PairArgs& A, int part) {
     case 4 * 8 + 1: launch_mixed_TV<4, 1, EV, PIECE>(c, A, part); break;
     case 4 * 8 + 4: launch_mixed_TV<4, 4, EV, PIECE>(c, A, part); break;
     case 8 * 8 + 1: launch_mixed_TV<8, 1, EV, PIECE>(c, A, part); break;
+    case 8 * 8 + 4: launch_mixed_TV<8, 4, EV, PIECE>(c, A, part); break;
+    case 16 * 8 + 4: launch_mixed_TV<16, 4, EV, PIECE>(c, A, part); break;
     case 16 * 8 + 1: launch_mixed_TV<16, 1, EV, PIECE>(c, A, part); break;
     default:
       return set_error(c, GBMD_ERR_INVALID, "unsupported launch: %d lanes x %d entries per atom", c->tpa, c->vec);

@@ -399,13 +399,13 @@ __device__ __forceinline__ int build_stage(const BuildCell& B, const float4* __r
 // Deferred FP64 re-test of an atom's band entries: recompute each entry's
 // FP32 d2 with the rounded operations of the staging and the walk, re-test
 // the band ones and compact the row in place.  Returns the entries dropped.
-__device__ __noinline__ int build_retest_row(uint32_t* row, int nkeep, int wsh, int W, int64_t stride,
+__device__ __noinline__ int build_retest_row(uint32_t* row, int nkeep, int wsh, int tsh, int W, int64_t stride,
                                              const float4* __restrict__ pf, float4 pi, const double* __restrict__ x,
                                              const double* __restrict__ y, const double* __restrict__ z, int i,
                                              int cx, int cy, int cz, const Grid g, double R2, float R2lo) {
   int wpos = 0;
   for (int p = 0; p < nkeep; ++p) {
-    const uint32_t w = row[(size_t)(p >> wsh) * stride + (p & (W - 1))];
+    const uint32_t w = row[(size_t)(p >> wsh) * stride + list_word(p & (W - 1), wsh, tsh)];
     const int k = (int)(w & GBMD_IDX_MASK);
     const uint32_t code = w >> GBMD_IDX_BITS;
     const float4 pj = pf[k];
@@ -419,7 +419,7 @@ __device__ __noinline__ int build_retest_row(uint32_t* row, int nkeep, int wsh, 
     bool keepit = true;
     if (d2f >= R2lo) keepit = exact_within(x, y, z, i, k, code, cx, cy, cz, g, R2);
     if (keepit) {
-      row[(size_t)(wpos >> wsh) * stride + (wpos & (W - 1))] = w;
+      row[(size_t)(wpos >> wsh) * stride + list_word(wpos & (W - 1), wsh, tsh)] = w;
       ++wpos;
     }
   }
@@ -437,7 +437,8 @@ __device__ __forceinline__ int build_walk(const BuildCell& B, const float4* __re
                                           const double* __restrict__ x, const double* __restrict__ y,
                                           const double* __restrict__ z, const Grid& g, double R2, float R2lo,
                                           float R2hi, uint32_t* __restrict__ nbr, int32_t* __restrict__ nnb,
-                                          int maxnb, int W, int wsh, int64_t stride, int* __restrict__ err,
+                                          int maxnb, int W, int wsh, int tsh, int64_t stride,
+                                          int* __restrict__ err,
                                           float4* stage, int lane) {
   const unsigned FULL = 0xffffffffu;
   const float FAR = 1e18f;
@@ -464,7 +465,7 @@ __device__ __forceinline__ int build_walk(const BuildCell& B, const float4* __re
       bhi.y = fmaxf(bhi.y, __shfl_xor_sync(FULL, bhi.y, o));
       bhi.z = fmaxf(bhi.z, __shfl_xor_sync(FULL, bhi.z, o));
     }
-    uint32_t* row = nbr + (size_t)i * W;  // slot k at row[(k >> wsh) * stride + (k & (W - 1))]
+    uint32_t* row = nbr + (size_t)i * W;  // slot k at row[(k >> wsh) * stride + list_word(k & (W - 1))]
     int cnt = 0;
     bool unc = false;
     for (int q0 = 0; q0 < B.total; q0 += BUILD_CHUNK) {
@@ -490,11 +491,11 @@ __device__ __forceinline__ int build_walk(const BuildCell& B, const float4* __re
         if (G == 16) {
           const int other = __shfl_xor_sync(FULL, (int)in, 16);
           const int pos = cnt + (half & other);  // candidate 2t goes first
-          uint32_t* dst = row + (size_t)(pos >> wsh) * stride + (pos & (W - 1));
+          uint32_t* dst = row + (size_t)(pos >> wsh) * stride + list_word(pos & (W - 1), wsh, tsh);
           if (in && pos < maxnb) *dst = w;
           cnt += (int)in + other;
         } else {
-          uint32_t* dst = row + (size_t)(cnt >> wsh) * stride + (cnt & (W - 1));
+          uint32_t* dst = row + (size_t)(cnt >> wsh) * stride + list_word(cnt & (W - 1), wsh, tsh);
           if (in && cnt < maxnb) *dst = w;
           cnt += (int)in;
         }
@@ -505,11 +506,11 @@ __device__ __forceinline__ int build_walk(const BuildCell& B, const float4* __re
       const int partner_unc = __shfl_xor_sync(FULL, (int)unc, 16);
       unc = unc || partner_unc != 0;
       __syncwarp();  // the high-half lanes' entries are visible to the low half
-      if (half == 0 && unc) cnt -= build_retest_row(row, min(cnt, maxnb), wsh, W, stride, pf, pi, x, y, z, i,
+      if (half == 0 && unc) cnt -= build_retest_row(row, min(cnt, maxnb), wsh, tsh, W, stride, pf, pi, x, y, z, i,
                                                     B.cx, B.cy, B.cz, g, R2, R2lo);
       cnt = __shfl_sync(FULL, cnt, hl);  // the high-half lane takes the corrected count
     } else if (unc) {
-      cnt -= build_retest_row(row, min(cnt, maxnb), wsh, W, stride, pf, pi, x, y, z, i, B.cx, B.cy, B.cz, g,
+      cnt -= build_retest_row(row, min(cnt, maxnb), wsh, tsh, W, stride, pf, pi, x, y, z, i, B.cx, B.cy, B.cz, g,
                               R2, R2lo);
     }
     if (hv && half == 0) {
@@ -537,7 +538,7 @@ template <bool LOOP, bool HALF>
 __global__ void __launch_bounds__(BUILD_WARPS * 32) k_build_list_cells(
     int64_t ncells, const float4* __restrict__ pf, const double* __restrict__ x, const double* __restrict__ y,
     const double* __restrict__ z, const int32_t* __restrict__ cstart, Grid g, double R2, float R2lo, float R2hi,
-    uint32_t* __restrict__ nbr, int32_t* __restrict__ nnb, int maxnb, int W, int64_t stride,
+    uint32_t* __restrict__ nbr, int32_t* __restrict__ nnb, int maxnb, int W, int tsh, int64_t stride,
     int* __restrict__ err, const int* __restrict__ gate) {
   const int lane = threadIdx.x & 31;
   if (gate && !*gate) return;
@@ -583,9 +584,9 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32) k_build_list_cells(
   B.nh = cstart[cell + 1] - B.hb;
   int warp_max;
   if (B.nh <= 16)
-    warp_max = build_walk<16, HALF>(B, pf, x, y, z, g, R2, R2lo, R2hi, nbr, nnb, maxnb, W, wsh, stride, err, stage, lane);
+    warp_max = build_walk<16, HALF>(B, pf, x, y, z, g, R2, R2lo, R2hi, nbr, nnb, maxnb, W, wsh, tsh, stride, err, stage, lane);
   else
-    warp_max = build_walk<32, HALF>(B, pf, x, y, z, g, R2, R2lo, R2hi, nbr, nnb, maxnb, W, wsh, stride, err, stage, lane);
+    warp_max = build_walk<32, HALF>(B, pf, x, y, z, g, R2, R2lo, R2hi, nbr, nnb, maxnb, W, wsh, tsh, stride, err, stage, lane);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) warp_max = max(warp_max, __shfl_xor_sync(FULL, warp_max, o));
   if (lane == 0 && warp_max > 0) atomicMax(&err[ERRW_MAXNB], warp_max);
@@ -637,7 +638,7 @@ static int build_list(gbmd_context* c, const int* gate) {
   auto kern = loop ? (c->newton3 ? k_build_list_cells<true, true> : k_build_list_cells<true, false>)
                    : (c->newton3 ? k_build_list_cells<false, true> : k_build_list_cells<false, false>);
   kern<<<blocks, 32 * BUILD_WARPS, 0, c->stream>>>(c->grid.ncells, c->POSF(), c->X(), c->Y(), c->Z(), c->cell_start,
-                                                  c->grid, R2, R2lo, R2hi, c->nbr, c->nnb, c->maxnb, W, stride,
+                                                  c->grid, R2, R2lo, R2hi, c->nbr, c->nnb, c->maxnb, W, log2_of(c->tpa), stride,
                                                   c->d_err, gate);
   return GBMD_OK;
 }
@@ -836,12 +837,13 @@ __global__ void k_save_outer(int64_t n, const double* __restrict__ r, double* __
   }
 }
 
-// One thread per atom: the entries of its outer row within R now, in order.
+// One thread per atom: the entries of its outer row within R now, in the
+// order of the row's words.
 // The FP32 distance of the cell-relative copies (the builder's expression)
 // decides outside the band [R2lo, R2hi]; band entries are re-tested in
 // FP64 with the pair-set rounding.  A row never grows, so the list has the
-// outer list's capacity.  V4 (rows interleaved in groups of a multiple of 4
-// entries): the row is read 4 entries per 16-byte load with the next load in
+// outer list's capacity.  V4 (4 entries per lane
+// and load): the row is read 4 words per 16-byte load with the next load in
 // flight, and the 4 neighbour positions are gathered together.
 struct FilterArgs {
   int64_t n;
@@ -852,7 +854,7 @@ struct FilterArgs {
   const int32_t* nnb_out;
   uint32_t* nbr;
   int32_t* nnb;
-  int maxnb_out, W, wsh;
+  int maxnb_out, W, wsh, tsh;
   int64_t stride;
   double R2;
   float R2lo, R2hi;
@@ -885,17 +887,21 @@ __global__ void __launch_bounds__(256) k_filter_list(FilterArgs A, Grid g, const
     uint32_t* row = A.nbr + (size_t)i * A.W;
     int cnt = 0;
     auto put = [&](uint32_t w) {
-      row[(size_t)(cnt >> A.wsh) * A.stride + (cnt & (A.W - 1))] = w;
+      row[(size_t)(cnt >> A.wsh) * A.stride + list_word(cnt & (A.W - 1), A.wsh, A.tsh)] = w;
       ++cnt;
     };
     if (V4) {
-      // slot k at orow[(k >> wsh) * stride + (k & (W - 1))]; W is a multiple
-      // of 4, so 4 consecutive slots from a multiple of 4 are one aligned uint4
-      // (rows hold maxnb_out slots, a multiple of W: the last load stays in)
+      // words k .. k + 3 (k a multiple of 4) of row k / W are one lane's
+      // aligned uint4: its entries q * T + lane, q = 0 .. 3.  Rows hold
+      // maxnb_out words, a multiple of W, so the loads of every row that
+      // holds an entry stay in
       auto group = [&](int k) {
         return *reinterpret_cast<const uint4*>(orow + (size_t)(k >> A.wsh) * A.stride + (k & (A.W - 1)));
       };
-      const int ng = (nn + 3) >> 2;
+      const int ng = ((nn + A.W - 1) >> A.wsh) << (A.wsh - 2);
+      auto entry_of = [&](int k, int q) {  // which entry word k + q holds
+        return (k & ~(A.W - 1)) + (q << A.tsh) + ((k & (A.W - 1)) >> 2);
+      };
       uint4 cur = ng > 0 ? group(0) : make_uint4(0u, 0u, 0u, 0u);
       for (int t = 0; t < ng; ++t) {
         const int k0 = t << 2;
@@ -904,15 +910,15 @@ __global__ void __launch_bounds__(256) k_filter_list(FilterArgs A, Grid g, const
         const uint32_t e[4] = {cur.x, cur.y, cur.z, cur.w};
         float4 pj[4];
 #pragma unroll
-        for (int q = 0; q < 4; ++q) pj[q] = A.pf[k0 + q < nn ? (int64_t)(e[q] & GBMD_IDX_MASK) : i];
+        for (int q = 0; q < 4; ++q) pj[q] = A.pf[entry_of(k0, q) < nn ? (int64_t)(e[q] & GBMD_IDX_MASK) : i];
 #pragma unroll
         for (int q = 0; q < 4; ++q)
-          if (k0 + q < nn && filter_keep(A, g, i, pi, e[q], pj[q], cx, cy, cz)) put(e[q]);
+          if (entry_of(k0, q) < nn && filter_keep(A, g, i, pi, e[q], pj[q], cx, cy, cz)) put(e[q]);
         cur = nxt;
       }
     } else {
       for (int k = 0; k < nn; ++k) {
-        const uint32_t w = orow[(size_t)(k >> A.wsh) * A.stride + (k & (A.W - 1))];
+        const uint32_t w = orow[(size_t)(k >> A.wsh) * A.stride + list_word(k & (A.W - 1), A.wsh, A.tsh)];
         const float4 pj = A.pf[w & GBMD_IDX_MASK];
         if (filter_keep(A, g, i, pi, w, pj, cx, cy, cz)) put(w);
       }
@@ -950,8 +956,6 @@ static int outer_chain(gbmd_context* c, bool check_capacity, const int* gate) {
 
 static int filter_list(gbmd_context* c, const int* gate) {
   const int W = list_width(c);
-  int wsh = 0;
-  while ((1 << wsh) < W) ++wsh;
   const int64_t stride = c->npad * W;
   const int64_t need = (int64_t)(c->maxnb_out / W) * stride;
   if (need > c->nbr_cap) {
@@ -978,20 +982,64 @@ static int filter_list(gbmd_context* c, const int* gate) {
   A.nnb = c->nnb;
   A.maxnb_out = c->maxnb_out;
   A.W = W;
-  A.wsh = wsh;
+  A.wsh = log2_of(W);
+  A.tsh = log2_of(c->tpa);
   A.stride = stride;
   A.R2 = R2;
   A.R2lo = R2lo;
   A.R2hi = R2hi;
   const unsigned blocks = gate ? chain_blocks(c, c->n, 256, gate, 8) : nblk(c->n, 256);
-  if (W % 4 == 0) k_filter_list<true><<<blocks, 256, 0, c->stream>>>(A, c->grid, gate);
+  if (c->vec == 4) k_filter_list<true><<<blocks, 256, 0, c->stream>>>(A, c->grid, gate);
   else k_filter_list<false><<<blocks, 256, 0, c->stream>>>(A, c->grid, gate);
   c->list_valid = true;
   if (!gate) c->list_builds++;
   return GBMD_OK;
 }
 
+// More lanes per atom while the atoms alone cannot fill the chip; then the
+// fewest, since each doubling adds a step of the shuffle reduction and of the
+// epilogue's exchange.  Two lanes win longest where the pair work per entry is
+// largest, because their gathers touch fewer cache lines (ListRows).
+// Measured on GB300, us, lanes 1 / 2 / 4 / 8 / 16; force evaluations:
+//   eam_alloy, one element      4,000 atoms    36 / 24 / 18 / 15 / 13
+//                              16,384          39 / 28 / 22 / 18 / 22
+//                              32,000          39 / 29 / 23 / 27 / 31
+//   LJ                          4,000          14 / 10 /  8 /  6 /  6
+//                              16,384          14 / 10 /  8 /  8 /  9
+//                              32,000          14 / 12 / 11 / 10 / 14
+// and 20 NVE steps with two rebuilds, lanes 1 / 2 / 4:
+//   eam_alloy, one element    108,000         1,286 / 1,305 / 1,248
+//                             256,000         2,742 / 2,576 / 2,590
+//                             864,000         7,738 / 7,641 / 8,144
+//                           4,000,000        32,289 / 32,939 / 35,542
+//   two elements              256,000         3,425 / 3,125 / 3,096
+//                           2,048,000        21,073 / 20,706 / 22,275
+//   LJ                         32,000           513 / 440 / 428
+//                              62,500           630 / 577 / 591
+//                             256,000         1,597 / 1,557 / 1,653
+//   LJ mixture                253,000         2,104 / 2,098 / 2,192
+// The analytic EAM functions, bound by the SFU, take one lane where LJ takes two.
+void choose_launch(gbmd_context* c) {
+  if (c->launch_set) return;
+  const bool alloy = c->pot == GBMD_POT_EAM_ALLOY, single = alloy && c->eam.nel == 1;
+  const bool lj = c->pot == GBMD_POT_LJ || c->pot == GBMD_POT_LJ_MULTI;
+  int tpa = 1;
+  if (c->n <= 8192) tpa = 16;
+  else if (c->n <= 24576) tpa = 8;
+  else if (c->n <= (single ? 160000 : alloy ? 327680 : 49152)) tpa = 4;
+  else if (single ? c->n <= 1500000 : alloy || (lj && c->n <= 262144)) tpa = 2;
+  if (c->newton3 || c->staged) tpa = 1;  // the layout of the half list and of the staged kernels
+  c->vec = 4;
+  c->block = tpa == 1 || (tpa == 2 && alloy && !single) ? 256 : 128;
+  if (tpa == c->tpa) return;
+  c->tpa = tpa;
+  const int W = list_width(c);
+  if (c->maxnb > 0) c->maxnb = ((c->maxnb + W - 1) / W) * W;
+  if (c->maxnb_out > 0) c->maxnb_out = ((c->maxnb_out + W - 1) / W) * W;
+}
+
 int rebuild(gbmd_context* c, bool check_capacity, const int* gate) {
+  if (!gate && !c->capturing) choose_launch(c);
   if (c->n == 0 || !two_level(c)) {
     const int rc = rebuild_chain(c, check_capacity, gate);
     if (rc == GBMD_OK && !gate) c->list_builds++;
@@ -1053,6 +1101,7 @@ int export_pairs(gbmd_context* c, int64_t cap, uint64_t* id_i, uint64_t* id_j, i
   *count = total;
   if (cap < total || !id_i) return GBMD_OK;
   const int W = list_width(c);
+  const int wsh = log2_of(W), tsh = log2_of(c->tpa);
   const int64_t stride = c->npad * W;
   std::vector<uint32_t> nb((size_t)c->nbr_cap);
   GBMD_CUDA(c, cudaMemcpy(nb.data(), c->nbr, sizeof(uint32_t) * c->nbr_cap, cudaMemcpyDeviceToHost));
@@ -1061,7 +1110,7 @@ int export_pairs(gbmd_context* c, int64_t cap, uint64_t* id_i, uint64_t* id_j, i
   for (int64_t i = 0; i < n; ++i) {
     const int cx = cp[i] & 1023, cy = (cp[i] >> 10) & 1023, cz = cp[i] >> 20;
     for (int k = 0; k < nnb[i] && k < c->maxnb; ++k) {
-      const uint32_t e = nb[(size_t)(k / W) * stride + (size_t)i * W + (k % W)];
+      const uint32_t e = nb[(size_t)(k / W) * stride + (size_t)i * W + list_word(k % W, wsh, tsh)];
       const uint32_t j = e & GBMD_IDX_MASK, code = e >> GBMD_IDX_BITS;
       const int d[3] = {int(code & 3) - 1, int((code >> 2) & 3) - 1, int((code >> 4) & 3) - 1};
       const int cc[3] = {cx + d[0], cy + d[1], cz + d[2]};

@@ -3,7 +3,8 @@
 // Thread mapping: T consecutive lanes own one atom i (atoms in cell order).
 // The list is stored in rows of W = T*V words per atom (V entries per lane per
 // load), consecutive atoms adjacent: row r of atom i is nbr[r*stride + i*W ..
-// + W), so a warp reads 32*V*4 contiguous bytes per load.  Per-atom sums are reduced across the T lanes
+// + W), so a warp reads 32*V*4 contiguous bytes per load; entry r*W + p sits
+// in word list_word(p) of the row.  Per-atom sums are reduced across the T lanes
 // with shuffles; lane 0 of the group runs the epilogue.
 //
 // Epilogue (lane 0): a = f/m (force_to_accel), optional ep / virial stores,
@@ -22,7 +23,7 @@ struct PairArgs {
   int64_t n;                  // atoms [i0, n) are processed (a piece of the cell order, or all)
   int64_t i0;
   int64_t stride;             // npad * W (words per list row)
-  int W, wsh;                 // words per atom per row (lanes x entries per lane), log2 W
+  int W, wsh, tsh;            // words per atom per row (lanes x entries per lane), log2 W, log2 lanes
   const uint32_t* nbr;
   const int32_t* nnb;
   int maxnb;
@@ -87,6 +88,43 @@ __device__ __forceinline__ void unpack_cell(int cp, int& cx, int& cy, int& cz) {
   cz = cp >> 20;
 }
 
+struct GeomF {
+  float dx, dy, dz, d2;
+};
+
+// Exact FP64 cutoff test of a pair whose FP32 d2 fell in the ambiguous band:
+// d2 <= rc2 and, for per-pair cutoffs, sqrt(d2) <= rc_pair (the reference's
+// two-stage test).  Kept out of line: it runs for ~1e-4 of the pairs.
+static __device__ __noinline__ bool exact_inside(const double4_32a* __restrict__ posd, int64_t i, uint32_t j,
+                                          uint32_t code, int cp, const Grid g, double rc2, double rc_pair) {
+  int cx, cy, cz;
+  unpack_cell(cp, cx, cy, cz);
+  double Sx, Sy, Sz, a, b, c;
+  image_shift(g, cx, cy, cz, code, Sx, Sy, Sz);
+  const double4_32a di = posd[i], dj = posd[j];
+  const double d2 = exact_d2(di.x, di.y, di.z, dj.x, dj.y, dj.z, Sx, Sy, Sz, a, b, c);
+  if (!(d2 <= rc2)) return false;
+  return rc_pair <= 0.0 || sqrt(d2) <= rc_pair;
+}
+
+// {0,1,2} -> -1.f, 0.f, +1.f exactly (small integer through the 2^23 mantissa
+// trick); the separation shift is then one FMA per axis.
+__device__ __forceinline__ float unit_of(uint32_t b) { return __int_as_float(0x4B000000u | b) - 8388609.0f; }
+
+__device__ __forceinline__ GeomF geom_f(uint32_t ent, const float4& pj, const float4& pi, const Grid& g) {
+  GeomF r;
+  r.dx = fmaf(unit_of((ent >> 26) & 3u), g.hf[0], pj.x - pi.x);
+  r.dy = fmaf(unit_of((ent >> 28) & 3u), g.hf[1], pj.y - pi.y);
+  r.dz = fmaf(unit_of(ent >> 30), g.hf[2], pj.z - pi.z);
+  r.d2 = fmaf(r.dx, r.dx, fmaf(r.dy, r.dy, r.dz * r.dz));
+  return r;
+}
+
+// Entry k of atom i's list row base (nbr + i * W).
+__device__ __forceinline__ size_t list_slot(const PairArgs& A, int k) {
+  return (size_t)(k >> A.wsh) * A.stride + list_word(k & (A.W - 1), A.wsh, A.tsh);
+}
+
 // Lane-0 epilogue for atom i: force -> acceleration, stores, fused push.
 // fx,fy,fz are the force in FP64; mixed kernels pass accelerations computed in
 // FP32 through `amixed` (then fx.. are ignored).
@@ -96,16 +134,20 @@ __device__ __forceinline__ void atom_epilogue(const PairArgs& A, int64_t i, int 
                                               const double* v9) {
   double ax, ay, az;
   if (MIXED) {
-    ax = (double)afx;
-    ay = (double)afy;
-    az = (double)afz;
+    ax = widen(afx);
+    ay = widen(afy);
+    az = widen(afz);
+    if (!(isfinite(afx) && isfinite(afy) && isfinite(afz))) {
+      atomicOr(&A.err[ERRW_FLAGS], GBMD_DEVERR_NONFINITE);
+      atomicCAS(&A.err[ERRW_BADATOM], -1, (int)i);
+    }
   } else {
     const double m = A.mass[t];
     ax = fx / m;
     ay = fy / m;
     az = fz / m;
   }
-  if (!(isfinite(ax) && isfinite(ay) && isfinite(az))) {
+  if (!MIXED && !(isfinite(ax) && isfinite(ay) && isfinite(az))) {
     atomicOr(&A.err[ERRW_FLAGS], GBMD_DEVERR_NONFINITE);
     atomicCAS(&A.err[ERRW_BADATOM], -1, (int)i);
   }

@@ -9,154 +9,301 @@
 // with dr = (x_j + n*L) - x_i and d2 rounded exactly like the list builder
 // and the oracle, so cutoff membership is identical.
 //
-// Per unit (one ordered list entry): 4 B of list, one 32 B position gather,
-// the cutoff test and, inside the cutoff, the pair function.
+// The FP64 pipe is the bound: an FP64 instruction of a warp takes 16 cycles
+// of an SM, as long as some 60 FP32 or integer ones over its four schedulers.
+// So everything that need not be FP64 is not: the cutoff is screened in FP32
+// (the mixed kernels' screen, exact outside its band), the knot index and the
+// float conversions are integer arithmetic, 1/r comes from an FP32 seed, image
+// shifts are added only in border cells, and the virial's six values carry
+// their factor at the end.  Cu, 108,000 atoms, with energies and virials:
+// density 437 -> 288 us, force 928 -> 577 us; LJ, 256,000
+// atoms: 3,456 -> 1,134 us.
 #include "gbmd_pair_common.cuh"
 
 namespace gbmd {
 
+// r = sqrt(d2), and 1/r with it where INV: the FP32 rsqrt as seed y0 (relative
+// error below 2^-22), one Householder step of third order, y = y0 (1 + e/2 +
+// 3 e^2/8) with e = 1 - d2 y0^2 (remainder e^3, below 2^-60), then a Newton
+// correction of r = d2 y and one of y towards 1/r.  Outside FP32's range the
+// library functions are taken.
+template <bool INV>
+__device__ __forceinline__ double root(double d2, double& y) {
+  const uint32_t hi = (uint32_t)__double2hiint(d2);
+  if (hi - 0x3a000000u < 0x0c000000u) {  // 2^-95 <= d2 < 2^97
+    const float s = __uint_as_float(((hi - 0x38000000u) << 3) | ((uint32_t)__double2loint(d2) >> 29));
+    const double y0 = widen(rsqrtf(s));
+    const double e = fma(-(d2 * y0), y0, 1.0);
+    y = fma(y0 * e, fma(e, 0.375, 0.5), y0);
+    double r = d2 * y;
+    r = fma(fma(-r, r, d2), 0.5 * y, r);
+    if (INV) y = fma(fma(-r, y, 1.0), y, y);
+    return r;
+  }
+  const double r = sqrt(d2);
+  y = 1.0 / r;
+  return r;
+}
+
+// 1/d2 from an FP32 seed y0: y0 (1 + e + e^2), e = 1 - d2 y0, remainder e^3.
+__device__ __forceinline__ double inverse(double d2) {
+  const uint32_t hi = (uint32_t)__double2hiint(d2);
+  if (hi - 0x3a000000u < 0x0c000000u) {
+    const float s = __uint_as_float(((hi - 0x38000000u) << 3) | ((uint32_t)__double2loint(d2) >> 29));
+    const double y0 = widen(__frcp_rn(s));
+    const double e = fma(-d2, y0, 1.0);
+    return fma(y0, fma(e, e, e), y0);
+  }
+  return 1.0 / d2;
+}
+
+// Knot m = floor(t), capped at nr - 1, and p = t - m, capped at 1: the integer
+// part of t in [1, 2^20) by shifts, the fraction by one subtraction.
+__device__ __forceinline__ int r_knot_d(double t, int nr, double& p) {
+  const long long b = __double_as_longlong(t);
+  const int ex = (int)(b >> 52) - 1023;
+  if ((unsigned)ex < 20u) {
+    const long long mant = b & 0xfffffffffffffll;
+    const int m = (int)((mant | 0x10000000000000ll) >> (52 - ex));
+    if (m < nr) {
+      p = __longlong_as_double(((mant << ex) & 0xfffffffffffffll) | 0x3ff0000000000000ll) - 1.0;
+      return m;
+    }
+  }
+  const int m = min((int)t, nr - 1);
+  p = fmin(t - m, 1.0);
+  return m;
+}
+
+// Where atom i's pairs start from: its positions and its cell.
+struct PairHome {
+  double4_32a pd;
+  float4 pf;
+  int cx, cy, cz, nn;
+  bool border;  // some stencil cell lies across the box face
+  const uint32_t* row;
+  __device__ __forceinline__ PairHome(const PairArgs& A, int64_t i, bool live)
+      : pd(make_double4_32a(0., 0., 0., 0.)), pf(make_float4(0.f, 0.f, 0.f, 0.f)), cx(0), cy(0), cz(0), nn(0),
+        row(A.nbr + (size_t)i * A.W) {
+    if (live) {
+      pd = A.posd[i];
+      pf = A.posf[i];
+      unpack_cell(A.cellpack[i], cx, cy, cz);
+      nn = min(A.nnb[i], A.maxnb);
+    }
+    border = cx == 0 || cy == 0 || cz == 0 || cx == A.g.nc[0] - 1 || cy == A.g.nc[1] - 1 || cz == A.g.nc[2] - 1;
+  }
+  // FP64 separation of entry ent and its squared length
+  __device__ __forceinline__ double separation(const PairArgs& A, uint32_t ent, double& dx, double& dy,
+                                               double& dz) const {
+    const double4_32a pj = A.posd[ent & GBMD_IDX_MASK];
+    double x = pj.x, y = pj.y, z = pj.z;
+    if (border) {
+      const uint32_t code = ent >> GBMD_IDX_BITS;
+      const int nx = image_of(cx, code_dx(code), A.g.nc[0]), ny = image_of(cy, code_dy(code), A.g.nc[1]),
+                nz = image_of(cz, code_dz(code), A.g.nc[2]);
+      if (nx) x = __dadd_rn(x, nx > 0 ? A.g.L[0] : -A.g.L[0]);
+      if (ny) y = __dadd_rn(y, ny > 0 ? A.g.L[1] : -A.g.L[1]);
+      if (nz) z = __dadd_rn(z, nz > 0 ? A.g.L[2] : -A.g.L[2]);
+    }
+    // the reference's rounding, which the oracle shares
+    dx = __dsub_rn(x, pd.x);
+    dy = __dsub_rn(y, pd.y);
+    dz = __dsub_rn(z, pd.z);
+    return __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+  }
+};
+
+// body(entry, type of j): the entries of a group's list within the cutoff,
+// every lane its own k = lane, lane + T, ...  A lane runs ahead over the
+// entries that the FP32 screen excludes, so a warp takes the FP64 body as
+// often as its fullest lane has pairs, not list entries (44 and 54, Cu).
+// limits(type): the screen's band and the exact cutoffs of the pair.
+struct PairLimits {
+  float lo, hi;
+  double rc2, rc;  // rc <= 0: no second test
+};
+
+template <int T, class Limits, class Body>
+__device__ __forceinline__ void for_pairs(const PairArgs& A, const PairHome& H, int64_t i, int lane, Limits limits,
+                                          Body body) {
+  int k = lane;
+  for (;;) {
+    uint32_t ent = 0;
+    int tj = 0;
+    bool found = false;
+    while (k < H.nn && !found) {
+      ent = __ldg(H.row + list_slot(A, k));
+      k += T;
+      const float4 pj = A.posf[ent & GBMD_IDX_MASK];
+      tj = __float_as_int(pj.w);
+      const PairLimits P = limits(tj);
+      const float d2 = geom_f(ent, pj, H.pf, A.g).d2;
+      found = d2 <= P.hi;
+      if (found && d2 >= P.lo)
+        found = exact_inside(A.posd, i, ent & GBMD_IDX_MASK, ent >> GBMD_IDX_BITS, A.cellpack[i], A.g, P.rc2, P.rc);
+    }
+    if (!found) break;
+    body(ent, tj);
+  }
+}
+
+// Epilogue of a block's atoms i0 .. i0 + blockDim / T: the sums f (3), e and
+// the virial xx yy zz xy xz yz (before its factor -1/2) of each group's first
+// lane pass to the block's first blockDim / T threads, one atom each, so that
+// the FP64 work per atom runs on full warps; the virial rows are written
+// contiguously.  A block whose lanes own an atom each keeps f and e in place.
+template <int T, bool EV>
+__device__ __forceinline__ void block_epilogue_d(const PairArgs& A, int64_t i0, int ti, double f0, double f1,
+                                                 double f2, double e, const double* v,
+                                                 const double* __restrict__ emb = nullptr) {
+  constexpr bool SHARED = T > 1 || EV;
+  constexpr int NF = T > 1 ? 4 : 0, NV = NF + (EV ? 6 : 0);
+  __shared__ double sums[SHARED ? NV : 1][SHARED ? 256 / T : 1];
+  const int nat = (int)blockDim.x / T;
+  if constexpr (SHARED) {
+    const int a = (int)threadIdx.x / T;
+    if (threadIdx.x % T == 0) {
+      if constexpr (T > 1) {
+        sums[0][a] = f0;
+        sums[1][a] = f1;
+        sums[2][a] = f2;
+        sums[3][a] = e;
+      }
+      if constexpr (EV) {
+#pragma unroll
+        for (int q = 0; q < 6; ++q) sums[NF + q][a] = -0.5 * v[q];
+      }
+    }
+    __syncthreads();
+    if constexpr (EV) {
+      const int m = A.want_virial ? (int)min((int64_t)nat, A.n - i0) * 9 : 0;
+      for (int k = threadIdx.x; k < m; k += blockDim.x)  // row-major 3x3
+        A.vir[9 * i0 + k] = sums[NF + (int)((0x254513430ll >> (4 * (k % 9))) & 15)][k / 9];
+    }
+    if ((int)threadIdx.x >= nat) return;
+    if constexpr (T > 1) {
+      f0 = sums[0][threadIdx.x];
+      f1 = sums[1][threadIdx.x];
+      f2 = sums[2][threadIdx.x];
+      e = sums[3][threadIdx.x];
+    }
+  }
+  const int64_t i = i0 + threadIdx.x;
+  if (i >= A.n) return;
+  if (T > 1) ti = __float_as_int(A.posf[i].w);
+  if (EV && emb) e += emb[i];
+  atom_epilogue<false>(A, i, ti, f0, f1, f2, 0.f, 0.f, 0.f, e, nullptr);
+}
+
 // ---------------------------------------------------------------------------
 // Lennard-Jones (single parameter set and per-type-pair tables)
 // ---------------------------------------------------------------------------
-struct LJSingle {
-  double eps, sig, ecut, rc2;
-};
-
 template <int T, bool EV, bool MULTI>
-__global__ void __launch_bounds__(256) k_lj(PairArgs A, LJSingle P, const LJPair* __restrict__ tab, int ntypes,
+__global__ void __launch_bounds__(256) k_lj(PairArgs A, LJPair P, const LJPair* __restrict__ tab, int ntypes,
                                             double rcmax2) {
-  __shared__ double sd[MULTI ? GBMD_MAX_TYPES * GBMD_MAX_TYPES * 5 : 1];
+  __shared__ double sd[MULTI ? GBMD_MAX_TYPES * GBMD_MAX_TYPES * 4 : 1];
+  __shared__ float2 sb[MULTI ? GBMD_MAX_TYPES * GBMD_MAX_TYPES : 1];
   if (MULTI) {
     for (int q = threadIdx.x; q < ntypes * ntypes; q += blockDim.x) {
       const LJPair& p = tab[q];
-      sd[5 * q + 0] = p.eps;
-      sd[5 * q + 1] = p.sig;
-      sd[5 * q + 2] = p.rc;
-      sd[5 * q + 3] = p.ecut;
-      sd[5 * q + 4] = p.rc2;
+      sd[4 * q + 0] = p.eps;
+      sd[4 * q + 1] = p.sig * p.sig;
+      sd[4 * q + 2] = p.rc;
+      sd[4 * q + 3] = p.ecut;
+      sb[q] = make_float2(p.rc2lo, p.rc2hi);
     }
     __syncthreads();
   }
-  const int64_t gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t i = A.i0 + gt / T;
-  const int lane = (int)(gt % T);
-  const bool live = i < A.n;
-  const int nn = live ? min(A.nnb[i], A.maxnb) : 0;
-  int cx = 0, cy = 0, cz = 0, ti = 0;
-  if (live) unpack_cell(A.cellpack[i], cx, cy, cz);
-
-  {
-    double fx = 0., fy = 0., fz = 0., e = 0.;
-    double v[9] = {0., 0., 0., 0., 0., 0., 0., 0., 0.};
-    double4_32a pi = make_double4_32a(0., 0., 0., 0.);
-    if (live) pi = A.posd[i];
-    ti = (int)pi.w;
-    const uint32_t* row = A.nbr + (size_t)i * A.W;
-    for (int k = lane; k < nn; k += T) {
-      const uint32_t ent = __ldg(row + list_slot(A, k));
-      const uint32_t j = ent & GBMD_IDX_MASK, code = ent >> GBMD_IDX_BITS;
-      const double4_32a pj = A.posd[j];
-      double Sx, Sy, Sz, dx, dy, dz;
-      image_shift(A.g, cx, cy, cz, code, Sx, Sy, Sz);
-      const double d2 = exact_d2(pi.x, pi.y, pi.z, pj.x, pj.y, pj.z, Sx, Sy, Sz, dx, dy, dz);
-      double eps, sig, ecut;
-      if (MULTI) {
-        const int pid = ti * ntypes + (int)pj.w;
-        if (!(d2 <= rcmax2)) continue;
-        const double r = sqrt(d2);
-        if (!(r <= sd[5 * pid + 2])) continue;
-        eps = sd[5 * pid]; sig = sd[5 * pid + 1]; ecut = sd[5 * pid + 3];
-      } else {
-        if (!(d2 <= P.rc2)) continue;
-        eps = P.eps; sig = P.sig; ecut = P.ecut;
-      }
-      const double r = sqrt(d2);
-      const double ratio = sig / r;
-      const double ratio2 = ratio * ratio;
-      const double ratio6 = ratio2 * ratio2 * ratio2;
-      const double ratio12 = ratio6 * ratio6;
-      double ee = 4. * eps * (ratio12 - ratio6);
-      double de = (-24. * eps * (2. * ratio12 - ratio6)) / r;
-      ee -= ecut;
-      de /= r;
-      const double fex = de * dx, fey = de * dy, fez = de * dz;
-      fx += fex; fy += fey; fz += fez;
-      if (EV) {
-        e += .5 * ee;
-        v[0] += fex * dx * -0.5; v[1] += fex * dy * -0.5; v[2] += fex * dz * -0.5;
-        v[3] += fey * dx * -0.5; v[4] += fey * dy * -0.5; v[5] += fey * dz * -0.5;
-        v[6] += fez * dx * -0.5; v[7] += fez * dy * -0.5; v[8] += fez * dz * -0.5;
-      }
-    }
-    fx = group_reduce_d<T>(fx);
-    fy = group_reduce_d<T>(fy);
-    fz = group_reduce_d<T>(fz);
+  const int64_t i0 = A.i0 + blockIdx.x * (int64_t)(blockDim.x / T);
+  const int64_t i = i0 + threadIdx.x / T;
+  const int lane = (int)threadIdx.x % T;
+  const PairHome H(A, i, i < A.n);
+  const int ti = __float_as_int(H.pf.w);
+  double fx = 0., fy = 0., fz = 0., e = 0.;
+  double v[6] = {0., 0., 0., 0., 0., 0.};
+  auto limits = [&](int tj) {
+    if (!MULTI) return PairLimits{P.rc2lo, P.rc2hi, P.rc2, 0.0};
+    const int q = ti * ntypes + tj;
+    return PairLimits{sb[q].x, sb[q].y, rcmax2, sd[4 * q + 2]};
+  };
+  for_pairs<T>(A, H, i, lane, limits, [&](uint32_t ent, int tj) {
+    double dx, dy, dz;
+    const double d2 = H.separation(A, ent, dx, dy, dz);
+    const double* p = sd + (MULTI ? 4 * (ti * ntypes + tj) : 0);
+    const double eps = MULTI ? p[0] : P.eps, sig2 = MULTI ? p[1] : P.sig * P.sig;
+    const double r2i = inverse(d2);
+    const double s2 = sig2 * r2i;
+    const double s6 = s2 * s2 * s2;
+    const double s12 = s6 * s6;
+    const double de = (-24. * eps) * (fma(2., s12, -s6) * r2i);
+    fx = fma(de, dx, fx);
+    fy = fma(de, dy, fy);
+    fz = fma(de, dz, fz);
     if (EV) {
-      e = group_reduce_d<T>(e);
-#pragma unroll
-      for (int q = 0; q < 9; ++q) v[q] = group_reduce_d<T>(v[q]);
+      e += fma(4. * eps, s12 - s6, -(MULTI ? p[3] : P.ecut));
+      const double fex = de * dx, fey = de * dy;
+      v[0] = fma(fex, dx, v[0]);
+      v[1] = fma(fey, dy, v[1]);
+      v[2] = fma(de * dz, dz, v[2]);
+      v[3] = fma(fex, dy, v[3]);
+      v[4] = fma(fex, dz, v[4]);
+      v[5] = fma(fey, dz, v[5]);
     }
-    if (live && lane == 0) atom_epilogue<false>(A, i, ti, fx, fy, fz, 0.f, 0.f, 0.f, e, EV ? v : nullptr);
+  });
+  fx = group_reduce_d<T>(fx);
+  fy = group_reduce_d<T>(fy);
+  fz = group_reduce_d<T>(fz);
+  if (EV) {
+    e = group_reduce_d<T>(e);
+#pragma unroll
+    for (int q = 0; q < 6; ++q) v[q] = group_reduce_d<T>(v[q]);
   }
+  block_epilogue_d<T, EV>(A, i0, ti, fx, fy, fz, 0.5 * e, v);
 }
 
 // ---------------------------------------------------------------------------
 // eam_alloy: density + embedding (one kernel), force (second kernel)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ int r_knot_d(double r, double rdr, int nr, double& p) {
-  double pp = r * rdr + 1.0;
-  int m = (int)pp;
-  m = min(m, nr - 1);
-  pp -= m;
-  p = fmin(pp, 1.0);
-  return m;
-}
-
 template <int T, bool EV>
 __global__ void __launch_bounds__(256) k_eam_rho(PairArgs A, EamDev E, double* __restrict__ fpd) {
-  const int64_t gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t i = A.i0 + gt / T;
-  const int lane = (int)(gt % T);
-  const bool live = i < A.n;
-  const int nn = live ? min(A.nnb[i], A.maxnb) : 0;
-  int cx = 0, cy = 0, cz = 0;
-  if (live) unpack_cell(A.cellpack[i], cx, cy, cz);
+  const int64_t i0 = A.i0 + blockIdx.x * (int64_t)(blockDim.x / T);
+  int64_t i = i0 + threadIdx.x / T;
+  double rho = 0.;
   {
-    double rho = 0.;
-    double4_32a pi = make_double4_32a(0., 0., 0., 0.);
-    if (live) pi = A.posd[i];
-    const int ti = (int)pi.w;
-    const uint32_t* row = A.nbr + (size_t)i * A.W;
-    for (int k = lane; k < nn; k += T) {
-      const uint32_t ent = __ldg(row + list_slot(A, k));
-      const uint32_t j = ent & GBMD_IDX_MASK, code = ent >> GBMD_IDX_BITS;
-      const double4_32a pj = A.posd[j];
-      double Sx, Sy, Sz, dx, dy, dz;
-      image_shift(A.g, cx, cy, cz, code, Sx, Sy, Sz);
-      const double d2 = exact_d2(pi.x, pi.y, pi.z, pj.x, pj.y, pj.z, Sx, Sy, Sz, dx, dy, dz);
-      if (!(d2 <= E.rcut2)) continue;
-      double q;
-      const int m = r_knot_d(sqrt(d2), E.rdr, E.nr, q);
-      const double* c = E.rhor + ((size_t)(int)pj.w * (E.nr + 1) + m) * 8;
+    const PairHome H(A, i, i < A.n);
+    auto limits = [&](int) { return PairLimits{E.rc2lo, E.rc2hi, E.rcut2, 0.0}; };
+    for_pairs<T>(A, H, i, (int)threadIdx.x % T, limits, [&](uint32_t ent, int tj) {
+      double dx, dy, dz, y, q;
+      const double r = root<false>(H.separation(A, ent, dx, dy, dz), y);
+      const int m = r_knot_d(fma(r, E.rdr, 1.0), E.nr, q);
+      const double* c = E.rhor + ((size_t)tj * (E.nr + 1) + m) * 8;
       rho += ((c[3] * q + c[4]) * q + c[5]) * q + c[6];
-    }
-    rho = group_reduce_d<T>(rho);
-    if (live && lane == 0) {
-      double q = rho * E.rdrho + 1.0;
-      int m = (int)q;
-      m = max(1, min(m, E.nrho - 1));
-      q -= m;
-      q = fmin(q, 1.0);
-      const double* c = E.frho + ((size_t)ti * (E.nrho + 1) + m) * 8;
-      double fp = (c[0] * q + c[1]) * q + c[2];
-      double phi = ((c[3] * q + c[4]) * q + c[5]) * q + c[6];
-      if (rho > E.rhomax) phi += fp * (rho - E.rhomax);
-      phi *= E.conv_frho;
-      fp *= E.conv_frho;
-      fpd[i] = fp;
-      if (EV) A.ep_emb[i] = phi;
-    }
+    });
   }
+  rho = group_reduce_d<T>(rho);
+  if (T > 1) {
+    __shared__ double sum[T > 1 ? 256 / T : 1];
+    if (threadIdx.x % T == 0) sum[threadIdx.x / T] = rho;
+    __syncthreads();
+    if (threadIdx.x >= blockDim.x / T) return;
+    rho = sum[threadIdx.x];
+    i = i0 + threadIdx.x;
+  }
+  if (i >= A.n) return;
+  double q = rho * E.rdrho + 1.0;
+  int m = (int)q;
+  m = max(1, min(m, E.nrho - 1));
+  q -= m;
+  q = fmin(q, 1.0);
+  const double* c = E.frho + ((size_t)__float_as_int(A.posf[i].w) * (E.nrho + 1) + m) * 8;
+  double fp = (c[0] * q + c[1]) * q + c[2];
+  double phi = ((c[3] * q + c[4]) * q + c[5]) * q + c[6];
+  if (rho > E.rhomax) phi += fp * (rho - E.rhomax);
+  phi *= E.conv_frho;
+  fp *= E.conv_frho;
+  fpd[i] = fp;
+  if (EV) A.ep_emb[i] = phi;
 }
 
 __device__ __forceinline__ int z2r_index(int a, int b) {
@@ -166,71 +313,59 @@ __device__ __forceinline__ int z2r_index(int a, int b) {
 
 template <int T, bool EV>
 __global__ void __launch_bounds__(256) k_eam_force(PairArgs A, EamDev E, const double* __restrict__ fpd) {
-  const int64_t gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t i = A.i0 + gt / T;
-  const int lane = (int)(gt % T);
-  const bool live = i < A.n;
-  const int nn = live ? min(A.nnb[i], A.maxnb) : 0;
-  int cx = 0, cy = 0, cz = 0;
-  if (live) unpack_cell(A.cellpack[i], cx, cy, cz);
-  {
-    double fx = 0., fy = 0., fz = 0., e = 0.;
-    double v[9] = {0., 0., 0., 0., 0., 0., 0., 0., 0.};
-    double4_32a pi = make_double4_32a(0., 0., 0., 0.);
-    double fpi = 0.;
-    if (live) {
-      pi = A.posd[i];
-      fpi = fpd[i];
-    }
-    const int ti = (int)pi.w;
-    const uint32_t* row = A.nbr + (size_t)i * A.W;
-    for (int k = lane; k < nn; k += T) {
-      const uint32_t ent = __ldg(row + list_slot(A, k));
-      const uint32_t j = ent & GBMD_IDX_MASK, code = ent >> GBMD_IDX_BITS;
-      const double4_32a pj = A.posd[j];
-      double Sx, Sy, Sz, dx, dy, dz;
-      image_shift(A.g, cx, cy, cz, code, Sx, Sy, Sz);
-      const double d2 = exact_d2(pi.x, pi.y, pi.z, pj.x, pj.y, pj.z, Sx, Sy, Sz, dx, dy, dz);
-      if (!(d2 <= E.rcut2)) continue;
-      const int tj = (int)pj.w;
-      const double r = sqrt(d2);
-      double q;
-      const int m = r_knot_d(r, E.rdr, E.nr, q);
+  const int64_t i0 = A.i0 + blockIdx.x * (int64_t)(blockDim.x / T);
+  const int64_t i = i0 + threadIdx.x / T;
+  const PairHome H(A, i, i < A.n);
+  const int ti = __float_as_int(H.pf.w);
+  const double fpi = i < A.n ? fpd[i] : 0.;
+  double fx = 0., fy = 0., fz = 0., e = 0.;
+  double v[6] = {0., 0., 0., 0., 0., 0.};
+  auto limits = [&](int) { return PairLimits{E.rc2lo, E.rc2hi, E.rcut2, 0.0}; };
+  for_pairs<T>(A, H, i, (int)threadIdx.x % T, limits, [&](uint32_t ent, int tj) {
+    const double fpj = __ldg(&fpd[ent & GBMD_IDX_MASK]);
+    double dx, dy, dz, recip, q;
+    const double r = root<true>(H.separation(A, ent, dx, dy, dz), recip);
+    const int m = r_knot_d(fma(r, E.rdr, 1.0), E.nr, q);
+    const double* cj = E.rhor + ((size_t)tj * (E.nr + 1) + m) * 8;
+    const double rhojp = (cj[0] * q + cj[1]) * q + cj[2];
+    double rhoip = rhojp;
+    if (ti != tj) {
       const double* ci = E.rhor + ((size_t)ti * (E.nr + 1) + m) * 8;
-      const double rhoip = (ci[0] * q + ci[1]) * q + ci[2];
-      const double* cj = E.rhor + ((size_t)tj * (E.nr + 1) + m) * 8;
-      const double rhojp = (cj[0] * q + cj[1]) * q + cj[2];
-      const double* c = E.z2r + ((size_t)z2r_index(ti, tj) * (E.nr + 1) + m) * 8;
-      const double z2p = (c[0] * q + c[1]) * q + c[2];
-      const double z2 = ((c[3] * q + c[4]) * q + c[5]) * q + c[6];
-      const double recip = 1.0 / r;
-      double phi = z2 * recip;
-      const double phip = (z2p * recip - phi * recip) * E.conv_z2r;
-      phi *= E.conv_z2r;
-      const double psip = fpi * rhojp + __ldg(&fpd[j]) * rhoip + phip;
-      const double fpair = psip * recip;
-      const double fex = dx * fpair, fey = dy * fpair, fez = dz * fpair;
-      fx += fex; fy += fey; fz += fez;
-      if (EV) {
-        e += .5 * phi;
-        v[0] += fex * dx * -0.5; v[1] += fex * dy * -0.5; v[2] += fex * dz * -0.5;
-        v[3] += fey * dx * -0.5; v[4] += fey * dy * -0.5; v[5] += fey * dz * -0.5;
-        v[6] += fez * dx * -0.5; v[7] += fez * dy * -0.5; v[8] += fez * dz * -0.5;
-      }
+      rhoip = (ci[0] * q + ci[1]) * q + ci[2];
     }
-    fx = group_reduce_d<T>(fx);
-    fy = group_reduce_d<T>(fy);
-    fz = group_reduce_d<T>(fz);
+    const double* c = E.z2r + ((size_t)z2r_index(ti, tj) * (E.nr + 1) + m) * 8;
+    const double z2p = (c[0] * q + c[1]) * q + c[2];
+    const double z2 = ((c[3] * q + c[4]) * q + c[5]) * q + c[6];
+    const double phi = z2 * recip;
+    const double phip = (z2p - phi) * recip;
+    const double psip = fma(phip, E.conv_z2r, fma(fpj, rhoip, fpi * rhojp));
+    const double fpair = psip * recip;
+    fx = fma(dx, fpair, fx);
+    fy = fma(dy, fpair, fy);
+    fz = fma(dz, fpair, fz);
     if (EV) {
-      e = group_reduce_d<T>(e);
+      e += phi;
+      const double fex = dx * fpair, fey = dy * fpair;
+      v[0] = fma(fex, dx, v[0]);
+      v[1] = fma(fey, dy, v[1]);
+      v[2] = fma(dz * fpair, dz, v[2]);
+      v[3] = fma(fex, dy, v[3]);
+      v[4] = fma(fex, dz, v[4]);
+      v[5] = fma(fey, dz, v[5]);
+    }
+  });
+  fx = group_reduce_d<T>(fx);
+  fy = group_reduce_d<T>(fy);
+  fz = group_reduce_d<T>(fz);
+  if (EV) {
+    e = group_reduce_d<T>(e);
 #pragma unroll
-      for (int q = 0; q < 9; ++q) v[q] = group_reduce_d<T>(v[q]);
-    }
-    if (live && lane == 0) {
-      const double epv = EV ? A.ep_emb[i] + e : 0.0;
-      atom_epilogue<false>(A, i, ti, fx, fy, fz, 0.f, 0.f, 0.f, epv, EV ? v : nullptr);
-    }
+    for (int q = 0; q < 6; ++q) v[q] = group_reduce_d<T>(v[q]);
   }
+  // the pair energy goes to the thread that finishes the atom, which adds
+  // the embedding energy to it
+  e *= 0.5 * E.conv_z2r;
+  block_epilogue_d<T, EV>(A, i0, ti, fx, fy, fz, e, v, EV ? A.ep_emb : nullptr);
 }
 
 // ---------------------------------------------------------------------------
@@ -298,11 +433,9 @@ static void launch_fp64_T(gbmd_context* c, const PairArgs& A, int part) {
   if (c->pot != GBMD_POT_EAM_ALLOY && part == 1) return;
   if (c->pot == GBMD_POT_LJ) {
     const LJPair& p = c->lj.p[0];
-    LJSingle P{p.eps, p.sig, p.ecut, p.rc2};
-    k_lj<T, EV, false><<<grid, B, 0, s>>>(A, P, nullptr, 1, c->lj.rcut_max2);
+    k_lj<T, EV, false><<<grid, B, 0, s>>>(A, p, nullptr, 1, c->lj.rcut_max2);
   } else if (c->pot == GBMD_POT_LJ_MULTI) {
-    LJSingle P{};
-    k_lj<T, EV, true><<<grid, B, 0, s>>>(A, P, c->lj_tab_d, c->lj.ntypes, c->lj.rcut_max2);
+    k_lj<T, EV, true><<<grid, B, 0, s>>>(A, LJPair{}, c->lj_tab_d, c->lj.ntypes, c->lj.rcut_max2);
   } else {
     if (part != 2) k_eam_rho<T, EV><<<grid, B, 0, s>>>(A, c->eam, c->fpd);
     if (part != 1) k_eam_force<T, EV><<<grid, B, 0, s>>>(A, c->eam, c->fpd);

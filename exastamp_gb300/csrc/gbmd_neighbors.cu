@@ -16,8 +16,8 @@
 //   k_cell_rank   canonical (id, upload index) order per cell   L1-resident
 //   k_gather      permute the FP64 state into cell order        HBM: ~130 B r/w
 //   k_posf        FP32 local + FP64 packed gather copies        HBM: 24 B r, 48 B w
-//   k_build_list_cells  warp per home cell over the 27-cell candidates, ballot
-//                 compaction in canonical order                 HBM: 4 B per entry
+//   k_build_list_cells  warp per home cell over the 27-cell candidates, rows
+//                 in canonical order                            HBM: 4 B per entry
 //
 // Every kernel of the chain takes a `gate` word: when it is non-null and
 // holds 0 the kernel returns at once.  The displacement-triggered step
@@ -26,6 +26,7 @@
 // to rebuild never goes through the host and the chain can sit inside a CUDA
 // graph.  That variant gathers into the spare buffers and copies back, so the
 // buffer parity the captured pointers rely on does not depend on the outcome.
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <utility>
@@ -339,258 +340,357 @@ __device__ __noinline__ bool exact_within(const double* __restrict__ x, const do
                   (double)nzi * g.L[2], a, b, c) <= R2;
 }
 
-constexpr int BUILD_CHUNK = 64;  // candidates staged per chunk
-constexpr int BUILD_WARPS = 4;   // warps per block
+// ---------------------------------------------------------------------------
+// The list builder: one warp per home cell (or several, each taking its share
+// of the cell's groups), the cell's atoms 16 at a time.
+//
+// Lanes l and l + 16 hold home atom l of the group.  The candidates, the atoms
+// of the 27 stencil cells in stencil order, are staged in shared memory 32 at
+// a time for each half-warp, shifted into the home cell's frame; those farther
+// than R from the bounding box of the group's atoms, about a quarter, are left
+// out.  The low half-warp tests the first half of the candidates in order and
+// appends to the front of the atom's row in shared memory; the high half-warp
+// tests the second half from the end backwards and fills the row from its end
+// towards the front.  So both know where a hit goes without asking the other,
+// and the row ends in the canonical order (stencil code, then cell order).
+//
+// The walk is bound by instruction issue: a test costs about nine
+// instructions (two candidates at a time in packed FP32, one broadcast read
+// of 16 bytes, one predicated shared-memory store), where appending straight to the rows in
+// global memory, with their 64-bit slot address and an exchange between the
+// half-warps on every step, took over thirty.  A row leaves shared memory
+// once, complete, as 16-byte stores of neighbouring atoms.
+// Whole rebuild: 4 M-atom Cu, R = 5.3, 2,380 -> 1,845 us; 16.6 M-atom LJ mixture, 111
+// entries an atom, 17.6 -> 13.1 ms; 1 M-atom LJ 888 -> 765 us.
+//
+// The walk keeps every candidate with FP32 d2 <= R2hi; atoms with a hit above
+// R2lo (the band of band_rel, below one per cent) have their band entries
+// re-tested in FP64 afterwards by the whole warp.
+// ---------------------------------------------------------------------------
+constexpr int BUILD_G = 16;       // home atoms per group
+constexpr int BUILD_CHUNK = 32;   // candidates staged per half-warp: one round of the warp
+constexpr int BUILD_WARPS = 4;    // warps per block, where shared memory allows
+constexpr int BUILD_SLACK = 16;   // row slots beyond maxnb: 8 tests at either end run unchecked
 
-// Per-warp state of the candidate walk shared by both groupings.
-struct BuildCell {
-  int cx, cy, cz, total, hb, nh;
-  int s_start, s_pre;
-  uint32_t s_code;
-  float s_sx, s_sy, s_sz;
+// One warp's shared memory, followed by its BUILD_G rows of (maxnb + BUILD_SLACK) entries.
+struct BuildSmem {
+  // x, y, z, w of the low half-warp's candidates, then of the high one's, 64
+  // bytes further so that both broadcasts of a step read different banks
+  float4 chunk[2 * BUILD_CHUNK + 4];
+  float4 shift[28];    // nonempty stencil cells in order: first atom - first candidate, shift into the home frame
+  uint32_t code[28];   // their stencil code << 26
+  int pre[28];         // their first candidate; pre[ncell] = all candidates
 };
 
-// Stage candidates q0 .. q0+63 (position shifted into the home cell's frame,
-// index | stencil code << 26) into this warp's shared-memory buffer, keeping
-// in order only those within reach of the home group's bounding box
-// [blo, bhi] (box distance^2 <= R2keep); the rest cannot pair with any home
-// atom of the group (about a quarter of the candidates: the far parts of the
-// edge and corner cells).  Returns the number kept; stage[kept] is a sentinel.
-__device__ __forceinline__ int build_stage(const BuildCell& B, const float4* __restrict__ pf, int q0,
-                                           float4* stage, int lane, const float3& blo, const float3& bhi,
-                                           float R2keep) {
-  const unsigned FULL = 0xffffffffu;
-  const float FAR = 1e18f;
-  int kept = 0;
-#pragma unroll
-  for (int r = 0; r < BUILD_CHUNK / 32; ++r) {
-    const int q = q0 + r * 32 + lane;
-    // stencil cell of candidate q: largest s with s_pre(s) <= q (5-step search)
-    int sc = 0;
-#pragma unroll
-    for (int step = 16; step > 0; step >>= 1) {
-      const int t = min(sc + step, 26);
-      const int pv = __shfl_sync(FULL, B.s_pre, t);
-      if (sc + step <= 26 && pv <= q) sc = t;
-    }
-    const int k = __shfl_sync(FULL, B.s_start, sc) + (q - __shfl_sync(FULL, B.s_pre, sc));
-    const uint32_t code = __shfl_sync(FULL, B.s_code, sc);
-    const float sx = __shfl_sync(FULL, B.s_sx, sc), sy = __shfl_sync(FULL, B.s_sy, sc),
-                sz = __shfl_sync(FULL, B.s_sz, sc);
-    float4 e = make_float4(FAR, FAR, FAR, __uint_as_float(0xffffffffu));
-    bool keep = false;
-    if (q < B.total) {
-      const float4 pj = pf[k];
-      e = make_float4(__fadd_rn(pj.x, sx), __fadd_rn(pj.y, sy), __fadd_rn(pj.z, sz),
-                      __uint_as_float((uint32_t)k | (code << GBMD_IDX_BITS)));
-      const float bx = fmaxf(0.f, fmaxf(blo.x - e.x, e.x - bhi.x));
-      const float by = fmaxf(0.f, fmaxf(blo.y - e.y, e.y - bhi.y));
-      const float bz = fmaxf(0.f, fmaxf(blo.z - e.z, e.z - bhi.z));
-      keep = fmaf(bx, bx, fmaf(by, by, bz * bz)) <= R2keep;
-    }
-    const unsigned km = __ballot_sync(FULL, keep);
-    if (keep) stage[kept + __popc(km & ((1u << lane) - 1u))] = e;
-    kept += __popc(km);
+__host__ __device__ inline int build_rowlen(int maxnb) { return (maxnb + BUILD_SLACK) | 1; }  // odd: rows start in different banks
+__host__ __device__ inline size_t build_smem(int maxnb, int homes) {
+  return sizeof(BuildSmem) + (size_t)((homes * build_rowlen(maxnb) + 3) & ~3) * sizeof(uint32_t);
+}
+
+struct BuildArgs {
+  int64_t ncells;
+  const float4* pf;
+  const double *x, *y, *z;
+  const int32_t* cstart;
+  double R2;
+  float R2lo, R2hi;
+  uint32_t* nbr;
+  int32_t* nnb;
+  int maxnb, W, wsh, tsh, homes, parts;  // homes: atoms per group; parts: warps per cell
+  int64_t stride;
+  int* err;
+};
+
+// One round of staging: the candidates qa .. qa + 31, in reverse with `rev`,
+// as far as they lie in [q0, q1).  Lane s describes stencil cell s: s_pre its
+// first candidate, s_any whether it has any.  fetch() reads a lane's candidate,
+// store() writes those near the box [blo, bhi], in order, to the front of
+// `dst`, fills the rest of the 32 slots with candidates out of reach, and
+// returns how many are in.
+struct BuildRound {
+  float4 pj, sh;
+  uint32_t w;
+  bool valid;
+  __device__ __forceinline__ void fetch(const BuildSmem& S, const float4* __restrict__ pf, int s_pre, bool s_any,
+                                        int qa, int q0, int q1, bool rev, int lane) {
+    const unsigned FULL = 0xffffffffu;
+    const int off = s_pre - qa, pos = rev ? 31 - lane : lane, q = qa + pos;
+    // cell of candidate qa + pos: the nonempty cells that start up to there
+    const unsigned starts = __reduce_or_sync(FULL, s_any && (unsigned)off < 32u ? 1u << off : 0u);
+    const int before = __popc(__ballot_sync(FULL, s_any && off < 0));
+    valid = q >= q0 && q < q1;
+    const int sc = valid ? before + __popc(starts & (0xffffffffu >> (31 - pos))) - 1 : 0;
+    sh = S.shift[sc];
+    const int k = valid ? q + __float_as_int(sh.x) : 0;
+    w = (uint32_t)k | S.code[sc];
+    pj = pf[k];
   }
-  if (lane == 0) stage[kept] = make_float4(FAR, FAR, FAR, __uint_as_float(0xffffffffu));
+  __device__ __forceinline__ int store(float4* dst, int lane, const float3& blo, const float3& bhi, float R2keep) {
+    const float ex = __fadd_rn(pj.x, sh.y), ey = __fadd_rn(pj.y, sh.z), ez = __fadd_rn(pj.z, sh.w);
+    const float bx = fmaxf(0.f, fmaxf(blo.x - ex, ex - bhi.x));
+    const float by = fmaxf(0.f, fmaxf(blo.y - ey, ey - bhi.y));
+    const float bz = fmaxf(0.f, fmaxf(blo.z - ez, ez - bhi.z));
+    const bool keep = valid && fmaf(bx, bx, fmaf(by, by, bz * bz)) <= R2keep;
+    const unsigned km = __ballot_sync(0xffffffffu, keep), lt = (1u << lane) - 1u;
+    const int kept = __popc(km), slot = keep ? __popc(km & lt) : kept + __popc(~km & lt);
+    float* d = reinterpret_cast<float*>(dst) + slot;
+    d[0] = keep ? ex : 1e18f;
+    d[BUILD_CHUNK] = ey;
+    d[2 * BUILD_CHUNK] = ez;
+    d[3 * BUILD_CHUNK] = __uint_as_float(w);
+    return kept;
+  }
+};
+
+// FP32 d2 of home atom pi and entry w, as the walk computes it.
+__device__ __forceinline__ float build_d2(const float4* __restrict__ pf, const Grid& g, const float4& pi, uint32_t w) {
+  const uint32_t code = w >> GBMD_IDX_BITS;
+  const float4 pj = pf[w & GBMD_IDX_MASK];
+  const float sx = __fmul_rn((float)((int)(code & 3u) - 1), g.hf[0]);
+  const float sy = __fmul_rn((float)((int)((code >> 2) & 3u) - 1), g.hf[1]);
+  const float sz = __fmul_rn((float)((int)(code >> 4) - 1), g.hf[2]);
+  const float dx = __fsub_rn(__fadd_rn(pj.x, sx), pi.x);
+  const float dy = __fsub_rn(__fadd_rn(pj.y, sy), pi.y);
+  const float dz = __fsub_rn(__fadd_rn(pj.z, sz), pi.z);
+  return fmaf(dx, dx, fmaf(dy, dy, __fmul_rn(dz, dz)));
+}
+
+__device__ __forceinline__ float4 shfl4(const float4& v, int src) {
+  return make_float4(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src),
+                     __shfl_sync(0xffffffffu, v.z, src), __shfl_sync(0xffffffffu, v.w, src));
+}
+
+// A row's n entries (front: the first `front`, the rest at the row's end)
+// without the band entries that FP64 excludes, packed at the front; returns
+// how many stay.  By the whole warp.
+__device__ __noinline__ int build_retest_row(const BuildArgs& A, const Grid& g, uint32_t* row, int rowlen, int front,
+                                             int n, float4 pi, int i, int cx, int cy, int cz, int lane) {
+  int kept = 0;
+  for (int p0 = 0; p0 < n; p0 += 32) {
+    const int p = p0 + lane;
+    uint32_t w = 0;
+    bool keep = p < n;
+    if (keep) {
+      w = row[p < front ? p : p + rowlen - n];
+      if (build_d2(A.pf, g, pi, w) >= A.R2lo)
+        keep = exact_within(A.x, A.y, A.z, i, (int64_t)(w & GBMD_IDX_MASK), w >> GBMD_IDX_BITS, cx, cy, cz, g, A.R2);
+    }
+    const unsigned km = __ballot_sync(0xffffffffu, keep);
+    // slots below p0 + 32: this step's entries are read, later ones lie above
+    if (keep) row[kept + __popc(km & ((1u << lane) - 1u))] = w;
+    kept += __popc(km);
+    __syncwarp();
+  }
   return kept;
 }
 
-// Deferred FP64 re-test of an atom's band entries: recompute each entry's
-// FP32 d2 with the rounded operations of the staging and the walk, re-test
-// the band ones and compact the row in place.  Returns the entries dropped.
-__device__ __noinline__ int build_retest_row(uint32_t* row, int nkeep, int wsh, int tsh, int W, int64_t stride,
-                                             const float4* __restrict__ pf, float4 pi, const double* __restrict__ x,
-                                             const double* __restrict__ y, const double* __restrict__ z, int i,
-                                             int cx, int cy, int cz, const Grid g, double R2, float R2lo) {
-  int wpos = 0;
-  for (int p = 0; p < nkeep; ++p) {
-    const uint32_t w = row[(size_t)(p >> wsh) * stride + list_word(p & (W - 1), wsh, tsh)];
-    const int k = (int)(w & GBMD_IDX_MASK);
-    const uint32_t code = w >> GBMD_IDX_BITS;
-    const float4 pj = pf[k];
-    const float sx = __fmul_rn((float)((int)(code & 3u) - 1), g.hf[0]);
-    const float sy = __fmul_rn((float)((int)((code >> 2) & 3u) - 1), g.hf[1]);
-    const float sz = __fmul_rn((float)((int)(code >> 4) - 1), g.hf[2]);
-    const float dx = __fsub_rn(__fadd_rn(pj.x, sx), pi.x);
-    const float dy = __fsub_rn(__fadd_rn(pj.y, sy), pi.y);
-    const float dz = __fsub_rn(__fadd_rn(pj.z, sz), pi.z);
-    const float d2f = fmaf(dx, dx, fmaf(dy, dy, __fmul_rn(dz, dz)));
-    bool keepit = true;
-    if (d2f >= R2lo) keepit = exact_within(x, y, z, i, k, code, cx, cy, cz, g, R2);
-    if (keepit) {
-      row[(size_t)(wpos >> wsh) * stride + list_word(wpos & (W - 1), wsh, tsh)] = w;
-      ++wpos;
+// All neighbours (FP32) of an atom whose row overflowed, for the regrow.  By
+// the whole warp.
+template <bool HALF>
+__device__ __noinline__ int build_count(const BuildArgs& A, const Grid& g, const BuildSmem& S, int ncell, float4 pi,
+                                        int i, int lane) {
+  int n = 0;
+  for (int c = 0; c < ncell; ++c)
+    for (int q = S.pre[c] + lane; q < S.pre[c + 1]; q += 32) {
+      const int k = q + __float_as_int(S.shift[c].x);
+      n += (HALF ? k > i : k != i) && build_d2(A.pf, g, pi, (uint32_t)k | S.code[c]) <= A.R2hi;
     }
-  }
-  return nkeep - wpos;
+  return __reduce_add_sync(0xffffffffu, n);
 }
 
-// The walk for home groups of G atoms: G = 32, one home atom per lane and one
-// candidate per step; G = 16, lanes l and l+16 hold the same home atom and a
-// step tests candidates 2t (low half) and 2t+1 (high half), the two lanes
-// exchanging their hit with one shuffle so both append in candidate order.
-// HALF keeps only candidates after the home atom in cell order (k > i): each
-// unordered pair once, for the Newton-3 force kernels.
-template <int G, bool HALF>
-__device__ __forceinline__ int build_walk(const BuildCell& B, const float4* __restrict__ pf,
-                                          const double* __restrict__ x, const double* __restrict__ y,
-                                          const double* __restrict__ z, const Grid& g, double R2, float R2lo,
-                                          float R2hi, uint32_t* __restrict__ nbr, int32_t* __restrict__ nnb,
-                                          int maxnb, int W, int wsh, int tsh, int64_t stride,
-                                          int* __restrict__ err,
-                                          float4* stage, int lane) {
+template <bool LOOP, bool HALF>
+__global__ void __launch_bounds__(BUILD_WARPS * 32, 6) k_build_list_cells(const __grid_constant__ BuildArgs A,
+                                                                       const __grid_constant__ Grid g,
+                                                                       const int* __restrict__ gate) {
+  if (gate && !*gate) return;
+  extern __shared__ float4 build_shared[];
   const unsigned FULL = 0xffffffffu;
   const float FAR = 1e18f;
-  const int half = G == 16 ? (lane >> 4) : 0;
-  const int hl = G == 16 ? (lane & 15) : lane;
-  // box distance bound with a margin far above the FP32 rounding of the
-  // walk's d2, so no candidate the walk would keep is dropped
-  const float R2keep = R2hi * (1.0f + 0x1p-10f);
-  int warp_max = 0;
-  for (int h0 = 0; h0 < B.nh; h0 += G) {
-    const bool hv = h0 + hl < B.nh;
-    const int i = B.hb + h0 + hl;
-    float4 pi = make_float4(FAR, FAR, FAR, 0.f);
-    if (hv) pi = pf[i];
-    // bounding box of the group's home atoms (cell frame)
-    float3 blo = make_float3(hv ? pi.x : FAR, hv ? pi.y : FAR, hv ? pi.z : FAR);
-    float3 bhi = make_float3(hv ? pi.x : -FAR, hv ? pi.y : -FAR, hv ? pi.z : -FAR);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      blo.x = fminf(blo.x, __shfl_xor_sync(FULL, blo.x, o));
-      blo.y = fminf(blo.y, __shfl_xor_sync(FULL, blo.y, o));
-      blo.z = fminf(blo.z, __shfl_xor_sync(FULL, blo.z, o));
-      bhi.x = fmaxf(bhi.x, __shfl_xor_sync(FULL, bhi.x, o));
-      bhi.y = fmaxf(bhi.y, __shfl_xor_sync(FULL, bhi.y, o));
-      bhi.z = fmaxf(bhi.z, __shfl_xor_sync(FULL, bhi.z, o));
+  const int lane = threadIdx.x & 31, half = lane >> 4, hl = lane & 15;
+  const int rowlen = build_rowlen(A.maxnb);
+  unsigned char* const mine =
+      reinterpret_cast<unsigned char*>(build_shared) + (threadIdx.x >> 5) * build_smem(A.maxnb, A.homes);
+  BuildSmem& S = *reinterpret_cast<BuildSmem*>(mine);
+  uint32_t* const rows = reinterpret_cast<uint32_t*>(mine + sizeof(BuildSmem));
+  const int64_t items = A.ncells * A.parts;
+  const int64_t warps = LOOP ? (int64_t)gridDim.x * (blockDim.x >> 5) : items;
+  for (int64_t item = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); item < items; item += warps) {
+    const int64_t cell = item / A.parts;
+    const int part = (int)(item - cell * A.parts);
+    const int hb = A.cstart[cell], nh = A.cstart[cell + 1] - hb;
+    if (part * A.homes >= nh) continue;
+    const int cx = (int)(cell % g.nc[0]), cy = (int)((cell / g.nc[0]) % g.nc[1]),
+              cz = (int)(cell / ((int64_t)g.nc[0] * g.nc[1]));
+    // stencil cell of this lane
+    int s_cnt = 0, s_start = 0;
+    uint32_t s_code = 0;
+    float s_sx = 0.f, s_sy = 0.f, s_sz = 0.f;
+    if (lane < 27) {
+      const int dx = lane % 3 - 1, dy = (lane / 3) % 3 - 1, dz = lane / 9 - 1;
+      const int nx = image_of(cx, dx, g.nc[0]), ny = image_of(cy, dy, g.nc[1]), nz = image_of(cz, dz, g.nc[2]);
+      const int64_t cj =
+          ((int64_t)(cz + dz - nz * g.nc[2]) * g.nc[1] + (cy + dy - ny * g.nc[1])) * g.nc[0] + (cx + dx - nx * g.nc[0]);
+      s_start = A.cstart[cj];
+      s_cnt = A.cstart[cj + 1] - s_start;
+      s_code = (uint32_t)(dx + 1) | ((uint32_t)(dy + 1) << 2) | ((uint32_t)(dz + 1) << 4);
+      s_sx = __fmul_rn((float)dx, g.hf[0]);
+      s_sy = __fmul_rn((float)dy, g.hf[1]);
+      s_sz = __fmul_rn((float)dz, g.hf[2]);
     }
-    uint32_t* row = nbr + (size_t)i * W;  // slot k at row[(k >> wsh) * stride + list_word(k & (W - 1))]
-    int cnt = 0;
-    bool unc = false;
-    for (int q0 = 0; q0 < B.total; q0 += BUILD_CHUNK) {
-      __syncwarp();
-      const int m = build_stage(B, pf, q0, stage, lane, blo, bhi, R2keep);
-      __syncwarp();
-#pragma unroll 8
-      for (int t = 0; t < m; t += (G == 16 ? 2 : 1)) {
-        const float4 e = stage[t + half];
-        const uint32_t w = __float_as_uint(e.w);
-        const float dx = __fsub_rn(e.x, pi.x);
-        const float dy = __fsub_rn(e.y, pi.y);
-        const float dz = __fsub_rn(e.z, pi.z);
-        const float d2f = fmaf(dx, dx, fmaf(dy, dy, __fmul_rn(dz, dz)));
-        // an atom never pairs with itself: its images sit at least one box
-        // edge >= R away, so k == i only ever matters in the home cell.
-        // Keep d2 <= R2hi; flag the atom when d2 >= R2lo.
-        const int k = (int)(w & GBMD_IDX_MASK);
-        const bool in = hv && (HALF ? k > i : k != i) && d2f <= R2hi;
-        unc |= in && d2f >= R2lo;
-        // the slot address is formed on every step and only the store is
-        // conditional, so the walk stays one straight-line block
-        if (G == 16) {
-          const int other = __shfl_xor_sync(FULL, (int)in, 16);
-          const int pos = cnt + (half & other);  // candidate 2t goes first
-          uint32_t* dst = row + (size_t)(pos >> wsh) * stride + list_word(pos & (W - 1), wsh, tsh);
-          if (in && pos < maxnb) *dst = w;
-          cnt += (int)in + other;
-        } else {
-          uint32_t* dst = row + (size_t)(cnt >> wsh) * stride + list_word(cnt & (W - 1), wsh, tsh);
-          if (in && cnt < maxnb) *dst = w;
-          cnt += (int)in;
+    int incl = s_cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(FULL, incl, o);
+      if (lane >= o) incl += t;
+    }
+    const int s_pre = incl - s_cnt, total = __shfl_sync(FULL, incl, 31);
+    const bool s_any = s_cnt > 0;
+    const unsigned any = __ballot_sync(FULL, s_any);
+    const int ncell = __popc(any);
+    if (s_any) {
+      const int c = __popc(any & ((1u << lane) - 1u));
+      S.shift[c] = make_float4(__int_as_float(s_start - s_pre), s_sx, s_sy, s_sz);
+      S.code[c] = s_code << GBMD_IDX_BITS;
+      S.pre[c] = s_pre;
+    }
+    if (lane == 0) S.pre[ncell] = total;
+    // the low half-warp's candidates: whole staging rounds
+    const int mid = min(total, (((total + 1) >> 1) + 31) & ~31);
+    // box distance bound with a margin far above the FP32 rounding of the
+    // walk's d2, so no candidate the walk would keep is dropped
+    const float R2keep = A.R2hi * (1.0f + 0x1p-10f);
+    int warp_max = 0;
+    for (int h0 = part * A.homes; h0 < nh; h0 += A.parts * A.homes) {
+      const bool hv = hl < A.homes && h0 + hl < nh;
+      const int i = hb + h0 + hl;
+      float4 pi = make_float4(FAR, FAR, FAR, 0.f);
+      if (hv) pi = A.pf[i];
+      // bounding box of the group's atoms (cell frame)
+      float3 blo = make_float3(hv ? pi.x : FAR, hv ? pi.y : FAR, hv ? pi.z : FAR);
+      float3 bhi = make_float3(hv ? pi.x : -FAR, hv ? pi.y : -FAR, hv ? pi.z : -FAR);
+#pragma unroll
+      for (int o = 8; o > 0; o >>= 1) {
+        blo.x = fminf(blo.x, __shfl_xor_sync(FULL, blo.x, o));
+        blo.y = fminf(blo.y, __shfl_xor_sync(FULL, blo.y, o));
+        blo.z = fminf(blo.z, __shfl_xor_sync(FULL, blo.z, o));
+        bhi.x = fmaxf(bhi.x, __shfl_xor_sync(FULL, bhi.x, o));
+        bhi.y = fmaxf(bhi.y, __shfl_xor_sync(FULL, bhi.y, o));
+        bhi.z = fmaxf(bhi.z, __shfl_xor_sync(FULL, bhi.z, o));
+      }
+      // shared-memory addresses of the lane's row end and of its next slot
+      const uint32_t row = (uint32_t)__cvta_generic_to_shared(rows + (hv ? hl : 0) * rowlen);
+      const uint32_t first = half ? row + 4 * (rowlen - 1) : row;
+      uint32_t put = first;
+      const int step = half ? -4 : 4;
+      float thr = hv ? A.R2hi : -1.f;  // -1: no candidate is a hit
+      float far2 = -1.f;               // largest d2 of the hits
+      bool full = false;
+      const float2 npx = make_float2(-pi.x, -pi.x), npy = make_float2(-pi.y, -pi.y), npz = make_float2(-pi.z, -pi.z);
+      const uint32_t self = (uint32_t)i | (21u << GBMD_IDX_BITS);
+      const float4* const cand = S.chunk + half * (BUILD_CHUNK + 4);
+      // Predicated, so that eight tests are one straight line.  An atom never
+      // pairs with itself: its images sit at least one box edge >= R away, so
+      // only its entry of the home cell is itself.
+      auto test = [&](float d2, float wf) {
+        const uint32_t w = __float_as_uint(wf);
+        if (HALF)
+          asm volatile("{\n.reg .pred p, q;\nsetp.gt.s32 q, %6, %7;\nsetp.le.and.f32 p, %2, %3, q;\n"
+                       "@p st.shared.u32 [%0], %4;\n@p max.f32 %1, %1, %2;\n@p add.s32 %0, %0, %5;\n}"
+                       : "+r"(put), "+f"(far2)
+                       : "f"(d2), "f"(thr), "r"(w), "r"(step), "r"((int)(w & GBMD_IDX_MASK)), "r"(i)
+                       : "memory");
+        else
+          asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 q, %4, %6;\nsetp.le.and.f32 p, %2, %3, q;\n"
+                       "@p st.shared.u32 [%0], %4;\n@p max.f32 %1, %1, %2;\n@p add.s32 %0, %0, %5;\n}"
+                       : "+r"(put), "+f"(far2)
+                       : "f"(d2), "f"(thr), "r"(w), "r"(step), "r"(self)
+                       : "memory");
+      };
+      for (int qa = 0; qa < mid; qa += BUILD_CHUNK) {
+        __syncwarp();  // the last chunk's reads, and S, are done
+        BuildRound lo, hi;
+        lo.fetch(S, A.pf, s_pre, s_any, qa, 0, mid, false, lane);
+        hi.fetch(S, A.pf, s_pre, s_any, total - qa - BUILD_CHUNK, mid, total, true, lane);
+        const int m0 = lo.store(S.chunk, lane, blo, bhi, R2keep);
+        const int m1 = hi.store(S.chunk + BUILD_CHUNK + 4, lane, blo, bhi, R2keep);
+        const int m = max(m0, m1);
+        __syncwarp();
+        for (int t = 0; t < m; t += 8) {
+          // fewer than 8 free slots: the row (more than maxnb entries) has overflowed
+          if (half ? put < row + 4 * 7 : put > row + 4 * (rowlen - 8)) {
+            thr = -1.f;
+            full = true;
+          }
+#pragma unroll
+          for (int u = 0; u < 8; u += 4) {
+            if (u && t + u >= m) break;
+            const float4* const c = cand + (t + u) / 4;
+            const float4 x = c[0], y = c[BUILD_CHUNK / 4], z = c[BUILD_CHUNK / 2], w = c[3 * BUILD_CHUNK / 4];
+            const float2 dx0 = __fadd2_rn(make_float2(x.x, x.y), npx), dx1 = __fadd2_rn(make_float2(x.z, x.w), npx);
+            const float2 dy0 = __fadd2_rn(make_float2(y.x, y.y), npy), dy1 = __fadd2_rn(make_float2(y.z, y.w), npy);
+            const float2 dz0 = __fadd2_rn(make_float2(z.x, z.y), npz), dz1 = __fadd2_rn(make_float2(z.z, z.w), npz);
+            const float2 d0 = __ffma2_rn(dx0, dx0, __ffma2_rn(dy0, dy0, __fmul2_rn(dz0, dz0)));
+            const float2 d1 = __ffma2_rn(dx1, dx1, __ffma2_rn(dy1, dy1, __fmul2_rn(dz1, dz1)));
+            test(d0.x, w.x);
+            test(d0.y, w.y);
+            test(d1.x, w.z);
+            test(d1.y, w.w);
+          }
         }
       }
+      __syncwarp();
+      // entries at the front and in all (stored); full, far2 of either half
+      const int mycnt = (half ? (int)(first - put) : (int)(put - first)) >> 2;
+      int front = __shfl_sync(FULL, mycnt, hl), n = front + __shfl_sync(FULL, mycnt, hl + 16);
+      full = (__ballot_sync(FULL, full) & (0x10001u << hl)) != 0;
+      far2 = fmaxf(far2, __shfl_xor_sync(FULL, far2, 16));
+      const bool over = hv && (full || n > A.maxnb);
+      int found = n;
+      unsigned todo = __ballot_sync(FULL, hv && half == 0 && !over && far2 >= A.R2lo);
+      while (todo) {
+        const int h = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const int k = build_retest_row(A, g, rows + h * rowlen, rowlen, __shfl_sync(FULL, front, h),
+                                       __shfl_sync(FULL, n, h), shfl4(pi, h), hb + h0 + h, cx, cy, cz, lane);
+        if (hl == h) front = n = found = k;
+      }
+      todo = __ballot_sync(FULL, half == 0 && over);
+      while (todo) {
+        const int h = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const int k = build_count<HALF>(A, g, S, ncell, shfl4(pi, h), hb + h0 + h, lane);
+        if (hl == h) found = k;
+      }
+      if (!hv) n = found = 0;
+      // rows out: unit (r, h, t) is what lane t of atom h's T lanes reads of
+      // list row r, V adjacent words.  An overflowed row's first maxnb slots
+      // hold entries too (stored counts above maxnb), so a reader stays in
+      // bounds until the host sees the error.
+      const int nrow = (min(__reduce_max_sync(FULL, n), A.maxnb) + A.W - 1) >> A.wsh;
+      const int units = nrow << (4 + A.tsh), T = 1 << A.tsh;
+      for (int u0 = 0; u0 < units; u0 += 32) {
+        const int u = u0 + lane, r = u >> (4 + A.tsh), h = (u >> A.tsh) & 15, t = u & (T - 1);
+        const int hn = __shfl_sync(FULL, n, h), hf = __shfl_sync(FULL, front, h);
+        if (u < units && r * A.W < hn) {
+          const uint32_t* const from = rows + h * rowlen;
+          auto entry = [&](int q) {
+            const int p = (r << A.wsh) + (q << A.tsh) + t;
+            return p >= hn ? 0u : from[p < hf ? p : p + rowlen - hn];
+          };
+          uint32_t* const to = A.nbr + (size_t)r * A.stride + (size_t)(hb + h0 + h) * A.W;
+          if (A.wsh - A.tsh == 2) *reinterpret_cast<uint4*>(to + 4 * t) = make_uint4(entry(0), entry(1), entry(2), entry(3));
+          else to[t] = entry(0);
+        }
+      }
+      if (hv && half == 0) {
+        A.nnb[i] = found;
+        if (found > A.maxnb) atomicOr(&A.err[ERRW_FLAGS], GBMD_DEVERR_NBR_OVERFLOW);
+        warp_max = max(warp_max, found);
+      }
     }
-    if (G == 16) {
-      // the shuffle runs on every lane (a short-circuit here would skip it)
-      const int partner_unc = __shfl_xor_sync(FULL, (int)unc, 16);
-      unc = unc || partner_unc != 0;
-      __syncwarp();  // the high-half lanes' entries are visible to the low half
-      if (half == 0 && unc) cnt -= build_retest_row(row, min(cnt, maxnb), wsh, tsh, W, stride, pf, pi, x, y, z, i,
-                                                    B.cx, B.cy, B.cz, g, R2, R2lo);
-      cnt = __shfl_sync(FULL, cnt, hl);  // the high-half lane takes the corrected count
-    } else if (unc) {
-      cnt -= build_retest_row(row, min(cnt, maxnb), wsh, tsh, W, stride, pf, pi, x, y, z, i, B.cx, B.cy, B.cz, g,
-                              R2, R2lo);
-    }
-    if (hv && half == 0) {
-      nnb[i] = cnt;
-      if (cnt > maxnb) atomicOr(&err[ERRW_FLAGS], GBMD_DEVERR_NBR_OVERFLOW);
-      warp_max = max(warp_max, cnt);
-    }
-  }
-  return warp_max;
-}
-
-// One warp per home cell.  Lane s < 27 describes stencil cell s (start,
-// count, code, FP32 shift); the 27 candidate ranges are concatenated in
-// stencil order and staged 64 at a time in shared memory, every candidate is
-// read as a shared-memory broadcast and tested against the home atoms held
-// in the lanes, hits are appended in candidate order -- the canonical order
-// (stencil code, then cell order) -- straight to the atoms' list rows.  Cells
-// of at most 16 atoms use the 16-atom grouping (two candidates per step),
-// fuller cells the 32-atom one.  The walk keeps every candidate with FP32
-// d2 <= R2hi and flags the atom when one lies above R2lo (the band of
-// band_rel); flagged atoms (below one per cent) rescan their row, re-test
-// those entries in FP64 and compact, so the walk has no call and no
-// divergent branch.
-template <bool LOOP, bool HALF>
-__global__ void __launch_bounds__(BUILD_WARPS * 32) k_build_list_cells(
-    int64_t ncells, const float4* __restrict__ pf, const double* __restrict__ x, const double* __restrict__ y,
-    const double* __restrict__ z, const int32_t* __restrict__ cstart, Grid g, double R2, float R2lo, float R2hi,
-    uint32_t* __restrict__ nbr, int32_t* __restrict__ nnb, int maxnb, int W, int tsh, int64_t stride,
-    int* __restrict__ err, const int* __restrict__ gate) {
-  const int lane = threadIdx.x & 31;
-  if (gate && !*gate) return;
-  const unsigned FULL = 0xffffffffu;
-  __shared__ float4 stage_all[BUILD_WARPS][BUILD_CHUNK + 1];
-  float4* stage = stage_all[threadIdx.x >> 5];
-  int wsh = 0;
-  while ((1 << wsh) < W) ++wsh;
-  // one cell per warp (LOOP: and per iteration, striding over the cells;
-  // used by the gated launch with its capped grid)
-  const int64_t warps = LOOP ? (int64_t)gridDim.x * (blockDim.x >> 5) : ncells;
-  for (int64_t cell = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); cell < ncells; cell += warps) {
-  BuildCell B;
-  B.cx = (int)(cell % g.nc[0]);
-  B.cy = (int)((cell / g.nc[0]) % g.nc[1]);
-  B.cz = (int)(cell / ((int64_t)g.nc[0] * g.nc[1]));
-  // stencil cell of this lane
-  int s_cnt = 0;
-  B.s_start = 0;
-  B.s_code = 0;
-  B.s_sx = B.s_sy = B.s_sz = 0.f;
-  if (lane < 27) {
-    const int dx = lane % 3 - 1, dy = (lane / 3) % 3 - 1, dz = lane / 9 - 1;
-    const int nx = image_of(B.cx, dx, g.nc[0]), ny = image_of(B.cy, dy, g.nc[1]), nz = image_of(B.cz, dz, g.nc[2]);
-    const int64_t cj = ((int64_t)(B.cz + dz - nz * g.nc[2]) * g.nc[1] + (B.cy + dy - ny * g.nc[1])) * g.nc[0] +
-                       (B.cx + dx - nx * g.nc[0]);
-    B.s_start = cstart[cj];
-    s_cnt = cstart[cj + 1] - B.s_start;
-    B.s_code = (uint32_t)(dx + 1) | ((uint32_t)(dy + 1) << 2) | ((uint32_t)(dz + 1) << 4);
-    B.s_sx = __fmul_rn((float)dx, g.hf[0]);
-    B.s_sy = __fmul_rn((float)dy, g.hf[1]);
-    B.s_sz = __fmul_rn((float)dz, g.hf[2]);
-  }
-  int incl = s_cnt;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int t = __shfl_up_sync(FULL, incl, o);
-    if (lane >= o) incl += t;
-  }
-  B.s_pre = incl - s_cnt;  // exclusive prefix of this lane's stencil cell
-  B.total = __shfl_sync(FULL, incl, 26);
-  B.hb = cstart[cell];
-  B.nh = cstart[cell + 1] - B.hb;
-  int warp_max;
-  if (B.nh <= 16)
-    warp_max = build_walk<16, HALF>(B, pf, x, y, z, g, R2, R2lo, R2hi, nbr, nnb, maxnb, W, wsh, tsh, stride, err, stage, lane);
-  else
-    warp_max = build_walk<32, HALF>(B, pf, x, y, z, g, R2, R2lo, R2hi, nbr, nnb, maxnb, W, wsh, tsh, stride, err, stage, lane);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) warp_max = max(warp_max, __shfl_xor_sync(FULL, warp_max, o));
-  if (lane == 0 && warp_max > 0) atomicMax(&err[ERRW_MAXNB], warp_max);
-  __syncwarp();  // the next cell restages this warp's buffer
+    warp_max = __reduce_max_sync(FULL, warp_max);
+    if (lane == 0 && warp_max > 0) atomicMax(&A.err[ERRW_MAXNB], warp_max);
+    __syncwarp();  // the next cell overwrites S
   }
 }
 
@@ -633,13 +733,45 @@ static int build_list(gbmd_context* c, const int* gate) {
   }
   c->npad = npad;
   if (!gate) GBMD_CUDA(c, cudaMemsetAsync(c->d_err + ERRW_MAXNB, 0, sizeof(int), c->stream));
-  const bool loop = gate && !c->full_chain_grids;  // capped grid striding over the cells (five blocks per SM fit)
-  const unsigned blocks = loop ? chain_blocks(c, c->grid.ncells, BUILD_WARPS, gate, 5) : nblk(c->grid.ncells, BUILD_WARPS);
+  BuildArgs A;
+  A.ncells = c->grid.ncells;
+  A.pf = c->POSF();
+  A.x = c->X(); A.y = c->Y(); A.z = c->Z();
+  A.cstart = c->cell_start;
+  A.R2 = R2;
+  A.R2lo = R2lo;
+  A.R2hi = R2hi;
+  A.nbr = c->nbr;
+  A.nnb = c->nnb;
+  A.maxnb = c->maxnb;
+  A.W = W;
+  A.wsh = log2_of(W);
+  A.tsh = log2_of(c->tpa);
+  A.stride = stride;
+  A.err = c->d_err;
+  // rows of 16 atoms fit a warp's shared memory up to some 3,000 entries an
+  // atom; beyond that a group takes fewer atoms
+  const size_t most = 200 * 1024;
+  A.homes = BUILD_G;
+  while (A.homes > 1 && build_smem(c->maxnb, A.homes) > most) --A.homes;
+  const size_t per_warp = build_smem(c->maxnb, A.homes);
+  if (per_warp > most) return set_error(c, GBMD_ERR_TOO_LARGE, "%d neighbours per atom", c->maxnb);
+  // the widest blocks of which an SM holds several
+  int nw = BUILD_WARPS;
+  while (nw > 1 && nw * per_warp > 56 * 1024) nw >>= 1;
+  // a second warp for a cell's second group while cells are few (an SM holds
+  // some 20 warps of this kernel)
+  A.parts = c->grid.ncells < 20ll * c->nsm ? 2 : 1;
+  const int64_t items = c->grid.ncells * A.parts;
+  const bool loop = gate && !c->full_chain_grids;  // capped grid striding over the cells
   auto kern = loop ? (c->newton3 ? k_build_list_cells<true, true> : k_build_list_cells<true, false>)
                    : (c->newton3 ? k_build_list_cells<false, true> : k_build_list_cells<false, false>);
-  kern<<<blocks, 32 * BUILD_WARPS, 0, c->stream>>>(c->grid.ncells, c->POSF(), c->X(), c->Y(), c->Z(), c->cell_start,
-                                                  c->grid, R2, R2lo, R2hi, c->nbr, c->nnb, c->maxnb, W, log2_of(c->tpa), stride,
-                                                  c->d_err, gate);
+  const size_t smem = nw * per_warp;
+  if (smem > 48 * 1024)
+    GBMD_CUDA(c, cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
+  const int per_sm = (int)std::max<size_t>(1, 220 * 1024 / (smem + 1024));
+  const unsigned blocks = loop ? chain_blocks(c, items, nw, gate, std::min(per_sm, 8)) : nblk(items, nw);
+  kern<<<blocks, 32 * nw, smem, c->stream>>>(A, c->grid, gate);
   return GBMD_OK;
 }
 

@@ -3,21 +3,29 @@
 // parameter adjoint of a force-matching + energy loss.
 //
 // One thread block owns one replica at a time (replicas are taken largest
-// first from an atomic queue, so the launch load-balances uneven sizes).
-// Everything a replica needs lives in shared memory: its cell-sorted FP32
-// cell-relative positions, cell ranges, F'(rho), the loss gradients with
-// respect to its per-atom forces and energies, and the adjoint
-// intermediates.  Pairs are found once per replica from the (2S+1)^3 cells
-// around each atom (S = 1 with cells >= rcut, or S = 2 with cells >= rcut/2;
-// the autotuner picks S and the block size), with the same FP32 screen +
-// FP64 re-test of the ambiguous band as the main path, so the in-cutoff pair
-// set is the FP64 one; they go to a pair list in the block's own global
-// scratch (128 entries per atom, slot-major), which the density, force and
-// adjoint passes read.  A replica with a fuller atom walks the cells in
-// every pass instead, with the same order and arithmetic.  Pair arithmetic is FP32 with compensated force and
-// density sums; per-replica sums (energy, virial, loss, gradient) are FP64
-// and written to the replica's own row, so results do not depend on which
-// block ran which replica.
+// first from an atomic queue, so the launch load-balances uneven sizes), with
+// T = 1 .. 32 lanes per atom so that a replica of any size keeps its block's
+// threads busy.  Everything a replica needs lives in shared memory: its
+// cell-sorted FP32 cell-relative positions with F'(rho), cell ranges, rho, and
+// the loss gradients with respect to its per-atom forces and energies.  Pairs
+// are found once per replica from the (2S+1)^3 cells around each atom (S = 1
+// with cells >= rcut, or S = 2 with cells >= rcut/2), with the same FP32
+// screen + FP64 re-test of the ambiguous band as the main path, so the
+// in-cutoff pair set is the FP64 one; they go to a pair list in the block's
+// own global scratch (at least 2 x 128 entries per atom), which the density, force
+// and adjoint passes read, four entries a lane in flight.  A replica with a
+// fuller atom walks the cells in every pass instead.  Pair arithmetic is FP32
+// with compensated force and density sums; per-replica sums (energy, virial,
+// loss, gradient) are FP64 and written to the replica's own row, so results do
+// not depend on which block ran which replica.
+//
+// What bounds it: with one lane per atom and one pair in flight, latency (256
+// replicas of 243 atoms took 538 us, forward and adjoint, now 192; 4,096 of
+// 32-2,048 atoms 11.2 ms, now 4.3).  Of the latter the derivative tables' reads
+// (358 KB in use, from L2) are a third, the list a sixth.  The FP64 pipe is slow (16 SM cycles a warp
+// instruction), so conversions and the periodic wrap are integer arithmetic,
+// the geometry is computed once per replica, and the block sums are
+// transposed as they are reduced.
 //
 // Physics restated (single element, eam_alloy.h L198-313 and
 // eam_force_op_multimat.h L114-343):
@@ -44,9 +52,10 @@ constexpr int BMAX_ATOMS = 2048;   // largest replica
 constexpr int BMAX_CELLS = 1024;
 constexpr int SMALL_ATOMS = 512;   // replicas up to this size run in the small-block kernel
 constexpr int SMALL_CELLS = 512;
-constexpr int NBL_MAX = 128;       // pair-list entries per atom
+constexpr int NBL_MAX = 256;       // pair-list entries per atom, half of them for either half-warp of the builder
 constexpr int BMAX_PARAMS = 9;
 constexpr int REP_ROW = 20;  // epot, virial[9], loss, grad[9]
+constexpr int MAX_TABLES = 24;  // derivative tables per knot: up to 2 x 9, padded to a multiple of 8
 
 struct BatchArgs {
   int nrep, single;
@@ -61,54 +70,72 @@ struct BatchArgs {
   int* queue;
   int* err;
   // tables (FP32 value coefficients c3..c6, scaled by conv)
-  const float4 *frho4, *rhor4, *rhod4, *z2r4;
+  const float4 *frho4, *rhor4;
+  const float4* fz8;  // per knot: rho' coefficients (3c3, 2c4, c5) / dr, z2r coefficients
   int nr, nrho;
   float rdr, rdrho, rhomax;
   double rcut, rcut2;
-  float rc2lo, rc2hi;
   int S;
   // adjoint
   int adjoint;
   const double *Ftx, *Fty, *Ftz, *Et;
   double wF, wE;
-  const float4 *dz2r4, *drhor4, *dfrho4;  // [k][knot] for the listed parameters
-  int nz2, nrh, nfr;
+  const float4* dtab;    // [knot][ktab]: derivative tables of z2r (nz2), then of rho (nrh), zero-padded
+  const float4* dfrho4;  // [k][knot] for the listed parameters
+  int nz2, nrh, nfr, ktab;
   uint32_t* nbl;  // MAXA * NBL_MAX entries per block: the current replica's pair list
   int pz2[BMAX_PARAMS], prh[BMAX_PARAMS], pfr[BMAX_PARAMS];
 };
 
-// Shared memory of one block: a replica of up to MAXA atoms in MAXC cells.
-template <int MAXA, int MAXC>
-struct SmemT {
-  float4 pos[MAXA];   // cell-relative FP32 position, w = local atom index bits
-  float4 gfe[MAXA];   // adjoint: dL/dF (xyz) and dL/dE (w)
-  int cstart[MAXC + 1];
-  int cfill[MAXC];
-  int cellof[MAXA];   // by local atom index
-  int order[MAXA];    // slot -> local atom index
-  float fp[MAXA];     // F'(rho) by slot
-  float eemb[MAXA];   // F(rho) by slot
-  float rho[MAXA];    // rho by slot
-  float G[MAXA];      // adjoint G by slot
-  int nnb[MAXA];      // pair-list length by slot
-  double red[32][REP_ROW];  // block reduction
-  int rep;
-  int list_ok;              // every atom's pairs fit in the list
-};
-
 struct RepGeom {
   int64_t base;
-  int n, nc[3], ncells;
+  int n, nc[3], ncells, tsh;  // 1 << tsh lanes per atom
   double lo[3], hi[3], L[3], h[3], inv_h[3];
-  float hf[3];
+  float hf[3], rc2lo, rc2hi;  // cell edges; FP64 re-test band of the cutoff
+};
+
+// One warp's 32 pairs on their way to the derivative tables: knot, and the
+// weights of the four coefficients of a z2r and of a rho table.
+struct PairRecord {
+  float4 z[32], r[32];
+  int m[32];
+};
+
+// Shared memory of one block: a replica of up to MAXA atoms in MAXC cells.
+template <int MAXA, int MAXC, int MAXT>
+struct SmemT {
+  static constexpr uint32_t ATOMS = MAXA;  // a power of two of at most 2,048
+  float4 pos[MAXA];   // by slot: cell-relative FP32 position, w = F'(rho)
+  float4 gfe[MAXA];   // adjoint: dL/dF (xyz) and dL/dE (w) by slot; before that, positions by atom
+  PairRecord rec[MAXT / 32];
+  double red[MAXT / 32][MAX_TABLES];  // block reductions
+  RepGeom geom;
+  float rho[MAXA];    // by slot: rho, then the adjoint's lambda
+  int cfill[MAXC];
+  unsigned short cstart[MAXC + 2];
+  unsigned short cellof[MAXA];   // by local atom index
+  unsigned short order[MAXA];    // slot -> local atom index
+  unsigned short nnb[MAXA];      // pair-list length by slot
+  unsigned short front[MAXA];    // entries in its first part
+  int rep;
+  int overflow;             // some atom's pairs do not fit in the list
 };
 
 __device__ __forceinline__ int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
 
+// A double's bits as an integer of the same order.
+__device__ __forceinline__ long long order_key(double v) {
+  const long long b = __double_as_longlong(v);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+
 // periodic wrap with the rounding of the main path's rebuild (and the oracle)
 __device__ __forceinline__ void wrap_cell(const RepGeom& g, double v, int d, double& w, int& c) {
-  if (v < g.lo[d]) v = __dadd_rn(v, g.L[d]);
-  else if (v >= g.hi[d]) v = __dsub_rn(v, g.L[d]);
+  const long long k = order_key(v);
+  if (k <= order_key(g.lo[d]) || k >= order_key(g.hi[d])) {  // outside, or on the face
+    if (v < g.lo[d]) v = __dadd_rn(v, g.L[d]);
+    else if (v >= g.hi[d]) v = __dsub_rn(v, g.L[d]);
+  }
   w = v;
   int q = (int)__dmul_rn(__dsub_rn(v, g.lo[d]), g.inv_h[d]);
   c = q < 0 ? 0 : (q > g.nc[d] - 1 ? g.nc[d] - 1 : q);
@@ -136,6 +163,15 @@ __device__ __forceinline__ float sdq(const float4& c, float q) {  // d value / d
   return fmaf(fmaf(3.f * c.x, q, 2.f * c.y), q, c.z);
 }
 
+// Embedding knot of rho, and the fraction (linear continuation above the table
+// is the caller's).
+__device__ __forceinline__ int embed_knot(const BatchArgs& A, float rho, float& q) {
+  q = fmaf(rho, A.rdrho, 1.f);
+  const int m = max(1, min((int)q, A.nrho - 1));
+  q = fminf(q - (float)m, 1.f);
+  return m;
+}
+
 __device__ __forceinline__ int knot(float t, int nmax, float& q) {
   const int m = min((int)t, nmax);
   q = fminf(t - (float)m, 1.0f);
@@ -152,10 +188,12 @@ __device__ __forceinline__ float pair_d2(const float4& pi, const float4& pj, flo
   return fmaf(ddx, ddx, fmaf(ddy, ddy, ddz * ddz));
 }
 
-// Visit every in-cutoff neighbour of slot s from the cells around it:
-// fn(k, dx, dy, dz, d2, code), code = the cell offset (dx+S) | (dy+S) << 3 | (dz+S) << 6.
+// Lane t of atom s's T lanes: every T-th candidate of each cell around slot s,
+// fn(k, dx, dy, dz, d2, code) where it lies within the cutoff, code = the cell
+// offset (dx+S) | (dy+S) << 3 | (dz+S) << 6.
 template <class SM, class Fn>
-__device__ __forceinline__ void for_pairs(const BatchArgs& A, const RepGeom& g, const SM& sm, int s, Fn fn) {
+__device__ __forceinline__ void for_pairs(const BatchArgs& A, const RepGeom& g, const SM& sm, int s, int t, int T,
+                                          Fn fn) {
   const int ai = sm.order[s];
   const int c = sm.cellof[ai];
   const int cx = c % g.nc[0], cy = (c / g.nc[0]) % g.nc[1], cz = c / (g.nc[0] * g.nc[1]);
@@ -171,13 +209,11 @@ __device__ __forceinline__ void for_pairs(const BatchArgs& A, const RepGeom& g, 
         const float sx = (float)dx * g.hf[0], sy = (float)dy * g.hf[1], sz = (float)dz * g.hf[2];
         const bool self_cell = (dx | dy | dz) == 0;
         const uint32_t code = (uint32_t)(dx + S) | ((uint32_t)(dy + S) << 3) | ((uint32_t)(dz + S) << 6);
-        for (int k = sm.cstart[cj]; k < sm.cstart[cj + 1]; ++k) {
+        for (int k = sm.cstart[cj] + t; k < sm.cstart[cj + 1]; k += T) {
           if (self_cell && k == s) continue;
-          const float4 pj = sm.pos[k];
           float ddx, ddy, ddz;
-          const float d2 = pair_d2(pi, pj, sx, sy, sz, ddx, ddy, ddz);
-          if (d2 > A.rc2hi) continue;
-          if (d2 >= A.rc2lo && !batch_exact(A, g, ai, sm.order[k], nx, ny, nz)) continue;
+          const float d2 = pair_d2(pi, sm.pos[k], sx, sy, sz, ddx, ddy, ddz);
+          if (!(d2 <= g.rc2hi) || (d2 >= g.rc2lo && !batch_exact(A, g, ai, sm.order[k], nx, ny, nz))) continue;
           fn(k, ddx, ddy, ddz, d2, code);
         }
       }
@@ -185,347 +221,701 @@ __device__ __forceinline__ void for_pairs(const BatchArgs& A, const RepGeom& g, 
   }
 }
 
-// The same neighbours, in the same order and with the same FP32 arithmetic,
-// from the replica's pair list (entry: slot k | code << 11, slot-major).
-template <class SM, class Fn>
-__device__ __forceinline__ void for_list(const RepGeom& g, const SM& sm, const uint32_t* __restrict__ nbl,
-                                         int n, int S, int s, Fn fn) {
-  const float4 pi = sm.pos[s];
-  const int cnt = sm.nnb[s];
-  for (int q = 0; q < cnt; ++q) {
-    const uint32_t e = nbl[(size_t)q * n + s];
-    const int k = (int)(e & 2047u);
-    const int dx = (int)((e >> 11) & 7u) - S, dy = (int)((e >> 14) & 7u) - S, dz = (int)((e >> 17) & 7u) - S;
-    const float sx = (float)dx * g.hf[0], sy = (float)dy * g.hf[1], sz = (float)dz * g.hf[2];
-    const float4 pj = sm.pos[k];
-    float ddx, ddy, ddz;
-    const float d2 = pair_d2(pi, pj, sx, sy, sz, ddx, ddy, ddz);
-    fn(k, ddx, ddy, ddz, d2);
+// The pair list of a replica of n atoms: entries (slot k | code << 11) in two
+// parts per atom of up to cap entries, entry q of part p of slot s in word
+// (p cap + q) n + s; the first `front` entries of the atom are its part 0, the
+// rest part 1.  Read past L1, which serves the tables.
+struct PairList {
+  const uint32_t* at;
+  int front, count, n, jump;
+  template <class SM>
+  __device__ __forceinline__ PairList(const SM& sm, const uint32_t* nbl, int n_, int cap, int s)
+      : at(nbl + s), front(min((int)sm.front[s], cap)), count(min((int)sm.nnb[s], front + cap)), n(n_), jump(cap - front) {}
+  __device__ __forceinline__ uint32_t operator[](int e) const {
+    uint32_t w;
+    asm volatile("ld.global.L1::no_allocate.u32 %0, [%1];" : "=r"(w) : "l"(at + (e < front ? e : e + jump) * n));
+    return w;
   }
-}
+};
 
-// fn(k, dx, dy, dz, d2) over the neighbours of slot s: from the list when
-// every atom's pairs fit in it, else from the cells.
-template <class SM, class Fn>
-__device__ __forceinline__ void visit(const BatchArgs& A, const RepGeom& g, const SM& sm,
-                                      const uint32_t* nbl, int n, int s, Fn fn) {
-  if (sm.list_ok)
-    for_list(g, sm, nbl, n, A.S, s, fn);
-  else
-    for_pairs(A, g, sm, s, [&](int k, float dx, float dy, float dz, float d2, uint32_t) { fn(k, dx, dy, dz, d2); });
-}
+// {0 .. 2S} -> -S .. S exactly (small integer through the 2^23 mantissa trick)
+__device__ __forceinline__ float cell_unit(uint32_t b, float bias) { return __int_as_float(0x4B000000u | b) - bias; }
 
-// The replica's pair list, one thread per atom walking the cells as
-// for_pairs does (same FP32 screen and FP64 band re-test, same order).  A
-// warp-per-cell walk with shared-memory broadcasts measured slower here: a
-// replica of a few hundred atoms has too few cells to keep 16 warps busy.
-template <class SM>
-__device__ void build_list(const BatchArgs& A, const RepGeom& g, SM& sm, uint32_t* __restrict__ nbl, int n) {
-  for (int s = threadIdx.x; s < n; s += blockDim.x) {
-    int cnt = 0;
-    for_pairs(A, g, sm, s, [&](int k, float, float, float, float, uint32_t code) {
-      if (cnt < NBL_MAX) nbl[(size_t)cnt * n + s] = (uint32_t)k | (code << 11);
-      ++cnt;
+// Lane t's share of the pairs of slot s, fn(k, dx, dy, dz, d2, ok), four at a
+// time with done() after each four; pairs with ok = false count nothing (their
+// separation is zero).  From the list, or from the cells (cap = 0) where some
+// atom's pairs do not fit in it.
+template <class SM, class Fn, class Done>
+__device__ __forceinline__ void visit(const BatchArgs& A, const RepGeom& g, const SM& sm, const uint32_t* nbl,
+                                      int cap, int s, int t, Fn fn, Done done) {
+  const int T = 1 << g.tsh;
+  if (cap == 0) {
+    for_pairs(A, g, sm, s, t, T, [&](int k, float dx, float dy, float dz, float d2, uint32_t) {
+      fn(k, dx, dy, dz, d2, true);
+      done();
     });
-    sm.nnb[s] = cnt;
-    if (cnt > NBL_MAX) sm.list_ok = 0;
+    return;
+  }
+  const float4 pi = sm.pos[s];
+  const PairList list(sm, nbl, g.n, cap, s);
+  const float bias = 8388608.0f + (float)A.S;
+  const uint32_t none = (uint32_t)s | (uint32_t)(A.S | (A.S << 3) | (A.S << 6)) << 11;
+  const int n = list.count;
+  uint32_t e[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) e[u] = t + u * T < n ? list[t + u * T] : none;
+  for (int q = t; q < n; q += 4 * T) {
+    uint32_t nxt[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) nxt[u] = q + (4 + u) * T < n ? list[q + (4 + u) * T] : none;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int k = (int)(e[u] & (SM::ATOMS - 1u));
+      const float sx = cell_unit((e[u] >> 11) & 7u, bias) * g.hf[0], sy = cell_unit((e[u] >> 14) & 7u, bias) * g.hf[1],
+                  sz = cell_unit((e[u] >> 17) & 7u, bias) * g.hf[2];
+      float ddx, ddy, ddz;
+      const float d2 = pair_d2(pi, sm.pos[k], sx, sy, sz, ddx, ddy, ddz);
+      fn(k, ddx, ddy, ddz, d2, q + u * T < n);
+    }
+    done();
+#pragma unroll
+    for (int u = 0; u < 4; ++u) e[u] = nxt[u];
   }
 }
 
-template <class SM>
-__device__ void block_reduce_row(SM& sm, double* v, int nv, double* out) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  for (int q = 0; q < nv; ++q) {
-    double a = v[q];
+// The replica's pair list, by warps: a warp takes 16 atoms of a cell, lanes l
+// and l + 16 hold atom l.  The candidates of up to 32 stencil cells at a time
+// are staged in shared memory, 32 for each half-warp, without those farther
+// than the cutoff from the group's bounding box; the low half-warp tests the
+// first half of them and writes its hits to part 0 of the atom's list, the high
+// one tests the second half and writes part 1.  The walk of the main path's
+// list builder, with the rows in the block's scratch (L2) instead of shared
+// memory.  A test costs some ten instructions of a warp; one lane walking the
+// cells of its own atom took 45, half of the whole evaluation (243 atoms:
+// 200,000 of 420,000 cycles).  A part of more than cap - 4 entries raises
+// sm.overflow, and the passes walk the cells.
+template <int MAXT, class SM>
+__device__ void build_list(const BatchArgs& A, const RepGeom& g, SM& sm, uint32_t* __restrict__ nbl, int cap) {
+  const unsigned FULL = 0xffffffffu;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int half = lane >> 4, hl = lane & 15, S = A.S, width = 2 * S + 1, ncells = width * width * width;
+  const int n = g.n;
+  // staging: x, y, z, entry of the low half's 32 candidates, then the high
+  // half's, 64 bytes further (other banks); the cells' shifts, x = (first slot
+  // - first candidate) << 9 | code
+  float* const chunk = reinterpret_cast<float*>(&sm.rec[wid]);
+  float4* const shift = sm.gfe + 32 * wid;
+  static_assert(sizeof(PairRecord) >= (2 * 128 + 16) * sizeof(float), "staging fits");
+  int item = wid;  // groups of 16 atoms, cell by cell, dealt to the warps in turn
+  for (int cell = 0; cell < g.ncells; ++cell) {
+    const int b = sm.cstart[cell], nh = sm.cstart[cell + 1] - b;
+    for (int h0 = 0; h0 < nh; h0 += 16, --item) {
+      if (item != 0) continue;
+      item = nw;
+      const bool hv = h0 + hl < nh;
+      const int s = b + h0 + hl;
+      const float FAR = 1e18f;
+      float4 pi = make_float4(FAR, FAR, FAR, 0.f);
+      if (hv) pi = sm.pos[s];
+      float3 blo = make_float3(pi.x, pi.y, pi.z);
+      float3 bhi = make_float3(hv ? pi.x : -FAR, hv ? pi.y : -FAR, hv ? pi.z : -FAR);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) a += __shfl_down_sync(0xffffffffu, a, o);
-    if (lane == 0) sm.red[w][q] = a;
+      for (int o = 8; o > 0; o >>= 1) {
+        blo.x = fminf(blo.x, __shfl_xor_sync(FULL, blo.x, o));
+        blo.y = fminf(blo.y, __shfl_xor_sync(FULL, blo.y, o));
+        blo.z = fminf(blo.z, __shfl_xor_sync(FULL, blo.z, o));
+        bhi.x = fmaxf(bhi.x, __shfl_xor_sync(FULL, bhi.x, o));
+        bhi.y = fmaxf(bhi.y, __shfl_xor_sync(FULL, bhi.y, o));
+        bhi.z = fmaxf(bhi.z, __shfl_xor_sync(FULL, bhi.z, o));
+      }
+      const float keep2 = g.rc2hi * (1.0f + 0x1p-10f);  // far above the rounding of the tests' d2
+      const float2 npx = make_float2(-pi.x, -pi.x), npy = make_float2(-pi.y, -pi.y), npz = make_float2(-pi.z, -pi.z);
+      const uint32_t self = (uint32_t)s | (uint32_t)(S | (S << 3) | (S << 6)) << 11;
+      const int cx = cell % g.nc[0], cy = (cell / g.nc[0]) % g.nc[1], cz = cell / (g.nc[0] * g.nc[1]);
+      uint32_t* const part = nbl + (size_t)half * cap * n + s;  // this lane's: entry q at part[q n]
+      uint32_t* put = part;
+      const uint32_t* const last = part + (size_t)(cap - 4) * n;
+      const long long step = 4ll * n;
+      int cnt = 0;
+      float thr = hv ? g.rc2hi : -1.f;  // -1: no candidate is a hit
+      float far2 = -1.f;                // largest d2 of the hits
+      for (int c0 = 0; c0 < ncells; c0 += 32) {
+        // stencil cell of this lane
+        int start = 0, many = 0;
+        float4 sh = make_float4(0.f, 0.f, 0.f, 0.f);
+        uint32_t code = 0;
+        if (c0 + lane < ncells) {
+          const int q = c0 + lane, dx = q % width - S, dy = (q / width) % width - S, dz = q / (width * width) - S;
+          const int vx = cx + dx, vy = cy + dy, vz = cz + dz;
+          const int wx = vx - floor_div(vx, g.nc[0]) * g.nc[0], wy = vy - floor_div(vy, g.nc[1]) * g.nc[1],
+                    wz = vz - floor_div(vz, g.nc[2]) * g.nc[2];
+          const int cj = (wz * g.nc[1] + wy) * g.nc[0] + wx;
+          start = sm.cstart[cj];
+          many = sm.cstart[cj + 1] - start;
+          sh = make_float4(0.f, (float)dx * g.hf[0], (float)dy * g.hf[1], (float)dz * g.hf[2]);
+          code = (uint32_t)(dx + S) | ((uint32_t)(dy + S) << 3) | ((uint32_t)(dz + S) << 6);
+        }
+        int incl = many;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(FULL, incl, o);
+          if (lane >= o) incl += v;
+        }
+        const int pre = incl - many, total = __shfl_sync(FULL, incl, 31);
+        const bool any = many > 0;
+        const unsigned anyb = __ballot_sync(FULL, any);
+        __syncwarp();
+        if (any) {
+          sh.x = __int_as_float(((start - pre) << 9) | (int)code);
+          shift[__popc(anyb & ((1u << lane) - 1u))] = sh;
+        }
+        const int mid = min(total, (((total + 1) >> 1) + 31) & ~31);
+        for (int qa = 0; qa < mid; qa += 32) {
+          __syncwarp();
+          int m[2];
+#pragma unroll
+          for (int side = 0; side < 2; ++side) {
+            const int w0 = side ? total - qa - 32 : qa, q0 = side ? mid : 0, q1 = side ? total : mid;
+            const int off = pre - w0, q = w0 + lane;
+            const unsigned starts = __reduce_or_sync(FULL, any && (unsigned)off < 32u ? 1u << off : 0u);
+            const int before = __popc(__ballot_sync(FULL, any && off < 0));
+            const bool valid = q >= q0 && q < q1;
+            const int sc = valid ? before + __popc(starts & (0xffffffffu >> (31 - lane))) - 1 : 0;
+            const float4 cs = shift[sc];
+            const int dc = __float_as_int(cs.x), k = valid ? q + (dc >> 9) : 0;
+            const float4 pj = sm.pos[k];
+            // the separation's rounding is pair_d2's, (p_j - p_i) + shift, below;
+            // here the shifted position serves the box test alone
+            const float ex = pj.x + cs.y, ey = pj.y + cs.z, ez = pj.z + cs.w;
+            const float bx = fmaxf(0.f, fmaxf(blo.x - ex, ex - bhi.x));
+            const float by = fmaxf(0.f, fmaxf(blo.y - ey, ey - bhi.y));
+            const float bz = fmaxf(0.f, fmaxf(blo.z - ez, ez - bhi.z));
+            const bool keep = valid && fmaf(bx, bx, fmaf(by, by, bz * bz)) <= keep2;
+            const unsigned km = __ballot_sync(FULL, keep), lt = (1u << lane) - 1u;
+            m[side] = __popc(km);
+            float* const d = chunk + side * (128 + 16) + (keep ? __popc(km & lt) : m[side] + __popc(~km & lt));
+            d[0] = keep ? ex : FAR;
+            d[32] = ey;
+            d[64] = ez;
+            d[96] = __uint_as_float((uint32_t)k | (uint32_t)(dc & 511) << 11);
+          }
+          __syncwarp();
+          const int mm = max(m[0], m[1]);
+          const float4* const cand = reinterpret_cast<const float4*>(chunk + half * (128 + 16));
+          for (int t = 0; t < mm; t += 4) {
+            if (put > last) {
+              thr = -1.f;
+              sm.overflow = 1;
+            }
+            const float4 x = cand[t / 4], y = cand[8 + t / 4], z = cand[16 + t / 4], w = cand[24 + t / 4];
+            const float2 dx0 = __fadd2_rn(make_float2(x.x, x.y), npx), dx1 = __fadd2_rn(make_float2(x.z, x.w), npx);
+            const float2 dy0 = __fadd2_rn(make_float2(y.x, y.y), npy), dy1 = __fadd2_rn(make_float2(y.z, y.w), npy);
+            const float2 dz0 = __fadd2_rn(make_float2(z.x, z.y), npz), dz1 = __fadd2_rn(make_float2(z.z, z.w), npz);
+            const float2 d0 = __ffma2_rn(dx0, dx0, __ffma2_rn(dy0, dy0, __fmul2_rn(dz0, dz0)));
+            const float2 d1 = __ffma2_rn(dx1, dx1, __ffma2_rn(dy1, dy1, __fmul2_rn(dz1, dz1)));
+            const float dd[4] = {d0.x, d0.y, d1.x, d1.y};
+            const uint32_t ww[4] = {__float_as_uint(w.x), __float_as_uint(w.y), __float_as_uint(w.z),
+                                    __float_as_uint(w.w)};
+#pragma unroll
+            for (int u = 0; u < 4; ++u)  // predicated: four tests are one straight line
+              asm volatile("{\n.reg .pred p, q;\nsetp.ne.u32 q, %5, %7;\nsetp.le.and.f32 p, %3, %4, q;\n"
+                           "@p st.global.u32 [%0], %5;\n@p add.s64 %0, %0, %6;\n@p add.s32 %1, %1, 1;\n"
+                           "@p max.f32 %2, %2, %3;\n}"
+                           : "+l"(put), "+r"(cnt), "+f"(far2)
+                           : "f"(dd[u]), "f"(thr), "r"(ww[u]), "l"(step), "r"(self)
+                           : "memory");
+          }
+        }
+      }
+      // exact re-test of the band entries, by the lane that wrote them
+      int kept = cnt;
+      if (hv && far2 >= g.rc2lo * (1.0f - 0x1p-20f)) {
+        int to = 0;
+        for (int q = 0; q < cnt; ++q) {
+          const uint32_t w = part[(size_t)q * n];
+          const int k = (int)(w & 2047u), dx = (int)((w >> 11) & 7u) - S, dy = (int)((w >> 14) & 7u) - S,
+                    dz = (int)(w >> 17) - S;
+          float ddx, ddy, ddz;
+          const float d2 = pair_d2(pi, sm.pos[k], (float)dx * g.hf[0], (float)dy * g.hf[1], (float)dz * g.hf[2], ddx,
+                                   ddy, ddz);
+          if (d2 < g.rc2lo || (d2 <= g.rc2hi && batch_exact(A, g, sm.order[s], sm.order[k], floor_div(cx + dx, g.nc[0]),
+                                                            floor_div(cy + dy, g.nc[1]), floor_div(cz + dz, g.nc[2]))))
+            part[(size_t)(to++) * n] = w;
+        }
+        kept = to;
+      }
+      const int other = __shfl_xor_sync(FULL, kept, 16);
+      if (hv && half == 0) {
+        sm.front[s] = (unsigned short)kept;
+        sm.nnb[s] = (unsigned short)(kept + other);
+      }
+    }
   }
+}
+
+// Merge the compensated sums of an atom's T lanes (all lanes of the warp).
+__device__ __forceinline__ void reduce_kahan(float& s, float& c, int T) {
+  for (int off = T >> 1; off > 0; off >>= 1) {
+    const float s2 = __shfl_xor_sync(0xffffffffu, s, off), c2 = __shfl_xor_sync(0xffffffffu, c, off);
+    kahan_merge(s, c, s2, c2);
+  }
+}
+__device__ __forceinline__ void reduce_plain(float& s, int T) {
+  for (int off = T >> 1; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+}
+
+__device__ __forceinline__ void knot_pair(const float4* p, float4& a, float4& b) {
+  asm("ld.global.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+      : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+      : "l"(p));
+}
+
+// Block barrier after code in which lanes of a warp part (a last warp with
+// fewer atoms than lanes, lists of different lengths): the warp comes together
+// first.  With one lane per atom nothing else brings the lanes of a short warp
+// together before the barrier, and it was seen to count such a warp twice.
+__device__ __forceinline__ void block_sync() {
+  __syncwarp();
   __syncthreads();
-  if (threadIdx.x < nv) {
+}
+
+// Sums of NV quantities over the block, to red[0][0 .. NV).
+template <int NV, class SM>
+__device__ __forceinline__ void block_sum(SM& sm, double (&v)[NV]) {
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int q = warp_sum_transposed<NV>(v, lane);
+  if (q >= 0) sm.red[w][q] = v[0];
+  block_sync();
+  if (threadIdx.x < NV) {
     double a = 0.0;
     for (int k = 0; k < (int)(blockDim.x >> 5); ++k) a += sm.red[k][threadIdx.x];
-    out[threadIdx.x] = a;
+    sm.red[0][threadIdx.x] = a;
   }
-  __syncthreads();
+  block_sync();
 }
 
-template <int MAXA, int MAXC>
-__global__ void __launch_bounds__(512, 1) k_batch(BatchArgs A) {
+template <int MAXA, int MAXC, int MAXT, int MINB, bool ADJ>
+__global__ void __launch_bounds__(MAXT, MINB) k_batch(const __grid_constant__ BatchArgs A) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  using SM = SmemT<MAXA, MAXC>;
+  using SM = SmemT<MAXA, MAXC, MAXT>;
   SM& sm = *reinterpret_cast<SM*>(smem_raw);
-  const int t = threadIdx.x, B = blockDim.x;
+  const int tid = threadIdx.x, B = blockDim.x;
+  RepGeom& g = sm.geom;
   // Persistent mode: take queue tickets until they run past nrep (each block
   // takes at most nrep + 1 tickets).  Single mode: exactly one replica.
   for (int iter = 0;; ++iter) {
-    if (t == 0) sm.rep = A.single >= 0 ? (iter == 0 ? A.single : A.nrep) : atomicAdd(A.queue, 1);
-    __syncthreads();
+    if (tid == 0) sm.rep = A.single >= 0 ? (iter == 0 ? A.single : A.nrep) : atomicAdd(A.queue, 1);
+    block_sync();
     const int qi = sm.rep;
-    __syncthreads();
     if (qi < 0 || qi >= A.nrep) break;
     const int r = A.single >= 0 ? qi : A.order[qi];
-    RepGeom g;
-    g.base = A.off[r];
-    g.n = (int)(A.off[r + 1] - g.base);
-    for (int d = 0; d < 3; ++d) {
-      g.lo[d] = A.lo[3 * r + d];
-      g.L[d] = A.L[3 * r + d];
-      g.hi[d] = A.hi[3 * r + d];
-    }
-    g.ncells = gbmd::batch_grid_dims(g.L, A.rcut, A.S, MAXC, g.nc);
-    for (int d = 0; d < 3; ++d) {
-      g.h[d] = g.L[d] / g.nc[d];
-      g.inv_h[d] = (double)g.nc[d] / g.L[d];
-      g.hf[d] = (float)g.h[d];
-    }
     double* row = A.rep + (size_t)r * REP_ROW;
-    if (g.n > MAXA || g.L[0] < A.rcut || g.L[1] < A.rcut || g.L[2] < A.rcut) {
-      if (t == 0) {
+    for (int c = tid; c < MAXC; c += B) sm.cfill[c] = 0;
+    if (tid < 3) {  // FP64 divisions take some 600 cycles each: few of them in a row
+      const int d = tid;
+      const double L3[3] = {A.L[3 * r], A.L[3 * r + 1], A.L[3 * r + 2]};
+      int nc[3];
+      const int ncells = gbmd::batch_grid_dims(L3, A.rcut, A.S, MAXC, nc);
+      const double L = L3[d];
+      const double n = small_double(d == 0 ? nc[0] : (d == 1 ? nc[1] : nc[2]));
+      g.lo[d] = A.lo[3 * r + d];
+      g.hi[d] = A.hi[3 * r + d];
+      g.L[d] = L;
+      g.nc[d] = (int)n;
+      g.h[d] = L / n;
+      g.inv_h[d] = n / L;
+      g.hf[d] = (float)g.h[d];
+      if (d == 0) {
+        g.base = A.off[r];
+        g.n = (int)(A.off[r + 1] - g.base);
+        g.ncells = ncells;
+        int tsh = 0;  // the most lanes per atom that take the replica in one go
+        while (tsh < 5 && (g.n << (tsh + 1)) <= B) ++tsh;
+        g.tsh = tsh;
+        sm.overflow = 0;
+        // the band covers the rounding of coordinates in cells of edge h, as
+        // band_rel's does for its cells
+        const float hmax = fmaxf((float)L3[0] / nc[0], fmaxf((float)L3[1] / nc[1], (float)L3[2] / nc[2]));
+        const float rc = (float)A.rcut, band = fminf(0x1p-16f * fmaxf(1.f, hmax / rc), 0.5f);
+        g.rc2lo = rc * rc * (1.f - band);
+        g.rc2hi = rc * rc * (1.f + band);
+      }
+    }
+    block_sync();
+    const int n = g.n;
+    if (n > MAXA || g.L[0] < A.rcut || g.L[1] < A.rcut || g.L[2] < A.rcut) {
+      if (tid == 0) {
         atomicOr(&A.err[0], 16);
         for (int q = 0; q < REP_ROW; ++q) row[q] = __longlong_as_double(0x7ff8000000000000ll);
       }
-      __syncthreads();
+      block_sync();
       continue;
     }
-    const int n = g.n;
     // ---- cell sort (deterministic order inside a cell: local atom index)
-    for (int c = t; c < g.ncells; c += B) sm.cfill[c] = 0;
-    __syncthreads();
-    for (int a = t; a < n; a += B) {
-      double w;
-      int c3[3];
+    for (int a = tid; a < n; a += B) {
       const double xs[3] = {A.x[g.base + a], A.y[g.base + a], A.z[g.base + a]};
-      for (int d = 0; d < 3; ++d) wrap_cell(g, xs[d], d, w, c3[d]);
+      int c3[3];
+      float lp[3];
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        double w;
+        wrap_cell(g, xs[d], d, w, c3[d]);
+        lp[d] = narrow(w - small_double(c3[d]) * g.h[d] - g.lo[d]);
+      }
       const int c = (c3[2] * g.nc[1] + c3[1]) * g.nc[0] + c3[0];
-      sm.cellof[a] = c;
+      sm.cellof[a] = (unsigned short)c;
+      sm.gfe[a] = make_float4(lp[0], lp[1], lp[2], 0.f);
       atomicAdd(&sm.cfill[c], 1);
     }
-    __syncthreads();
-    if (t < 32) {  // warp scan of the cell counts
+    block_sync();
+    if (tid < 32) {  // warp scan of the cell counts
       const int per = (g.ncells + 31) / 32;
       int loc = 0;
       for (int k = 0; k < per; ++k) {
-        const int c = t * per + k;
+        const int c = tid * per + k;
         if (c < g.ncells) loc += sm.cfill[c];
       }
       int inc = loc;
       for (int o = 1; o < 32; o <<= 1) {
         const int v = __shfl_up_sync(0xffffffffu, inc, o);
-        if (t >= o) inc += v;
+        if (tid >= o) inc += v;
       }
       int run = inc - loc;
       for (int k = 0; k < per; ++k) {
-        const int c = t * per + k;
+        const int c = tid * per + k;
         if (c < g.ncells) {
-          sm.cstart[c] = run;
+          sm.cstart[c] = (unsigned short)run;
           run += sm.cfill[c];
           sm.cfill[c] = 0;
         }
       }
-      if (t == 31) sm.cstart[g.ncells] = inc;
+      if (tid == 31) sm.cstart[g.ncells] = (unsigned short)inc;
     }
-    __syncthreads();
-    for (int a = t; a < n; a += B) {
+    block_sync();
+    for (int a = tid; a < n; a += B) {  // any order first
       const int c = sm.cellof[a];
-      sm.order[sm.cstart[c] + atomicAdd(&sm.cfill[c], 1)] = a;
+      sm.nnb[sm.cstart[c] + atomicAdd(&sm.cfill[c], 1)] = (unsigned short)a;
     }
-    __syncthreads();
-    for (int c = t; c < g.ncells; c += B) {  // insertion sort of the cell's atoms
-      const int b = sm.cstart[c], e = sm.cstart[c + 1];
-      for (int k = b + 1; k < e; ++k) {
-        const int v = sm.order[k];
-        int m = k - 1;
-        while (m >= b && sm.order[m] > v) {
-          sm.order[m + 1] = sm.order[m];
-          --m;
-        }
-        sm.order[m + 1] = v;
-      }
+    block_sync();
+    for (int s = tid; s < n; s += B) {  // then by rank among the cell's atoms
+      const int a = sm.nnb[s], c = sm.cellof[a], b = sm.cstart[c], e = sm.cstart[c + 1];
+      int rank = b;
+      for (int k = b; k < e; ++k) rank += sm.nnb[k] < a;
+      sm.order[rank] = (unsigned short)a;
+      sm.pos[rank] = sm.gfe[a];
     }
-    __syncthreads();
-    for (int s = t; s < n; s += B) {
-      const int a = sm.order[s], c = sm.cellof[a];
-      const int c3[3] = {c % g.nc[0], (c / g.nc[0]) % g.nc[1], c / (g.nc[0] * g.nc[1])};
-      const double xs[3] = {A.x[g.base + a], A.y[g.base + a], A.z[g.base + a]};
-      float lp[3];
-      for (int d = 0; d < 3; ++d) {
-        double w;
-        int cc;
-        wrap_cell(g, xs[d], d, w, cc);
-        lp[d] = (float)(w - (double)c3[d] * g.h[d] - g.lo[d]);
-      }
-      sm.pos[s] = make_float4(lp[0], lp[1], lp[2], __int_as_float(a));
-    }
-    if (t == 0) sm.list_ok = 1;
-    __syncthreads();
+    block_sync();
+    const int T = 1 << g.tsh, t = tid & (T - 1), ns = B >> g.tsh;  // ns atoms at a time
     // ---- pair list: one walk over the cells (FP32 screen, FP64 band
     // re-test), then every pass below reads the list
     uint32_t* nbl = A.nbl + (A.single >= 0 ? (size_t)0 : (size_t)blockIdx.x * MAXA * NBL_MAX);
-    build_list(A, g, sm, nbl, n);
-    __syncthreads();
+    const int cap = MAXA * NBL_MAX / (2 * max(n, 1));  // entries in either part
+    build_list<MAXT>(A, g, sm, nbl, cap);
+    block_sync();
+    const bool list_ok = !sm.overflow;
+    const int listed = list_ok ? cap : 0;
     // ---- density + embedding
-    for (int s = t; s < n; s += B) {
-      float acc = 0.f, comp = 0.f;
-      visit(A, g, sm, nbl, n, s, [&](int k, float dx, float dy, float dz, float d2) {
-        const float rr = d2 * rsqrtf(d2);
-        float q;
-        const int m = knot(fmaf(rr, A.rdr, 1.f), A.nr - 1, q);
-        kahan_add(acc, comp, sval(A.rhor4[m], q));
-      });
-      const float R = acc - comp;
-      float q = fmaf(R, A.rdrho, 1.f);
-      int m = (int)q;
-      m = max(1, min(m, A.nrho - 1));
-      q = fminf(q - (float)m, 1.f);
-      const float4 c = A.frho4[m];
-      const float fp = sdq(c, q) * A.rdrho;
-      float e = sval(c, q);
-      if (R > A.rhomax) e = fmaf(fp, R - A.rhomax, e);
-      sm.fp[s] = fp;
-      sm.eemb[s] = e;
-      sm.rho[s] = R;
+    for (int s0 = 0; s0 < n; s0 += ns) {
+      const int s = s0 + (tid >> g.tsh);
+      float acc = 0.f, comp = 0.f, part = 0.f;
+      if (s < n)
+        visit(A, g, sm, nbl, listed, s, t,
+              [&](int k, float dx, float dy, float dz, float d2, bool ok) {
+                const float rr = d2 * rsqrtf(d2);
+                float q;
+                const int m = knot(fmaf(rr, A.rdr, 1.f), A.nr - 1, q);
+                const float val = sval(A.rhor4[m], q);
+                part += ok ? val : 0.f;
+              },
+              [&]() {
+                kahan_add(acc, comp, part);
+                part = 0.f;
+              });
+      reduce_kahan(acc, comp, T);
+      if (s < n && t == 0) sm.rho[s] = acc - comp;
     }
-    __syncthreads();
+    block_sync();
+    // F'(rho); E = F(rho) is formed again where it is needed
+    for (int s = tid; s < n; s += B) {
+      float q;
+      const float4 c = A.frho4[embed_knot(A, sm.rho[s], q)];
+      sm.pos[s].w = sdq(c, q) * A.rdrho;
+    }
+    block_sync();
     // ---- forces, energies, virial; loss residuals
-    // per-thread sums: energy, virial, loss (static indices) and the
-    // parameter gradient by parameter slot
-    double acc_rep[REP_ROW];
-    double acc_par[BMAX_PARAMS];
-    for (int q = 0; q < REP_ROW; ++q) acc_rep[q] = 0.0;
-    for (int q = 0; q < BMAX_PARAMS; ++q) acc_par[q] = 0.0;
-    for (int s = t; s < n; s += B) {
+    // block sums: energy, virial xx yy zz xy xz yz, loss
+    constexpr int NV = ADJ ? 8 : 7;
+    double sum[NV];
+#pragma unroll
+    for (int q = 0; q < NV; ++q) sum[q] = 0.0;
+    for (int s0 = 0; s0 < n; s0 += ns) {
+      const int s = s0 + (tid >> g.tsh);
       float fx = 0.f, fy = 0.f, fz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f, ee = 0.f, ce = 0.f;
+      float px = 0.f, py = 0.f, pz = 0.f, pe = 0.f;
       float v[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-      const float fpi = sm.fp[s];
-      visit(A, g, sm, nbl, n, s, [&](int k, float dx, float dy, float dz, float d2) {
+      if (s < n) {
+        const float fpi = sm.pos[s].w;
+        visit(A, g, sm, nbl, listed, s, t,
+              [&](int k, float dx, float dy, float dz, float d2, bool ok) {
+                const float rs = rsqrtf(d2), rr = d2 * rs;
+                float q;
+                const int m = knot(fmaf(rr, A.rdr, 1.f), A.nr - 1, q);
+                float4 dr, cz2;
+                knot_pair(A.fz8 + 2 * m, dr, cz2);
+                const float rhop = fmaf(fmaf(dr.x, q, dr.y), q, dr.z);
+                const float z2 = sval(cz2, q), z2d = sdq(cz2, q) * A.rdr;
+                const float phi = z2 * rs;
+                const float phip = (z2d - phi) * rs;
+                const float psip = fmaf(fpi + sm.pos[k].w, rhop, phip);
+                const float fpair = ok ? psip * rs : 0.f;
+                px = fmaf(dx, fpair, px);
+                py = fmaf(dy, fpair, py);
+                pz = fmaf(dz, fpair, pz);
+                pe += ok ? 0.5f * phi : 0.f;
+                const float hh = -0.5f * fpair;
+                v[0] = fmaf(hh * dx, dx, v[0]);
+                v[1] = fmaf(hh * dy, dy, v[1]);
+                v[2] = fmaf(hh * dz, dz, v[2]);
+                v[3] = fmaf(hh * dx, dy, v[3]);
+                v[4] = fmaf(hh * dx, dz, v[4]);
+                v[5] = fmaf(hh * dy, dz, v[5]);
+              },
+              [&]() {
+                kahan_add(fx, cx, px);
+                kahan_add(fy, cy, py);
+                kahan_add(fz, cz, pz);
+                kahan_add(ee, ce, pe);
+                px = py = pz = pe = 0.f;
+              });
+      }
+      reduce_kahan(fx, cx, T);
+      reduce_kahan(fy, cy, T);
+      reduce_kahan(fz, cz, T);
+      reduce_kahan(ee, ce, T);
+#pragma unroll
+      for (int q = 0; q < 6; ++q) reduce_plain(v[q], T);
+      if (s < n && t == 0) {
+        const int64_t ga = g.base + sm.order[s];
+        const double Fx = widen(fx - cx), Fy = widen(fy - cy), Fz = widen(fz - cz);
+        const float R = sm.rho[s];
+        float q;
+        const float4 c = A.frho4[embed_knot(A, R, q)];
+        float emb = sval(c, q);
+        if (R > A.rhomax) emb = fmaf(sm.pos[s].w, R - A.rhomax, emb);
+        const double E = widen(emb) + widen(ee - ce);
+        A.fx[ga] = Fx;
+        A.fy[ga] = Fy;
+        A.fz[ga] = Fz;
+        A.ep[ga] = E;
+        sum[0] += E;
+#pragma unroll
+        for (int u = 0; u < 6; ++u) sum[1 + u] += widen(v[u]);
+        if (ADJ) {
+          const double ex = Fx - A.Ftx[ga], ey = Fy - A.Fty[ga], ez = Fz - A.Ftz[ga], de = E - A.Et[ga];
+          sum[ADJ ? 7 : 0] += A.wF * (ex * ex + ey * ey + ez * ez) + A.wE * de * de;
+          const double twF = 2.0 * A.wF;
+          sm.gfe[s] = make_float4(narrow(twF * ex), narrow(twF * ey), narrow(twF * ez), narrow(2.0 * A.wE * de));
+        }
+      }
+    }
+    block_sum<NV>(sm, sum);
+    if (tid < (ADJ ? 11 : 10)) {
+      // row-major virial from xx yy zz xy xz yz
+      const int q = tid == 0 ? 0 : (tid == 10 ? 7 : 1 + (int)((0x254513430ll >> (4 * (tid - 1))) & 15));
+      row[tid] = sm.red[0][q];
+    }
+    if (!ADJ && tid >= 10 && tid < REP_ROW) row[tid] = 0.0;
+    if constexpr (ADJ) {
+      double fr[BMAX_PARAMS];  // dF/dtheta terms
+#pragma unroll
+      for (int p = 0; p < BMAX_PARAMS; ++p) fr[p] = 0.0;
+      // ---- adjoint sweep 1: G_i, then the embedding terms and lambda_i
+      for (int s0 = 0; s0 < n; s0 += ns) {
+        const int s = s0 + (tid >> g.tsh);
+        float Gs = 0.f;
+        float4 gi = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (s < n) {
+          gi = sm.gfe[s];
+          visit(A, g, sm, nbl, listed, s, t,
+                [&](int k, float dx, float dy, float dz, float d2, bool ok) {
+                  const float rs = rsqrtf(d2), rr = d2 * rs;
+                  float q;
+                  const int m = knot(fmaf(rr, A.rdr, 1.f), A.nr - 1, q);
+                  const float ux = dx * rs, uy = dy * rs, uz = dz * rs;
+                  const float4 gk = sm.gfe[k];
+                  const float sij = fmaf(gi.x, ux, fmaf(gi.y, uy, gi.z * uz));
+                  const float sji = -fmaf(gk.x, ux, fmaf(gk.y, uy, gk.z * uz));
+                  const float4 dr = A.fz8[2 * m];
+                  const float rhop = fmaf(fmaf(dr.x, q, dr.y), q, dr.z);
+                  Gs = ok ? fmaf(sij + sji, rhop, Gs) : Gs;
+                },
+                []() {});
+        }
+        reduce_plain(Gs, T);
+        if (s < n && t == 0) {
+          const float R = sm.rho[s];
+          float q;
+          const int m = embed_knot(A, R, q);
+          const float4 c = A.frho4[m];
+          const bool over = R > A.rhomax;
+          const float f2 = over ? 0.f : fmaf(6.f * c.x, q, 2.f * c.y) * A.rdrho * A.rdrho;
+          sm.rho[s] = fmaf(gi.w, sm.pos[s].w, Gs * f2);
+#pragma unroll
+          for (int p = 0; p < BMAX_PARAMS; ++p)
+            if (p < A.nfr) {
+              const float4 dc = A.dfrho4[(size_t)p * (A.nrho + 1) + m];
+              const float dfp = sdq(dc, q) * A.rdrho;
+              fr[p] += widen(fmaf(gi.w, sval(dc, q) + (over ? dfp * (R - A.rhomax) : 0.f), Gs * dfp));
+            }
+        }
+      }
+      block_sync();  // red is read
+      block_sum<BMAX_PARAMS>(sm, fr);
+      if (tid < BMAX_PARAMS) {
+        double v = 0.0;
+        for (int p = 0; p < A.nfr; ++p)
+          if (A.pfr[p] == tid) v += sm.red[0][p];
+        row[11 + tid] = v;
+      }
+      // ---- adjoint sweep 2: the tables' terms.  A pair's contribution to the
+      // gradient of any z2r (rho) parameter is the same four weights times its
+      // table's four coefficients at the pair's knot.  A lane forms the weights
+      // of its pair; then eight lanes take the tables of one pair, 16 bytes of
+      // one or a few 128-byte lines each (a lane reading all tables of its own
+      // pair costs 32 lines a read).
+      const int lane = tid & 31, wid = tid >> 5;
+      PairRecord& rec = sm.rec[wid];
+      const int nb = A.ktab >> 3;  // table batches of eight
+      float acc[MAX_TABLES / 8];
+      double accd[MAX_TABLES / 8];
+#pragma unroll
+      for (int b = 0; b < MAX_TABLES / 8; ++b) {
+        acc[b] = 0.f;
+        accd[b] = 0.0;
+      }
+      auto weights = [&](const float4& gi, float fpi, float lam, int k, float dx, float dy, float dz, float d2, bool ok) {
         const float rs = rsqrtf(d2), rr = d2 * rs;
         float q;
         const int m = knot(fmaf(rr, A.rdr, 1.f), A.nr - 1, q);
-        const float4 dr = A.rhod4[m];
-        const float rhop = fmaf(fmaf(dr.x, q, dr.y), q, dr.z);
-        const float4 cz2 = A.z2r4[m];
-        const float z2 = sval(cz2, q), z2d = sdq(cz2, q) * A.rdr;
-        const float phi = z2 * rs;
-        const float phip = (z2d - phi) * rs;
-        const float psip = fmaf(fpi + sm.fp[k], rhop, phip);
-        const float fpair = psip * rs;
-        kahan_add(fx, cx, dx * fpair);
-        kahan_add(fy, cy, dy * fpair);
-        kahan_add(fz, cz, dz * fpair);
-        kahan_add(ee, ce, 0.5f * phi);
-        const float hh = -0.5f * fpair;
-        v[0] = fmaf(hh * dx, dx, v[0]);
-        v[1] = fmaf(hh * dy, dy, v[1]);
-        v[2] = fmaf(hh * dz, dz, v[2]);
-        v[3] = fmaf(hh * dx, dy, v[3]);
-        v[4] = fmaf(hh * dx, dz, v[4]);
-        v[5] = fmaf(hh * dy, dz, v[5]);
-      });
-      const int a = sm.order[s];
-      const int64_t ga = g.base + a;
-      const double Fx = (double)(fx - cx), Fy = (double)(fy - cy), Fz = (double)(fz - cz);
-      const double E = (double)sm.eemb[s] + (double)(ee - ce);
-      A.fx[ga] = Fx;
-      A.fy[ga] = Fy;
-      A.fz[ga] = Fz;
-      A.ep[ga] = E;
-      acc_rep[0] += E;
-      acc_rep[1] += v[0]; acc_rep[2] += v[3]; acc_rep[3] += v[4];
-      acc_rep[4] += v[3]; acc_rep[5] += v[1]; acc_rep[6] += v[5];
-      acc_rep[7] += v[4]; acc_rep[8] += v[5]; acc_rep[9] += v[2];
-      if (A.adjoint) {
-        const double ex = Fx - A.Ftx[ga], ey = Fy - A.Fty[ga], ez = Fz - A.Ftz[ga], de = E - A.Et[ga];
-        acc_rep[10] += A.wF * (ex * ex + ey * ey + ez * ez) + A.wE * de * de;
-        sm.gfe[s] = make_float4((float)(2.0 * A.wF * ex), (float)(2.0 * A.wF * ey), (float)(2.0 * A.wF * ez),
-                                (float)(2.0 * A.wE * de));
-      }
-    }
-    if (A.adjoint) {
-      __syncthreads();
-      // ---- adjoint sweep 1: G_i, and the phi / phi' / rho' parameter terms
-      for (int s = t; s < n; s += B) {
-        const float4 gi = sm.gfe[s];
-        const float fpi = sm.fp[s];
-        float Gs = 0.f;
-        // this atom's parameter terms, FP32 over its pairs (static indices:
-        // registers), folded into the FP64 per-thread sums once per atom
-        float gz[BMAX_PARAMS], gr[BMAX_PARAMS];
+        const float sij = fmaf(gi.x, dx, fmaf(gi.y, dy, gi.z * dz)) * rs;
+        const float wv = (0.5f * gi.w - sij * rs) * rs;        // weight of dz2
+        const float wd = sij * rs * A.rdr;                     // of d(dz2)/dq
+        const float wr = sij * (fpi + sm.pos[k].w) * A.rdr;    // of d(drho)/dq; lam: of drho
+        rec.m[lane] = ok ? m : 0;
+        rec.z[lane] = ok ? make_float4(fmaf(wv, q, 3.f * wd) * q * q, fmaf(wv, q, 2.f * wd) * q, fmaf(wv, q, wd), wv)
+                         : make_float4(0.f, 0.f, 0.f, 0.f);
+        rec.r[lane] = ok ? make_float4(fmaf(lam, q, 3.f * wr) * q * q, fmaf(lam, q, 2.f * wr) * q, fmaf(lam, q, wr), lam)
+                         : make_float4(0.f, 0.f, 0.f, 0.f);
+      };
+      auto tables = [&]() {  // the warp's 32 recorded pairs
+        __syncwarp();
+        const int kt = lane & 7;
+        for (int b = 0; b < nb; ++b) {
+          const float4* const w = kt + 8 * b < A.nz2 ? rec.z : rec.r;
+          float a = 0.f;
 #pragma unroll
-        for (int p = 0; p < BMAX_PARAMS; ++p) gz[p] = gr[p] = 0.f;
-        visit(A, g, sm, nbl, n, s, [&](int k, float dx, float dy, float dz, float d2) {
-          const float rs = rsqrtf(d2), rr = d2 * rs;
-          float q;
-          const int m = knot(fmaf(rr, A.rdr, 1.f), A.nr - 1, q);
-          const float ux = dx * rs, uy = dy * rs, uz = dz * rs;
-          const float4 gk = sm.gfe[k];
-          const float sij = fmaf(gi.x, ux, fmaf(gi.y, uy, gi.z * uz));
-          const float sji = -fmaf(gk.x, ux, fmaf(gk.y, uy, gk.z * uz));
-          const float4 dr = A.rhod4[m];
-          const float rhop = fmaf(fmaf(dr.x, q, dr.y), q, dr.z);
-          Gs = fmaf(sij + sji, rhop, Gs);
-          const float wv = (0.5f * gi.w - sij * rs) * rs;  // weight of dz2
-          const float wd = sij * rs * A.rdr;              // weight of dz2/dq
-          const float wr = sij * (fpi + sm.fp[k]) * A.rdr; // weight of drho/dq
-#pragma unroll
-          for (int p = 0; p < BMAX_PARAMS; ++p) {
-            if (p < A.nz2) {
-              const float4 c = A.dz2r4[(size_t)p * (A.nr + 1) + m];
-              gz[p] += fmaf(wv, sval(c, q), wd * sdq(c, q));
-            }
-            if (p < A.nrh) {
-              const float4 c = A.drhor4[(size_t)p * (A.nr + 1) + m];
-              gr[p] = fmaf(wr, sdq(c, q), gr[p]);
-            }
+          for (int u = 0; u < 8; ++u) {
+            const int pr = 4 * u + (lane >> 3);
+            const float4 c = A.dtab[(size_t)rec.m[pr] * A.ktab + kt + 8 * b], f = w[pr];
+            a = fmaf(c.x, f.x, fmaf(c.y, f.y, fmaf(c.z, f.z, fmaf(c.w, f.w, a))));
           }
-        });
-        sm.G[s] = Gs;
 #pragma unroll
-        for (int p = 0; p < BMAX_PARAMS; ++p) {
-          if (p < A.nz2) acc_par[A.pz2[p]] += (double)gz[p];
-          if (p < A.nrh) acc_par[A.prh[p]] += (double)gr[p];
+          for (int bb = 0; bb < MAX_TABLES / 8; ++bb)
+            if (bb == b) acc[bb] += a;
         }
+        __syncwarp();
+      };
+      auto settle = [&]() {
+#pragma unroll
+        for (int b = 0; b < MAX_TABLES / 8; ++b)
+          if (b < nb) {
+            accd[b] += widen(acc[b]);
+            acc[b] = 0.f;
+          }
+      };
+      block_sync();  // lambda is complete; red is read
+      if (nb > 0) {
+        const float bias = 8388608.0f + (float)A.S;
+        const uint32_t none = (uint32_t)(A.S | (A.S << 3) | (A.S << 6)) << 11;
+        for (int s0 = 0; s0 < n && list_ok; s0 += ns) {
+          const bool live = s0 + (tid >> g.tsh) < n;
+          const int s = live ? s0 + (tid >> g.tsh) : n - 1;
+          const float4 gi = sm.gfe[s], pi = sm.pos[s];
+          const float lam = sm.rho[s];
+          const PairList list(sm, nbl, n, cap, s);
+          const int mine = live ? list.count : 0;
+          const int steps = __reduce_max_sync(0xffffffffu, mine);
+          uint32_t e = t < mine ? list[t] : none | s;
+          for (int q = t; q - t < steps; q += T) {
+            const uint32_t nxt = q + T < mine ? list[q + T] : none | s;
+            const int k = (int)(e & (SM::ATOMS - 1u));
+            float dx, dy, dz;
+            const float d2 = pair_d2(pi, sm.pos[k], cell_unit((e >> 11) & 7u, bias) * g.hf[0],
+                                     cell_unit((e >> 14) & 7u, bias) * g.hf[1],
+                                     cell_unit((e >> 17) & 7u, bias) * g.hf[2], dx, dy, dz);
+            weights(gi, pi.w, lam, k, dx, dy, dz, d2, q < mine);
+            tables();
+            if (((q >> g.tsh) & 3) == 3) settle();
+            e = nxt;
+          }
+          settle();
       }
-      __syncthreads();
-      // ---- adjoint sweep 2: embedding terms and lam_i * drho
-      for (int s = t; s < n; s += B) {
-        const float4 gi = sm.gfe[s];
-        const float R = sm.rho[s];
-        float q = fmaf(R, A.rdrho, 1.f);
-        int m = (int)q;
-        m = max(1, min(m, A.nrho - 1));
-        q = fminf(q - (float)m, 1.f);
-        const float4 c = A.frho4[m];
-        const bool over = R > A.rhomax;
-        const float f2 = over ? 0.f : fmaf(6.f * c.x, q, 2.f * c.y) * A.rdrho * A.rdrho;
-        const float Gs = sm.G[s];
-        const float lam = fmaf(gi.w, sm.fp[s], Gs * f2);
-        for (int p = 0; p < A.nfr; ++p) {
-          const float4 dc = A.dfrho4[(size_t)p * (A.nrho + 1) + m];
-          const float dfp = sdq(dc, q) * A.rdrho;
-          acc_par[A.pfr[p]] += (double)fmaf(gi.w, sval(dc, q) + (over ? dfp * (R - A.rhomax) : 0.f), Gs * dfp);
+        for (int b = 0; b < nb && !list_ok; ++b) {
+          // from the cells: a lane reads eight tables of each of its own pairs
+          double sum8[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) sum8[k] = 0.0;
+          for (int s = tid >> g.tsh; s < n; s += ns) {
+            const float4 gi = sm.gfe[s];
+            const float fpi = sm.pos[s].w, lam = sm.rho[s];
+            float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            for_pairs(A, g, sm, s, t, T, [&](int k, float dx, float dy, float dz, float d2, uint32_t) {
+              weights(gi, fpi, lam, k, dx, dy, dz, d2, true);
+              const float4* const c = A.dtab + (size_t)rec.m[lane] * A.ktab + 8 * b;
+#pragma unroll
+              for (int q = 0; q < 8; ++q) {
+                const float4 f = q + 8 * b < A.nz2 ? rec.z[lane] : rec.r[lane];
+                a[q] = fmaf(c[q].x, f.x, fmaf(c[q].y, f.y, fmaf(c[q].z, f.z, fmaf(c[q].w, f.w, a[q]))));
+              }
+            });
+#pragma unroll
+            for (int q = 0; q < 8; ++q) sum8[q] += widen(a[q]);
+          }
+          __syncwarp();
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            double v = sum8[q];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+#pragma unroll
+            for (int bb = 0; bb < MAX_TABLES / 8; ++bb)
+              if (bb == b && lane == q) accd[bb] = v;
+          }
         }
-        // lam_i * sum_j drho(r_ij): the pair sums in FP32, lam once per atom
-        float gd[BMAX_PARAMS];
 #pragma unroll
-        for (int p = 0; p < BMAX_PARAMS; ++p) gd[p] = 0.f;
-        visit(A, g, sm, nbl, n, s, [&](int k, float dx, float dy, float dz, float d2) {
-          const float rr = d2 * rsqrtf(d2);
-          float qq;
-          const int mm = knot(fmaf(rr, A.rdr, 1.f), A.nr - 1, qq);
-#pragma unroll
-          for (int p = 0; p < BMAX_PARAMS; ++p)
-            if (p < A.nrh) gd[p] += sval(A.drhor4[(size_t)p * (A.nr + 1) + mm], qq);
-        });
-#pragma unroll
-        for (int p = 0; p < BMAX_PARAMS; ++p)
-          if (p < A.nrh) acc_par[A.prh[p]] += (double)(lam * gd[p]);
+        for (int b = 0; b < MAX_TABLES / 8; ++b) {
+          accd[b] += __shfl_xor_sync(0xffffffffu, accd[b], 8);
+          accd[b] += __shfl_xor_sync(0xffffffffu, accd[b], 16);
+          if (lane < 8) sm.red[wid][lane + 8 * b] = accd[b];
+        }
+        block_sync();
+        if (tid < MAX_TABLES) {
+          double a = 0.0;
+          for (int k = 0; k < (B >> 5); ++k) a += sm.red[k][tid];
+          sm.red[0][tid] = a;
+        }
+        block_sync();
+        if (tid < BMAX_PARAMS) {
+          double v = row[11 + tid];
+          for (int p = 0; p < A.nz2; ++p)
+            if (A.pz2[p] == tid) v += sm.red[0][p];
+          for (int p = 0; p < A.nrh; ++p)
+            if (A.prh[p] == tid) v += sm.red[0][A.nz2 + p];
+          row[11 + tid] = v;
+        }
       }
     }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < BMAX_PARAMS; ++q) acc_rep[11 + q] = acc_par[q];
-    block_reduce_row(sm, acc_rep, REP_ROW, row);
+    block_sync();  // the next replica overwrites the shared memory
   }
 }
 
@@ -550,8 +940,8 @@ struct gbmd_batch {
   float4* dtab = nullptr;
   BatchArgs a{};
   bool have_pot = false, have_targets = false;
-  int block = 256, S = 1;
-  int small_block = 128;         // threads per block of the small-replica kernel
+  int block = 512, S = 1;
+  int small_block = 0;           // threads per block of the small-replica kernel (0: by the number of replicas)
   cudaStream_t side = nullptr;   // runs the small-replica kernel beside the large one
   cudaEvent_t fork = nullptr, join = nullptr;
   int nbig = 0;                  // replicas of more than SMALL_ATOMS atoms (first in `order`)
@@ -607,10 +997,33 @@ void table_f4(int n, double delta, const double* vals, double scale, std::vector
                               (float)(s[m * 8 + 5] * scale), (float)(s[m * 8 + 6] * scale)));
 }
 
-constexpr size_t SMEM_BIG = sizeof(SmemT<BMAX_ATOMS, BMAX_CELLS>);
-constexpr size_t SMEM_SMALL = sizeof(SmemT<SMALL_ATOMS, SMALL_CELLS>);
-auto* const K_BIG = &k_batch<BMAX_ATOMS, BMAX_CELLS>;
-auto* const K_SMALL = &k_batch<SMALL_ATOMS, SMALL_CELLS>;
+// 512 threads at most: large replicas at 128 registers (1,024 threads at 64:
+// 4,480 against 4,340 us for 4,096 replicas of 32-2,048 atoms), small ones two
+// blocks of 512 (or four of 256) per SM at 64 registers (one at 128: 210
+// against 192 us for 256 replicas of 243 atoms).
+constexpr int BIG_THREADS = 512, SMALL_THREADS = 512;
+constexpr size_t SMEM_BIG = sizeof(SmemT<BMAX_ATOMS, BMAX_CELLS, BIG_THREADS>);
+constexpr size_t SMEM_SMALL = sizeof(SmemT<SMALL_ATOMS, SMALL_CELLS, SMALL_THREADS>);
+using BatchKernel = void (*)(BatchArgs);
+BatchKernel big_kernel(int adjoint) {
+  return adjoint ? &k_batch<BMAX_ATOMS, BMAX_CELLS, BIG_THREADS, 1, true>
+                 : &k_batch<BMAX_ATOMS, BMAX_CELLS, BIG_THREADS, 1, false>;
+}
+BatchKernel small_kernel(int adjoint) {
+  return adjoint ? &k_batch<SMALL_ATOMS, SMALL_CELLS, SMALL_THREADS, 2, true>
+                 : &k_batch<SMALL_ATOMS, SMALL_CELLS, SMALL_THREADS, 2, false>;
+}
+
+// Threads per block of the small-replica kernel: with few replicas per SM,
+// many threads (and lanes per atom) for each (256 replicas of 243 atoms, 512 /
+// 256 / 128 threads: 192 / 211 / 307 us); with many, more blocks (4,000 of
+// 32-500 atoms, 256 / 128: 1,558 / 1,832 us).
+int small_threads(const gbmd_batch* b) {
+  if (b->small_block) return b->small_block;
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
+  return b->nrep - b->nbig <= 4 * sms ? 512 : 256;
+}
 
 }  // namespace
 
@@ -636,8 +1049,10 @@ int gbmd_batch_create(gbmd_batch** out, int device, void* stream) {
   }
   if (cudaMalloc(&b->queue, sizeof(int) * 2) != cudaSuccess || cudaMalloc(&b->d_err, sizeof(int) * 4) != cudaSuccess ||
       cudaMemset(b->d_err, 0, sizeof(int) * 4) != cudaSuccess ||
-      cudaFuncSetAttribute(K_BIG, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BIG) != cudaSuccess ||
-      cudaFuncSetAttribute(K_SMALL, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_SMALL) != cudaSuccess ||
+      cudaFuncSetAttribute(big_kernel(0), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BIG) != cudaSuccess ||
+      cudaFuncSetAttribute(big_kernel(1), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_BIG) != cudaSuccess ||
+      cudaFuncSetAttribute(small_kernel(0), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_SMALL) != cudaSuccess ||
+      cudaFuncSetAttribute(small_kernel(1), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_SMALL) != cudaSuccess ||
       cudaStreamCreateWithFlags(&b->side, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&b->join, cudaEventDisableTiming) != cudaSuccess) {
@@ -681,29 +1096,31 @@ int gbmd_batch_set_eam_alloy(gbmd_batch* b, int nrho, double drho, int nr, doubl
                              double conv_frho) {
   if (!b || nrho < 5 || nr < 5 || !(drho > 0) || !(dr > 0) || !frho || !rhor || !z2r || !(rcut > 0))
     return berr(b, GBMD_ERR_INVALID, "bad eam_alloy tables");
-  std::vector<float4> h;
-  table_f4(nrho, drho, frho, conv_frho, h);
-  table_f4(nr, dr, rhor, 1.0, h);
-  table_f4(nr, dr, z2r, conv_z2r, h);
-  // rho' coefficients (3c3, 2c4, c5) / dr
+  std::vector<float4> h, z;
+  // rho' coefficients (3c3, 2c4, c5) / dr beside the pair function's, so that
+  // the force pass reads one 32-byte knot
+  table_f4(nr, dr, z2r, conv_z2r, z);
   {
     std::vector<double> f(nr + 1, 0.0), s((size_t)(nr + 1) * 8);
     for (int k = 0; k < nr; ++k) f[k + 1] = rhor[k];
     gbmd::spline7(nr, dr, f.data(), s.data());
-    for (int m = 0; m <= nr; ++m)
+    for (int m = 0; m <= nr; ++m) {
       h.push_back(make_float4((float)(3.0 * s[m * 8 + 3] / dr), (float)(2.0 * s[m * 8 + 4] / dr),
                               (float)(s[m * 8 + 5] / dr), 0.f));
+      h.push_back(z[m]);
+    }
   }
+  table_f4(nrho, drho, frho, conv_frho, h);
+  table_f4(nr, dr, rhor, 1.0, h);
   cudaSetDevice(b->device);
   cudaFree(b->tab);
   b->tab = nullptr;
   BCUDA(b, cudaMalloc(&b->tab, sizeof(float4) * h.size()));
   BCUDA(b, cudaMemcpy(b->tab, h.data(), sizeof(float4) * h.size(), cudaMemcpyHostToDevice));
   BatchArgs& A = b->a;
-  A.frho4 = b->tab;
+  A.fz8 = b->tab;
+  A.frho4 = A.fz8 + 2 * (nr + 1);
   A.rhor4 = A.frho4 + (nrho + 1);
-  A.z2r4 = A.rhor4 + (nr + 1);
-  A.rhod4 = A.z2r4 + (nr + 1);
   A.nr = nr;
   A.nrho = nrho;
   A.rdr = (float)(1.0 / dr);
@@ -711,10 +1128,8 @@ int gbmd_batch_set_eam_alloy(gbmd_batch* b, int nrho, double drho, int nr, doubl
   A.rhomax = (float)((nrho - 1) * drho);
   A.rcut = rcut;
   A.rcut2 = rcut * rcut;
-  A.rc2lo = (float)(A.rcut2 * (1.0 - 0x1p-12));
-  A.rc2hi = (float)(A.rcut2 * (1.0 + 0x1p-12));
   b->have_pot = true;
-  A.nz2 = A.nrh = A.nfr = 0;
+  A.nz2 = A.nrh = A.nfr = A.ktab = 0;
   drop_graph(b);
   return GBMD_OK;
 }
@@ -747,18 +1162,24 @@ int gbmd_batch_set_param_derivatives(gbmd_batch* b, int nparam, const double* df
       A.pz2[A.nz2++] = p;
     }
   }
+  // the pair tables knot by knot, a multiple of eight of them
+  A.ktab = (A.nz2 + A.nrh + 7) / 8 * 8;
   std::vector<float4> h;
+  for (int m = 0; m <= nr; ++m)
+    for (int k = 0; k < A.ktab; ++k) {
+      if (k < A.nz2) h.push_back(zz[(size_t)k * (nr + 1) + m]);
+      else if (k < A.nz2 + A.nrh) h.push_back(rh[(size_t)(k - A.nz2) * (nr + 1) + m]);
+      else h.push_back(make_float4(0.f, 0.f, 0.f, 0.f));
+    }
+  const size_t pair_tables = h.size();
   h.insert(h.end(), fr.begin(), fr.end());
-  h.insert(h.end(), rh.begin(), rh.end());
-  h.insert(h.end(), zz.begin(), zz.end());
   cudaSetDevice(b->device);
   cudaFree(b->dtab);
   b->dtab = nullptr;
   BCUDA(b, cudaMalloc(&b->dtab, sizeof(float4) * (h.size() + 1)));
   BCUDA(b, cudaMemcpy(b->dtab, h.data(), sizeof(float4) * h.size(), cudaMemcpyHostToDevice));
-  A.dfrho4 = b->dtab;
-  A.drhor4 = A.dfrho4 + fr.size();
-  A.dz2r4 = A.drhor4 + rh.size();
+  A.dtab = b->dtab;
+  A.dfrho4 = A.dtab + pair_tables;
   drop_graph(b);
   return GBMD_OK;
 }
@@ -850,13 +1271,13 @@ int gbmd_batch_set_launch(gbmd_batch* b, int block, int stencil) {
 // Blocks of a persistent launch: as many as fit on the device at once, at
 // most one per replica of its queue.  big: the large-replica kernel (the
 // autotuned block), else the small-replica kernel (b->small_block threads).
-static int persistent_grid(gbmd_batch* b, bool big) {
+static int persistent_grid(gbmd_batch* b, bool big, int adjoint) {
   int dev_sms = 0, per_sm = 0;
   cudaDeviceGetAttribute(&dev_sms, cudaDevAttrMultiProcessorCount, b->device);
   if (big)
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, K_BIG, b->block, SMEM_BIG);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, big_kernel(adjoint), b->block, SMEM_BIG);
   else
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, K_SMALL, b->small_block, SMEM_SMALL);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, small_kernel(adjoint), small_threads(b), SMEM_SMALL);
   const int nq = big ? b->nbig : b->nrep - b->nbig;
   return std::max(1, std::min(nq, dev_sms * std::max(per_sm, 1)));
 }
@@ -883,9 +1304,9 @@ static int ensure_nbl(gbmd_batch* b, int regions, int small_regions) {
 }
 
 // Replicas of more than SMALL_ATOMS atoms run in the large-replica kernel
-// (one block of up to 512 threads and 136 KB of shared memory per SM), the
-// rest in the small-replica kernel (64-256 threads, 36 KB, several blocks per
-// SM); each takes its replicas from its own queue, largest first.
+// (blocks of up to 512 threads), the rest in the small-replica kernel (64-512
+// threads, less shared memory, several blocks per SM); each takes its
+// replicas from its own queue, largest first.
 static int batch_launch(gbmd_batch* b, int adjoint, int per_replica) {
   BatchArgs A = b->a;
   A.nrep = b->nrep;
@@ -907,10 +1328,10 @@ static int batch_launch(gbmd_batch* b, int adjoint, int per_replica) {
       A.single = r;
       if (b->rep_atoms[r] > SMALL_ATOMS) {
         A.nbl = b->nbl;
-        K_BIG<<<1, b->block, SMEM_BIG, b->stream>>>(A);
+        big_kernel(adjoint)<<<1, b->block, SMEM_BIG, b->stream>>>(A);
       } else {
         A.nbl = b->nbl_small;
-        K_SMALL<<<1, b->small_block, SMEM_SMALL, b->stream>>>(A);
+        small_kernel(adjoint)<<<1, small_threads(b), SMEM_SMALL, b->stream>>>(A);
       }
     }
   } else {
@@ -924,22 +1345,22 @@ static int batch_launch(gbmd_batch* b, int adjoint, int per_replica) {
       BCUDA(b, cudaStreamWaitEvent(b->side, b->fork, 0));
     }
     if (b->nbig > 0) {
-      const int grid = persistent_grid(b, true);
+      const int grid = persistent_grid(b, true, adjoint);
       if ((size_t)grid > b->nbl_regions) return berr(b, GBMD_ERR_INVALID, "pair-list scratch not sized");
       BatchArgs Ab = A;
       Ab.nrep = b->nbig;
       Ab.nbl = b->nbl;
-      K_BIG<<<grid, b->block, SMEM_BIG, b->stream>>>(Ab);
+      big_kernel(adjoint)<<<grid, b->block, SMEM_BIG, b->stream>>>(Ab);
     }
     if (b->nrep > b->nbig) {
-      const int grid = persistent_grid(b, false);
+      const int grid = persistent_grid(b, false, adjoint);
       if ((size_t)grid > b->nbl_small_regions) return berr(b, GBMD_ERR_INVALID, "pair-list scratch not sized");
       BatchArgs As = A;
       As.nrep = b->nrep - b->nbig;
       As.order = b->order + b->nbig;
       As.queue = b->queue + 1;
       As.nbl = b->nbl_small;
-      K_SMALL<<<grid, b->small_block, SMEM_SMALL, both ? b->side : b->stream>>>(As);
+      small_kernel(adjoint)<<<grid, small_threads(b), SMEM_SMALL, both ? b->side : b->stream>>>(As);
     }
     if (both) {
       BCUDA(b, cudaEventRecord(b->join, b->side));
@@ -957,8 +1378,8 @@ int gbmd_batch_run(gbmd_batch* b, int adjoint, int per_replica, int use_graph) {
   cudaSetDevice(b->device);
   {
     const int rc = per_replica ? ensure_nbl(b, 1, 1)
-                               : ensure_nbl(b, b->nbig > 0 ? persistent_grid(b, true) : 0,
-                                            b->nrep > b->nbig ? persistent_grid(b, false) : 0);
+                               : ensure_nbl(b, b->nbig > 0 ? persistent_grid(b, true, adjoint) : 0,
+                                            b->nrep > b->nbig ? persistent_grid(b, false, adjoint) : 0);
     if (rc) return rc;
   }
   if (use_graph && !per_replica) {

@@ -175,6 +175,7 @@ __device__ __forceinline__ void block_epilogue_d(const PairArgs& A, int64_t i0, 
         for (int q = 0; q < 6; ++q) sums[NF + q][a] = -0.5 * v[q];
       }
     }
+    __syncwarp();  // the lanes' lists differ in length
     __syncthreads();
     if constexpr (EV) {
       const int m = A.want_virial ? (int)min((int64_t)nat, A.n - i0) * 9 : 0;

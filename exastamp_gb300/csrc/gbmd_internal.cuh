@@ -426,6 +426,45 @@ __device__ __forceinline__ void kahan_add(float& s, float& comp, float v) {
   s = t;
 }
 
+// (float)x in integer instructions, rounded to nearest even.
+__device__ __forceinline__ float narrow(double x) {
+  const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
+  const uint32_t m = (hi & 0x7fffffffu) - 0x38100000u;  // exponent - that of FP32's smallest normal
+  if (m >= 0x0fd00000u) return (float)x;  // zero, tiny, huge, infinity, NaN
+  uint32_t f = ((m + 0x00100000u) << 3) | (lo >> 29);
+  const uint32_t rest = lo & 0x1fffffffu;
+  f += rest > 0x10000000u - (f & 1u);  // above a half, or a half with an odd last bit
+  return __uint_as_float((hi & 0x80000000u) | f);
+}
+
+// (double)c for 0 <= c < 2^20 in integer instructions.
+__device__ __forceinline__ double small_double(int c) {
+  const int e = 31 - __clz(c);
+  return c == 0 ? 0.0 : __hiloint2double(((1023 + e) << 20) | ((c << (20 - e)) & 0xfffff), 0);
+}
+
+// Sums of NV quantities over a warp: each of the five steps hands half of the
+// remaining quantities to the partner lane, so a lane ends with one quantity's
+// total in v[0] after about NV additions instead of 5 NV.  Returns which
+// quantity that is, -1 for none.
+template <int NV>
+__device__ __forceinline__ int warp_sum_transposed(double (&v)[NV], int lane) {
+  int first = 0, n = NV;  // this lane's quantities: first .. first + n of the NV
+#pragma unroll
+  for (int o = 16, w = NV; o > 0; o >>= 1, w = (w + 1) / 2) {
+    const int h = (w + 1) / 2;  // the lower lanes keep v[0 .. h), the upper ones v[h .. w)
+    const bool up = lane & o;
+#pragma unroll
+    for (int k = 0; k < h; ++k) {
+      const double a = v[k], b = k + h < w ? v[k + h] : 0.0;
+      v[k] = (up ? b : a) + __shfl_xor_sync(0xffffffffu, up ? a : b, o);
+    }
+    first += up ? h : 0;
+    n = up ? n - h : min(n, h);
+  }
+  return n > 0 ? first : -1;
+}
+
 // Combine two compensated sums (s1 - c1) + (s2 - c2) with an exact two-sum.
 __device__ __forceinline__ void kahan_merge(float& s, float& comp, float s2, float c2) {
   const float t = s + s2;

@@ -390,6 +390,7 @@ __device__ __forceinline__ void block_epilogue(const PairArgs& A, int64_t i0, co
         for (int q = 0; q < 6; ++q) sums[4 + q][a] = S.v[q];
       }
     }
+    __syncwarp();  // the lanes' lists differ in length
     __syncthreads();
     if (EV && A.want_virial) {
       const int m = (int)min((int64_t)nat, A.n - i0) * 9;

@@ -433,7 +433,8 @@ int gbmd_batch_set_targets(gbmd_batch* b, const double* fx, const double* fy, co
  * cell stencil radius (1: cells >= rcut, 2: cells >= rcut/2) */
 int gbmd_batch_set_launch(gbmd_batch* b, int block, int stencil);
 /* Replicas of at most 512 atoms run in a second kernel with smaller blocks
- * (several per SM): its threads per block, 64-256 (default 128). */
+ * (several per SM): its threads per block, 64-256 (unless set: 512 with at
+ * most four such replicas per SM, 256 with more). */
 int gbmd_batch_set_small_block(gbmd_batch* b, int block);
 /* per_replica != 0: one launch per replica (the comparison mode);
  * use_graph != 0: the persistent launch is captured once and replayed */

@@ -364,8 +364,8 @@ int pipe_issue(gbmd_context* c, double dt, const double* const host[9], const do
     if (r) return r;
     forced[s] = 1;
     forced_mask |= 1ull << s;
-    GBMD_CUDA(c, cudaEventRecord(c->pipe_f_ev[s], st));
     if ((r = trace_mark(c, st, GBMD_PIPE_MARK_FORCE, s))) return r;
+    GBMD_CUDA(c, cudaEventRecord(c->pipe_f_ev[s], st));
     bool waited = false;
     for (int k = 0; k < P; ++k) {
       if (outd[k] || (c->pipe_mask[k] & ~forced_mask)) continue;
@@ -399,8 +399,9 @@ int pipe_issue(gbmd_context* c, double dt, const double* const host[9], const do
         const cudaStream_t st = take();
         GBMD_CUDA(c, cudaStreamWaitEvent(st, c->pipe_in_ev[k], 0));
         if ((rc = piece(s, 1, st))) return rc;
-        GBMD_CUDA(c, cudaEventRecord(c->pipe_d_ev[s], st));
+        // the mark first: whoever waits for the event runs after it
         if ((rc = trace_mark(c, st, GBMD_PIPE_MARK_DENSITY, s))) return rc;
+        GBMD_CUDA(c, cudaEventRecord(c->pipe_d_ev[s], st));
         dens[s] = 1;
       } else if ((rc = force_piece(s))) {
         return rc;

@@ -195,6 +195,22 @@ __global__ void k_to_user_multi(int64_t n, int64_t cap, Arrays9 src, const int32
   for (int k = 0; k < count; ++k) stage[k * cap + u] = src.a[k][p];
 }
 
+// Several per-atom fields in caller order, one after the other in `out`.
+struct PackArgs {
+  const double* src[11];
+  int width[11];
+  int64_t off[11];
+  int count;
+};
+
+__global__ void k_pack_to_user(int64_t n, PackArgs f, const int32_t* __restrict__ user, double* __restrict__ out) {
+  const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (p >= n) return;
+  const int64_t u = user[p];
+  for (int k = 0; k < f.count; ++k)
+    for (int q = 0; q < f.width[k]; ++q) out[f.off[k] + u * f.width[k] + q] = f.src[k][p * f.width[k] + q];
+}
+
 // inv[user[p]] = p: caller index -> cell-sorted index
 __global__ void k_invert_user(int64_t n, const int32_t* __restrict__ user, int32_t* __restrict__ inv) {
   const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -408,16 +424,13 @@ static int rebuild_if_displaced(gbmd_context* c) {
 }
 
 // folds the device-side counts of displacement-triggered rebuilds and of
-// outer list builds into list_builds and outer_builds (stream synchronised)
+// outer list builds into list_builds and outer_builds (h_err holds the device's
+// words)
 static int collect_device_rebuilds(gbmd_context* c) {
-  int cnt[5] = {0, 0, 0, 0, 0};
-  static_assert(ERRW_OUTER_BUILDS - ERRW_REBUILDS == 4, "counter words");
-  GBMD_CUDA(c, cudaMemcpyAsync(cnt, c->d_err + ERRW_REBUILDS, sizeof(cnt), cudaMemcpyDeviceToHost, c->stream));
   GBMD_CUDA(c, cudaMemsetAsync(c->d_err + ERRW_REBUILDS, 0, sizeof(int), c->stream));
   GBMD_CUDA(c, cudaMemsetAsync(c->d_err + ERRW_OUTER_BUILDS, 0, sizeof(int), c->stream));
-  GBMD_CUDA(c, cudaStreamSynchronize(c->stream));
-  c->list_builds += cnt[0];
-  c->outer_builds += cnt[4];
+  c->list_builds += c->h_err[ERRW_REBUILDS];
+  c->outer_builds += c->h_err[ERRW_OUTER_BUILDS];
   return GBMD_OK;
 }
 
@@ -485,12 +498,14 @@ int gbmd_create(gbmd_context** out, int device, void* stream) {
   }
   if (cudaMalloc(&c->d_err, sizeof(int) * ERRW_WORDS) != cudaSuccess ||
       cudaMallocHost(&c->h_err, sizeof(int) * ERRW_WORDS) != cudaSuccess ||
-      cudaMalloc(&c->d_thermo, sizeof(double) * 27) != cudaSuccess ||
-      cudaMallocHost(&c->h_thermo, sizeof(double) * 27) != cudaSuccess ||
+      cudaMalloc(&c->d_thermo, sizeof(double) * (32 + PACK_DOUBLES)) != cudaSuccess ||
+      cudaMallocHost(&c->h_thermo, sizeof(double) * (32 + PACK_DOUBLES)) != cudaSuccess ||
       cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, device) != cudaSuccess) {
     gbmd_destroy(c);
     return GBMD_ERR_CUDA;
   }
+  c->d_pack = c->d_thermo + 32;
+  c->h_pack = c->h_thermo + 32;
   int init[ERRW_WORDS] = {0, 0, 0, -1, -1};
   cudaMemcpy(c->d_err, init, sizeof(init), cudaMemcpyHostToDevice);
   *out = c;
@@ -723,6 +738,37 @@ int gbmd_download(gbmd_context* c, double* rx, double* ry, double* rz, double* v
   } f[11] = {{rx, c->X(), 1}, {ry, c->Y(), 1}, {rz, c->Z(), 1}, {vx, c->VX(), 1}, {vy, c->VY(), 1},
              {vz, c->VZ(), 1}, {ax, c->AX(), 1}, {ay, c->AY(), 1}, {az, c->AZ(), 1}, {ep, c->ep, 1},
              {vir, c->vir, 9}};
+  // small: all fields packed in caller order, one copy and one wait (forces,
+  // energies and virials of 500 atoms with their download: 103 -> 49 us)
+  int64_t total = 0;
+  for (const F& q : f)
+    if (q.host && q.dev) total += n * q.width;
+  if (total > 0 && total <= PACK_DOUBLES) {
+    PackArgs P{};
+    int64_t off = 0;
+    for (const F& q : f) {
+      if (!q.host || !q.dev) continue;
+      P.src[P.count] = q.dev;
+      P.width[P.count] = q.width;
+      P.off[P.count++] = off;
+      off += n * q.width;
+    }
+    k_pack_to_user<<<nblk(n, 128), 128, 0, s>>>(n, P, c->USER(), c->d_pack);
+    GBMD_CUDA(c, cudaMemcpyAsync(c->h_pack, c->d_pack, sizeof(double) * total, cudaMemcpyDeviceToHost, s));
+    GBMD_CUDA(c, cudaStreamSynchronize(s));
+    off = 0;
+    for (const F& q : f) {
+      if (!q.host) continue;
+      const size_t bytes = sizeof(double) * n * q.width;
+      if (!q.dev) {
+        std::memset(q.host, 0, bytes);
+        continue;
+      }
+      std::memcpy(q.host, c->h_pack + off, bytes);
+      off += n * q.width;
+    }
+    return GBMD_OK;
+  }
   // r, v, a: one un-permutation kernel into separate staging slots, then the
   // copies over several copy streams; ep and vir one by one
   Arrays9 src{};
@@ -1183,9 +1229,8 @@ static int ensure_virial(gbmd_context* c) {
   return GBMD_OK;
 }
 
-static int check_device_errors(gbmd_context* c) {
-  int rc = sync_error_word(c);
-  if (rc) return rc;
+// the errors in h_err, which holds the device's words
+static int report_device_errors(gbmd_context* c) {
   const int f = c->h_err[ERRW_FLAGS];
   if (!f) return GBMD_OK;
   int init[ERRW_WORDS] = {0, 0, 0, -1, -1};
@@ -1200,6 +1245,11 @@ static int check_device_errors(gbmd_context* c) {
     return set_error(c, GBMD_ERR_TOO_LARGE,
                      "a Newton-3 pair force beyond 2^16 x 24 eps/sigma (the fixed-point range); use the full list");
   return set_error(c, GBMD_ERR_CUDA, "device error flags %d", f);
+}
+
+static int check_device_errors(gbmd_context* c) {
+  const int rc = sync_error_word(c);
+  return rc ? rc : report_device_errors(c);
 }
 
 int gbmd_check_errors(gbmd_context* c) {
@@ -1468,15 +1518,19 @@ int gbmd_run_nve(gbmd_context* c, int nsteps, double dt, int rebuild_every, int 
     ++s;
   }
   GBMD_CUDA(c, cudaGetLastError());
+  // the rows and the error words with one wait
+  const bool packed = 27 * nrows <= PACK_DOUBLES;
   if (want_thermo && thermo_out)
-    GBMD_CUDA(c, cudaMemcpyAsync(thermo_out, rows, sizeof(double) * 27 * nrows, cudaMemcpyDeviceToHost, c->stream));
-  GBMD_CUDA(c, cudaStreamSynchronize(c->stream));
+    GBMD_CUDA(c, cudaMemcpyAsync(packed ? c->h_pack : thermo_out, rows, sizeof(double) * 27 * nrows,
+                                 cudaMemcpyDeviceToHost, c->stream));
+  if ((rc = sync_error_word(c))) return rc;
+  if (want_thermo && thermo_out && packed) std::memcpy(thermo_out, c->h_pack, sizeof(double) * 27 * nrows);
   c->step += nsteps;
   c->energy_step = -1, c->forces_valid_step = c->step;
   // the last step computed energies and virials when it was a thermo step
   if (want_thermo && nsteps % thermo_every == 0) c->energy_step = c->step;
   if ((trigger || two_level(c)) && (rc = collect_device_rebuilds(c))) return rc;
-  return check_device_errors(c);
+  return report_device_errors(c);
 }
 
 int gbmd_run_nve_host(gbmd_context* c, int nsteps, double dt, int rebuild_every, double* rx, double* ry, double* rz,
@@ -1599,8 +1653,9 @@ int gbmd_run_minimize(gbmd_context* c, int nsteps, double dt, double tolF, int r
   }
   c->energy_step = -1, c->forces_valid_step = c->rho_valid_step = -1;
   GBMD_CUDA(c, cudaStreamSynchronize(c->stream));
+  if ((rc = sync_error_word(c))) return rc;
   if ((trigger || two_level(c)) && (rc = collect_device_rebuilds(c))) return rc;
-  return check_device_errors(c);
+  return report_device_errors(c);
 }
 
 // lj_compute_force parameter adjoint (gbmd_adjoint_lj.cu): forces and

@@ -950,6 +950,7 @@ struct gbmd_batch {
   size_t nbl_regions = 0;
   uint32_t* nbl_small = nullptr; // and of the small-replica kernel's blocks
   size_t nbl_small_regions = 0;
+  double* h_rows = nullptr;      // page-locked: the replicas' rows, then the error words
   cudaGraphExec_t graph = nullptr;
   int graph_adjoint = -1;
 };
@@ -976,6 +977,8 @@ void free_atoms(gbmd_batch* b) {
   void* ps[] = {b->off, b->lo, b->hi, b->L, b->x, b->y, b->z, b->fx, b->fy, b->fz, b->ep, b->rep,
                 b->Ftx, b->Fty, b->Ftz, b->Et, b->order};
   for (void* p : ps) cudaFree(p);
+  if (b->h_rows) cudaFreeHost(b->h_rows);
+  b->h_rows = nullptr;
   b->off = nullptr; b->lo = b->hi = b->L = b->x = b->y = b->z = nullptr;
   b->fx = b->fy = b->fz = b->ep = b->rep = nullptr;
   b->Ftx = b->Fty = b->Ftz = b->Et = nullptr;
@@ -1223,6 +1226,7 @@ int gbmd_batch_upload(gbmd_batch* b, int nrep, const int64_t* offsets, const dou
   BCUDA(b, cudaMalloc(&b->hi, sizeof(double) * 3 * nrep));
   BCUDA(b, cudaMalloc(&b->order, sizeof(int) * nrep));
   BCUDA(b, cudaMalloc(&b->rep, sizeof(double) * REP_ROW * nrep));
+  BCUDA(b, cudaMallocHost(&b->h_rows, sizeof(double) * ((size_t)REP_ROW * nrep + 2)));
   double** arrs[] = {&b->x, &b->y, &b->z, &b->fx, &b->fy, &b->fz, &b->ep, &b->Ftx, &b->Fty, &b->Ftz, &b->Et};
   for (double** p : arrs) BCUDA(b, cudaMalloc(p, nb));
   BCUDA(b, cudaMemcpy(b->off, offsets, sizeof(int64_t) * (nrep + 1), cudaMemcpyHostToDevice));
@@ -1416,15 +1420,19 @@ int gbmd_batch_synchronize(gbmd_batch* b) {
 int gbmd_batch_download(gbmd_batch* b, double* fx, double* fy, double* fz, double* ep, double* rep_energy,
                         double* rep_virial, double* loss, double* grad) {
   if (!b || !b->x) return GBMD_ERR_INVALID;
-  int rc = gbmd_batch_synchronize(b);
-  if (rc) return rc;
-  const size_t nb = sizeof(double) * (size_t)b->n;
-  if (fx) BCUDA(b, cudaMemcpy(fx, b->fx, nb, cudaMemcpyDeviceToHost));
-  if (fy) BCUDA(b, cudaMemcpy(fy, b->fy, nb, cudaMemcpyDeviceToHost));
-  if (fz) BCUDA(b, cudaMemcpy(fz, b->fz, nb, cudaMemcpyDeviceToHost));
-  if (ep) BCUDA(b, cudaMemcpy(ep, b->ep, nb, cudaMemcpyDeviceToHost));
-  std::vector<double> rows((size_t)REP_ROW * b->nrep);
-  BCUDA(b, cudaMemcpy(rows.data(), b->rep, sizeof(double) * rows.size(), cudaMemcpyDeviceToHost));
+  // everything queued behind the run, one wait at the end
+  cudaSetDevice(b->device);
+  const size_t nb = sizeof(double) * (size_t)b->n, nrow = (size_t)REP_ROW * b->nrep;
+  double* const rows = b->h_rows;
+  int* const err = reinterpret_cast<int*>(rows + nrow);
+  BCUDA(b, cudaMemcpyAsync(rows, b->rep, sizeof(double) * nrow, cudaMemcpyDeviceToHost, b->stream));
+  BCUDA(b, cudaMemcpyAsync(err, b->d_err, sizeof(int) * 4, cudaMemcpyDeviceToHost, b->stream));
+  if (fx) BCUDA(b, cudaMemcpyAsync(fx, b->fx, nb, cudaMemcpyDeviceToHost, b->stream));
+  if (fy) BCUDA(b, cudaMemcpyAsync(fy, b->fy, nb, cudaMemcpyDeviceToHost, b->stream));
+  if (fz) BCUDA(b, cudaMemcpyAsync(fz, b->fz, nb, cudaMemcpyDeviceToHost, b->stream));
+  if (ep) BCUDA(b, cudaMemcpyAsync(ep, b->ep, nb, cudaMemcpyDeviceToHost, b->stream));
+  BCUDA(b, cudaStreamSynchronize(b->stream));
+  if (err[0] & 16) return berr(b, GBMD_ERR_TOO_LARGE, "a replica exceeded the per-block limits (atoms or box)");
   double L = 0.0, G[BMAX_PARAMS] = {0};
   for (int r = 0; r < b->nrep; ++r) {  // replica order: fixed summation order
     const double* row = &rows[(size_t)r * REP_ROW];

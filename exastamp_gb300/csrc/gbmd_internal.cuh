@@ -253,6 +253,8 @@ struct gbmd_context {
   int64_t part_cap = 0;
   double* d_thermo = nullptr;   // 27
   double* h_thermo = nullptr;   // pinned 27
+  double* d_pack = nullptr;     // PACK_DOUBLES: small downloads, packed on the device
+  double* h_pack = nullptr;     // and their page-locked copy
   double* d_rows = nullptr;     // thermo rows of a run (27 per row)
   int64_t rows_cap = 0;
 
@@ -318,6 +320,10 @@ void spline7(int n, double delta, const double* f, double* s);
 int check_cuda(gbmd_context* c, cudaError_t e, const char* what);
 int ensure_atom_capacity(gbmd_context* c, int64_t n);
 int sync_error_word(gbmd_context* c);  // copies device error word, returns status
+// Downloads of up to this many doubles (a, ep and virial of 5,041 atoms) go
+// through one kernel, one copy to page-locked memory and one wait.  Beyond, the
+// copy out of the page-locked memory costs what the separate copies do.
+constexpr int64_t PACK_DOUBLES = 65536;
 
 // neighbours (gbmd_neighbors.cu)
 int grid_dims(const double lo[3], const double hi[3], double R, int nc[3]);

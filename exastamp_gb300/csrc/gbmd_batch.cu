@@ -123,12 +123,6 @@ struct SmemT {
 
 __device__ __forceinline__ int floor_div(int a, int b) { return a >= 0 ? a / b : -((-a + b - 1) / b); }
 
-// A double's bits as an integer of the same order.
-__device__ __forceinline__ long long order_key(double v) {
-  const long long b = __double_as_longlong(v);
-  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
-}
-
 // periodic wrap with the rounding of the main path's rebuild (and the oracle)
 __device__ __forceinline__ void wrap_cell(const RepGeom& g, double v, int d, double& w, int& c) {
   const long long k = order_key(v);

@@ -20,14 +20,6 @@ namespace gbmd {
 
 static inline unsigned nblk(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
 
-__device__ __forceinline__ void refresh_gather(const Grid& g, int64_t i, int cp, int t, double x, double y,
-                                               double z, float4* pf, double4_32a* pd) {
-  const double cx = (double)(cp & 1023), cy = (double)((cp >> 10) & 1023), cz = (double)(cp >> 20);
-  pf[i] = make_float4((float)(x - cx * g.h[0] - g.lo[0]), (float)(y - cy * g.h[1] - g.lo[1]),
-                      (float)(z - cz * g.h[2] - g.lo[2]), __int_as_float(t));
-  pd[i] = make_double4_32a(x, y, z, (double)t);
-}
-
 struct PushArgs {
   int64_t n;
   double *x, *y, *z, *vx, *vy, *vz, *ax, *ay, *az;
@@ -53,7 +45,7 @@ __global__ void k_push_f_v_r(PushArgs P, double h, double h2) {
   P.x[i] = x;
   P.y[i] = y;
   P.z[i] = z;
-  if (P.refresh) refresh_gather(P.g, i, P.cellpack[i], P.type[i], x, y, z, P.pf, P.pd);
+  if (P.refresh) store_gather(P.g, i, P.cellpack[i], P.type[i], x, y, z, P.pf, P.pd);
 }
 
 __global__ void k_push_f_v(PushArgs P, double h) {
@@ -79,7 +71,7 @@ __global__ void k_first_half(PushArgs P, double h, double h2, double hv) {
   P.vx[i] = __dadd_rn(vx, __dmul_rn(ax, hv));
   P.vy[i] = __dadd_rn(vy, __dmul_rn(ay, hv));
   P.vz[i] = __dadd_rn(vz, __dmul_rn(az, hv));
-  if (P.refresh) refresh_gather(P.g, i, P.cellpack[i], P.type[i], x, y, z, P.pf, P.pd);
+  if (P.refresh) store_gather(P.g, i, P.cellpack[i], P.type[i], x, y, z, P.pf, P.pd);
   if (P.gate) displacement_test(P.gate, P.rref, P.rcap, P.thr2, i, x, y, z);
 }
 
@@ -101,7 +93,7 @@ __global__ void k_push_min(PushArgs P, double h2, double tolF) {
   P.x[i] = x;
   P.y[i] = y;
   P.z[i] = z;
-  if (P.refresh) refresh_gather(P.g, i, P.cellpack[i], P.type[i], x, y, z, P.pf, P.pd);
+  if (P.refresh) store_gather(P.g, i, P.cellpack[i], P.type[i], x, y, z, P.pf, P.pd);
 }
 
 static PushArgs push_args(gbmd_context* c) {
@@ -195,7 +187,7 @@ __global__ void k_host_first_half(PushArgs P, HostState9 H, const int32_t* __res
     P.ax[i] = q[6];
     P.ay[i] = q[7];
     P.az[i] = q[8];
-    if (P.refresh) refresh_gather(P.g, i, P.cellpack[i], P.type[i], x, y, z, P.pf, P.pd);
+    if (P.refresh) store_gather(P.g, i, P.cellpack[i], P.type[i], x, y, z, P.pf, P.pd);
     if (P.gate) displacement_test(P.gate, P.rref, P.rcap, P.thr2, i, x, y, z);
     if (rout.a[0]) {
       const_cast<double*>(rout.a[0])[u] = x;
@@ -253,10 +245,20 @@ struct ThermoArgs {
   double mass[GBMD_MAX_TYPES];
 };
 
+// The sums kept apart, TH_SUMS of them (three fewer where the virial rows are
+// symmetric): virial xx yy zz xy xz yz (yx zx zy), kinetic xx yy zz xy xz yz,
+// momentum, potential energy, mass.  The FP64 pipe is the bound: 20 FP64
+// instructions an atom (it was 38 and 130 more a warp for its sums; 4 M atoms
+// 322 -> 171 us, 108,000 42 -> 14.5).
+constexpr int TH_SUMS = 20;
+
+template <bool SYM>
 __global__ void __launch_bounds__(TH_THREADS) k_thermo_part(ThermoArgs T, double* __restrict__ part) {
-  double s[26];
+  constexpr int NVIR = SYM ? 6 : 9, NV = NVIR + 11;
+  double s[NV];
 #pragma unroll
-  for (int q = 0; q < 26; ++q) s[q] = 0.0;
+  for (int q = 0; q < NV; ++q) s[q] = 0.0;
+  constexpr int at[9] = {0, 4, 8, 1, 2, 5, 3, 6, 7};  // row-major place of each virial sum
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < T.n; i += (int64_t)gridDim.x * blockDim.x) {
     // a type outside [0, ntypes) has no mass: it makes the mass-weighted
     // sums NaN instead of reading past the table
@@ -265,53 +267,58 @@ __global__ void __launch_bounds__(TH_THREADS) k_thermo_part(ThermoArgs T, double
     const double v[3] = {T.vx[i], T.vy[i], T.vz[i]};
     if (T.vir) {
 #pragma unroll
-      for (int q = 0; q < 9; ++q) s[q] += T.vir[9 * i + q];
+      for (int q = 0; q < NVIR; ++q) s[q] += T.vir[9 * i + at[q]];
     }
+    const double p[3] = {v[0] * m, v[1] * m, v[2] * m};
 #pragma unroll
-    for (int a = 0; a < 3; ++a)
+    for (int a = 0; a < 3; ++a) s[NVIR + a] = fma(p[a], v[a], s[NVIR + a]);
+    s[NVIR + 3] = fma(p[0], v[1], s[NVIR + 3]);
+    s[NVIR + 4] = fma(p[0], v[2], s[NVIR + 4]);
+    s[NVIR + 5] = fma(p[1], v[2], s[NVIR + 5]);
 #pragma unroll
-      for (int b = 0; b < 3; ++b) s[9 + 3 * a + b] += v[a] * v[b] * m;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) s[18 + a] += v[a] * m;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) s[21 + a] += v[a] * v[a] * m;
-    if (T.ep) s[24] += T.ep[i];
-    s[25] += m;
+    for (int a = 0; a < 3; ++a) s[NVIR + 6 + a] += p[a];
+    if (T.ep) s[NVIR + 9] += T.ep[i];
+    s[NVIR + 10] += m;
   }
-  __shared__ double red[TH_THREADS / 32][26];
+  __shared__ double red[TH_THREADS / 32][NV];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-#pragma unroll
-  for (int q = 0; q < 26; ++q) {
-    double v = s[q];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if (lane == 0) red[w][q] = v;
-  }
+  __syncwarp();
+  const int q = warp_sum_transposed<NV>(s, lane);
+  if (q >= 0) red[w][q] = s[0];
+  __syncwarp();
   __syncthreads();
-  if (threadIdx.x < 26) {
+  if (threadIdx.x < NV) {
     double v = 0.0;
     for (int k = 0; k < TH_THREADS / 32; ++k) v += red[k][threadIdx.x];
-    part[(size_t)blockIdx.x * 26 + threadIdx.x] = v;
+    // symmetric rows: the virial's lower half is its upper one
+    part[(size_t)blockIdx.x * TH_SUMS + (threadIdx.x < NVIR ? threadIdx.x : threadIdx.x + 9 - NVIR)] = v;
+    if (SYM && threadIdx.x >= 3 && threadIdx.x < 6) part[(size_t)blockIdx.x * TH_SUMS + threadIdx.x + 3] = v;
   }
 }
 
-// one warp per reduced quantity: lane-strided partial sums, then a fixed
-// shuffle tree -- the summation order depends only on the block count
+// one warp per sum: lane-strided partial sums, eight loads in flight, then a
+// fixed shuffle tree -- the summation order depends only on the block count
 __global__ void k_thermo_final(const double* __restrict__ part, int nb, int64_t n, double* __restrict__ out) {
   const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (q >= 27) return;
-  if (q == 26) {
-    if (lane == 0) out[26] = (double)n;
-    return;
-  }
+  __shared__ double sum[TH_SUMS];
   double v = 0.0;
-  for (int b = lane; b < nb; b += 32) v += part[(size_t)b * 26 + q];
+#pragma unroll 8
+  for (int b = lane; b < nb; b += 32) v += part[(size_t)b * TH_SUMS + q];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-  if (lane == 0) {
-    if ((q >= 9 && q < 18) || (q >= 21 && q < 24)) v *= 0.5;
-    out[q] = v;
-  }
+  if (lane == 0) sum[q] = v;
+  __syncthreads();
+  if (threadIdx.x >= 27) return;
+  const int k = threadIdx.x;
+  // virial (row-major), kinetic tensor and its diagonal (halved), momentum, energy, mass
+  const int vir[9] = {0, 3, 4, 6, 1, 5, 7, 8, 2}, kin[9] = {0, 3, 4, 3, 1, 5, 4, 5, 2};
+  double r;
+  if (k < 9) r = sum[vir[k]];
+  else if (k < 18) r = 0.5 * sum[9 + kin[k - 9]];
+  else if (k < 21) r = sum[15 + k - 18];
+  else if (k < 24) r = 0.5 * sum[9 + k - 21];
+  else r = k == 24 ? sum[18] : (k == 25 ? sum[19] : (double)n);
+  out[k] = r;
 }
 
 // The same two reduction kernels on caller-provided device arrays, with a
@@ -328,8 +335,8 @@ void launch_thermo_raw(int64_t n, const double* vx, const double* vy, const doub
   T.ntypes = ntypes;
   for (int t = 0; t < GBMD_MAX_TYPES; ++t) T.mass[t] = t < ntypes ? mass[t] : 1.0;
   const int nb = thermo_blocks(n);
-  k_thermo_part<<<nb, TH_THREADS, 0, s>>>(T, part);
-  k_thermo_final<<<1, 27 * 32, 0, s>>>(part, nb, n, out);
+  k_thermo_part<false><<<nb, TH_THREADS, 0, s>>>(T, part);  // any caller's virial
+  k_thermo_final<<<1, TH_SUMS * 32, 0, s>>>(part, nb, n, out);
 }
 
 void launch_thermo(gbmd_context* c, bool with_virial) {
@@ -342,8 +349,11 @@ void launch_thermo(gbmd_context* c, bool with_virial) {
   T.ntypes = c->ntypes > 0 ? c->ntypes : GBMD_MAX_TYPES;
   for (int t = 0; t < GBMD_MAX_TYPES; ++t) T.mass[t] = t < c->ntypes ? c->mass[t] : 1.0;
   const int nb = thermo_blocks(c->n);
-  k_thermo_part<<<nb, TH_THREADS, 0, c->stream>>>(T, c->d_part);
-  k_thermo_final<<<1, 27 * 32, 0, c->stream>>>(c->d_part, nb, c->n, c->d_thermo);
+  // the LJ and eam_alloy kernels write symmetric virial rows
+  const bool sym = c->pot != GBMD_POT_EAM_JOHNSON && c->pot != GBMD_POT_EAM_SUTTON_CHEN;
+  if (sym) k_thermo_part<true><<<nb, TH_THREADS, 0, c->stream>>>(T, c->d_part);
+  else k_thermo_part<false><<<nb, TH_THREADS, 0, c->stream>>>(T, c->d_part);
+  k_thermo_final<<<1, TH_SUMS * 32, 0, c->stream>>>(c->d_part, nb, c->n, c->d_thermo);
 }
 
 }  // namespace gbmd

@@ -14,6 +14,7 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+#include <cstring>
 #include <string>
 #include <vector>
 
@@ -415,21 +416,22 @@ int thermo_blocks(int64_t n);
     if (e_ != cudaSuccess) return gbmd::check_cuda((c), e_, #call); \
   } while (0)
 
-// particle_displ_over for one atom at its new position: raise the gate when
-// it moved more than sqrt(thr2) since the last rebuild (|dr|^2 summed x, y, z
-// without contraction, as the standalone test kernel does).
-__device__ __forceinline__ void displacement_test(int* gate, const double* __restrict__ rref, int64_t cap,
-                                                  double thr2, int64_t i, double x, double y, double z) {
-  const double dx = __dsub_rn(x, rref[i]), dy = __dsub_rn(y, rref[cap + i]), dz = __dsub_rn(z, rref[2 * cap + i]);
-  const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
-  if (d2 > thr2) *gate = 1;
-}
-
 __device__ __forceinline__ void kahan_add(float& s, float& comp, float v) {
   const float y = v - comp;
   const float t = s + y;
   comp = (t - s) - y;
   s = t;
+}
+
+// A double's bits as an integer of the same order.
+__device__ __forceinline__ long long order_key(double v) {
+  const long long b = __double_as_longlong(v);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
+}
+inline long long order_key_host(double v) {
+  long long b;
+  std::memcpy(&b, &v, sizeof(b));
+  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
 }
 
 // (float)x in integer instructions, rounded to nearest even.
@@ -447,6 +449,44 @@ __device__ __forceinline__ float narrow(double x) {
 __device__ __forceinline__ double small_double(int c) {
   const int e = 31 - __clz(c);
   return c == 0 ? 0.0 : __hiloint2double(((1023 + e) << 20) | ((c << (20 - e)) & 0xfffff), 0);
+}
+
+// (double)x in integer instructions (exact; the FP64 pipe, where the
+// conversion runs, takes 16 SM cycles an instruction).
+__device__ __forceinline__ double widen(float x) {
+  const uint32_t b = __float_as_uint(x), m = b & 0x7fffffffu;
+  if (m - 0x00800000u >= 0x7f000000u) return (double)x;  // zero, subnormal, infinity, NaN
+  return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + 0x38000000u)), (int)(b << 29));
+}
+
+// One axis of an atom's home-cell-relative FP32 position, float(x - c h - lo).
+__device__ __forceinline__ float cell_local(double x, int c, double h, double lo) {
+  double u = fma(-small_double(c), h, x);
+  if (__double_as_longlong(lo) != 0) u -= lo;
+  return narrow(u);
+}
+
+// The FP32 and FP64 gather copies of atom i (cp: its home cell, t: its type).
+// Conversions and small integers in integer instructions: an FP64 one takes
+// 16 SM cycles a warp, and these were two thirds of the FP64 work per atom.
+__device__ __forceinline__ void store_gather(const gbmd::Grid& g, int64_t i, int cp, int t, double x, double y,
+                                             double z, float4* pf, double4_32a* pd) {
+  pf[i] = make_float4(cell_local(x, cp & 1023, g.h[0], g.lo[0]), cell_local(y, (cp >> 10) & 1023, g.h[1], g.lo[1]),
+                      cell_local(z, cp >> 20, g.h[2], g.lo[2]), __int_as_float(t));
+  pd[i] = make_double4_32a(x, y, z, small_double(t));
+}
+
+// particle_displ_over for one atom at its new position: raise the gate when
+// it moved more than sqrt(thr2) since the last rebuild (|dr|^2 summed x, y, z
+// without contraction, as the standalone test kernel does).  FP32 tells the
+// atoms that clearly have not.
+__device__ __forceinline__ void displacement_test(int* gate, const double* __restrict__ rref, int64_t cap,
+                                                  double thr2, int64_t i, double x, double y, double z) {
+  const double dx = __dsub_rn(x, rref[i]), dy = __dsub_rn(y, rref[cap + i]), dz = __dsub_rn(z, rref[2 * cap + i]);
+  const float fx = narrow(dx), fy = narrow(dy), fz = narrow(dz);
+  if (fmaf(fx, fx, fmaf(fy, fy, fz * fz)) < narrow(thr2) * (1.0f - 0x1p-20f)) return;
+  const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+  if (d2 > thr2) *gate = 1;
 }
 
 // Sums of NV quantities over a warp: each of the five steps hands half of the
@@ -538,12 +578,4 @@ inline int log2_of(int p2) {
 // it as the (p / T)-th of its V = W / T adjacent words, T = 2^tsh.
 __host__ __device__ __forceinline__ int list_word(int p, int wsh, int tsh) {
   return ((p & ((1 << tsh) - 1)) << (wsh - tsh)) | (p >> tsh);
-}
-
-// (double)x in integer instructions (exact; the FP64 pipe, where the
-// conversion runs, takes 16 SM cycles an instruction).
-__device__ __forceinline__ double widen(float x) {
-  const uint32_t b = __float_as_uint(x), m = b & 0x7fffffffu;
-  if (m - 0x00800000u >= 0x7f000000u) return (double)x;  // zero, subnormal, infinity, NaN
-  return __hiloint2double((int)((b & 0x80000000u) | ((m >> 3) + 0x38000000u)), (int)(b << 29));
 }

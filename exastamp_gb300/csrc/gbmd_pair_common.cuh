@@ -174,12 +174,7 @@ __device__ __forceinline__ void atom_epilogue(const PairArgs& A, int64_t i, int 
       A.yo[i] = y;
       A.zo[i] = z;
       if (A.gate) displacement_test(A.gate, A.rref, A.rcap, A.thr2, i, x, y, z);
-      int cx, cy, cz;
-      unpack_cell(A.cellpack[i], cx, cy, cz);
-      A.posf_o[i] = make_float4((float)(x - (double)cx * A.g.h[0] - A.g.lo[0]),
-                                (float)(y - (double)cy * A.g.h[1] - A.g.lo[1]),
-                                (float)(z - (double)cz * A.g.h[2] - A.g.lo[2]), __int_as_float(t));
-      A.posd_o[i] = make_double4_32a(x, y, z, (double)t);
+      store_gather(A.g, i, A.cellpack[i], t, x, y, z, A.posf_o, A.posd_o);
     }
     A.vxo[i] = vx;
     A.vyo[i] = vy;

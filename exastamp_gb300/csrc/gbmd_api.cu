@@ -314,10 +314,15 @@ static int staged_copies(gbmd_context* c, double* const* host, int count, bool t
   return GBMD_OK;
 }
 
+__global__ void k_copy_planes(int64_t n, const double* __restrict__ from, double* __restrict__ to, int64_t cap) {
+  const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  if (p >= n) return;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) to[d * cap + p] = from[d * cap + p];
+}
+
 static int copy_rref(gbmd_context* c) {
-  for (int d = 0; d < 3; ++d)
-    GBMD_CUDA(c, cudaMemcpyAsync(c->rref + d * c->cap, c->rbuf[c->cur] + d * c->cap, sizeof(double) * c->n,
-                                 cudaMemcpyDeviceToDevice, c->stream));
+  if (c->n) k_copy_planes<<<nblk(c->n, 256), 256, 0, c->stream>>>(c->n, c->rbuf[c->cur], c->rref, c->cap);
   return GBMD_OK;
 }
 

@@ -57,6 +57,7 @@ __global__ void k_wrap_bin(int64_t n, double* __restrict__ x, double* __restrict
                            double* __restrict__ z, BoxArgs b, int32_t* __restrict__ cell_of,
                            int32_t* __restrict__ cell_count, int* __restrict__ err, const int* __restrict__ gate) {
   if (gate && !*gate) return;
+  if (!gate && blockIdx.x == 0 && threadIdx.x == 0) err[ERRW_MAXNB] = 0;  // of the list this chain builds
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
   double* r[3] = {x, y, z};
   int c[3];
@@ -182,7 +183,35 @@ __global__ void k_scan_add(int32_t* __restrict__ out, int64_t n, const int32_t* 
   }
 }
 
+// The same in one block of 1,024 threads: for a few thousand cells the three
+// launches above are all latency (1,331 cells: 12 us).
+constexpr int SCAN_SMALL = 1024 * 16;
+
+__global__ void __launch_bounds__(1024) k_scan_small(const int32_t* __restrict__ in, int32_t* __restrict__ out, int n,
+                                                     const int* __restrict__ gate) {
+  if (gate && !*gate) return;
+  __shared__ int smem[33];
+  const int base = (int)threadIdx.x * 16;
+  int it[16], s = 0;
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    it[k] = base + k < n ? in[base + k] : 0;
+    s += it[k];
+  }
+  int total;
+  int off = block_exclusive(s, smem, total);
+#pragma unroll
+  for (int k = 0; k < 16; ++k) {
+    if (base + k <= n) out[base + k] = off;
+    off += it[k];
+  }
+}
+
 static int scan(gbmd_context* c, const int32_t* in, int32_t* out, int64_t n, const int* gate) {
+  if (n + 1 <= SCAN_SMALL) {
+    k_scan_small<<<1, 1024, 0, c->stream>>>(in, out, (int)n, gate);
+    return GBMD_OK;
+  }
   const int64_t nb = (n + 1 + SCAN_B - 1) / SCAN_B;
   if (c->scan_cap < nb) {
     if (c->scan_tmp) cudaFree(c->scan_tmp);
@@ -205,8 +234,10 @@ __global__ void k_scatter(int64_t n, const int32_t* __restrict__ cell_of, const 
     // by k_cell_rank, so any slot assignment will do
     const unsigned peers = __match_any_sync(__activemask(), cl);
     const int leader = __ffs(peers) - 1;
+    // counting the cell's atoms down: all counts are zero again at the end,
+    // ready for the next chain
     int base = 0;
-    if (lane == leader) base = atomicAdd(&fill[cl], __popc(peers));
+    if (lane == leader) base = atomicSub(&fill[cl], __popc(peers)) - __popc(peers);
     base = __shfl_sync(peers, base, leader);
     order[cstart[cl] + base + __popc(peers & ((1u << lane) - 1u))] = (int32_t)i;
   }
@@ -317,11 +348,6 @@ __global__ void k_copy_back(int64_t n, GatherArgs g, const int* __restrict__ gat
   const_cast<int32_t*>(g.u0)[p] = g.u1[p];
   const_cast<double*>(g.ep0)[p] = g.ep1[p];
   }
-}
-
-__global__ void k_fill_gated(int32_t* __restrict__ p, int64_t n, const int* __restrict__ gate) {
-  if (!*gate) return;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) p[i] = 0;
 }
 
 __global__ void k_posf(int64_t n, const double* __restrict__ x, const double* __restrict__ y,
@@ -740,7 +766,6 @@ static int build_list(gbmd_context* c, const int* gate) {
     c->nbr_cap = need;
   }
   c->npad = npad;
-  if (!gate) GBMD_CUDA(c, cudaMemsetAsync(c->d_err + ERRW_MAXNB, 0, sizeof(int), c->stream));
   BuildArgs A;
   A.ncells = c->grid.ncells;
   A.pf = c->POSF();
@@ -816,6 +841,7 @@ static int rebuild_chain(gbmd_context* c, bool check_capacity, const int* gate) 
       if (c->cell_fill) cudaFree(c->cell_fill);
       GBMD_CUDA(c, cudaMalloc(&c->cell_start, sizeof(int32_t) * (g.ncells + 1)));
       GBMD_CUDA(c, cudaMalloc(&c->cell_fill, sizeof(int32_t) * (g.ncells + 1)));
+      GBMD_CUDA(c, cudaMemsetAsync(c->cell_fill, 0, sizeof(int32_t) * (g.ncells + 1), c->stream));
       c->cells_cap = g.ncells + 1;
     }
     c->grid_valid = true;
@@ -833,17 +859,11 @@ static int rebuild_chain(gbmd_context* c, bool check_capacity, const int* gate) 
   }
   const int64_t n = c->n;
   cudaStream_t s = c->stream;
-  auto zero_fill = [&]() -> int {
-    if (gate) k_fill_gated<<<chain_blocks(c, g.ncells + 1, 256, gate, 8), 256, 0, s>>>(c->cell_fill, g.ncells + 1, gate);
-    else GBMD_CUDA(c, cudaMemsetAsync(c->cell_fill, 0, sizeof(int32_t) * (g.ncells + 1), s));
-    return GBMD_OK;
-  };
-  int rc = zero_fill();
-  if (rc) return rc;
+  // cell_fill is zero here: cleared when allocated, counted down by k_scatter
+  int rc;
   k_wrap_bin<<<chain_blocks(c, n, 256, gate, 8), 256, 0, s>>>(n, c->X(), c->Y(), c->Z(), b, c->cell_of, c->cell_fill,
                                                             c->d_err, gate);
   if ((rc = scan(c, c->cell_fill, c->cell_start, g.ncells, gate))) return rc;
-  if ((rc = zero_fill())) return rc;
   k_scatter<<<chain_blocks(c, n, 256, gate, 8), 256, 0, s>>>(n, c->cell_of, c->cell_start, c->cell_fill, c->order,
                                                            gate);
   k_cell_rank<<<chain_blocks(c, g.ncells * 32, 256, gate, 8), 256, 0, s>>>(g.ncells, c->cell_start, c->order, c->ID(),

@@ -51,6 +51,8 @@ static void free_atoms(gbmd_context* c) {
   cudaFree(c->ep); cudaFree(c->vir); cudaFree(c->cellpack); cudaFree(c->cell_of);
   cudaFree(c->order); cudaFree(c->src); cudaFree(c->fpf); cudaFree(c->fpd); cudaFree(c->epf);
   cudaFree(c->pfp);
+  cudaFree(c->f0);
+  c->f0 = nullptr;
   cudaFree(c->stage); cudaFree(c->rref); cudaFree(c->nnb); cudaFree(c->d_part); cudaFree(c->stage_r);
   cudaFree(c->h3acc);
   cudaFree(c->epd);
@@ -92,6 +94,7 @@ int ensure_atom_capacity(gbmd_context* c, int64_t n) {
   GBMD_CUDA(c, cudaMalloc(&c->fpf, sizeof(float) * cap));
   GBMD_CUDA(c, cudaMalloc(&c->epf, sizeof(float) * cap));
   GBMD_CUDA(c, cudaMalloc(&c->pfp, sizeof(float4) * cap));
+  GBMD_CUDA(c, cudaMalloc(&c->f0, sizeof(float4) * cap));
   GBMD_CUDA(c, cudaMalloc(&c->fpd, sizeof(double) * cap));
   GBMD_CUDA(c, cudaMalloc(&c->stage, sizeof(double) * 9 * cap));
   GBMD_CUDA(c, cudaMalloc(&c->rref, d3));
@@ -523,7 +526,7 @@ int gbmd_destroy(gbmd_context* c) {
   if (c->stream) cudaStreamSynchronize(c->stream);
   drop_graph(c);
   free_atoms(c);
-  cudaFree(c->cell_start); cudaFree(c->cell_fill); cudaFree(c->scan_tmp); cudaFree(c->nbr); cudaFree(c->nbr_out);
+  cudaFree(c->cell_start); cudaFree(c->cell_fill); cudaFree(c->scan_tmp); cudaFree(c->nbr); cudaFree(c->nbr_out); cudaFree(c->bpair);
   cudaFree(c->eam_d); cudaFree(c->eam_f); cudaFree(c->lj_tab_d);
   cudaFree(c->d_err); cudaFree(c->d_thermo); cudaFree(c->d_rows); cudaFree(c->adj_scratch);
   if (c->h_err) cudaFreeHost(c->h_err);
@@ -894,7 +897,7 @@ int gbmd_set_eam_alloy(gbmd_context* c, int nel, int nrho, double drho, int nr, 
   // on a 32-byte boundary so a knot's two float4 share one sector
   const size_t nf0 = nel * kp + nel * kr + npairs * kr + nel * kr;
   const size_t fz_off = (nf0 + 1) & ~(size_t)1;
-  const size_t nf = nel == 1 ? fz_off + 2 * kr : nf0;
+  const size_t nf = nel == 1 ? fz_off + 4 * kr : nf0;
   cudaFree(c->eam_d);
   cudaFree(c->eam_f);
   c->eam_d = nullptr;
@@ -929,6 +932,8 @@ int gbmd_set_eam_alloy(gbmd_context* c, int nel, int nrho, double drho, int nr, 
     for (size_t m = 0; m < kr; ++m) {
       hf[fz_off + 2 * m] = hf[nel * kp + nel * kr + npairs * kr + m];  // rho' coefficients
       hf[fz_off + 2 * m + 1] = hf[nel * kp + nel * kr + m];           // z2r coefficients
+      hf[fz_off + 2 * (kr + m)] = hf[nel * kp + m];                   // rho coefficients
+      hf[fz_off + 2 * (kr + m) + 1] = hf[nel * kp + nel * kr + m];
     }
   GBMD_CUDA(c, cudaMemcpy(c->eam_d, hd.data(), sizeof(double) * nd, cudaMemcpyHostToDevice));
   GBMD_CUDA(c, cudaMemcpy(c->eam_f, hf.data(), sizeof(float4) * nf, cudaMemcpyHostToDevice));
@@ -952,6 +957,7 @@ int gbmd_set_eam_alloy(gbmd_context* c, int nel, int nrho, double drho, int nr, 
   E.z2r4 = E.rhor4 + nel * kr;
   E.rhod4 = E.z2r4 + npairs * kr;
   E.fz8 = nel == 1 ? c->eam_f + fz_off : nullptr;
+  E.rz8 = nel == 1 ? E.fz8 + 2 * kr : nullptr;
   E.rdrf = (float)E.rdr;
   E.rdrhof = (float)E.rdrho;
   E.rhomaxf = (float)E.rhomax;
@@ -1049,6 +1055,10 @@ int gbmd_set_precision(gbmd_context* c, int precision) {
     c->precision = precision;
     c->energy_step = -1, c->forces_valid_step = c->rho_valid_step = -1;
     drop_graph(c);
+    if (c->list_valid && c->n) {
+      cudaSetDevice(c->device);
+      ensure_bpair(c);
+    }
   }
   return GBMD_OK;
 }

@@ -401,6 +401,8 @@ PairArgs make_args(gbmd_context* c, const ForceFlags& f) {
   A.vxo = f.v_out ? f.v_out : A.vx;
   A.vyo = f.v_out ? f.v_out + c->cap : A.vy;
   A.vzo = f.v_out ? f.v_out + 2 * c->cap : A.vz;
+  A.f0 = c->f0;
+  A.bpair = c->bpair;
   A.ep = c->ep;
   A.ep_emb = c->epd;
   A.vir = c->vir;

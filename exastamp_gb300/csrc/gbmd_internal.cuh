@@ -75,6 +75,7 @@ struct EamDev {
   const float4* z2r4;  // npairs x (nr+1)      z2r * conv_z2r
   const float4* rhod4; // nel x (nr+1)         rho' coefficients (3c3, 2c4, c5) / dr
   const float4* fz8;   // one element: (nr+1) x {rhod4, z2r4}, 32-byte aligned knots
+  const float4* rz8;   // one element: (nr+1) x {rhor4, z2r4}, 32-byte aligned knots
   float rdrf, rdrhof, rhomaxf, rc2f, rc2lo, rc2hi;
 };
 
@@ -171,6 +172,10 @@ struct gbmd_context {
   int32_t* src = nullptr;                 // scratch: new position -> old position
   float* fpf = nullptr;                   // EAM F'(rho) FP32 (mixed)
   float4* pfp = nullptr;                  // single-element EAM: FP32 position with F'(rho) in w (mixed)
+  float4* f0 = nullptr;                   // mixed one-element EAM without energies: sum phi' u from the density pass
+  float* bpair = nullptr;                 // and rho'(r)/r per list entry, in the list's layout
+  int64_t bpair_cap = 0;
+  bool rho_bonds = false;                 // the last density pass left f0 and bpair
   double* adj_scratch = nullptr;          // LJ adjoint: targets + per-atom terms (lazily allocated)
   int64_t adj_cap = 0;
   double* fpd = nullptr;                  // EAM rho_dEmb FP64
@@ -327,6 +332,8 @@ int sync_error_word(gbmd_context* c);  // copies device error word, returns stat
 constexpr int64_t PACK_DOUBLES = 65536;
 
 // neighbours (gbmd_neighbors.cu)
+// one-element EAM: room for one float per list entry (bpair), if it can be had
+void ensure_bpair(gbmd_context* c);
 int grid_dims(const double lo[3], const double hi[3], double R, int nc[3]);
 // gate: device word; non-null makes every kernel of the chain return at once
 // while it holds 0, and keeps the buffer indices unchanged (see gbmd_neighbors.cu)

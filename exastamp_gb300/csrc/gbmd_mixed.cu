@@ -118,6 +118,7 @@ template <int N>
 struct RowPart {
   uint32_t e[N];
   bool ok[N];
+  size_t at;  // the first entry's word, from the lane's first
 };
 
 template <int T, int V, class Body>
@@ -128,6 +129,7 @@ __device__ __forceinline__ void for_rows(const ListRows<T, V>& L, Body body) {
   for (int r = 0; r < L.nfull; ++r) {
     if (r + 1 < L.nrow) L.load(r + 1, nxt);
     RowPart<V> P;
+    P.at = (size_t)r * L.stride;
 #pragma unroll
     for (int q = 0; q < V; ++q) {
       P.e[q] = ent[q];
@@ -141,6 +143,7 @@ __device__ __forceinline__ void for_rows(const ListRows<T, V>& L, Body body) {
   for (int h = 0; h < V; h += H) {
     if (L.rem > h * T) {
       RowPart<H> P;
+      P.at = (size_t)L.nfull * L.stride + h;
 #pragma unroll
       for (int q = 0; q < H; ++q) {
         P.ok[q] = L.in_tail(h + q);
@@ -373,7 +376,8 @@ __device__ __forceinline__ void atom_finish(const PairArgs& A, int64_t i, const 
 // row touches 32 sectors per store, nine times.
 template <int T, bool EV>
 __device__ __forceinline__ void block_epilogue(const PairArgs& A, int64_t i0, const PairSums& S,
-                                               const float* __restrict__ epf) {
+                                               const float* __restrict__ epf,
+                                               const float4* __restrict__ f0 = nullptr) {
   constexpr int NV = EV ? 10 : 3;
   constexpr bool SHARED = T > 1 || EV;
   __shared__ float sums[SHARED ? NV : 1][SHARED ? 256 / T : 1];
@@ -408,6 +412,12 @@ __device__ __forceinline__ void block_epilogue(const PairArgs& A, int64_t i0, co
   }
   const int64_t i = i0 + threadIdx.x;
   if (i >= A.n) return;
+  if (f0) {
+    const float4 f = f0[i];
+    R.f[0] += f.x;
+    R.f[1] += f.y;
+    R.f[2] += f.z;
+  }
   const int ti = __float_as_int(A.posf[i].w);
   const float im = A.inv_massf[ti];
   atom_epilogue<true>(A, i, ti, 0., 0., 0., R.f[0] * im, R.f[1] * im, R.f[2] * im,
@@ -534,7 +544,7 @@ __device__ __forceinline__ float eam_rho_atom(const PairArgs& A, const EamDev& E
 // writes pfp[i] = (position, F'(rho_i)) so the force pass gathers both in one
 // 16 B load.
 template <bool EV, bool SINGLE>
-__device__ __forceinline__ void eam_embed(const PairArgs& A, const EamDev& E, int64_t i, float R,
+__device__ __forceinline__ float eam_embed(const PairArgs& A, const EamDev& E, int64_t i, float R,
                                           float* __restrict__ fpf, float* __restrict__ epf,
                                           float4* __restrict__ pfp) {
   const float4 pi = A.posf[i];
@@ -552,6 +562,7 @@ __device__ __forceinline__ void eam_embed(const PairArgs& A, const EamDev& E, in
     if (R > E.rhomaxf) phi = fmaf(fp, R - E.rhomaxf, phi);
     epf[i] = phi;
   }
+  return fp;
 }
 
 template <int T, int V, bool EV, bool SINGLE, bool PIECE>
@@ -724,6 +735,219 @@ __global__ void __launch_bounds__(256) k_eam_force_staged(PairArgs A, EamDev E, 
     const PairSums S = ok ? eam_force_atom<1, 4, EV, true>(A, E, fpf, i, 0, true, StagedFetch{staged_pos, rows})
                           : eam_force_atom<1, 4, EV, true>(A, E, fpf, i, 0, true, GlobalFetch{pfp});
     atom_finish<EV>(A, i, S, EV ? epf[i] : 0.f);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// One-element eam_alloy forces without energies.  The force on i is
+//   sum_j phi'(r) u + sum_j (F'_i + F'_j) rho'(r) u.
+// The density pass has every pair's knot at hand, so it forms the first sum
+// (f0) too and leaves rho'(r) / r for each list entry in `bpair`, laid out as
+// the list.  The force pass is left with the second: per entry 4 + 4 streamed
+// bytes, one 16 B gather and some 25 instructions, where the pair terms' own
+// knots (32 B a lane, 28 lines a warp) made it the larger of the two.  The
+// streamed floats go through HBM, which both passes left at a fifth of its
+// rate; they bypass L1, which serves the gathers.
+// 4 M-atom Cu, density + force: 529 + 768 -> 796 + 411 us (72 registers in the
+// density pass; 64: 810, 56: 972).
+// (Two elements: the entry's two rho' differ, and the sum over F'_i has to be
+// formed in the density pass as well; that was slower than the plain passes,
+// 2 M atoms 933 against 874 us.)
+// ---------------------------------------------------------------------------
+struct BondSums {
+  float rho, f[3];
+};
+
+template <int T, class Fetch>
+__device__ __forceinline__ BondSums eam_rho_bonds_atom(const PairArgs& A, const EamDev& E, int64_t i, int lane,
+                                                       bool live, const Fetch& fetch) {
+  const int nn = live ? min(A.nnb[i], A.maxnb) : 0;
+  const float4 pi = live ? A.posf[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const int nr = E.nr;
+  const float rdr = E.rdrf;
+  float s[4], c[4];  // rho, sum phi'/r d
+#pragma unroll
+  for (int k = 0; k < 4; ++k) s[k] = c[k] = 0.f;
+  const ListRows<T, 4> L(A.nbr, i, lane, A.stride, nn);
+  float* const bonds = A.bpair + (L.p - A.nbr);
+  for_rows(L, [&](const auto& R) {
+    constexpr int N = sizeof(R.e) / sizeof(R.e[0]);
+    float4 pj[N];
+#pragma unroll
+    for (int q = 0; q < N; ++q) pj[q] = fetch(R.e[q], R.e[q] & GBMD_IDX_MASK);
+    float p[4], b[N];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) p[k] = 0.f;
+#pragma unroll
+    for (int q = 0; q < N; ++q) {
+      const GeomF G = geom_f(R.e[q], pj[q], pi, A.g);
+      bool in = G.d2 < E.rc2lo;
+      if (!in && G.d2 <= E.rc2hi && R.ok[q])
+        in = exact_inside(A.posd, i, R.e[q] & GBMD_IDX_MASK, R.e[q] >> GBMD_IDX_BITS, A.cellpack[i], A.g, E.rcut2,
+                          0.0);
+      const float rs = rsqrtf(G.d2);
+      const float rd = G.d2 * rs;
+      float t;
+      const int m = knot_f(rd, rdr, nr, t);
+      float4 cr, cz;
+      ldg_knot_pair(&E.rz8[2 * m], cr, cz);
+      const float t1 = fmaf(cz.x, t, cz.y);
+      const float z2 = fmaf(fmaf(t1, t, cz.z), t, cz.w);
+      const float z2d = fmaf(fmaf(cz.x, t, t1 + t1), t, cz.z);
+      const float phi = z2 * rs;
+      const float phip = fmaf(z2d * rdr, rs, -phi * rs);
+      const float fa = in ? phip * rs : 0.f;
+      b[q] = in ? spline_der(cr, t, rdr) * rs : 0.f;
+      p[0] += in ? spline_val(cr, t) : 0.f;
+      p[1] = fmaf(G.dx, fa, p[1]);
+      p[2] = fmaf(G.dy, fa, p[2]);
+      p[3] = fmaf(G.dz, fa, p[3]);
+    }
+    if constexpr (N == 4)
+      asm volatile("st.global.L1::no_allocate.v4.f32 [%0], {%1,%2,%3,%4};" ::"l"(bonds + R.at), "f"(b[0]), "f"(b[1]),
+                   "f"(b[2]), "f"(b[3])
+                   : "memory");
+    else
+      *reinterpret_cast<float2*>(bonds + R.at) = make_float2(b[0], b[1]);
+#pragma unroll
+    for (int k = 0; k < 4; ++k) kahan_add(s[k], c[k], p[k]);
+  });
+#pragma unroll
+  for (int k = 0; k < 4; ++k) group_reduce_kahan<T>(s[k], c[k]);
+  return BondSums{s[0] - c[0], {s[1] - c[1], s[2] - c[2], s[3] - c[3]}};
+}
+
+template <int T, bool PIECE>
+__global__ void __launch_bounds__(128, 7) k_eam_rho_bonds(const __grid_constant__ PairArgs A,
+                                                          const __grid_constant__ EamDev E,
+                                                          float* __restrict__ fpf, float4* __restrict__ pfp) {
+  const int64_t gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  int64_t i = PIECE ? A.i0 + gt / T : gt / T;
+  BondSums S = eam_rho_bonds_atom<T>(A, E, i, (int)(gt % T), i < A.n, GlobalFetch{A.posf});
+  if (T > 1) {
+    // the embedding of the block's atoms on its first blockDim / T threads
+    __shared__ float sums[4][T > 1 ? 128 / T : 1];
+    const int nat = (int)blockDim.x / T;
+    if (threadIdx.x % T == 0) {
+      sums[0][threadIdx.x / T] = S.rho;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) sums[1 + k][threadIdx.x / T] = S.f[k];
+    }
+    __syncwarp();
+    __syncthreads();
+    if ((int)threadIdx.x >= nat) return;
+    S.rho = sums[0][threadIdx.x];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) S.f[k] = sums[1 + k][threadIdx.x];
+    i = (PIECE ? A.i0 : 0) + blockIdx.x * (int64_t)nat + threadIdx.x;
+  }
+  if (i >= A.n) return;
+  eam_embed<false, true>(A, E, i, S.rho, fpf, nullptr, pfp);
+  A.f0[i] = make_float4(S.f[0], S.f[1], S.f[2], 0.f);
+}
+
+template <int T, class Fetch>
+__device__ __forceinline__ PairSums eam_force_bonds_atom(const PairArgs& A, const float* __restrict__ fpf, int64_t i,
+                                                         int lane, bool live, const Fetch& fetch) {
+  const int nn = live ? min(A.nnb[i], A.maxnb) : 0;
+  const float4 pi = live ? A.posf[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const float fpi = live ? fpf[i] : 0.f;
+  float s[3] = {0.f, 0.f, 0.f}, c[3] = {0.f, 0.f, 0.f};
+  const ListRows<T, 4> L(A.nbr, i, lane, A.stride, nn);
+  const float* const bonds = A.bpair + (L.p - A.nbr);
+  auto load = [&](int r, uint32_t (&e)[4], float (&b)[4]) {
+    L.load(r, e);
+    asm("ld.global.nc.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];"
+        : "=f"(b[0]), "=f"(b[1]), "=f"(b[2]), "=f"(b[3])
+        : "l"(bonds + (size_t)r * L.stride));
+  };
+  uint32_t ent[4], nxt[4];
+  float b[4], nb[4];
+  if (L.nrow > 0) load(0, ent, b);
+  for (int r = 0; r < L.nrow; ++r) {
+    if (r + 1 < L.nrow) load(r + 1, nxt, nb);
+    if (r >= L.nfull) {  // the last, partial row
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (!L.in_tail(q)) {
+          ent[q] = L.standin;
+          b[q] = 0.f;
+        }
+    }
+    float4 pj[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) pj[q] = fetch(ent[q], ent[q] & GBMD_IDX_MASK);
+    float p[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float w = (fpi + pj[q].w) * b[q];
+      p[0] = fmaf(fmaf(unit_of((ent[q] >> 26) & 3u), A.g.hf[0], pj[q].x - pi.x), w, p[0]);
+      p[1] = fmaf(fmaf(unit_of((ent[q] >> 28) & 3u), A.g.hf[1], pj[q].y - pi.y), w, p[1]);
+      p[2] = fmaf(fmaf(unit_of(ent[q] >> 30), A.g.hf[2], pj[q].z - pi.z), w, p[2]);
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) kahan_add(s[k], c[k], p[k]);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      ent[q] = nxt[q];
+      b[q] = nb[q];
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < 3; ++k) group_reduce_kahan<T>(s[k], c[k]);
+  PairSums S;
+  S.f[0] = s[0] - c[0];
+  S.f[1] = s[1] - c[1];
+  S.f[2] = s[2] - c[2];
+  S.e = 0.f;
+  return S;
+}
+
+template <int T, bool PIECE>
+__global__ void __launch_bounds__(256, 4) k_eam_force_bonds(const __grid_constant__ PairArgs A,
+                                                            const float* __restrict__ fpf,
+                                                            const float4* __restrict__ pfp) {
+  const int64_t gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+  const int64_t i = PIECE ? A.i0 + gt / T : gt / T;
+  const PairSums S = eam_force_bonds_atom<T>(A, fpf, i, (int)(gt % T), i < A.n, GlobalFetch{pfp});
+  block_epilogue<T, false>(A, (PIECE ? A.i0 : 0) + blockIdx.x * (int64_t)(blockDim.x / T), S, nullptr, A.f0);
+}
+
+// The same with the neighbour positions from the block's staged cells.
+__global__ void __launch_bounds__(256) k_eam_rho_bonds_staged(const __grid_constant__ PairArgs A,
+                                                              const __grid_constant__ EamDev E,
+                                                              float* __restrict__ fpf, float4* __restrict__ pfp,
+                                                              const int32_t* __restrict__ cstart, int K, int cap) {
+  __shared__ int4 rows[16];
+  __shared__ int sh[56];
+  extern __shared__ float4 staged_pos[];
+  int64_t a0, a1;
+  const bool ok = stage_cells(A.g, cstart, A.posf, K, cap, staged_pos, rows, sh, a0, a1);
+  for (int64_t i = a0 + threadIdx.x; i < a1; i += blockDim.x) {
+    const BondSums S = ok ? eam_rho_bonds_atom<1>(A, E, i, 0, true, StagedFetch{staged_pos, rows})
+                          : eam_rho_bonds_atom<1>(A, E, i, 0, true, GlobalFetch{A.posf});
+    eam_embed<false, true>(A, E, i, S.rho, fpf, nullptr, pfp);
+    A.f0[i] = make_float4(S.f[0], S.f[1], S.f[2], 0.f);
+  }
+}
+
+__global__ void __launch_bounds__(256) k_eam_force_bonds_staged(const __grid_constant__ PairArgs A,
+                                                                const float* __restrict__ fpf,
+                                                                const float4* __restrict__ pfp,
+                                                                const int32_t* __restrict__ cstart, int K, int cap) {
+  __shared__ int4 rows[16];
+  __shared__ int sh[56];
+  extern __shared__ float4 staged_pos[];
+  int64_t a0, a1;
+  const bool ok = stage_cells(A.g, cstart, pfp, K, cap, staged_pos, rows, sh, a0, a1);
+  for (int64_t i = a0 + threadIdx.x; i < a1; i += blockDim.x) {
+    PairSums S = ok ? eam_force_bonds_atom<1>(A, fpf, i, 0, true, StagedFetch{staged_pos, rows})
+                    : eam_force_bonds_atom<1>(A, fpf, i, 0, true, GlobalFetch{pfp});
+    const float4 f = A.f0[i];
+    S.f[0] += f.x;
+    S.f[1] += f.y;
+    S.f[2] += f.z;
+    atom_finish<false>(A, i, S, 0.f);
   }
 }
 
@@ -1243,6 +1467,8 @@ int configure_staged_kernels() {
   set((const void*)k_eam_rho_staged<true>);
   set((const void*)k_eam_force_staged<false>);
   set((const void*)k_eam_force_staged<true>);
+  set((const void*)k_eam_rho_bonds_staged);
+  set((const void*)k_eam_force_bonds_staged);
   return e == cudaSuccess ? GBMD_OK : GBMD_ERR_CUDA;
 }
 
@@ -1271,6 +1497,10 @@ static bool launch_staged(gbmd_context* c, const PairArgs& A, int part) {
     LJF P{};
     k_lj_staged<EV, true><<<grid, B, smem, s>>>(A, P, c->lj_tab_d, c->lj.ntypes, c->lj.rcut_max2, c->cell_start,
                                                  K, cap);
+  } else if (!EV && c->rho_bonds) {
+    if (part != 2)
+      k_eam_rho_bonds_staged<<<grid, B, smem, s>>>(A, c->eam, c->fpf, c->pfp, c->cell_start, K, cap);
+    if (part != 1) k_eam_force_bonds_staged<<<grid, B, smem, s>>>(A, c->fpf, c->pfp, c->cell_start, K, cap);
   } else {
     if (part != 2)
       k_eam_rho_staged<EV><<<grid, B, smem, s>>>(A, c->eam, c->fpf, c->epf, c->pfp, c->cell_start, K, cap);
@@ -1278,6 +1508,36 @@ static bool launch_staged(gbmd_context* c, const PairArgs& A, int part) {
       k_eam_force_staged<EV><<<grid, B, smem, s>>>(A, c->eam, c->fpf, c->epf, c->pfp, c->cell_start, K, cap);
   }
   return true;
+}
+
+template <int T, bool PIECE>
+static void launch_bonds_T(gbmd_context* c, const PairArgs& A, int part) {
+  const int64_t threads = (A.n - A.i0) * T;
+  const int B = c->block, Bd = std::min(128, c->block_rho ? c->block_rho : B);
+  cudaStream_t s = c->stream;
+  if (part != 2) k_eam_rho_bonds<T, PIECE><<<(unsigned)((threads + Bd - 1) / Bd), Bd, 0, s>>>(A, c->eam, c->fpf, c->pfp);
+  if (part != 1) k_eam_force_bonds<T, PIECE><<<(unsigned)((threads + B - 1) / B), B, 0, s>>>(A, c->fpf, c->pfp);
+}
+
+template <bool PIECE>
+static void launch_bonds(gbmd_context* c, const PairArgs& A, int part) {
+  switch (c->tpa) {
+    case 1: launch_bonds_T<1, PIECE>(c, A, part); break;
+    case 2: launch_bonds_T<2, PIECE>(c, A, part); break;
+    case 4: launch_bonds_T<4, PIECE>(c, A, part); break;
+    case 8: launch_bonds_T<8, PIECE>(c, A, part); break;
+    default: launch_bonds_T<16, PIECE>(c, A, part); break;
+  }
+}
+
+// One-element eam_alloy without energies goes through the bond passes; a force
+// pass on its own, the way of its density pass (of the whole system, or all
+// its pieces).
+static bool take_bonds(gbmd_context* c, const PairArgs& A, int part, bool ev) {
+  if (c->pot != GBMD_POT_EAM_ALLOY || c->eam.nel != 1) return false;
+  const bool can = !ev && !c->newton3 && c->vec == 4 && c->bpair_cap >= (int64_t)(c->maxnb / A.W) * A.stride;
+  if (part != 2) c->rho_bonds = can;
+  return can && c->rho_bonds;
 }
 
 template <bool EV, bool PIECE>
@@ -1317,7 +1577,16 @@ int launch_mixed(gbmd_context* c, const PairArgs& A, int part, bool ev) {
   // list, no staging, checked by launch_forces)
   if (A.i0 != 0 || A.n != c->n) {
     if (ev) return set_error(c, GBMD_ERR_INVALID, "atom ranges: no energies or virials");
+    if (take_bonds(c, A, part, false)) {
+      launch_bonds<true>(c, A, part);
+      return GBMD_OK;
+    }
     return launch_mixed_shape<false, true>(c, A, part);
+  }
+  const bool bonds = take_bonds(c, A, part, ev);
+  if (bonds && !(c->staged && c->tpa == 1)) {
+    launch_bonds<false>(c, A, part);
+    return GBMD_OK;
   }
   return ev ? launch_mixed_E<true>(c, A, part) : launch_mixed_E<false>(c, A, part);
 }

@@ -1153,6 +1153,7 @@ static int filter_list(gbmd_context* c, const int* gate) {
   A.R2lo = R2lo;
   A.R2hi = R2hi;
   const unsigned blocks = gate ? chain_blocks(c, c->n, 256, gate, 8) : nblk(c->n, 256);
+  if (!gate && !c->capturing) ensure_bpair(c);
   if (c->vec == 4) k_filter_list<true><<<blocks, 256, 0, c->stream>>>(A, c->grid, gate);
   else k_filter_list<false><<<blocks, 256, 0, c->stream>>>(A, c->grid, gate);
   c->list_valid = true;
@@ -1167,15 +1168,15 @@ static int filter_list(gbmd_context* c, const int* gate) {
 // Measured on GB300, us, lanes 1 / 2 / 4 / 8 / 16; force evaluations:
 //   eam_alloy, one element      4,000 atoms    36 / 24 / 18 / 15 / 13
 //                              16,384          39 / 28 / 22 / 18 / 22
-//                              32,000          39 / 29 / 23 / 27 / 31
 //   LJ                          4,000          14 / 10 /  8 /  6 /  6
 //                              16,384          14 / 10 /  8 /  8 /  9
 //                              32,000          14 / 12 / 11 / 10 / 14
 // and 20 NVE steps with two rebuilds, lanes 1 / 2 / 4:
-//   eam_alloy, one element    108,000         1,286 / 1,305 / 1,248
-//                             256,000         2,742 / 2,576 / 2,590
-//                             864,000         7,738 / 7,641 / 8,144
-//                           4,000,000        32,289 / 32,939 / 35,542
+//   eam_alloy, one element     32,000           760 / 549 / 489
+//                              62,500           878 / 726 / 786
+//                             256,000         2,364 / 2,335 / 2,521
+//                             864,000         7,013 / 7,007 / 7,769
+//                           4,000,000        29,841 / 30,355 / 33,621
 //   two elements              256,000         3,425 / 3,125 / 3,096
 //                           2,048,000        21,073 / 20,706 / 22,275
 //   LJ                         32,000           513 / 440 / 428
@@ -1190,7 +1191,7 @@ void choose_launch(gbmd_context* c) {
   int tpa = 1;
   if (c->n <= 8192) tpa = 16;
   else if (c->n <= 24576) tpa = 8;
-  else if (c->n <= (single ? 160000 : alloy ? 327680 : 49152)) tpa = 4;
+  else if (c->n <= (alloy && !single ? 327680 : 49152)) tpa = 4;
   else if (single ? c->n <= 1500000 : alloy || (lj && c->n <= 262144)) tpa = 2;
   if (c->newton3 || c->staged) tpa = 1;  // the layout of the half list and of the staged kernels
   c->vec = 4;
@@ -1202,11 +1203,32 @@ void choose_launch(gbmd_context* c) {
   if (c->maxnb_out > 0) c->maxnb_out = ((c->maxnb_out + W - 1) / W) * W;
 }
 
+// Words of the list the pair kernels read.
+static int64_t list_words(const gbmd_context* c) {
+  return (int64_t)(c->maxnb / list_width(c)) * c->npad * list_width(c);
+}
+
+void ensure_bpair(gbmd_context* c) {
+  if (c->precision != GBMD_PRECISION_MIXED || c->pot != GBMD_POT_EAM_ALLOY || c->eam.nel != 1 || c->newton3 ||
+      c->vec != 4 || list_words(c) <= c->bpair_cap)
+    return;
+  cudaFree(c->bpair);
+  c->bpair = nullptr;
+  c->bpair_cap = 0;
+  const int64_t need = list_words(c);
+  // without it the force pass forms the pair terms again
+  if (cudaMalloc(&c->bpair, sizeof(float) * (size_t)need) == cudaSuccess) c->bpair_cap = need;
+  else (void)cudaGetLastError();
+}
+
 int rebuild(gbmd_context* c, bool check_capacity, const int* gate) {
   if (!gate && !c->capturing) choose_launch(c);
   if (c->n == 0 || !two_level(c)) {
     const int rc = rebuild_chain(c, check_capacity, gate);
-    if (rc == GBMD_OK && !gate) c->list_builds++;
+    if (rc == GBMD_OK && !gate) {
+      c->list_builds++;
+      if (!c->capturing) ensure_bpair(c);
+    }
     return rc;
   }
   if (gate && !c->outer_valid) return set_error(c, GBMD_ERR_INVALID, "gated rebuild needs an outer list");

@@ -37,6 +37,8 @@ struct PairArgs {
   double4_32a* posd_o;
   double *vx, *vy, *vz, *ax, *ay, *az;
   double *vxo, *vyo, *vzo;    // velocities after the fused halves (vx.. in place, or another buffer)
+  float4* f0;                 // EAM density pass -> force pass (gbmd_context::f0, bpair)
+  float* bpair;
   double* ep;
   double* ep_emb;             // FP64 EAM: embedding energy F(rho_i) from the density pass
   double* vir;

@@ -7,8 +7,8 @@
 //   cellpack (i32): home cell at the last rebuild, cx | cy<<10 | cz<<20
 //   posf (float4): FP32 position relative to the home-cell corner, w = type bits
 //   posd (double4_32a): FP64 absolute position, w = type bits (FP64 path gathers)
-//   nbr (u32): full neighbour list entries j | code<<26, code = (dx+1)|(dy+1)<<2|(dz+1)<<4
-//              the stencil offset of j's cell; laid out for T lanes per atom as
+//   nbr (u32): full neighbour list entries j | code<<26, code = the stencil offset of
+//              j's cell, two bits an axis in two's complement (code_of); laid out for T lanes per atom as
 //              nbr[(k/W)*(npad*W) + i*W + list_word(k%W)], W = T * entries per load
 //   nnb (i32): neighbours per atom
 #pragma once
@@ -98,7 +98,7 @@ struct SuttonChenDev {
 struct Grid {
   int nc[3];
   double h[3], L[3], lo[3];
-  float hf[3];
+  float hf[3], hh[3];  // cell edge and half of it
   int64_t ncells;
 };
 
@@ -545,14 +545,19 @@ __device__ __forceinline__ double group_reduce_d(double v) {
 }
 
 // stencil code -> offsets in {-1,0,1}
-__device__ __forceinline__ int code_dx(uint32_t code) { return int(code & 3u) - 1; }
-__device__ __forceinline__ int code_dy(uint32_t code) { return int((code >> 2) & 3u) - 1; }
-__device__ __forceinline__ int code_dz(uint32_t code) { return int((code >> 4) & 3u) - 1; }
-
-__device__ __forceinline__ float code_shift(uint32_t bits2, float h) {
-  // bits2 in {0,1,2} -> -h, 0, +h
-  return bits2 == 0u ? -h : (bits2 == 2u ? h : 0.0f);
+__host__ __device__ __forceinline__ int code_dx(uint32_t code) { return (int)(code << 30) >> 30; }
+__host__ __device__ __forceinline__ int code_dy(uint32_t code) { return (int)(code << 28) >> 30; }
+__host__ __device__ __forceinline__ int code_dz(uint32_t code) { return (int)(code << 26) >> 30; }
+__host__ __device__ __forceinline__ uint32_t code_of(int dx, int dy, int dz) {
+  return ((uint32_t)dx & 3u) | (((uint32_t)dy & 3u) << 2) | (((uint32_t)dz & 3u) << 4);
 }
+
+// Twice a list entry's stencil offset along each axis as a float, in one or
+// two instructions: an axis's two bits moved to the top are the sign and the
+// exponent of 0, +2 or -2.  Times half the cell edge it is the shift, exactly.
+__device__ __forceinline__ float twice_dx(uint32_t ent) { return __uint_as_float((ent << 4) & 0xc0000000u); }
+__device__ __forceinline__ float twice_dy(uint32_t ent) { return __uint_as_float((ent << 2) & 0xc0000000u); }
+__device__ __forceinline__ float twice_dz(uint32_t ent) { return __uint_as_float(ent & 0xc0000000u); }
 
 __device__ __forceinline__ int image_of(int c, int d, int nc) {
   const int cj = c + d;

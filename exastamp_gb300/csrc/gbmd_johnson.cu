@@ -261,7 +261,6 @@ __device__ __noinline__ bool ej_exact_inside(const double4_32a* __restrict__ pos
   return exact_d2(di.x, di.y, di.z, dj.x, dj.y, dj.z, Sx, Sy, Sz, a, b, c) <= rc2;
 }
 
-__device__ __forceinline__ float ej_unit(uint32_t b) { return __int_as_float(0x4B000000u | b) - 8388609.0f; }
 
 struct EjGeom {
   float dx, dy, dz, d2;
@@ -272,9 +271,9 @@ template <class Params>
 __device__ __forceinline__ EjGeom ej_geom(const PairArgs& A, const Params& P, uint32_t ent, const float4& pj,
                                           const float4& pi, int64_t i, int cp) {
   EjGeom G;
-  G.dx = fmaf(ej_unit((ent >> 26) & 3u), A.g.hf[0], pj.x - pi.x);
-  G.dy = fmaf(ej_unit((ent >> 28) & 3u), A.g.hf[1], pj.y - pi.y);
-  G.dz = fmaf(ej_unit(ent >> 30), A.g.hf[2], pj.z - pi.z);
+  G.dx = fmaf(twice_dx(ent), A.g.hh[0], pj.x - pi.x);
+  G.dy = fmaf(twice_dy(ent), A.g.hh[1], pj.y - pi.y);
+  G.dz = fmaf(twice_dz(ent), A.g.hh[2], pj.z - pi.z);
   G.d2 = fmaf(G.dx, G.dx, fmaf(G.dy, G.dy, G.dz * G.dz));
   G.in = G.d2 < P.rc2lo;
   if (!G.in && G.d2 <= P.rc2hi)

@@ -40,9 +40,9 @@ __device__ __forceinline__ GeomF2 geom_f2(uint32_t ea, uint32_t eb, const float4
                                           const float2& npx, const float2& npy, const float2& npz, const float2& hx,
                                           const float2& hy, const float2& hz) {
   GeomF2 r;
-  r.dx = __ffma2_rn(f2(unit_of((ea >> 26) & 3u), unit_of((eb >> 26) & 3u)), hx, __fadd2_rn(f2(pa.x, pb.x), npx));
-  r.dy = __ffma2_rn(f2(unit_of((ea >> 28) & 3u), unit_of((eb >> 28) & 3u)), hy, __fadd2_rn(f2(pa.y, pb.y), npy));
-  r.dz = __ffma2_rn(f2(unit_of(ea >> 30), unit_of(eb >> 30)), hz, __fadd2_rn(f2(pa.z, pb.z), npz));
+  r.dx = __ffma2_rn(f2(twice_dx(ea), twice_dx(eb)), hx, __fadd2_rn(f2(pa.x, pb.x), npx));
+  r.dy = __ffma2_rn(f2(twice_dy(ea), twice_dy(eb)), hy, __fadd2_rn(f2(pa.y, pb.y), npy));
+  r.dz = __ffma2_rn(f2(twice_dz(ea), twice_dz(eb)), hz, __fadd2_rn(f2(pa.z, pb.z), npz));
   r.d2 = __ffma2_rn(r.dx, r.dx, __ffma2_rn(r.dy, r.dy, __fmul2_rn(r.dz, r.dz)));
   return r;
 }
@@ -51,8 +51,8 @@ __device__ __forceinline__ GeomF2 geom_f2(uint32_t ea, uint32_t eb, const float4
 struct PairFrame {
   float2 npx, npy, npz, hx, hy, hz;
   __device__ __forceinline__ PairFrame(const float4& pi, const Grid& g)
-      : npx(f2(-pi.x, -pi.x)), npy(f2(-pi.y, -pi.y)), npz(f2(-pi.z, -pi.z)), hx(f2(g.hf[0], g.hf[0])),
-        hy(f2(g.hf[1], g.hf[1])), hz(f2(g.hf[2], g.hf[2])) {}
+      : npx(f2(-pi.x, -pi.x)), npy(f2(-pi.y, -pi.y)), npz(f2(-pi.z, -pi.z)), hx(f2(g.hh[0], g.hh[0])),
+        hy(f2(g.hh[1], g.hh[1])), hz(f2(g.hh[2], g.hh[2])) {}
   __device__ __forceinline__ GeomF2 geom(uint32_t ea, uint32_t eb, const float4& pa, const float4& pb) const {
     return geom_f2(ea, eb, pa, pb, npx, npy, npz, hx, hy, hz);
   }
@@ -93,7 +93,7 @@ struct ListRows {
     nrow = (nn + W - 1) / W;
     nfull = nn / W;
     rem = nn - nfull * W;
-    standin = (uint32_t)i | ((2u | (1u << 2) | (1u << 4)) << GBMD_IDX_BITS);
+    standin = (uint32_t)i | (code_of(1, 0, 0) << GBMD_IDX_BITS);
   }
   __device__ __forceinline__ void load(int r, uint32_t (&e)[V]) const {
     const uint32_t* q = p + (size_t)r * stride;
@@ -174,7 +174,7 @@ struct GlobalFetch {
 
 struct StagedFetch {
   const float4* pos;   // staged positions (shared memory)
-  const int4* rows;    // 16 entries by (dy+1) | (dz+1) << 2: {delta0, g1, n1, delta1}
+  const int4* rows;    // 16 entries by the entry's bits of dy, dz: {delta0, g1, n1, delta1}
   __device__ __forceinline__ float4 operator()(uint32_t ent, uint32_t j) const {
     const int4 t = rows[(ent >> 28) & 15u];
     const int jj = (int)j;
@@ -220,7 +220,7 @@ __device__ bool stage_cells(const Grid& g, const int32_t* __restrict__ cstart, c
       const int ga = sh[4 * s], na = sh[4 * s + 1], gb = sh[4 * s + 2], nb = sh[4 * s + 3];
       const int oa = off, ob = off + na;
       off += na + nb;
-      const int key = (s % 3) | ((s / 3) << 2);
+      const int key = (int)code_of(s % 3 - 1, s / 3 - 1, 0);
       rows[key] = make_int4(ga - oa, gb, nb, gb - ob);
       sh[36 + 2 * s] = oa;
       sh[36 + 2 * s + 1] = ob;
@@ -272,6 +272,22 @@ __device__ __forceinline__ void lj_load_table(LJTabSmem& t, const LJPair* __rest
   __syncthreads();
 }
 
+// geom_f with the stencil offset through the 2^23 mantissa trick, an FP32
+// addition an axis in place of geom_f's second integer instruction: for the
+// kernels that the L1 data path or registers bound, not instruction issue
+// (LJ mixtures without energies; one-element bond passes: 4M atoms 1,197
+// against 1,224 us with geom_f).
+__device__ __forceinline__ float unit_of(uint32_t b) { return __int_as_float((b & 3u) ^ 0x4b000002u) - 8388610.0f; }
+
+__device__ __forceinline__ GeomF geom_u(uint32_t ent, const float4& pj, const float4& pi, const Grid& g) {
+  GeomF r;
+  r.dx = fmaf(unit_of(ent >> 26), g.hf[0], pj.x - pi.x);
+  r.dy = fmaf(unit_of(ent >> 28), g.hf[1], pj.y - pi.y);
+  r.dz = fmaf(unit_of(ent >> 30), g.hf[2], pj.z - pi.z);
+  r.d2 = fmaf(r.dx, r.dx, fmaf(r.dy, r.dy, r.dz * r.dz));
+  return r;
+}
+
 // One atom's pair sums, reduced over its T lanes (v: virial xx yy zz xy xz yz).
 struct PairSums {
   float f[3], e, v[6];
@@ -280,6 +296,13 @@ struct PairSums {
 template <int T, int V, bool EV, bool MULTI, class Fetch>
 __device__ __forceinline__ PairSums lj_atom(const PairArgs& A, const LJF& P, const LJTabSmem& tab, int ntypes,
                                             double rcmax2, int64_t i, int lane, bool live, const Fetch& fetch) {
+  // ROW: the cutoffs of a row's entries first, with one branch for the (rare)
+  // entries in the band, where a branch an entry issues four times as many
+  // instructions: 1M-atom LJ 144 -> 129 us, with energies 217 -> 183; 1M-atom
+  // mixture with energies 315 -> 269.  A mixture without energies keeps the
+  // branch an entry: at 64 registers a row's pairs spill 76 bytes (252 against
+  // 227 us), and at 80 three blocks instead of four fit (264).
+  constexpr bool ROW = !MULTI || EV;
   const int nn = live ? min(A.nnb[i], A.maxnb) : 0;
   const float4 pi = live ? A.posf[i] : make_float4(0.f, 0.f, 0.f, 0.f);
   const int ti = __float_as_int(pi.w);
@@ -292,9 +315,57 @@ __device__ __forceinline__ PairSums lj_atom(const PairArgs& A, const LJF& P, con
 #pragma unroll
     for (int q = 0; q < N; ++q) pj[q] = fetch(R.e[q], R.e[q] & GBMD_IDX_MASK);
     float rx = 0.f, ry = 0.f, rz = 0.f, re = 0.f;
+    auto term = [&](const GeomF& G, float sig2, float eps24, float eps4, float ecut, bool in) {
+      // hardware reciprocal (within 1 ulp): the pair term's error budget is
+      // ~1e-7 relative against a 1e-5 force tolerance
+      float r2i;
+      asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r2i) : "f"(G.d2));
+      const float s2 = sig2 * r2i;
+      const float s6 = s2 * s2 * s2;
+      const float s12 = s6 * s6;
+      const float fpair = in ? eps24 * fmaf(2.f, s12, -s6) * r2i : 0.f;  // -(dE/dr)/r
+      rx = fmaf(-fpair, G.dx, rx);
+      ry = fmaf(-fpair, G.dy, ry);
+      rz = fmaf(-fpair, G.dz, rz);
+      if (EV) {
+        re += in ? 0.5f * fmaf(eps4, s12 - s6, -ecut) : 0.f;
+        const float h = 0.5f * fpair;
+        v[0] = fmaf(h * G.dx, G.dx, v[0]);
+        v[1] = fmaf(h * G.dy, G.dy, v[1]);
+        v[2] = fmaf(h * G.dz, G.dz, v[2]);
+        v[3] = fmaf(h * G.dx, G.dy, v[3]);
+        v[4] = fmaf(h * G.dx, G.dz, v[4]);
+        v[5] = fmaf(h * G.dy, G.dz, v[5]);
+      }
+    };
+    if constexpr (ROW) {
+      GeomF Gs[N];
+      int pids[N];
+      bool ins[N], near = false;
+#pragma unroll
+      for (int q = 0; q < N; ++q) {
+        Gs[q] = geom_f(R.e[q], pj[q], pi, A.g);
+        pids[q] = MULTI ? ti * ntypes + __float_as_int(pj[q].w) : 0;
+        const float2 lim = MULTI ? tab.b[pids[q]] : make_float2(P.rc2lo, P.rc2hi);
+        ins[q] = Gs[q].d2 < lim.x;
+        near |= !ins[q] && Gs[q].d2 <= lim.y;
+      }
+      if (near) {
+#pragma unroll
+        for (int q = 0; q < N; ++q)
+          if (!ins[q] && Gs[q].d2 <= (MULTI ? tab.b[pids[q]].y : P.rc2hi) && R.ok[q])
+            ins[q] = exact_inside(A.posd, i, R.e[q] & GBMD_IDX_MASK, R.e[q] >> GBMD_IDX_BITS, A.cellpack[i], A.g,
+                                  MULTI ? rcmax2 : P.rc2, MULTI ? tab.r[pids[q]] : 0.0);
+      }
+#pragma unroll
+      for (int q = 0; q < N; ++q) {
+        const float4 a = MULTI ? tab.a[pids[q]] : make_float4(P.sig2, P.eps24, P.eps4, P.ecut);
+        term(Gs[q], a.x, a.y, a.z, a.w, ins[q]);
+      }
+    } else {
 #pragma unroll
     for (int q = 0; q < N; ++q) {
-      const GeomF G = geom_f(R.e[q], pj[q], pi, A.g);
+      const GeomF G = geom_u(R.e[q], pj[q], pi, A.g);
       float sig2, eps24, eps4, ecut, rlo, rhi;
       int pid = 0;
       if (MULTI) {
@@ -330,6 +401,7 @@ __device__ __forceinline__ PairSums lj_atom(const PairArgs& A, const LJF& P, con
         v[4] = fmaf(h * G.dx, G.dz, v[4]);
         v[5] = fmaf(h * G.dy, G.dz, v[5]);
       }
+    }
     }
     kahan_add(fx, cfx, rx);
     kahan_add(fy, cfy, ry);
@@ -780,7 +852,7 @@ __device__ __forceinline__ BondSums eam_rho_bonds_atom(const PairArgs& A, const 
     for (int k = 0; k < 4; ++k) p[k] = 0.f;
 #pragma unroll
     for (int q = 0; q < N; ++q) {
-      const GeomF G = geom_f(R.e[q], pj[q], pi, A.g);
+      const GeomF G = geom_u(R.e[q], pj[q], pi, A.g);
       bool in = G.d2 < E.rc2lo;
       if (!in && G.d2 <= E.rc2hi && R.ok[q])
         in = exact_inside(A.posd, i, R.e[q] & GBMD_IDX_MASK, R.e[q] >> GBMD_IDX_BITS, A.cellpack[i], A.g, E.rcut2,
@@ -881,8 +953,8 @@ __device__ __forceinline__ PairSums eam_force_bonds_atom(const PairArgs& A, cons
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
       const float w = (fpi + pj[q].w) * b[q];
-      p[0] = fmaf(fmaf(unit_of((ent[q] >> 26) & 3u), A.g.hf[0], pj[q].x - pi.x), w, p[0]);
-      p[1] = fmaf(fmaf(unit_of((ent[q] >> 28) & 3u), A.g.hf[1], pj[q].y - pi.y), w, p[1]);
+      p[0] = fmaf(fmaf(unit_of(ent[q] >> 26), A.g.hf[0], pj[q].x - pi.x), w, p[0]);
+      p[1] = fmaf(fmaf(unit_of(ent[q] >> 28), A.g.hf[1], pj[q].y - pi.y), w, p[1]);
       p[2] = fmaf(fmaf(unit_of(ent[q] >> 30), A.g.hf[2], pj[q].z - pi.z), w, p[2]);
     }
 #pragma unroll

@@ -366,9 +366,9 @@ __global__ void k_posf(int64_t n, const double* __restrict__ x, const double* __
 __device__ __noinline__ bool exact_within(const double* __restrict__ x, const double* __restrict__ y,
                                           const double* __restrict__ z, int64_t i, int64_t k, uint32_t code,
                                           int cx, int cy, int cz, const Grid g, double R2) {
-  const int nxi = image_of(cx, int(code & 3u) - 1, g.nc[0]);
-  const int nyi = image_of(cy, int((code >> 2) & 3u) - 1, g.nc[1]);
-  const int nzi = image_of(cz, int((code >> 4) & 3u) - 1, g.nc[2]);
+  const int nxi = image_of(cx, code_dx(code), g.nc[0]);
+  const int nyi = image_of(cy, code_dy(code), g.nc[1]);
+  const int nzi = image_of(cz, code_dz(code), g.nc[2]);
   double a, b, c;
   return exact_d2(x[i], y[i], z[i], x[k], y[k], z[k], (double)nxi * g.L[0], (double)nyi * g.L[1],
                   (double)nzi * g.L[2], a, b, c) <= R2;
@@ -480,9 +480,9 @@ struct BuildRound {
 __device__ __forceinline__ float build_d2(const float4* __restrict__ pf, const Grid& g, const float4& pi, uint32_t w) {
   const uint32_t code = w >> GBMD_IDX_BITS;
   const float4 pj = pf[w & GBMD_IDX_MASK];
-  const float sx = __fmul_rn((float)((int)(code & 3u) - 1), g.hf[0]);
-  const float sy = __fmul_rn((float)((int)((code >> 2) & 3u) - 1), g.hf[1]);
-  const float sz = __fmul_rn((float)((int)(code >> 4) - 1), g.hf[2]);
+  const float sx = __fmul_rn((float)code_dx(code), g.hf[0]);
+  const float sy = __fmul_rn((float)code_dy(code), g.hf[1]);
+  const float sz = __fmul_rn((float)code_dz(code), g.hf[2]);
   const float dx = __fsub_rn(__fadd_rn(pj.x, sx), pi.x);
   const float dy = __fsub_rn(__fadd_rn(pj.y, sy), pi.y);
   const float dz = __fsub_rn(__fadd_rn(pj.z, sz), pi.z);
@@ -566,7 +566,7 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32, 6) k_build_list_cells(const 
           ((int64_t)(cz + dz - nz * g.nc[2]) * g.nc[1] + (cy + dy - ny * g.nc[1])) * g.nc[0] + (cx + dx - nx * g.nc[0]);
       s_start = A.cstart[cj];
       s_cnt = A.cstart[cj + 1] - s_start;
-      s_code = (uint32_t)(dx + 1) | ((uint32_t)(dy + 1) << 2) | ((uint32_t)(dz + 1) << 4);
+      s_code = code_of(dx, dy, dz);
       s_sx = __fmul_rn((float)dx, g.hf[0]);
       s_sy = __fmul_rn((float)dy, g.hf[1]);
       s_sz = __fmul_rn((float)dz, g.hf[2]);
@@ -620,7 +620,7 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32, 6) k_build_list_cells(const 
       float far2 = -1.f;               // largest d2 of the hits
       bool full = false;
       const float2 npx = make_float2(-pi.x, -pi.x), npy = make_float2(-pi.y, -pi.y), npz = make_float2(-pi.z, -pi.z);
-      const uint32_t self = (uint32_t)i | (21u << GBMD_IDX_BITS);
+      const uint32_t self = (uint32_t)i;
       const float4* const cand = S.chunk + half * (BUILD_CHUNK + 4);
       // Predicated, so that eight tests are one straight line.  An atom never
       // pairs with itself: its images sit at least one box edge >= R away, so
@@ -834,6 +834,7 @@ static int rebuild_chain(gbmd_context* c, bool check_capacity, const int* gate) 
       g.L[d] = c->hi[d] - c->lo[d];
       g.h[d] = g.L[d] / nc[d];
       g.hf[d] = (float)g.h[d];
+      g.hh[d] = 0.5f * g.hf[d];
       g.lo[d] = c->lo[d];
     }
     if (c->cells_cap < g.ncells + 1) {
@@ -1027,9 +1028,9 @@ struct FilterArgs {
 __device__ __forceinline__ bool filter_keep(const FilterArgs& A, const Grid& g, int64_t i, const float4& pi,
                                             uint32_t w, const float4& pj, int cx, int cy, int cz) {
   const uint32_t code = w >> GBMD_IDX_BITS;
-  const float sx = __fmul_rn((float)((int)(code & 3u) - 1), g.hf[0]);
-  const float sy = __fmul_rn((float)((int)((code >> 2) & 3u) - 1), g.hf[1]);
-  const float sz = __fmul_rn((float)((int)(code >> 4) - 1), g.hf[2]);
+  const float sx = __fmul_rn((float)code_dx(code), g.hf[0]);
+  const float sy = __fmul_rn((float)code_dy(code), g.hf[1]);
+  const float sz = __fmul_rn((float)code_dz(code), g.hf[2]);
   const float dx = __fsub_rn(__fadd_rn(pj.x, sx), pi.x);
   const float dy = __fsub_rn(__fadd_rn(pj.y, sy), pi.y);
   const float dz = __fsub_rn(__fadd_rn(pj.z, sz), pi.z);
@@ -1298,7 +1299,7 @@ int export_pairs(gbmd_context* c, int64_t cap, uint64_t* id_i, uint64_t* id_j, i
     for (int k = 0; k < nnb[i] && k < c->maxnb; ++k) {
       const uint32_t e = nb[(size_t)(k / W) * stride + (size_t)i * W + list_word(k % W, wsh, tsh)];
       const uint32_t j = e & GBMD_IDX_MASK, code = e >> GBMD_IDX_BITS;
-      const int d[3] = {int(code & 3) - 1, int((code >> 2) & 3) - 1, int((code >> 4) & 3) - 1};
+      const int d[3] = {code_dx(code), code_dy(code), code_dz(code)};
       const int cc[3] = {cx + d[0], cy + d[1], cz + d[2]};
       id_i[row] = ids[i];
       id_j[row] = ids[j];

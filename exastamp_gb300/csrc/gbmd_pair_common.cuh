@@ -109,15 +109,11 @@ static __device__ __noinline__ bool exact_inside(const double4_32a* __restrict__
   return rc_pair <= 0.0 || sqrt(d2) <= rc_pair;
 }
 
-// {0,1,2} -> -1.f, 0.f, +1.f exactly (small integer through the 2^23 mantissa
-// trick); the separation shift is then one FMA per axis.
-__device__ __forceinline__ float unit_of(uint32_t b) { return __int_as_float(0x4B000000u | b) - 8388609.0f; }
-
 __device__ __forceinline__ GeomF geom_f(uint32_t ent, const float4& pj, const float4& pi, const Grid& g) {
   GeomF r;
-  r.dx = fmaf(unit_of((ent >> 26) & 3u), g.hf[0], pj.x - pi.x);
-  r.dy = fmaf(unit_of((ent >> 28) & 3u), g.hf[1], pj.y - pi.y);
-  r.dz = fmaf(unit_of(ent >> 30), g.hf[2], pj.z - pi.z);
+  r.dx = fmaf(twice_dx(ent), g.hh[0], pj.x - pi.x);
+  r.dy = fmaf(twice_dy(ent), g.hh[1], pj.y - pi.y);
+  r.dz = fmaf(twice_dz(ent), g.hh[2], pj.z - pi.z);
   r.d2 = fmaf(r.dx, r.dx, fmaf(r.dy, r.dy, r.dz * r.dz));
   return r;
 }

@@ -125,14 +125,11 @@ static void invalidate_list(gbmd_context* c) {
   drop_graph(c);
 }
 
-// The FP64 re-test bands of the current potential for the current list radius.
-static int set_bands(gbmd_context* c) {
-  const double reach = c->rlist + c->list_buffer;
-  auto band = [&](double rc, float& lo, float& hi) {
-    const double w = band_rel(reach, rc);
-    lo = (float)(rc * rc * (1.0 - w));
-    hi = (float)(rc * rc * (1.0 + w));
-  };
+// The FP64 re-test bands of the current potential for the current cells; where
+// none are laid out, rebuild_chain calls again when it has done so.
+int set_bands(gbmd_context* c) {
+  const double tol = c->grid_valid ? c->grid.tol : band_tol(c->rlist + c->list_buffer, 0.0);
+  auto band = [&](double rc, float& lo, float& hi) { band_limits(rc, tol, lo, hi); };
   if (c->pot == GBMD_POT_LJ || c->pot == GBMD_POT_LJ_MULTI) {
     const int nt = c->lj.ntypes;
     for (int q = 0; q < nt * nt; ++q) band(c->lj.p[q].rc, c->lj.p[q].rc2lo, c->lj.p[q].rc2hi);

@@ -528,7 +528,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch(const __grid_constant__ Ba
         g.tsh = tsh;
         sm.overflow = 0;
         // the band covers the rounding of coordinates in cells of edge h, as
-        // band_rel's does for its cells
+        // band_tol's does for its cells
         const float hmax = fmaxf((float)L3[0] / nc[0], fmaxf((float)L3[1] / nc[1], (float)L3[2] / nc[2]));
         const float rc = (float)A.rcut, band = fminf(0x1p-16f * fmaxf(1.f, hmax / rc), 0.5f);
         g.rc2lo = rc * rc * (1.f - band);

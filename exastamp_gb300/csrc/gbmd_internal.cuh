@@ -99,21 +99,28 @@ struct Grid {
   int nc[3];
   double h[3], L[3], lo[3];
   float hf[3], hh[3];  // cell edge and half of it
+  double tol;          // band_tol of these cells
   int64_t ncells;
 };
 
-// Relative half-width of the band around rc^2 inside which a pair's FP32 d2
+// Half-width of the band around a radius inside which a pair's FP32 separation
 // may fall on the wrong side, so that it is re-tested in FP64.  With cells of
-// edge h < 2 reach (reach = the radius the cells are built for) and
-// home-cell-relative coordinates of at most 2 h, the coordinates' rounding
-// (2^-24 each of 2 h), that of their difference and of the shift add up to
-// 8.5 x 2^-24 h an axis, sqrt(3) of it in d, twice that relative to rc in d2:
-// 2^-18.1 reach / rc.  2^-16 leaves four times that, for atoms that drift on
-// between rebuilds.  The width decides only how many pairs take the FP64 test
-// (Cu, 2^-12: one row of four entries in 14 of a warp; now one in 200).
-inline double band_rel(double reach, double rc) {
-  const double w = 0x1p-16 * (reach > rc ? reach / rc : 1.0);
-  return w < 0.5 ? w : 0.5;
+// longest edge h and home-cell-relative coordinates of at most 2 h, the
+// coordinates' rounding (2^-24 each of 2 h), that of their difference and of
+// the shift add up to 8.5 x 2^-24 h an axis, sqrt(3) of it in d: 2^-20.1 h.
+// 2^-18 h leaves four times that, for atoms that drift on between rebuilds.
+// h is below 2 reach (the radius the cells are built for) but for boxes of
+// more than 1,024 cells along an axis, whose cells grow with the box; the width
+// is that of h = 2 reach at least.  It decides only how many pairs take the FP64
+// test (Cu, 2^-12 of rc^2: one row of four entries in 14 of a warp; now, 2^-16,
+// one in 200).
+inline double band_tol(double reach, double h) { return 0x1p-18 * (h > 2.0 * reach ? h : 2.0 * reach); }
+
+// The band of radius rc in terms of d^2.
+inline void band_limits(double rc, double tol, float& lo, float& hi) {
+  const double in = rc > tol ? rc - tol : 0.0, out = rc + tol;
+  lo = (float)(in * in);
+  hi = (float)(out * out);
 }
 
 struct StepParams {
@@ -335,6 +342,7 @@ constexpr int64_t PACK_DOUBLES = 65536;
 // one-element EAM: room for one float per list entry (bpair), if it can be had
 void ensure_bpair(gbmd_context* c);
 int grid_dims(const double lo[3], const double hi[3], double R, int nc[3]);
+int set_bands(gbmd_context* c);
 // gate: device word; non-null makes every kernel of the chain return at once
 // while it holds 0, and keeps the buffer indices unchanged (see gbmd_neighbors.cu)
 // A full list build: wrap, sort into cells and build the list the pair

@@ -9,7 +9,7 @@
 // stencil offset of j's cell, exact to ~1e-7 relative.  Forces, densities
 // and energies are summed with compensated (Kahan) FP32 sums; per-atom
 // results are converted to FP64 once.  Cutoff membership matches FP64
-// exactly: pairs with FP32 d2 within band_rel of rcut^2 are re-tested in FP64.
+// exactly: pairs with FP32 d2 within band_tol of rcut are re-tested in FP64.
 //
 // Loop structure: each lane reads V list entries with one coalesced load
 // (V = 4: 16 B per lane, streamed past L1 so the gathers keep it), the next

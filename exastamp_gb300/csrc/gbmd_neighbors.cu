@@ -6,7 +6,7 @@
 // src/debug/atom_neighbors_stats.cpp L169-228: every (i, j, image n) with
 // d2 <= (rcut_max + skin)^2, d2 computed in FP64 from ((x_j + n*L) - x_i)
 // without contraction.  Candidates are screened in FP32 on home-cell-relative
-// coordinates; only those within band_rel of the radius are re-tested in FP64,
+// coordinates; only those within band_tol of the radius are re-tested in FP64,
 // so the list is bit-identical to an all-FP64 build.
 //
 // Kernels (per rebuild):
@@ -398,7 +398,7 @@ __device__ __noinline__ bool exact_within(const double* __restrict__ x, const do
 // entries an atom, 17.6 -> 13.1 ms; 1 M-atom LJ 888 -> 765 us.
 //
 // The walk keeps every candidate with FP32 d2 <= R2hi; atoms with a hit above
-// R2lo (the band of band_rel, below one per cent) have their band entries
+// R2lo (the band of band_tol, below one per cent) have their band entries
 // re-tested in FP64 afterwards by the whole warp.
 // ---------------------------------------------------------------------------
 constexpr int BUILD_G = 16;       // home atoms per group
@@ -752,9 +752,8 @@ void launch_posf(gbmd_context* c, const int* gate) {
 static int build_list(gbmd_context* c, const int* gate) {
   const double R = c->rlist;
   const double R2 = R * R;
-  // cells are at least R wide here: the band of reach = R
-  const float R2lo = (float)(R2 * (1.0 - band_rel(R, R)));
-  const float R2hi = (float)(R2 * (1.0 + band_rel(R, R)));
+  float R2lo, R2hi;
+  band_limits(R, c->grid.tol, R2lo, R2hi);
   const int64_t npad = ((c->n + 31) / 32) * 32;
   const int W = list_width(c);
   const int64_t stride = npad * W;
@@ -837,6 +836,7 @@ static int rebuild_chain(gbmd_context* c, bool check_capacity, const int* gate) 
       g.hh[d] = 0.5f * g.hf[d];
       g.lo[d] = c->lo[d];
     }
+    g.tol = band_tol(R, std::max(g.h[0], std::max(g.h[1], g.h[2])));
     if (c->cells_cap < g.ncells + 1) {
       if (c->cell_start) cudaFree(c->cell_start);
       if (c->cell_fill) cudaFree(c->cell_fill);
@@ -846,6 +846,8 @@ static int rebuild_chain(gbmd_context* c, bool check_capacity, const int* gate) 
       c->cells_cap = g.ncells + 1;
     }
     c->grid_valid = true;
+    const int rb = set_bands(c);
+    if (rb) return rb;
   }
   Grid& g = c->grid;
   BoxArgs b;
@@ -1133,9 +1135,8 @@ static int filter_list(gbmd_context* c, const int* gate) {
   }
   c->maxnb = c->maxnb_out;
   const double R2 = c->rlist * c->rlist;
-  const double band = band_rel(c->rlist + c->list_buffer, c->rlist);
-  const float R2lo = (float)(R2 * (1.0 - band));
-  const float R2hi = (float)(R2 * (1.0 + band));
+  float R2lo, R2hi;
+  band_limits(c->rlist, c->grid.tol, R2lo, R2hi);
   FilterArgs A;
   A.n = c->n;
   A.pf = c->POSF();

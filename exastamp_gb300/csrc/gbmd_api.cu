@@ -128,7 +128,7 @@ static void invalidate_list(gbmd_context* c) {
 // The FP64 re-test bands of the current potential for the current cells; where
 // none are laid out, rebuild_chain calls again when it has done so.
 int set_bands(gbmd_context* c) {
-  const double tol = c->grid_valid ? c->grid.tol : band_tol(c->rlist + c->list_buffer, 0.0);
+  const double tol = c->band_margin * (c->grid_valid ? c->grid.tol : band_tol(c->rlist + c->list_buffer, 0.0));
   auto band = [&](double rc, float& lo, float& hi) { band_limits(rc, tol, lo, hi); };
   if (c->pot == GBMD_POT_LJ || c->pot == GBMD_POT_LJ_MULTI) {
     const int nt = c->lj.ntypes;
@@ -143,6 +143,31 @@ int set_bands(gbmd_context* c) {
     band(c->esc.rcut, c->esc.rc2lo, c->esc.rc2hi);
   }
   return GBMD_OK;
+}
+
+// The re-test band for `more` position updates to come without a rebuild or a
+// displacement test.  band_tol covers drifts of several list radii; 100 updates
+// of a simulation stay far below that.  A list kept longer (rebuild_every 0, a
+// caller that never asks for an update) may see its atoms travel together, so
+// the band is then 16 times as wide, for drifts of a hundred radii (more FP64
+// tests: some 5 % of a force pass).
+static int plan_moves(gbmd_context* c, int64_t more) {
+  const int margin = c->moves + more > 100 ? 16 : 1;
+  if (margin == c->band_margin) return GBMD_OK;
+  c->band_margin = margin;
+  drop_graph(c);
+  return set_bands(c);
+}
+
+// The same for a run of nsteps with a rebuild every R steps (0: none, below 0:
+// tests of every step), and the count of updates that it leaves.
+static int plan_run(gbmd_context* c, int nsteps, int R) {
+  return plan_moves(c, R < 0 ? 0 : (R == 0 ? nsteps : std::min(R, nsteps)));
+}
+static void count_run(gbmd_context* c, int nsteps, int R) {
+  if (R < 0) c->moves = 0;
+  else if (R > 0 && nsteps >= R) c->moves = nsteps % R;
+  else c->moves += nsteps;
 }
 
 static int set_rlist(gbmd_context* c, double rcut_max) {
@@ -332,6 +357,7 @@ static int copy_rref(gbmd_context* c) {
 static int do_rebuild(gbmd_context* c, bool check) {
   int rc = two_level(c) ? rebuild_two_level(c, check) : rebuild(c, check);
   if (rc) return rc;
+  if (!c->capturing) c->moves = 0;
   return copy_rref(c);
 }
 
@@ -340,6 +366,7 @@ static int do_rebuild(gbmd_context* c, bool check) {
 static int do_full_rebuild(gbmd_context* c, bool check) {
   int rc = rebuild(c, check);
   if (rc) return rc;
+  c->moves = 0;
   return copy_rref(c);
 }
 
@@ -695,6 +722,7 @@ static int after_new_positions(gbmd_context* c) {
                                                c->d_err + ERRW_DISPL);
   int rc = sync_error_word(c);
   if (rc) return rc;
+  c->moves = 0;
   if (c->h_err[ERRW_DISPL]) invalidate_list(c);
   else launch_posf(c);
   return GBMD_OK;
@@ -1205,7 +1233,10 @@ int gbmd_update_neighbors(gbmd_context* c, int* rebuilt) {
                                                  c->d_err + ERRW_DISPL);
     int rc = sync_error_word(c);
     if (rc) return rc;
-    if (!c->h_err[ERRW_DISPL]) return GBMD_OK;
+    if (!c->h_err[ERRW_DISPL]) {
+      c->moves = 0;
+      return GBMD_OK;
+    }
   }
   int rc = do_rebuild(c, true);
   if (rc) return rc;
@@ -1276,6 +1307,7 @@ int gbmd_compute_forces(gbmd_context* c, int flags) {
   cudaSetDevice(c->device);
   int rc = ensure_list(c);
   if (rc) return rc;
+  if ((rc = plan_moves(c, 0))) return rc;
   ForceFlags f;
   f.energy = (flags & GBMD_FORCE_ENERGY) != 0;
   f.virial = (flags & GBMD_FORCE_VIRIAL) != 0;
@@ -1312,6 +1344,7 @@ int gbmd_compute_forces(gbmd_context* c, int flags) {
 int gbmd_push_f_v_r(gbmd_context* c, double dt, double dt_scale) {
   if (!c) return GBMD_ERR_INVALID;
   launch_push_f_v_r(c, dt, dt_scale);
+  ++c->moves;
   c->energy_step = -1, c->forces_valid_step = c->rho_valid_step = -1;
   GBMD_CUDA(c, cudaGetLastError());
   return GBMD_OK;
@@ -1327,6 +1360,7 @@ int gbmd_push_f_v(gbmd_context* c, double dt, double dt_scale) {
 int gbmd_push_min(gbmd_context* c, double dt, double dt_scale, double tolF) {
   if (!c) return GBMD_ERR_INVALID;
   launch_push_min(c, dt, dt_scale, tolF);
+  ++c->moves;
   c->energy_step = -1, c->forces_valid_step = c->rho_valid_step = -1;
   GBMD_CUDA(c, cudaGetLastError());
   return GBMD_OK;
@@ -1452,6 +1486,7 @@ int gbmd_run_nve(gbmd_context* c, int nsteps, double dt, int rebuild_every, int 
   cudaSetDevice(c->device);
   int rc = ensure_list(c);
   if (rc) return rc;
+  if ((rc = plan_run(c, nsteps, rebuild_every))) return rc;
   if ((rc = ensure_virial(c))) return rc;
   const bool want_thermo = thermo_every > 0;
   // thermo rows are collected on the device and copied out once at the end,
@@ -1536,6 +1571,7 @@ int gbmd_run_nve(gbmd_context* c, int nsteps, double dt, int rebuild_every, int 
     GBMD_CUDA(c, cudaMemcpyAsync(packed ? c->h_pack : thermo_out, rows, sizeof(double) * 27 * nrows,
                                  cudaMemcpyDeviceToHost, c->stream));
   if ((rc = sync_error_word(c))) return rc;
+  count_run(c, nsteps, R);
   if (want_thermo && thermo_out && packed) std::memcpy(thermo_out, c->h_pack, sizeof(double) * 27 * nrows);
   c->step += nsteps;
   c->energy_step = -1, c->forces_valid_step = c->step;
@@ -1559,6 +1595,8 @@ int gbmd_run_nve_host(gbmd_context* c, int nsteps, double dt, int rebuild_every,
     // test of the pushed positions -- check_and_update_particles after
     // verlet_first_half -- decides a rebuild, which can regrow the list; the
     // given accelerations are the forces of the given positions
+    c->moves = 0;
+    if ((rc = plan_moves(c, 1))) return rc;
     GBMD_CUDA(c, cudaMemsetAsync(c->d_err + ERRW_GATE, 0, sizeof(int), c->stream));
     const double* hdev[9];
     for (int k = 0; k < 9; ++k) hdev[k] = hd.a[k];
@@ -1655,6 +1693,7 @@ int gbmd_run_minimize(gbmd_context* c, int nsteps, double dt, double tolF, int r
   if (!c || nsteps < 0 || rebuild_every < GBMD_REBUILD_ON_DISPLACEMENT) return GBMD_ERR_INVALID;
   int rc = ensure_list(c);
   if (rc) return rc;
+  if ((rc = plan_run(c, nsteps, rebuild_every))) return rc;
   const bool trigger = rebuild_every == GBMD_REBUILD_ON_DISPLACEMENT;
   for (int s = 1; s <= nsteps; ++s) {
     ForceFlags f;
@@ -1666,6 +1705,7 @@ int gbmd_run_minimize(gbmd_context* c, int nsteps, double dt, double tolF, int r
   c->energy_step = -1, c->forces_valid_step = c->rho_valid_step = -1;
   GBMD_CUDA(c, cudaStreamSynchronize(c->stream));
   if ((rc = sync_error_word(c))) return rc;
+  count_run(c, nsteps, rebuild_every);
   if ((trigger || two_level(c)) && (rc = collect_device_rebuilds(c))) return rc;
   return report_device_errors(c);
 }

@@ -81,6 +81,7 @@ struct PairHome {
   float4 pf;
   int cx, cy, cz, nn;
   bool border;  // some stencil cell lies across the box face
+  float slack;
   const uint32_t* row;
   __device__ __forceinline__ PairHome(const PairArgs& A, int64_t i, bool live)
       : pd(make_double4_32a(0., 0., 0., 0.)), pf(make_float4(0.f, 0.f, 0.f, 0.f)), cx(0), cy(0), cz(0), nn(0),
@@ -91,6 +92,7 @@ struct PairHome {
       unpack_cell(A.cellpack[i], cx, cy, cz);
       nn = min(A.nnb[i], A.maxnb);
     }
+    slack = drift_slack(A.g, pf);
     border = cx == 0 || cy == 0 || cz == 0 || cx == A.g.nc[0] - 1 || cy == A.g.nc[1] - 1 || cz == A.g.nc[2] - 1;
   }
   // FP64 separation of entry ent and its squared length
@@ -139,8 +141,8 @@ __device__ __forceinline__ void for_pairs(const PairArgs& A, const PairHome& H, 
       tj = __float_as_int(pj.w);
       const PairLimits P = limits(tj);
       const float d2 = geom_f(ent, pj, H.pf, A.g).d2;
-      found = d2 <= P.hi;
-      if (found && d2 >= P.lo)
+      found = d2 <= P.hi + H.slack;
+      if (found && d2 >= P.lo - H.slack)
         found = exact_inside(A.posd, i, ent & GBMD_IDX_MASK, ent >> GBMD_IDX_BITS, A.cellpack[i], A.g, P.rc2, P.rc);
     }
     if (!found) break;

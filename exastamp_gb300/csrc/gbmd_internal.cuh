@@ -100,6 +100,7 @@ struct Grid {
   double h[3], L[3], lo[3];
   float hf[3], hh[3];  // cell edge and half of it
   double tol;          // band_tol of these cells
+  float far, reach2;   // drift_slack's: coordinates that tol covers, twice the radius the cells are built for
   int64_t ncells;
 };
 
@@ -108,8 +109,8 @@ struct Grid {
 // longest edge h and home-cell-relative coordinates of at most 2 h, the
 // coordinates' rounding (2^-24 each of 2 h), that of their difference and of
 // the shift add up to 8.5 x 2^-24 h an axis, sqrt(3) of it in d: 2^-20.1 h.
-// 2^-18 h leaves four times that, for atoms that drift on between rebuilds.
-// h is below 2 reach (the radius the cells are built for) but for boxes of
+// 2^-18 h leaves four times that, for atoms that drift on between rebuilds
+// (further: plan_moves, drift_slack).  h is below 2 reach (the radius the cells are built for) but for boxes of
 // more than 1,024 cells along an axis, whose cells grow with the box; the width
 // is that of h = 2 reach at least.  It decides only how many pairs take the FP64
 // test (Cu, 2^-12 of rc^2: one row of four entries in 14 of a warp; now, 2^-16,
@@ -229,6 +230,8 @@ struct gbmd_context {
   int block = 256;              // threads per block of the pair / force kernels
   int block_rho = 128;          // threads per block of the EAM density kernels (autotuned; 0 = block)
   double skin = 0.0, rlist = 0.0;
+  int64_t moves = 0;            // position updates since the list was built or its atoms' displacements tested
+  int band_margin = 1;          // times band_tol (plan_moves)
   bool list_valid = false;
   int64_t list_builds = 0;
   // two-level list (gbmd_set_list_buffer): an outer list of radius rlist +

@@ -837,6 +837,8 @@ static int rebuild_chain(gbmd_context* c, bool check_capacity, const int* gate) 
       g.lo[d] = c->lo[d];
     }
     g.tol = band_tol(R, std::max(g.h[0], std::max(g.h[1], g.h[2])));
+    g.far = (float)(0x1p19 * g.tol);
+    g.reach2 = (float)(2.0 * R);
     if (c->cells_cap < g.ncells + 1) {
       if (c->cell_start) cudaFree(c->cell_start);
       if (c->cell_fill) cudaFree(c->cell_fill);

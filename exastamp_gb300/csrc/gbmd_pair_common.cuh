@@ -109,6 +109,18 @@ static __device__ __noinline__ bool exact_inside(const double4_32a* __restrict__
   return rc_pair <= 0.0 || sqrt(d2) <= rc_pair;
 }
 
+// What the band around rc^2 is short of for an atom at cell-relative position p
+// that has left the coordinates band_tol covers (2 h, four list radii at least):
+// a list kept while its atoms drift.  With coordinates up to m > far >= h + 2 reach,
+// a neighbour's up to m + reach + h, the errors add up to 4.25 x 2^-24 m an axis,
+// 2^-21.1 m in d; four times that, 2^-19 m =: t, moves d^2 by t (2 rc + t) at
+// most.  For the kernels with registers to spare; the others take a wider band
+// (band_margin) where atoms may have drifted.
+__device__ __forceinline__ float drift_slack(const Grid& g, const float4& p) {
+  const float m = fmaxf(fmaxf(fabsf(p.x), fabsf(p.y)), fabsf(p.z)), t = m * 0x1p-19f;
+  return m > g.far ? t * (g.reach2 + t) : 0.f;
+}
+
 __device__ __forceinline__ GeomF geom_f(uint32_t ent, const float4& pj, const float4& pi, const Grid& g) {
   GeomF r;
   r.dx = fmaf(twice_dx(ent), g.hh[0], pj.x - pi.x);

@@ -212,7 +212,6 @@ struct gbmd_context {
   int32_t *cell_start = nullptr, *cell_fill = nullptr;
   int64_t cells_cap = 0;
   int32_t* scan_tmp = nullptr;
-  int64_t scan_cap = 0;
   uint32_t* nbr = nullptr;
   int32_t* nnb = nullptr;
   int64_t nbr_cap = 0;          // entries allocated

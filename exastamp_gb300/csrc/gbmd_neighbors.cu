@@ -207,20 +207,34 @@ __global__ void __launch_bounds__(1024) k_scan_small(const int32_t* __restrict__
   }
 }
 
-static int scan(gbmd_context* c, const int32_t* in, int32_t* out, int64_t n, const int* gate) {
+static int64_t scan_blocks(int64_t n) { return (n + 1 + SCAN_B - 1) / SCAN_B; }
+
+// scan_tmp holds scan_blocks(n) words (ensure_cells): nothing here can fail.
+static void scan(gbmd_context* c, const int32_t* in, int32_t* out, int64_t n, const int* gate) {
   if (n + 1 <= SCAN_SMALL) {
     k_scan_small<<<1, 1024, 0, c->stream>>>(in, out, (int)n, gate);
-    return GBMD_OK;
+    return;
   }
-  const int64_t nb = (n + 1 + SCAN_B - 1) / SCAN_B;
-  if (c->scan_cap < nb) {
-    if (c->scan_tmp) cudaFree(c->scan_tmp);
-    GBMD_CUDA(c, cudaMalloc(&c->scan_tmp, sizeof(int32_t) * nb));
-    c->scan_cap = nb;
-  }
+  const int64_t nb = scan_blocks(n);
   k_scan_block<<<(unsigned)nb, SCAN_T, 0, c->stream>>>(in, out, n, c->scan_tmp, gate);
   k_scan_sums<<<1, SCAN_T, 0, c->stream>>>(c->scan_tmp, (int)nb, gate);
   k_scan_add<<<(unsigned)nb, SCAN_T, 0, c->stream>>>(out, n, c->scan_tmp, gate);
+}
+
+// The per-cell arrays for `ncells` cells, with the counts cleared.  An
+// allocation that fails leaves none, so that the next call starts afresh.
+static int ensure_cells(gbmd_context* c, int64_t ncells) {
+  if (c->cells_cap >= ncells + 1) return GBMD_OK;
+  cudaFree(c->cell_start);
+  cudaFree(c->cell_fill);
+  cudaFree(c->scan_tmp);
+  c->cell_start = c->cell_fill = c->scan_tmp = nullptr;
+  c->cells_cap = 0;
+  GBMD_CUDA(c, cudaMalloc(&c->cell_start, sizeof(int32_t) * (ncells + 1)));
+  GBMD_CUDA(c, cudaMalloc(&c->cell_fill, sizeof(int32_t) * (ncells + 1)));
+  GBMD_CUDA(c, cudaMalloc(&c->scan_tmp, sizeof(int32_t) * scan_blocks(ncells)));
+  GBMD_CUDA(c, cudaMemsetAsync(c->cell_fill, 0, sizeof(int32_t) * (ncells + 1), c->stream));
+  c->cells_cap = ncells + 1;
   return GBMD_OK;
 }
 
@@ -759,8 +773,9 @@ static int build_list(gbmd_context* c, const int* gate) {
   const int64_t stride = npad * W;
   const int64_t need = (int64_t)(c->maxnb / W) * stride;
   if (need > c->nbr_cap) {
-    if (c->nbr) cudaFree(c->nbr);
+    cudaFree(c->nbr);
     c->nbr = nullptr;
+    c->nbr_cap = 0;
     GBMD_CUDA(c, cudaMalloc(&c->nbr, sizeof(uint32_t) * (size_t)need));
     c->nbr_cap = need;
   }
@@ -839,17 +854,10 @@ static int rebuild_chain(gbmd_context* c, bool check_capacity, const int* gate) 
     g.tol = band_tol(R, std::max(g.h[0], std::max(g.h[1], g.h[2])));
     g.far = (float)(0x1p19 * g.tol);
     g.reach2 = (float)(2.0 * R);
-    if (c->cells_cap < g.ncells + 1) {
-      if (c->cell_start) cudaFree(c->cell_start);
-      if (c->cell_fill) cudaFree(c->cell_fill);
-      GBMD_CUDA(c, cudaMalloc(&c->cell_start, sizeof(int32_t) * (g.ncells + 1)));
-      GBMD_CUDA(c, cudaMalloc(&c->cell_fill, sizeof(int32_t) * (g.ncells + 1)));
-      GBMD_CUDA(c, cudaMemsetAsync(c->cell_fill, 0, sizeof(int32_t) * (g.ncells + 1), c->stream));
-      c->cells_cap = g.ncells + 1;
-    }
+    int ra = ensure_cells(c, g.ncells);
+    if (ra) return ra;
     c->grid_valid = true;
-    const int rb = set_bands(c);
-    if (rb) return rb;
+    if ((ra = set_bands(c))) return ra;
   }
   Grid& g = c->grid;
   BoxArgs b;
@@ -864,11 +872,11 @@ static int rebuild_chain(gbmd_context* c, bool check_capacity, const int* gate) 
   }
   const int64_t n = c->n;
   cudaStream_t s = c->stream;
-  // cell_fill is zero here: cleared when allocated, counted down by k_scatter
-  int rc;
+  // cell_fill is zero here: cleared when allocated, counted up by k_wrap_bin and
+  // down again by k_scatter, with nothing between the two that can fail
   k_wrap_bin<<<chain_blocks(c, n, 256, gate, 8), 256, 0, s>>>(n, c->X(), c->Y(), c->Z(), b, c->cell_of, c->cell_fill,
                                                             c->d_err, gate);
-  if ((rc = scan(c, c->cell_fill, c->cell_start, g.ncells, gate))) return rc;
+  scan(c, c->cell_fill, c->cell_start, g.ncells, gate);
   k_scatter<<<chain_blocks(c, n, 256, gate, 8), 256, 0, s>>>(n, c->cell_of, c->cell_start, c->cell_fill, c->order,
                                                            gate);
   k_cell_rank<<<chain_blocks(c, g.ncells * 32, 256, gate, 8), 256, 0, s>>>(g.ncells, c->cell_start, c->order, c->ID(),
@@ -903,7 +911,7 @@ static int rebuild_chain(gbmd_context* c, bool check_capacity, const int* gate) 
     int m = (int)(mean * 1.35) + 16;
     c->maxnb = ((m + list_width(c) - 1) / list_width(c)) * list_width(c);
   }
-  rc = build_list(c, gate);
+  int rc = build_list(c, gate);
   if (rc) return rc;
   c->list_valid = true;
   if (check_capacity) {

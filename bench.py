@@ -763,8 +763,8 @@ def measure(args, w, ws, dev, stream, torch, *, steps, fp64_steps, e2e_steps, dr
                       "outer_list_builds_in_timed_region": outer_builds,
                       "warmup_steps_run": warm,
                       "neighbours_per_atom": npairs / s.n, "cells": nc.tolist(),
-                      "lanes_per_atom": ctx.get_launch_ex()[0], "list_entries_per_load": ctx.get_launch_ex()[1],
-                      "block": ctx.get_launch_ex()[2], "density_block": ctx.get_density_block(),
+                      "lanes_per_atom": ctx.get_launch_used()[0], "list_entries_per_load": ctx.get_launch_used()[1],
+                      "block": ctx.get_launch_used()[2], "density_block": ctx.get_density_block(),
                       "staged_neighbour_positions": ctx.get_neighbor_staging(),
                       "newton3_half_list": ctx.get_newton3(),
                       "parallelism": "replicas" if ws > 1 else "single-gpu",

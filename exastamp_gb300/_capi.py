@@ -82,6 +82,8 @@ def lib(path: str = LIB_PATH):
             "gbmd_get_density_block": ([vp, P(i32)], i32),
             "gbmd_get_neighbor_staging": ([vp, P(i32)], i32),
             "gbmd_get_launch_ex": ([vp, P(i32), P(i32), P(i32)], i32),
+            "gbmd_set_launch_auto": ([vp], i32),
+            "gbmd_get_launch_used": ([vp, P(i32), P(i32), P(i32)], i32),
             "gbmd_set_skin": ([vp, dbl], i32),
             "gbmd_set_list_buffer": ([vp, dbl], i32),
             "gbmd_get_list_buffer": ([vp, P(dbl), P(i64)], i32),
@@ -282,6 +284,16 @@ class Context:
         self._chk(self._L.gbmd_get_launch_ex(self.h, C.byref(t), C.byref(v), C.byref(b)))
         return t.value, v.value, b.value
 
+    def set_launch_auto(self):
+        """Back to the launch the library picks, after a set_launch."""
+        self._chk(self._L.gbmd_set_launch_auto(self.h))
+
+    def get_launch_used(self):
+        """get_launch_ex's triple as the list last laid out has it."""
+        t, v, b = C.c_int(), C.c_int(), C.c_int()
+        self._chk(self._L.gbmd_get_launch_used(self.h, C.byref(t), C.byref(v), C.byref(b)))
+        return t.value, v.value, b.value
+
     def set_skin(self, skin):
         self._chk(self._L.gbmd_set_skin(self.h, float(skin)))
 
@@ -471,6 +483,7 @@ _BATCH_SIG = {
     "gbmd_batch_set_targets": (["vp", "vp", "vp", "vp", "vp", "dbl", "dbl"], "i32"),
     "gbmd_batch_set_launch": (["vp", "i32", "i32"], "i32"),
     "gbmd_batch_set_small_block": (["vp", "i32"], "i32"),
+    "gbmd_batch_set_small_block_auto": (["vp"], "i32"),
     "gbmd_batch_run": (["vp", "i32", "i32", "i32"], "i32"),
     "gbmd_batch_synchronize": (["vp"], "i32"),
     "gbmd_batch_download": (["vp", "vp", "vp", "vp", "vp", "vp", "vp", "vp", "vp"], "i32"),
@@ -557,6 +570,10 @@ class Batch:
     def set_small_block(self, block):
         """Threads per block of the kernel for replicas of at most 512 atoms."""
         self._chk(self._L.gbmd_batch_set_small_block(self.h, int(block)))
+
+    def set_small_block_auto(self):
+        """Back to the library's choice, after a set_small_block."""
+        self._chk(self._L.gbmd_batch_set_small_block_auto(self.h))
 
     def run(self, adjoint=False, per_replica=False, use_graph=False):
         self._chk(self._L.gbmd_batch_run(self.h, 1 if adjoint else 0, 1 if per_replica else 0,

@@ -1111,6 +1111,22 @@ int gbmd_set_launch_ex(gbmd_context* c, int tpa, int vec, int block) {
   return GBMD_OK;
 }
 
+int gbmd_set_launch_auto(gbmd_context* c) {
+  if (!c) return GBMD_ERR_INVALID;
+  if (!c->launch_set) return GBMD_OK;
+  c->launch_set = false;
+  invalidate_list(c);  // choose_launch picks when the list is laid out again
+  return GBMD_OK;
+}
+
+int gbmd_get_launch_used(const gbmd_context* c, int* tpa, int* vec, int* block) {
+  if (!c) return GBMD_ERR_INVALID;
+  if (tpa) *tpa = c->tpa;
+  if (vec) *vec = c->vec;
+  if (block) *block = c->block;
+  return GBMD_OK;
+}
+
 int gbmd_set_launch(gbmd_context* c, int tpa, int block) {
   if (!c) return GBMD_ERR_INVALID;
   return gbmd_set_launch_ex(c, tpa, 1, block);

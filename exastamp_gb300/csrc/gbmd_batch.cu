@@ -1257,6 +1257,13 @@ int gbmd_batch_set_small_block(gbmd_batch* b, int block) {
   return GBMD_OK;
 }
 
+int gbmd_batch_set_small_block_auto(gbmd_batch* b) {
+  if (!b) return GBMD_ERR_INVALID;
+  b->small_block = 0;
+  drop_graph(b);
+  return GBMD_OK;
+}
+
 int gbmd_batch_set_launch(gbmd_batch* b, int block, int stencil) {
   if (!b || block < 64 || block > 512 || block % 32 || (stencil != 1 && stencil != 2))
     return berr(b, GBMD_ERR_INVALID, "block in [64,512] (multiple of 32), stencil 1 or 2");

@@ -172,6 +172,13 @@ int gbmd_get_launch(const gbmd_context* ctx, int* lanes_per_atom, int* block);
  * atom).  The list rows are laid out lanes_per_atom * entries wide. */
 int gbmd_set_launch_ex(gbmd_context* ctx, int lanes_per_atom, int entries_per_load, int block);
 int gbmd_get_launch_ex(const gbmd_context* ctx, int* lanes_per_atom, int* entries_per_load, int* block);
+/* Unless a launch is set the library picks one for the number of atoms and
+ * the potential when it lays out a list (up to 16 lanes x 4 entries for small
+ * systems), and gbmd_get_launch(_ex) report the nominal (1, 4, 256).
+ * gbmd_set_launch_auto returns to that after a gbmd_set_launch(_ex);
+ * gbmd_get_launch_used reports the launch of the list last laid out. */
+int gbmd_set_launch_auto(gbmd_context* ctx);
+int gbmd_get_launch_used(const gbmd_context* ctx, int* lanes_per_atom, int* entries_per_load, int* block);
 /* Threads per block of the EAM density kernels (0 = the pair kernels'
  * block).  On GB300 the density pass prefers smaller blocks than the force
  * pass (4 M-atom Cu: 128 vs 256); the autotuner sets both. */
@@ -436,6 +443,7 @@ int gbmd_batch_set_launch(gbmd_batch* b, int block, int stencil);
  * (several per SM): its threads per block, 64-256 (unless set: 512 with at
  * most four such replicas per SM, 256 with more). */
 int gbmd_batch_set_small_block(gbmd_batch* b, int block);
+int gbmd_batch_set_small_block_auto(gbmd_batch* b); /* as if never set */
 /* per_replica != 0: one launch per replica (the comparison mode);
  * use_graph != 0: the persistent launch is captured once and replayed */
 int gbmd_batch_run(gbmd_batch* b, int adjoint, int per_replica, int use_graph);

@@ -128,7 +128,7 @@ static void invalidate_list(gbmd_context* c) {
 // The FP64 re-test bands of the current potential for the current cells; where
 // none are laid out, rebuild_chain calls again when it has done so.
 int set_bands(gbmd_context* c) {
-  const double tol = c->band_margin * (c->grid_valid ? c->grid.tol : band_tol(c->rlist + c->list_buffer, 0.0));
+  const double tol = c->band_margin * (c->grid_valid ? c->grid_tol : band_tol(c->rlist + c->list_buffer, 0.0));
   auto band = [&](double rc, float& lo, float& hi) { band_limits(rc, tol, lo, hi); };
   if (c->pot == GBMD_POT_LJ || c->pot == GBMD_POT_LJ_MULTI) {
     const int nt = c->lj.ntypes;

@@ -92,7 +92,7 @@ struct PairHome {
       unpack_cell(A.cellpack[i], cx, cy, cz);
       nn = min(A.nnb[i], A.maxnb);
     }
-    slack = drift_slack(A.g, pf);
+    slack = drift_slack(A, pf);
     border = cx == 0 || cy == 0 || cz == 0 || cx == A.g.nc[0] - 1 || cy == A.g.nc[1] - 1 || cz == A.g.nc[2] - 1;
   }
   // FP64 separation of entry ent and its squared length
@@ -393,6 +393,8 @@ PairArgs make_args(gbmd_context* c, const ForceFlags& f) {
   A.y = c->Y();
   A.z = c->Z();
   const int o = c->cur ^ 1;
+  A.far = (float)(0x1p19 * c->grid_tol);
+  A.reach2 = (float)(2.0 * c->grid_reach);
   A.xo = c->rbuf[o];
   A.yo = c->rbuf[o] + c->cap;
   A.zo = c->rbuf[o] + 2 * c->cap;

@@ -99,8 +99,6 @@ struct Grid {
   int nc[3];
   double h[3], L[3], lo[3];
   float hf[3], hh[3];  // cell edge and half of it
-  double tol;          // band_tol of these cells
-  float far, reach2;   // drift_slack's: coordinates that tol covers, twice the radius the cells are built for
   int64_t ncells;
 };
 
@@ -209,6 +207,8 @@ struct gbmd_context {
   // cell grid + neighbour list
   gbmd::Grid grid{};
   bool grid_valid = false;
+  double grid_tol = 0.0;        // band_tol of the grid's cells
+  double grid_reach = 0.0;      // radius they are built for
   int32_t *cell_start = nullptr, *cell_fill = nullptr;
   int64_t cells_cap = 0;
   int32_t* scan_tmp = nullptr;

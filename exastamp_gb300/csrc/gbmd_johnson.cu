@@ -276,7 +276,7 @@ __device__ __forceinline__ EjGeom ej_geom(const PairArgs& A, const Params& P, ui
   G.dz = fmaf(twice_dz(ent), A.g.hh[2], pj.z - pi.z);
   G.d2 = fmaf(G.dx, G.dx, fmaf(G.dy, G.dy, G.dz * G.dz));
   G.in = G.d2 < P.rc2lo;
-  const float s = drift_slack(A.g, pi);
+  const float s = drift_slack(A, pi);
   if (s > 0.f) G.in = G.d2 < P.rc2lo - s;
   if (!G.in && G.d2 <= P.rc2hi + s)
     G.in = ej_exact_inside(A.posd, i, ent & GBMD_IDX_MASK, ent >> GBMD_IDX_BITS, cp, A.g, P.rcut2);

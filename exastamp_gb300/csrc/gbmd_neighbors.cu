@@ -767,7 +767,7 @@ static int build_list(gbmd_context* c, const int* gate) {
   const double R = c->rlist;
   const double R2 = R * R;
   float R2lo, R2hi;
-  band_limits(R, c->grid.tol, R2lo, R2hi);
+  band_limits(R, c->grid_tol, R2lo, R2hi);
   const int64_t npad = ((c->n + 31) / 32) * 32;
   const int W = list_width(c);
   const int64_t stride = npad * W;
@@ -851,9 +851,10 @@ static int rebuild_chain(gbmd_context* c, bool check_capacity, const int* gate) 
       g.hh[d] = 0.5f * g.hf[d];
       g.lo[d] = c->lo[d];
     }
-    g.tol = band_tol(R, std::max(g.h[0], std::max(g.h[1], g.h[2])));
-    g.far = (float)(0x1p19 * g.tol);
-    g.reach2 = (float)(2.0 * R);
+    // not in Grid: the exact tests take it by value, and 16 bytes more put it on
+    // the stack (list builder 215 -> 238 us, 256,000-atom LJ)
+    c->grid_tol = band_tol(R, std::max(g.h[0], std::max(g.h[1], g.h[2])));
+    c->grid_reach = R;
     int ra = ensure_cells(c, g.ncells);
     if (ra) return ra;
     c->grid_valid = true;
@@ -1146,7 +1147,7 @@ static int filter_list(gbmd_context* c, const int* gate) {
   c->maxnb = c->maxnb_out;
   const double R2 = c->rlist * c->rlist;
   float R2lo, R2hi;
-  band_limits(c->rlist, c->grid.tol, R2lo, R2hi);
+  band_limits(c->rlist, c->grid_tol, R2lo, R2hi);
   FilterArgs A;
   A.n = c->n;
   A.pf = c->POSF();

@@ -31,6 +31,7 @@ struct PairArgs {
   const double4_32a* posd;
   const int32_t* cellpack;
   Grid g;
+  float far, reach2;          // drift_slack: coordinates that band_tol covers, twice the radius the cells are built for
   const double *x, *y, *z;    // current FP64 positions
   double *xo, *yo, *zo;       // next positions (fuse 2)
   float4* posf_o;
@@ -116,9 +117,9 @@ static __device__ __noinline__ bool exact_inside(const double4_32a* __restrict__
 // 2^-21.1 m in d; four times that, 2^-19 m =: t, moves d^2 by t (2 rc + t) at
 // most.  For the kernels with registers to spare; the others take a wider band
 // (band_margin) where atoms may have drifted.
-__device__ __forceinline__ float drift_slack(const Grid& g, const float4& p) {
+__device__ __forceinline__ float drift_slack(const PairArgs& A, const float4& p) {
   const float m = fmaxf(fmaxf(fabsf(p.x), fabsf(p.y)), fabsf(p.z)), t = m * 0x1p-19f;
-  return m > g.far ? t * (g.reach2 + t) : 0.f;
+  return m > A.far ? t * (A.reach2 + t) : 0.f;
 }
 
 __device__ __forceinline__ GeomF geom_f(uint32_t ent, const float4& pj, const float4& pi, const Grid& g) {

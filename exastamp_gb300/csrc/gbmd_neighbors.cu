@@ -418,6 +418,7 @@ __device__ __noinline__ bool exact_within(const double* __restrict__ x, const do
 constexpr int BUILD_G = 16;       // home atoms per group
 constexpr int BUILD_CHUNK = 32;   // candidates staged per half-warp: one round of the warp
 constexpr int BUILD_WARPS = 4;    // warps per block, where shared memory allows
+constexpr int BUILD_LONG = 900;   // row capacity from which k_build_list_long builds the list
 constexpr int BUILD_SLACK = 16;   // row slots beyond maxnb: 8 tests at either end run unchecked
 
 // One warp's shared memory, followed by its BUILD_G rows of (maxnb + BUILD_SLACK) entries.
@@ -431,8 +432,8 @@ struct BuildSmem {
 };
 
 __host__ __device__ inline int build_rowlen(int maxnb) { return (maxnb + BUILD_SLACK) | 1; }  // odd: rows start in different banks
-__host__ __device__ inline size_t build_smem(int maxnb, int homes) {
-  return sizeof(BuildSmem) + (size_t)((homes * build_rowlen(maxnb) + 3) & ~3) * sizeof(uint32_t);
+__host__ __device__ inline size_t build_smem(int maxnb) {
+  return sizeof(BuildSmem) + (size_t)(BUILD_G * build_rowlen(maxnb)) * sizeof(uint32_t);
 }
 
 struct BuildArgs {
@@ -444,9 +445,11 @@ struct BuildArgs {
   float R2lo, R2hi;
   uint32_t* nbr;
   int32_t* nnb;
-  int maxnb, W, wsh, tsh, homes, parts;  // homes: atoms per group; parts: warps per cell
+  int maxnb, W, wsh, tsh, parts;  // parts: warps per cell
   int64_t stride;
   int* err;
+  int64_t n;
+  const int32_t* cellpack;
 };
 
 // One round of staging: the candidates qa .. qa + 31, in reverse with `rev`,
@@ -557,7 +560,7 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32, 6) k_build_list_cells(const 
   const int lane = threadIdx.x & 31, half = lane >> 4, hl = lane & 15;
   const int rowlen = build_rowlen(A.maxnb);
   unsigned char* const mine =
-      reinterpret_cast<unsigned char*>(build_shared) + (threadIdx.x >> 5) * build_smem(A.maxnb, A.homes);
+      reinterpret_cast<unsigned char*>(build_shared) + (threadIdx.x >> 5) * build_smem(A.maxnb);
   BuildSmem& S = *reinterpret_cast<BuildSmem*>(mine);
   uint32_t* const rows = reinterpret_cast<uint32_t*>(mine + sizeof(BuildSmem));
   const int64_t items = A.ncells * A.parts;
@@ -566,7 +569,7 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32, 6) k_build_list_cells(const 
     const int64_t cell = item / A.parts;
     const int part = (int)(item - cell * A.parts);
     const int hb = A.cstart[cell], nh = A.cstart[cell + 1] - hb;
-    if (part * A.homes >= nh) continue;
+    if (part * BUILD_G >= nh) continue;
     const int cx = (int)(cell % g.nc[0]), cy = (int)((cell / g.nc[0]) % g.nc[1]),
               cz = (int)(cell / ((int64_t)g.nc[0] * g.nc[1]));
     // stencil cell of this lane
@@ -608,8 +611,8 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32, 6) k_build_list_cells(const 
     // walk's d2, so no candidate the walk would keep is dropped
     const float R2keep = A.R2hi * (1.0f + 0x1p-10f);
     int warp_max = 0;
-    for (int h0 = part * A.homes; h0 < nh; h0 += A.parts * A.homes) {
-      const bool hv = hl < A.homes && h0 + hl < nh;
+    for (int h0 = part * BUILD_G; h0 < nh; h0 += A.parts * BUILD_G) {
+      const bool hv = h0 + hl < nh;
       const int i = hb + h0 + hl;
       float4 pi = make_float4(FAR, FAR, FAR, 0.f);
       if (hv) pi = A.pf[i];
@@ -742,6 +745,57 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32, 6) k_build_list_cells(const 
   }
 }
 
+// The same list where rows are long: a warp per atom, 32 candidates at a time,
+// the hits straight to the row in global memory.  The walk above holds 16 rows
+// a warp in shared memory: at BUILD_LONG entries an SM has 4 of its warps, from
+// 3,000 entries on a group has fewer atoms, and a row of 51,000 does not fit at
+// all.  Rebuild, us, walk above / this: 256,000 atoms, capacity 560: 1,492 / 2,091;
+// 728: 2,217 / 2,485; 1,000: 3,761 / 3,035; 62,500 atoms, 560: 623 / 623;
+// 1,000: 1,330 / 861; 2,750: 8,400 / 2,270; 8,788 atoms, 6,200: 39,000 / 3,290;
+// 19,600: 6,150,000 / 157,000.
+template <bool HALF>
+__global__ void __launch_bounds__(128) k_build_list_long(const __grid_constant__ BuildArgs A,
+                                                         const __grid_constant__ Grid g,
+                                                         const int* __restrict__ gate) {
+  if (gate && !*gate) return;
+  const int lane = threadIdx.x & 31;
+  int longest = 0;
+  for (int64_t a = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5; a < A.n;
+       a += ((int64_t)gridDim.x * blockDim.x) >> 5) {
+    const int i = (int)a, cp = A.cellpack[a], cx = cp & 1023, cy = (cp >> 10) & 1023, cz = cp >> 20;
+    const float4 pi = A.pf[a];
+    uint32_t* const row = A.nbr + (size_t)a * A.W;
+    int found = 0;
+    for (int s = 0; s < 27; ++s) {
+      const int dx = s % 3 - 1, dy = (s / 3) % 3 - 1, dz = s / 9 - 1;
+      const int64_t x = cx + dx - image_of(cx, dx, g.nc[0]) * g.nc[0], y = cy + dy - image_of(cy, dy, g.nc[1]) * g.nc[1],
+                    z = cz + dz - image_of(cz, dz, g.nc[2]) * g.nc[2], c = (z * g.nc[1] + y) * g.nc[0] + x;
+      const uint32_t code = code_of(dx, dy, dz), self = (uint32_t)i;
+      const int end = A.cstart[c + 1];
+      for (int q = A.cstart[c]; q < end; q += 32) {
+        const int k = q + lane;
+        const uint32_t w = (uint32_t)k | code << GBMD_IDX_BITS;
+        bool hit = k < end && (HALF ? k > i : w != self);
+        if (hit) {
+          const float d2 = build_d2(A.pf, g, pi, w);
+          hit = d2 <= A.R2hi;
+          if (hit && d2 >= A.R2lo) hit = exact_within(A.x, A.y, A.z, i, k, code, cx, cy, cz, g, A.R2);
+        }
+        const unsigned hits = __ballot_sync(0xffffffffu, hit);
+        const int p = found + __popc(hits & ((1u << lane) - 1u));
+        if (hit && p < A.maxnb) row[(size_t)(p >> A.wsh) * A.stride + list_word(p & (A.W - 1), A.wsh, A.tsh)] = w;
+        found += __popc(hits);
+      }
+    }
+    if (lane == 0) {
+      A.nnb[a] = found;
+      if (found > A.maxnb) atomicOr(&A.err[ERRW_FLAGS], GBMD_DEVERR_NBR_OVERFLOW);
+    }
+    longest = max(longest, found);
+  }
+  if (lane == 0 && longest > 0) atomicMax(&A.err[ERRW_MAXNB], longest);
+}
+
 static inline unsigned nblk(int64_t n, int b) { return (unsigned)((n + b - 1) / b); }
 
 // Blocks of a rebuild-chain launch.  Ungated launches cover the data once;
@@ -796,13 +850,14 @@ static int build_list(gbmd_context* c, const int* gate) {
   A.tsh = log2_of(c->tpa);
   A.stride = stride;
   A.err = c->d_err;
-  // rows of 16 atoms fit a warp's shared memory up to some 3,000 entries an
-  // atom; beyond that a group takes fewer atoms
-  const size_t most = 200 * 1024;
-  A.homes = BUILD_G;
-  while (A.homes > 1 && build_smem(c->maxnb, A.homes) > most) --A.homes;
-  const size_t per_warp = build_smem(c->maxnb, A.homes);
-  if (per_warp > most) return set_error(c, GBMD_ERR_TOO_LARGE, "%d neighbours per atom", c->maxnb);
+  A.n = c->n;
+  A.cellpack = c->cellpack;
+  if (c->maxnb >= BUILD_LONG) {
+    auto kern = c->newton3 ? k_build_list_long<true> : k_build_list_long<false>;
+    kern<<<chain_blocks(c, c->n, 4, gate, 8), 128, 0, c->stream>>>(A, c->grid, gate);
+    return GBMD_OK;
+  }
+  const size_t per_warp = build_smem(c->maxnb);
   // the widest blocks of which an SM holds several
   int nw = BUILD_WARPS;
   while (nw > 1 && nw * per_warp > 56 * 1024) nw >>= 1;
@@ -813,7 +868,7 @@ static int build_list(gbmd_context* c, const int* gate) {
   const bool loop = gate && !c->full_chain_grids;  // capped grid striding over the cells
   auto kern = loop ? (c->newton3 ? k_build_list_cells<true, true> : k_build_list_cells<true, false>)
                    : (c->newton3 ? k_build_list_cells<false, true> : k_build_list_cells<false, false>);
-  const size_t smem = nw * per_warp;
+  const size_t smem = nw * per_warp, most = 64 * 1024;  // (a warp's rows of BUILD_LONG entries: 60 KB)
   if (smem > 48 * 1024)
     GBMD_CUDA(c, cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
   const int per_sm = (int)std::max<size_t>(1, 220 * 1024 / (smem + 1024));

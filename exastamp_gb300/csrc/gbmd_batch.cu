@@ -15,7 +15,7 @@
 // own global scratch (at least 2 x 128 entries per atom), which the density, force
 // and adjoint passes read, four entries a lane in flight.  A replica with a
 // fuller atom walks the cells in every pass instead.  Pair arithmetic is FP32
-// with compensated force and density sums; per-replica sums (energy, virial,
+// with force, energy and density sums compensated pair by pair; per-replica sums (energy, virial,
 // loss, gradient) are FP64 and written to the replica's own row, so results do
 // not depend on which block ran which replica.
 //
@@ -236,17 +236,15 @@ struct PairList {
 __device__ __forceinline__ float cell_unit(uint32_t b, float bias) { return __int_as_float(0x4B000000u | b) - bias; }
 
 // Lane t's share of the pairs of slot s, fn(k, dx, dy, dz, d2, ok), four at a
-// time with done() after each four; pairs with ok = false count nothing (their
-// separation is zero).  From the list, or from the cells (cap = 0) where some
+// time; pairs with ok = false count nothing (their separation is zero).  From the list, or from the cells (cap = 0) where some
 // atom's pairs do not fit in it.
-template <class SM, class Fn, class Done>
+template <class SM, class Fn>
 __device__ __forceinline__ void visit(const BatchArgs& A, const RepGeom& g, const SM& sm, const uint32_t* nbl,
-                                      int cap, int s, int t, Fn fn, Done done) {
+                                      int cap, int s, int t, Fn fn) {
   const int T = 1 << g.tsh;
   if (cap == 0) {
     for_pairs(A, g, sm, s, t, T, [&](int k, float dx, float dy, float dz, float d2, uint32_t) {
       fn(k, dx, dy, dz, d2, true);
-      done();
     });
     return;
   }
@@ -271,7 +269,6 @@ __device__ __forceinline__ void visit(const BatchArgs& A, const RepGeom& g, cons
       const float d2 = pair_d2(pi, sm.pos[k], sx, sy, sz, ddx, ddy, ddz);
       fn(k, ddx, ddy, ddz, d2, q + u * T < n);
     }
-    done();
 #pragma unroll
     for (int u = 0; u < 4; ++u) e[u] = nxt[u];
   }
@@ -611,7 +608,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch(const __grid_constant__ Ba
     // ---- density + embedding
     for (int s0 = 0; s0 < n; s0 += ns) {
       const int s = s0 + (tid >> g.tsh);
-      float acc = 0.f, comp = 0.f, part = 0.f;
+      float acc = 0.f, comp = 0.f;
       if (s < n)
         visit(A, g, sm, nbl, listed, s, t,
               [&](int k, float dx, float dy, float dz, float d2, bool ok) {
@@ -619,11 +616,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch(const __grid_constant__ Ba
                 float q;
                 const int m = knot(fmaf(rr, A.rdr, 1.f), A.nr - 1, q);
                 const float val = sval(A.rhor4[m], q);
-                part += ok ? val : 0.f;
-              },
-              [&]() {
-                kahan_add(acc, comp, part);
-                part = 0.f;
+                kahan_add(acc, comp, ok ? val : 0.f);
               });
       reduce_kahan(acc, comp, T);
       if (s < n && t == 0) sm.rho[s] = acc - comp;
@@ -645,7 +638,6 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch(const __grid_constant__ Ba
     for (int s0 = 0; s0 < n; s0 += ns) {
       const int s = s0 + (tid >> g.tsh);
       float fx = 0.f, fy = 0.f, fz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f, ee = 0.f, ce = 0.f;
-      float px = 0.f, py = 0.f, pz = 0.f, pe = 0.f;
       float v[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
       if (s < n) {
         const float fpi = sm.pos[s].w;
@@ -662,10 +654,10 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch(const __grid_constant__ Ba
                 const float phip = (z2d - phi) * rs;
                 const float psip = fmaf(fpi + sm.pos[k].w, rhop, phip);
                 const float fpair = ok ? psip * rs : 0.f;
-                px = fmaf(dx, fpair, px);
-                py = fmaf(dy, fpair, py);
-                pz = fmaf(dz, fpair, pz);
-                pe += ok ? 0.5f * phi : 0.f;
+                kahan_add(fx, cx, dx * fpair);
+                kahan_add(fy, cy, dy * fpair);
+                kahan_add(fz, cz, dz * fpair);
+                kahan_add(ee, ce, ok ? 0.5f * phi : 0.f);
                 const float hh = -0.5f * fpair;
                 v[0] = fmaf(hh * dx, dx, v[0]);
                 v[1] = fmaf(hh * dy, dy, v[1]);
@@ -673,13 +665,6 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch(const __grid_constant__ Ba
                 v[3] = fmaf(hh * dx, dy, v[3]);
                 v[4] = fmaf(hh * dx, dz, v[4]);
                 v[5] = fmaf(hh * dy, dz, v[5]);
-              },
-              [&]() {
-                kahan_add(fx, cx, px);
-                kahan_add(fy, cy, py);
-                kahan_add(fz, cz, pz);
-                kahan_add(ee, ce, pe);
-                px = py = pz = pe = 0.f;
               });
       }
       reduce_kahan(fx, cx, T);
@@ -742,8 +727,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch(const __grid_constant__ Ba
                   const float4 dr = A.fz8[2 * m];
                   const float rhop = fmaf(fmaf(dr.x, q, dr.y), q, dr.z);
                   Gs = ok ? fmaf(sij + sji, rhop, Gs) : Gs;
-                },
-                []() {});
+                });
         }
         reduce_plain(Gs, T);
         if (s < n && t == 0) {

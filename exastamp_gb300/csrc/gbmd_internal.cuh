@@ -178,7 +178,7 @@ struct gbmd_context {
   int32_t* src = nullptr;                 // scratch: new position -> old position
   float* fpf = nullptr;                   // EAM F'(rho) FP32 (mixed)
   float4* pfp = nullptr;                  // single-element EAM: FP32 position with F'(rho) in w (mixed)
-  float4* f0 = nullptr;                   // mixed one-element EAM without energies: sum phi' u from the density pass
+  float4* f0 = nullptr;                   // mixed one-element EAM without energies: sum phi' u from the density pass (pack_f0)
   float* bpair = nullptr;                 // and rho'(r)/r per list entry, in the list's layout
   int64_t bpair_cap = 0;
   bool rho_bonds = false;                 // the last density pass left f0 and bpair

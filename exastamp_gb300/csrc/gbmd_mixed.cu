@@ -448,8 +448,7 @@ __device__ __forceinline__ void atom_finish(const PairArgs& A, int64_t i, const 
 // row touches 32 sectors per store, nine times.
 template <int T, bool EV>
 __device__ __forceinline__ void block_epilogue(const PairArgs& A, int64_t i0, const PairSums& S,
-                                               const float* __restrict__ epf,
-                                               const float4* __restrict__ f0 = nullptr) {
+                                               const float* __restrict__ epf) {
   constexpr int NV = EV ? 10 : 3;
   constexpr bool SHARED = T > 1 || EV;
   __shared__ float sums[SHARED ? NV : 1][SHARED ? 256 / T : 1];
@@ -484,12 +483,6 @@ __device__ __forceinline__ void block_epilogue(const PairArgs& A, int64_t i0, co
   }
   const int64_t i = i0 + threadIdx.x;
   if (i >= A.n) return;
-  if (f0) {
-    const float4 f = f0[i];
-    R.f[0] += f.x;
-    R.f[1] += f.y;
-    R.f[2] += f.z;
-  }
   const int ti = __float_as_int(A.posf[i].w);
   const float im = A.inv_massf[ti];
   atom_epilogue<true>(A, i, ti, 0., 0., 0., R.f[0] * im, R.f[1] * im, R.f[2] * im,
@@ -827,8 +820,46 @@ __global__ void __launch_bounds__(256) k_eam_force_staged(PairArgs A, EamDev E, 
 // 2 M atoms 933 against 874 us.)
 // ---------------------------------------------------------------------------
 struct BondSums {
-  float rho, f[3];
+  float rho, s[3], c[3];  // force sum s - c, unrounded
 };
+
+// f0 keeps both parts, so that the force is rounded once, as one compensated sum
+// over both passes would be: f, and in w the three low parts, 10 bits each, in
+// units of 2^-9 of the last place of f (below half of which they lie), to and
+// from integers through the mantissa.
+__device__ __forceinline__ int low_part(float f, float lo) {
+  const float to = __int_as_float(0x7f000000 - (__float_as_int(f) & 0x7f800000));  // 1 / the power of two below f
+  return __float_as_int(fmaf(lo * to, 0x1p32f, 12582912.0f)) & 1023;
+}
+__device__ __forceinline__ float low_part_of(float f, int bits) {
+  const float q = __int_as_float(0x4b000000 | ((bits & 1023) ^ 512)) - 8389120.0f;
+  return __int_as_float(__float_as_int(f) & 0x7f800000) * (q * 0x1p-32f);
+}
+__device__ __forceinline__ float4 pack_f0(const BondSums& S) {
+  float f[3];
+  int w = 0;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    f[k] = S.s[k] - S.c[k];
+    w |= low_part(f[k], (S.s[k] - f[k]) - S.c[k]) << (10 * k);
+  }
+  return make_float4(f[0], f[1], f[2], __int_as_float(w));
+}
+
+// (a + alo) + (b + blo), rounded once but for the low parts' own rounding.
+__device__ __forceinline__ float sum_parts(float a, float alo, float b, float blo) {
+  const float t = a + b, z = t - a, e = (a - (t - z)) + (b - z);
+  return t + (e + (alo + blo));
+}
+
+// The force sum of both passes from the force pass's.
+__device__ __forceinline__ void add_f0(const PairArgs& A, int64_t i, const BondSums& S, float (&f)[3]) {
+  const float4 a = __ldg(&A.f0[i]);
+  const int w = __float_as_int(a.w);
+  f[0] = sum_parts(a.x, low_part_of(a.x, w), S.s[0], -S.c[0]);
+  f[1] = sum_parts(a.y, low_part_of(a.y, w >> 10), S.s[1], -S.c[1]);
+  f[2] = sum_parts(a.z, low_part_of(a.z, w >> 20), S.s[2], -S.c[2]);
+}
 
 template <int T, class Fetch>
 __device__ __forceinline__ BondSums eam_rho_bonds_atom(const PairArgs& A, const EamDev& E, int64_t i, int lane,
@@ -886,7 +917,7 @@ __device__ __forceinline__ BondSums eam_rho_bonds_atom(const PairArgs& A, const 
   });
 #pragma unroll
   for (int k = 0; k < 4; ++k) group_reduce_kahan<T>(s[k], c[k]);
-  return BondSums{s[0] - c[0], {s[1] - c[1], s[2] - c[2], s[3] - c[3]}};
+  return BondSums{s[0] - c[0], {s[1], s[2], s[3]}, {c[1], c[2], c[3]}};
 }
 
 template <int T, bool PIECE>
@@ -895,31 +926,37 @@ __global__ void __launch_bounds__(128, 7) k_eam_rho_bonds(const __grid_constant_
                                                           float* __restrict__ fpf, float4* __restrict__ pfp) {
   const int64_t gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
   int64_t i = PIECE ? A.i0 + gt / T : gt / T;
-  BondSums S = eam_rho_bonds_atom<T>(A, E, i, (int)(gt % T), i < A.n, GlobalFetch{A.posf});
+  const BondSums S = eam_rho_bonds_atom<T>(A, E, i, (int)(gt % T), i < A.n, GlobalFetch{A.posf});
+  float rho = S.rho;
+  float4 f0 = pack_f0(S);
   if (T > 1) {
-    // the embedding of the block's atoms on its first blockDim / T threads
-    __shared__ float sums[4][T > 1 ? 128 / T : 1];
+    // the embedding of the block's atoms on its first blockDim / T threads.  Five
+    // floats an atom: with seven (the sums unpacked) the seven blocks of an SM
+    // take the next size of shared memory from L1 (864,000 atoms: 184 -> 192 us)
+    __shared__ float sums[5][T > 1 ? 128 / T : 1];
     const int nat = (int)blockDim.x / T;
     if (threadIdx.x % T == 0) {
-      sums[0][threadIdx.x / T] = S.rho;
-#pragma unroll
-      for (int k = 0; k < 3; ++k) sums[1 + k][threadIdx.x / T] = S.f[k];
+      const int a = (int)threadIdx.x / T;
+      sums[0][a] = rho;
+      sums[1][a] = f0.x;
+      sums[2][a] = f0.y;
+      sums[3][a] = f0.z;
+      sums[4][a] = f0.w;
     }
     __syncwarp();
     __syncthreads();
     if ((int)threadIdx.x >= nat) return;
-    S.rho = sums[0][threadIdx.x];
-#pragma unroll
-    for (int k = 0; k < 3; ++k) S.f[k] = sums[1 + k][threadIdx.x];
+    rho = sums[0][threadIdx.x];
+    f0 = make_float4(sums[1][threadIdx.x], sums[2][threadIdx.x], sums[3][threadIdx.x], sums[4][threadIdx.x]);
     i = (PIECE ? A.i0 : 0) + blockIdx.x * (int64_t)nat + threadIdx.x;
   }
   if (i >= A.n) return;
-  eam_embed<false, true>(A, E, i, S.rho, fpf, nullptr, pfp);
-  A.f0[i] = make_float4(S.f[0], S.f[1], S.f[2], 0.f);
+  A.f0[i] = f0;
+  eam_embed<false, true>(A, E, i, rho, fpf, nullptr, pfp);
 }
 
 template <int T, class Fetch>
-__device__ __forceinline__ PairSums eam_force_bonds_atom(const PairArgs& A, const float* __restrict__ fpf, int64_t i,
+__device__ __forceinline__ BondSums eam_force_bonds_atom(const PairArgs& A, const float* __restrict__ fpf, int64_t i,
                                                          int lane, bool live, const Fetch& fetch) {
   const int nn = live ? min(A.nnb[i], A.maxnb) : 0;
   const float4 pi = live ? A.posf[i] : make_float4(0.f, 0.f, 0.f, 0.f);
@@ -967,12 +1004,7 @@ __device__ __forceinline__ PairSums eam_force_bonds_atom(const PairArgs& A, cons
   }
 #pragma unroll
   for (int k = 0; k < 3; ++k) group_reduce_kahan<T>(s[k], c[k]);
-  PairSums S;
-  S.f[0] = s[0] - c[0];
-  S.f[1] = s[1] - c[1];
-  S.f[2] = s[2] - c[2];
-  S.e = 0.f;
-  return S;
+  return BondSums{0.f, {s[0], s[1], s[2]}, {c[0], c[1], c[2]}};
 }
 
 template <int T, bool PIECE>
@@ -980,9 +1012,35 @@ __global__ void __launch_bounds__(256, 4) k_eam_force_bonds(const __grid_constan
                                                             const float* __restrict__ fpf,
                                                             const float4* __restrict__ pfp) {
   const int64_t gt = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-  const int64_t i = PIECE ? A.i0 + gt / T : gt / T;
-  const PairSums S = eam_force_bonds_atom<T>(A, fpf, i, (int)(gt % T), i < A.n, GlobalFetch{pfp});
-  block_epilogue<T, false>(A, (PIECE ? A.i0 : 0) + blockIdx.x * (int64_t)(blockDim.x / T), S, nullptr, A.f0);
+  int64_t i = PIECE ? A.i0 + gt / T : gt / T;
+  BondSums S = eam_force_bonds_atom<T>(A, fpf, i, (int)(gt % T), i < A.n, GlobalFetch{pfp});
+  // the epilogue of the block's atoms on its first blockDim / T threads, as block_epilogue's
+  if (T > 1) {
+    __shared__ float sums[6][T > 1 ? 256 / T : 1];
+    const int nat = (int)blockDim.x / T;
+    if (threadIdx.x % T == 0) {
+#pragma unroll
+      for (int k = 0; k < 3; ++k) {
+        sums[k][threadIdx.x / T] = S.s[k];
+        sums[3 + k][threadIdx.x / T] = S.c[k];
+      }
+    }
+    __syncwarp();
+    __syncthreads();
+    if ((int)threadIdx.x >= nat) return;
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      S.s[k] = sums[k][threadIdx.x];
+      S.c[k] = sums[3 + k][threadIdx.x];
+    }
+    i = (PIECE ? A.i0 : 0) + blockIdx.x * (int64_t)nat + threadIdx.x;
+  }
+  if (i >= A.n) return;
+  float f[3];
+  add_f0(A, i, S, f);
+  const int ti = __float_as_int(A.posf[i].w);
+  const float im = A.inv_massf[ti];
+  atom_epilogue<true>(A, i, ti, 0., 0., 0., f[0] * im, f[1] * im, f[2] * im, 0.0, nullptr);
 }
 
 // The same with the neighbour positions from the block's staged cells.
@@ -999,7 +1057,7 @@ __global__ void __launch_bounds__(256) k_eam_rho_bonds_staged(const __grid_const
     const BondSums S = ok ? eam_rho_bonds_atom<1>(A, E, i, 0, true, StagedFetch{staged_pos, rows})
                           : eam_rho_bonds_atom<1>(A, E, i, 0, true, GlobalFetch{A.posf});
     eam_embed<false, true>(A, E, i, S.rho, fpf, nullptr, pfp);
-    A.f0[i] = make_float4(S.f[0], S.f[1], S.f[2], 0.f);
+    A.f0[i] = pack_f0(S);
   }
 }
 
@@ -1013,12 +1071,11 @@ __global__ void __launch_bounds__(256) k_eam_force_bonds_staged(const __grid_con
   int64_t a0, a1;
   const bool ok = stage_cells(A.g, cstart, pfp, K, cap, staged_pos, rows, sh, a0, a1);
   for (int64_t i = a0 + threadIdx.x; i < a1; i += blockDim.x) {
-    PairSums S = ok ? eam_force_bonds_atom<1>(A, fpf, i, 0, true, StagedFetch{staged_pos, rows})
-                    : eam_force_bonds_atom<1>(A, fpf, i, 0, true, GlobalFetch{pfp});
-    const float4 f = A.f0[i];
-    S.f[0] += f.x;
-    S.f[1] += f.y;
-    S.f[2] += f.z;
+    const BondSums B = ok ? eam_force_bonds_atom<1>(A, fpf, i, 0, true, StagedFetch{staged_pos, rows})
+                          : eam_force_bonds_atom<1>(A, fpf, i, 0, true, GlobalFetch{pfp});
+    PairSums S;
+    add_f0(A, i, B, S.f);
+    S.e = 0.f;
     atom_finish<false>(A, i, S, 0.f);
   }
 }

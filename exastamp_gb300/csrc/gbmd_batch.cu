@@ -12,12 +12,13 @@
 // with cells >= rcut, or S = 2 with cells >= rcut/2), with the same FP32
 // screen + FP64 re-test of the ambiguous band as the main path, so the
 // in-cutoff pair set is the FP64 one; they go to a pair list in the block's
-// own global scratch (at least 2 x 128 entries per atom), which the density, force
-// and adjoint passes read, four entries a lane in flight.  A replica with a
+// own global scratch (at least 2 x 128 entries per atom), which the density,
+// force and adjoint passes read, four entries a lane in flight.  A replica with a
 // fuller atom walks the cells in every pass instead.  Pair arithmetic is FP32
-// with force, energy and density sums compensated pair by pair; per-replica sums (energy, virial,
-// loss, gradient) are FP64 and written to the replica's own row, so results do
-// not depend on which block ran which replica.
+// with force, energy and density sums compensated pair by pair; per-replica sums
+// (energy, virial, loss, gradient) are FP64 and written to the replica's own row.
+// Neither depends on which block ran the replica, nor for replicas of up to 512
+// atoms on the block's size: their results are the same bit for bit in any batch.
 //
 // What bounds it: with one lane per atom and one pair in flight, latency (256
 // replicas of 243 atoms took 538 us, forward and adjoint, now 192; 4,096 of
@@ -105,6 +106,10 @@ struct PairRecord {
 template <int MAXA, int MAXC, int MAXT>
 struct SmemT {
   static constexpr uint32_t ATOMS = MAXA;  // a power of two of at most 2,048
+  static constexpr int ROWS = MAXT / 32;
+  // replicas that MAXT threads take in one go: every turn of a smaller block has
+  // its own rows of red; larger replicas take several goes of the block as it is
+  static constexpr bool TURNS = MAXA <= MAXT;
   float4 pos[MAXA];   // by slot: cell-relative FP32 position, w = F'(rho)
   float4 gfe[MAXA];   // adjoint: dL/dF (xyz) and dL/dE (w) by slot; before that, positions by atom
   PairRecord rec[MAXT / 32];
@@ -470,16 +475,23 @@ __device__ __forceinline__ void block_sync() {
   __syncthreads();
 }
 
-// Sums of NV quantities over the block, to red[0][0 .. NV).
+// The block's sums of NV quantities, in two steps: a warp's to row `row` of red,
+// and the first `rows` rows' to red[0][0 .. NV).  The atoms are dealt out over
+// MAXT threads whatever the block has: a block of fewer takes them in several
+// turns, and each turn of each of its warps has a row of its own, so that a
+// replica's sums are added in one order whatever the block (SmemT::turn_row).
 template <int NV, class SM>
-__device__ __forceinline__ void block_sum(SM& sm, double (&v)[NV]) {
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const int q = warp_sum_transposed<NV>(v, lane);
-  if (q >= 0) sm.red[w][q] = v[0];
+__device__ __forceinline__ void warp_sums(SM& sm, double (&v)[NV], int row) {
+  const int q = warp_sum_transposed<NV>(v, threadIdx.x & 31);
+  if (q >= 0 && row < SM::ROWS) sm.red[row][q] = v[0];
+}
+
+template <int NV, class SM>
+__device__ __forceinline__ void block_sums(SM& sm, int rows) {
   block_sync();
   if (threadIdx.x < NV) {
     double a = 0.0;
-    for (int k = 0; k < (int)(blockDim.x >> 5); ++k) a += sm.red[k][threadIdx.x];
+    for (int k = 0; k < rows; ++k) a += sm.red[k][threadIdx.x];
     sm.red[0][threadIdx.x] = a;
   }
   block_sync();
@@ -520,8 +532,8 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch(const __grid_constant__ Ba
         g.base = A.off[r];
         g.n = (int)(A.off[r + 1] - g.base);
         g.ncells = ncells;
-        int tsh = 0;  // the most lanes per atom that take the replica in one go
-        while (tsh < 5 && (g.n << (tsh + 1)) <= B) ++tsh;
+        int tsh = 0;  // the most lanes per atom with which MAXT threads take the replica in one go
+        while (tsh < 5 && (g.n << (tsh + 1)) <= (SM::TURNS ? MAXT : B)) ++tsh;
         g.tsh = tsh;
         sm.overflow = 0;
         // the band covers the rounding of coordinates in cells of edge h, as
@@ -597,6 +609,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch(const __grid_constant__ Ba
     }
     block_sync();
     const int T = 1 << g.tsh, t = tid & (T - 1), ns = B >> g.tsh;  // ns atoms at a time
+    const int rows = SM::TURNS ? ((n << g.tsh) + 31) >> 5 : B >> 5;  // of red that hold sums
     // ---- pair list: one walk over the cells (FP32 screen, FP64 band
     // re-test), then every pass below reads the list
     uint32_t* nbl = A.nbl + (A.single >= 0 ? (size_t)0 : (size_t)blockIdx.x * MAXA * NBL_MAX);
@@ -635,6 +648,7 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch(const __grid_constant__ Ba
     double sum[NV];
 #pragma unroll
     for (int q = 0; q < NV; ++q) sum[q] = 0.0;
+    int row_of = tid >> 5;
     for (int s0 = 0; s0 < n; s0 += ns) {
       const int s = s0 + (tid >> g.tsh);
       float fx = 0.f, fy = 0.f, fz = 0.f, cx = 0.f, cy = 0.f, cz = 0.f, ee = 0.f, ce = 0.f;
@@ -696,8 +710,15 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch(const __grid_constant__ Ba
           sm.gfe[s] = make_float4(narrow(twF * ex), narrow(twF * ey), narrow(twF * ez), narrow(2.0 * A.wE * de));
         }
       }
+      if (SM::TURNS || s0 + ns >= n) {
+        __syncwarp();
+        warp_sums<NV>(sm, sum, row_of);
+        row_of += B >> 5;
+#pragma unroll
+        for (int q = 0; q < NV; ++q) sum[q] = 0.0;
+      }
     }
-    block_sum<NV>(sm, sum);
+    block_sums<NV>(sm, rows);
     if (tid < (ADJ ? 11 : 10)) {
       // row-major virial from xx yy zz xy xz yz
       const int q = tid == 0 ? 0 : (tid == 10 ? 7 : 1 + (int)((0x254513430ll >> (4 * (tid - 1))) & 15));
@@ -708,6 +729,8 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch(const __grid_constant__ Ba
       double fr[BMAX_PARAMS];  // dF/dtheta terms
 #pragma unroll
       for (int p = 0; p < BMAX_PARAMS; ++p) fr[p] = 0.0;
+      block_sync();  // red is read
+      row_of = tid >> 5;
       // ---- adjoint sweep 1: G_i, then the embedding terms and lambda_i
       for (int s0 = 0; s0 < n; s0 += ns) {
         const int s = s0 + (tid >> g.tsh);
@@ -746,9 +769,15 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch(const __grid_constant__ Ba
               fr[p] += widen(fmaf(gi.w, sval(dc, q) + (over ? dfp * (R - A.rhomax) : 0.f), Gs * dfp));
             }
         }
+        if (SM::TURNS || s0 + ns >= n) {
+          __syncwarp();
+          warp_sums<BMAX_PARAMS>(sm, fr, row_of);
+          row_of += B >> 5;
+#pragma unroll
+          for (int p = 0; p < BMAX_PARAMS; ++p) fr[p] = 0.0;
+        }
       }
-      block_sync();  // red is read
-      block_sum<BMAX_PARAMS>(sm, fr);
+      block_sums<BMAX_PARAMS>(sm, rows);
       if (tid < BMAX_PARAMS) {
         double v = 0.0;
         for (int p = 0; p < A.nfr; ++p)
@@ -811,7 +840,19 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch(const __grid_constant__ Ba
             acc[b] = 0.f;
           }
       };
+      // a turn's sums of eight tables at a time, to its row of red
+      auto store_tables = [&]() {
+#pragma unroll
+        for (int b = 0; b < MAX_TABLES / 8; ++b) {
+          accd[b] += __shfl_xor_sync(0xffffffffu, accd[b], 8);
+          accd[b] += __shfl_xor_sync(0xffffffffu, accd[b], 16);
+          if (lane < 8 && row_of < SM::ROWS) sm.red[row_of][lane + 8 * b] = accd[b];
+          accd[b] = 0.0;
+        }
+        row_of += B >> 5;
+      };
       block_sync();  // lambda is complete; red is read
+      row_of = wid;
       if (nb > 0) {
         const float bias = 8388608.0f + (float)A.S;
         const uint32_t none = (uint32_t)(A.S | (A.S << 3) | (A.S << 6)) << 11;
@@ -837,52 +878,40 @@ __global__ void __launch_bounds__(MAXT, MINB) k_batch(const __grid_constant__ Ba
             e = nxt;
           }
           settle();
-      }
-        for (int b = 0; b < nb && !list_ok; ++b) {
+          if (SM::TURNS || s0 + ns >= n) store_tables();
+        }
+        for (int s0 = 0; s0 < n && !list_ok; s0 += ns) {
           // from the cells: a lane reads eight tables of each of its own pairs
-          double sum8[8];
-#pragma unroll
-          for (int k = 0; k < 8; ++k) sum8[k] = 0.0;
-          for (int s = tid >> g.tsh; s < n; s += ns) {
-            const float4 gi = sm.gfe[s];
-            const float fpi = sm.pos[s].w, lam = sm.rho[s];
+          const int s = s0 + (tid >> g.tsh);
+          for (int b = 0; b < nb; ++b) {
             float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-            for_pairs(A, g, sm, s, t, T, [&](int k, float dx, float dy, float dz, float d2, uint32_t) {
-              weights(gi, fpi, lam, k, dx, dy, dz, d2, true);
-              const float4* const c = A.dtab + (size_t)rec.m[lane] * A.ktab + 8 * b;
+            if (s < n) {
+              const float4 gi = sm.gfe[s];
+              const float fpi = sm.pos[s].w, lam = sm.rho[s];
+              for_pairs(A, g, sm, s, t, T, [&](int k, float dx, float dy, float dz, float d2, uint32_t) {
+                weights(gi, fpi, lam, k, dx, dy, dz, d2, true);
+                const float4* const c = A.dtab + (size_t)rec.m[lane] * A.ktab + 8 * b;
 #pragma unroll
-              for (int q = 0; q < 8; ++q) {
-                const float4 f = q + 8 * b < A.nz2 ? rec.z[lane] : rec.r[lane];
-                a[q] = fmaf(c[q].x, f.x, fmaf(c[q].y, f.y, fmaf(c[q].z, f.z, fmaf(c[q].w, f.w, a[q]))));
-              }
-            });
+                for (int q = 0; q < 8; ++q) {
+                  const float4 f = q + 8 * b < A.nz2 ? rec.z[lane] : rec.r[lane];
+                  a[q] = fmaf(c[q].x, f.x, fmaf(c[q].y, f.y, fmaf(c[q].z, f.z, fmaf(c[q].w, f.w, a[q]))));
+                }
+              });
+            }
+            __syncwarp();
 #pragma unroll
-            for (int q = 0; q < 8; ++q) sum8[q] += widen(a[q]);
+            for (int q = 0; q < 8; ++q) {
+              double v = widen(a[q]);
+#pragma unroll
+              for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+#pragma unroll
+              for (int bb = 0; bb < MAX_TABLES / 8; ++bb)
+                if (bb == b && lane == q) accd[bb] += v;
+            }
           }
-          __syncwarp();
-#pragma unroll
-          for (int q = 0; q < 8; ++q) {
-            double v = sum8[q];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-#pragma unroll
-            for (int bb = 0; bb < MAX_TABLES / 8; ++bb)
-              if (bb == b && lane == q) accd[bb] = v;
-          }
+          if (SM::TURNS || s0 + ns >= n) store_tables();
         }
-#pragma unroll
-        for (int b = 0; b < MAX_TABLES / 8; ++b) {
-          accd[b] += __shfl_xor_sync(0xffffffffu, accd[b], 8);
-          accd[b] += __shfl_xor_sync(0xffffffffu, accd[b], 16);
-          if (lane < 8) sm.red[wid][lane + 8 * b] = accd[b];
-        }
-        block_sync();
-        if (tid < MAX_TABLES) {
-          double a = 0.0;
-          for (int k = 0; k < (B >> 5); ++k) a += sm.red[k][tid];
-          sm.red[0][tid] = a;
-        }
-        block_sync();
+        block_sums<MAX_TABLES>(sm, rows);
         if (tid < BMAX_PARAMS) {
           double v = row[11 + tid];
           for (int p = 0; p < A.nz2; ++p)

@@ -76,34 +76,33 @@ int ensure_atom_capacity(gbmd_context* c, int64_t n) {
   const int64_t cap = n;
   const size_t d3 = sizeof(double) * 3 * cap;
   for (int b = 0; b < 2; ++b) {
-    GBMD_CUDA(c, cudaMalloc(&c->rbuf[b], d3));
-    GBMD_CUDA(c, cudaMalloc(&c->vbuf[b], d3));
-    GBMD_CUDA(c, cudaMalloc(&c->abuf[b], d3));
-    GBMD_CUDA(c, cudaMalloc(&c->posf[b], sizeof(float4) * cap));
-    GBMD_CUDA(c, cudaMalloc(&c->posd[b], sizeof(double4_32a) * cap));
-    GBMD_CUDA(c, cudaMalloc(&c->typeb[b], cap));
-    GBMD_CUDA(c, cudaMalloc(&c->idb[b], sizeof(uint64_t) * cap));
-    GBMD_CUDA(c, cudaMalloc(&c->userb[b], sizeof(int32_t) * cap));
+    GBMD_CUDA(c, dev_malloc(c, (void**)&c->rbuf[b], d3));
+    GBMD_CUDA(c, dev_malloc(c, (void**)&c->vbuf[b], d3));
+    GBMD_CUDA(c, dev_malloc(c, (void**)&c->abuf[b], d3));
+    GBMD_CUDA(c, dev_malloc(c, (void**)&c->posf[b], sizeof(float4) * cap));
+    GBMD_CUDA(c, dev_malloc(c, (void**)&c->posd[b], sizeof(double4_32a) * cap));
+    GBMD_CUDA(c, dev_malloc(c, (void**)&c->typeb[b], cap));
+    GBMD_CUDA(c, dev_malloc(c, (void**)&c->idb[b], sizeof(uint64_t) * cap));
+    GBMD_CUDA(c, dev_malloc(c, (void**)&c->userb[b], sizeof(int32_t) * cap));
   }
-  GBMD_CUDA(c, cudaMalloc(&c->ep, sizeof(double) * cap));
-  GBMD_CUDA(c, cudaMalloc(&c->epd, sizeof(double) * cap));
-  GBMD_CUDA(c, cudaMalloc(&c->cellpack, sizeof(int32_t) * cap));
-  GBMD_CUDA(c, cudaMalloc(&c->cell_of, sizeof(int32_t) * cap));
-  GBMD_CUDA(c, cudaMalloc(&c->order, sizeof(int32_t) * cap));
-  GBMD_CUDA(c, cudaMalloc(&c->src, sizeof(int32_t) * cap));
-  GBMD_CUDA(c, cudaMalloc(&c->fpf, sizeof(float) * cap));
-  GBMD_CUDA(c, cudaMalloc(&c->epf, sizeof(float) * cap));
-  GBMD_CUDA(c, cudaMalloc(&c->pfp, sizeof(float4) * cap));
-  GBMD_CUDA(c, cudaMalloc(&c->f0, sizeof(float4) * cap));
-  GBMD_CUDA(c, cudaMalloc(&c->fpd, sizeof(double) * cap));
-  GBMD_CUDA(c, cudaMalloc(&c->stage, sizeof(double) * 9 * cap));
-  GBMD_CUDA(c, cudaMalloc(&c->rref, d3));
-  GBMD_CUDA(c, cudaMalloc(&c->nnb, sizeof(int32_t) * cap));
-  GBMD_CUDA(c, cudaMalloc(&c->d_part, sizeof(double) * 26 * thermo_blocks(cap)));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->ep, sizeof(double) * cap));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->epd, sizeof(double) * cap));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->cellpack, sizeof(int32_t) * cap));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->cell_of, sizeof(int32_t) * cap));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->order, sizeof(int32_t) * cap));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->src, sizeof(int32_t) * cap));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->fpf, sizeof(float) * cap));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->epf, sizeof(float) * cap));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->pfp, sizeof(float4) * cap));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->fpd, sizeof(double) * cap));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->stage, sizeof(double) * 9 * cap));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->rref, d3));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->nnb, sizeof(int32_t) * cap));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->d_part, sizeof(double) * 26 * thermo_blocks(cap)));
   c->cap = cap;
   if (c->newton3) {
     // zeroed once; the Newton-3 epilogue clears each atom's slots after reading them
-    GBMD_CUDA(c, cudaMalloc(&c->h3acc, sizeof(long long) * 10 * cap));
+    GBMD_CUDA(c, dev_malloc(c, (void**)&c->h3acc, sizeof(long long) * 10 * cap));
     GBMD_CUDA(c, cudaMemset(c->h3acc, 0, sizeof(long long) * 10 * cap));
   }
   c->cur = c->cur_s = 0;
@@ -116,6 +115,23 @@ static void drop_graph(gbmd_context* c) {
       if (g.exec) cudaGraphExecDestroy(g.exec);
       g.exec = nullptr;
     }
+}
+
+cudaError_t dev_malloc(gbmd_context* c, void** p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation || !c->bpair) return e;
+  (void)cudaGetLastError();
+  release_bpair(c);
+  return cudaMalloc(p, bytes);
+}
+
+void release_bpair(gbmd_context* c) {
+  if (!c->bpair) return;
+  drop_graph(c);
+  cudaFree(c->bpair);
+  c->bpair = nullptr;
+  c->bpair_cap = 0;
+  c->rho_bonds = false;
 }
 
 static void invalidate_list(gbmd_context* c) {
@@ -668,7 +684,7 @@ static int32_t* inverse_user(gbmd_context* c) {
 // the force pass runs; copy_join[0] marks the end.
 static int download_r_async(gbmd_context* c) {
   const int64_t n = c->n;
-  if (!c->stage_r) GBMD_CUDA(c, cudaMalloc(&c->stage_r, sizeof(double) * 3 * c->cap));
+  if (!c->stage_r) GBMD_CUDA(c, dev_malloc(c, (void**)&c->stage_r, sizeof(double) * 3 * c->cap));
   int rc = ensure_copy_streams(c);
   if (rc) return rc;
   Arrays9 src{}, dst{};
@@ -892,7 +908,7 @@ int gbmd_set_lj_multi(gbmd_context* c, int ntypes, const double* eps, const doub
   c->lj.ntypes = ntypes;
   c->lj.rcut_max = rmax;
   c->lj.rcut_max2 = rmax * rmax;
-  if (!c->lj_tab_d) GBMD_CUDA(c, cudaMalloc(&c->lj_tab_d, sizeof(LJPair) * GBMD_MAX_TYPES * GBMD_MAX_TYPES));
+  if (!c->lj_tab_d) GBMD_CUDA(c, dev_malloc(c, (void**)&c->lj_tab_d, sizeof(LJPair) * GBMD_MAX_TYPES * GBMD_MAX_TYPES));
   return set_rlist(c, rmax);
 }
 
@@ -927,8 +943,8 @@ int gbmd_set_eam_alloy(gbmd_context* c, int nel, int nrho, double drho, int nr, 
   cudaFree(c->eam_f);
   c->eam_d = nullptr;
   c->eam_f = nullptr;
-  GBMD_CUDA(c, cudaMalloc(&c->eam_d, sizeof(double) * nd));
-  GBMD_CUDA(c, cudaMalloc(&c->eam_f, sizeof(float4) * nf));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->eam_d, sizeof(double) * nd));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->eam_f, sizeof(float4) * nf));
   std::vector<double> hd;
   hd.reserve(nd);
   hd.insert(hd.end(), c->eam_host_frho.begin(), c->eam_host_frho.end());
@@ -1080,7 +1096,8 @@ int gbmd_set_precision(gbmd_context* c, int precision) {
     c->precision = precision;
     c->energy_step = -1, c->forces_valid_step = c->rho_valid_step = -1;
     drop_graph(c);
-    if (c->list_valid && c->n) {
+    // (a change to FP64 gives the bond terms' room back at the next rebuild)
+    if (c->list_valid && c->n && precision == GBMD_PRECISION_MIXED) {
       cudaSetDevice(c->device);
       ensure_bpair(c);
     }
@@ -1170,7 +1187,7 @@ int gbmd_set_newton3(gbmd_context* c, int enable) {
   cudaSetDevice(c->device);
   if ((enable != 0) == c->newton3) return GBMD_OK;
   if (enable && c->cap > 0 && !c->h3acc) {
-    GBMD_CUDA(c, cudaMalloc(&c->h3acc, sizeof(long long) * 10 * c->cap));
+    GBMD_CUDA(c, dev_malloc(c, (void**)&c->h3acc, sizeof(long long) * 10 * c->cap));
     GBMD_CUDA(c, cudaMemset(c->h3acc, 0, sizeof(long long) * 10 * c->cap));
   }
   c->newton3 = enable != 0;
@@ -1284,7 +1301,7 @@ static int ensure_list(gbmd_context* c) {
 }
 
 static int ensure_virial(gbmd_context* c) {
-  if (!c->vir && c->cap > 0) GBMD_CUDA(c, cudaMalloc(&c->vir, sizeof(double) * 9 * c->cap));
+  if (!c->vir && c->cap > 0) GBMD_CUDA(c, dev_malloc(c, (void**)&c->vir, sizeof(double) * 9 * c->cap));
   return GBMD_OK;
 }
 
@@ -1511,7 +1528,7 @@ int gbmd_run_nve(gbmd_context* c, int nsteps, double dt, int rebuild_every, int 
   if (nrows > c->rows_cap) {
     cudaFree(c->d_rows);
     c->d_rows = nullptr;
-    GBMD_CUDA(c, cudaMalloc(&c->d_rows, sizeof(double) * 27 * nrows));
+    GBMD_CUDA(c, dev_malloc(c, (void**)&c->d_rows, sizeof(double) * 27 * nrows));
     c->rows_cap = nrows;
   }
   double* rows = c->d_rows;
@@ -1745,7 +1762,7 @@ int gbmd_lj_loss_grad(gbmd_context* c, const double* fx_target, const double* fy
   if (need > c->adj_cap) {
     cudaFree(c->adj_scratch);
     c->adj_scratch = nullptr;
-    GBMD_CUDA(c, cudaMalloc(&c->adj_scratch, sizeof(double) * need));
+    GBMD_CUDA(c, dev_malloc(c, (void**)&c->adj_scratch, sizeof(double) * need));
     c->adj_cap = need;
   }
   double* t = c->adj_scratch;
@@ -1787,7 +1804,7 @@ int gbmd_lj_multi_loss_grad(gbmd_context* c, const double* fx_target, const doub
   if (need > c->adj_cap) {
     cudaFree(c->adj_scratch);
     c->adj_scratch = nullptr;
-    GBMD_CUDA(c, cudaMalloc(&c->adj_scratch, sizeof(double) * need));
+    GBMD_CUDA(c, dev_malloc(c, (void**)&c->adj_scratch, sizeof(double) * need));
     c->adj_cap = need;
   }
   double* t = c->adj_scratch;

@@ -341,8 +341,13 @@ int sync_error_word(gbmd_context* c);  // copies device error word, returns stat
 constexpr int64_t PACK_DOUBLES = 65536;
 
 // neighbours (gbmd_neighbors.cu)
-// one-element EAM: room for one float per list entry (bpair), if it can be had
+// one-element EAM in mixed precision: f0, and room for one float per list entry
+// (bpair), if they can be had; otherwise the room is given back
 void ensure_bpair(gbmd_context* c);
+void release_bpair(gbmd_context* c);
+// cudaMalloc for everything else a context holds: bpair, which is not needed, is
+// given up before an allocation fails
+cudaError_t dev_malloc(gbmd_context* c, void** p, size_t bytes);
 int grid_dims(const double lo[3], const double hi[3], double R, int nc[3]);
 int set_bands(gbmd_context* c);
 // gate: device word; non-null makes every kernel of the chain return at once

@@ -1664,7 +1664,7 @@ static void launch_bonds(gbmd_context* c, const PairArgs& A, int part) {
 // its pieces).
 static bool take_bonds(gbmd_context* c, const PairArgs& A, int part, bool ev) {
   if (c->pot != GBMD_POT_EAM_ALLOY || c->eam.nel != 1) return false;
-  const bool can = !ev && !c->newton3 && c->vec == 4 && c->bpair_cap >= (int64_t)(c->maxnb / A.W) * A.stride;
+  const bool can = !ev && !c->newton3 && c->vec == 4 && c->f0 && c->bpair_cap >= (int64_t)(c->maxnb / A.W) * A.stride;
   if (part != 2) c->rho_bonds = can;
   return can && c->rho_bonds;
 }

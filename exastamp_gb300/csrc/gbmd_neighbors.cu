@@ -230,9 +230,9 @@ static int ensure_cells(gbmd_context* c, int64_t ncells) {
   cudaFree(c->scan_tmp);
   c->cell_start = c->cell_fill = c->scan_tmp = nullptr;
   c->cells_cap = 0;
-  GBMD_CUDA(c, cudaMalloc(&c->cell_start, sizeof(int32_t) * (ncells + 1)));
-  GBMD_CUDA(c, cudaMalloc(&c->cell_fill, sizeof(int32_t) * (ncells + 1)));
-  GBMD_CUDA(c, cudaMalloc(&c->scan_tmp, sizeof(int32_t) * scan_blocks(ncells)));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->cell_start, sizeof(int32_t) * (ncells + 1)));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->cell_fill, sizeof(int32_t) * (ncells + 1)));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->scan_tmp, sizeof(int32_t) * scan_blocks(ncells)));
   GBMD_CUDA(c, cudaMemsetAsync(c->cell_fill, 0, sizeof(int32_t) * (ncells + 1), c->stream));
   c->cells_cap = ncells + 1;
   return GBMD_OK;
@@ -830,7 +830,7 @@ static int build_list(gbmd_context* c, const int* gate) {
     cudaFree(c->nbr);
     c->nbr = nullptr;
     c->nbr_cap = 0;
-    GBMD_CUDA(c, cudaMalloc(&c->nbr, sizeof(uint32_t) * (size_t)need));
+    GBMD_CUDA(c, dev_malloc(c, (void**)&c->nbr, sizeof(uint32_t) * (size_t)need));
     c->nbr_cap = need;
   }
   c->npad = npad;
@@ -1019,8 +1019,8 @@ void free_outer(gbmd_context* c) {
 static int ensure_outer(gbmd_context* c) {
   if (c->rout && c->outer_cap >= c->cap) return GBMD_OK;
   free_outer(c);
-  GBMD_CUDA(c, cudaMalloc(&c->rout, sizeof(double) * 3 * c->cap));
-  GBMD_CUDA(c, cudaMalloc(&c->nnb_out, sizeof(int32_t) * c->cap));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->rout, sizeof(double) * 3 * c->cap));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->nnb_out, sizeof(int32_t) * c->cap));
   c->outer_cap = c->cap;
   return GBMD_OK;
 }
@@ -1196,7 +1196,7 @@ static int filter_list(gbmd_context* c, const int* gate) {
     if (c->nbr) cudaFree(c->nbr);
     c->nbr = nullptr;
     c->nbr_cap = 0;
-    GBMD_CUDA(c, cudaMalloc(&c->nbr, sizeof(uint32_t) * (size_t)need));
+    GBMD_CUDA(c, dev_malloc(c, (void**)&c->nbr, sizeof(uint32_t) * (size_t)need));
     c->nbr_cap = need;
   }
   c->maxnb = c->maxnb_out;
@@ -1278,15 +1278,24 @@ static int64_t list_words(const gbmd_context* c) {
 
 void ensure_bpair(gbmd_context* c) {
   if (c->precision != GBMD_PRECISION_MIXED || c->pot != GBMD_POT_EAM_ALLOY || c->eam.nel != 1 || c->newton3 ||
-      c->vec != 4 || list_words(c) <= c->bpair_cap)
+      c->vec != 4) {
+    release_bpair(c);  // nothing reads it
     return;
-  cudaFree(c->bpair);
-  c->bpair = nullptr;
-  c->bpair_cap = 0;
+  }
+  // without them the force pass forms the pair terms again
+  if (!c->f0 && cudaMalloc(&c->f0, sizeof(float4) * c->cap) != cudaSuccess) {
+    (void)cudaGetLastError();
+    c->f0 = nullptr;
+    return;
+  }
   const int64_t need = list_words(c);
-  // without it the force pass forms the pair terms again
+  if (need <= c->bpair_cap) return;
+  release_bpair(c);
+  // no more than half of what is free: the caller's memory comes first
+  size_t free_bytes = 0, total = 0;
+  if (cudaMemGetInfo(&free_bytes, &total) != cudaSuccess || sizeof(float) * (size_t)need > free_bytes / 2) return;
   if (cudaMalloc(&c->bpair, sizeof(float) * (size_t)need) == cudaSuccess) c->bpair_cap = need;
-  else (void)cudaGetLastError();
+  else (void)cudaGetLastError(), c->bpair = nullptr;
 }
 
 int rebuild(gbmd_context* c, bool check_capacity, const int* gate) {

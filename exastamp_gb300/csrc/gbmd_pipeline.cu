@@ -158,7 +158,7 @@ int ensure_pipe(gbmd_context* c) {
     GBMD_CUDA(c, cudaEventCreateWithFlags(&c->pipe_f_ev[k], cudaEventDisableTiming));
     GBMD_CUDA(c, cudaEventCreateWithFlags(&c->pipe_d_ev[k], cudaEventDisableTiming));
   }
-  GBMD_CUDA(c, cudaMalloc(&c->pipe_dev, sizeof(int) * SCRATCH_INTS));
+  GBMD_CUDA(c, dev_malloc(c, (void**)&c->pipe_dev, sizeof(int) * SCRATCH_INTS));
   GBMD_CUDA(c, cudaMallocHost(&c->pipe_host, sizeof(int) * SCRATCH_INTS));
   return GBMD_OK;
 }
@@ -272,7 +272,7 @@ int pipe_issue(gbmd_context* c, double dt, const double* const host[9], const do
     if (c->pipe_stage) cudaFree(c->pipe_stage);
     c->pipe_stage = nullptr;
     c->pipe_stage_cap = 0;
-    GBMD_CUDA(c, cudaMalloc(&c->pipe_stage, sizeof(double) * 9 * c->cap));
+    GBMD_CUDA(c, dev_malloc(c, (void**)&c->pipe_stage, sizeof(double) * 9 * c->cap));
     c->pipe_stage_cap = c->cap;
   }
   const int64_t sc = c->pipe_stage_cap;

@@ -30,10 +30,10 @@ def test_nothing_can_fail_between_the_count_and_the_scatter():
     up, down = chain.index("k_wrap_bin<<<"), chain.index("k_scatter<<<")
     assert up < down
     between = chain[up:down]
-    assert not re.search(r"\breturn\b|GBMD_CUDA|cudaMalloc", between)
+    assert not re.search(r"\breturn\b|GBMD_CUDA|alloc\(", between)
     assert "scan(" in between
     scan = re.search(r"static (\w+) scan\(", src)
-    assert scan.group(1) == "void" and "cudaMalloc" not in _body(src, scan.group(0))
+    assert scan.group(1) == "void" and "alloc(" not in _body(src, scan.group(0))
 
 
 def test_a_failed_allocation_leaves_no_capacity():
@@ -41,4 +41,4 @@ def test_a_failed_allocation_leaves_no_capacity():
     for head, cap in (("static int ensure_cells(", "cells_cap = 0"), ("static int build_list(", "nbr_cap = 0"),
                       ("static int filter_list(", "nbr_cap = 0")):
         body = _body(src, head)
-        assert body.index(cap) < body.index("cudaMalloc(")
+        assert body.index(cap) < body.index("alloc(")

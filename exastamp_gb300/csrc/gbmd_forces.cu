@@ -1,13 +1,19 @@
 // gbmd_forces.cu -- plain-FP64 LJ and eam_alloy pair kernels for sm_103a, and
 // the force dispatch (FP64 here, mixed precision in gbmd_mixed.cu).
 //
-// The FP64 kernels restate the reference arithmetic exactly:
+// The functions of the reference, in FP64 throughout:
 //   LJ       lennard_jones.h L41-50 + force_op_impl2.hxx L33-68 (e -= ecut, de /= r,
 //            fe = de*dr, ep += e/2, vir += -1/2 fe (x) dr)
 //   LJ multi pair_potential_force_op_multiparam.h L92-118 (r <= rcut_pair test)
 //   EAM      eam_alloy.h L198-313 + eam_force_op_multimat.h L114-343
-// with dr = (x_j + n*L) - x_i and d2 rounded exactly like the list builder
-// and the oracle, so cutoff membership is identical.
+// dr = (x_j + n*L) - x_i and d2 are rounded exactly like the list builder and the
+// oracle, so cutoff membership is identical.  The rest is not the reference's
+// arithmetic operation for operation: LJ is a function of 1/d2 where the
+// reference divides by r, sums are fused, factors common to all pairs are taken
+// at the end, and sqrt and 1/x are gbmd_fp64.cuh's (each within one unit in the
+// last place of the correctly rounded value).  A pair's force differs by a few
+// units in the last place: against quad precision LJ is off by 1.4e-15 (the
+// reference's form: 1.8e-15), Cu by 1.9e-15 (1.9e-15).
 //
 // The FP64 pipe is the bound: an FP64 instruction of a warp takes 16 cycles
 // of an SM, as long as some 60 FP32 or integer ones over its four schedulers.
@@ -18,62 +24,10 @@
 // their factor at the end.  Cu, 108,000 atoms, with energies and virials:
 // density 437 -> 288 us, force 928 -> 577 us; LJ, 256,000
 // atoms: 3,456 -> 1,134 us.
+#include "gbmd_fp64.cuh"
 #include "gbmd_pair_common.cuh"
 
 namespace gbmd {
-
-// r = sqrt(d2), and 1/r with it where INV: the FP32 rsqrt as seed y0 (relative
-// error below 2^-22), one Householder step of third order, y = y0 (1 + e/2 +
-// 3 e^2/8) with e = 1 - d2 y0^2 (remainder e^3, below 2^-60), then a Newton
-// correction of r = d2 y and one of y towards 1/r.  Outside FP32's range the
-// library functions are taken.
-template <bool INV>
-__device__ __forceinline__ double root(double d2, double& y) {
-  const uint32_t hi = (uint32_t)__double2hiint(d2);
-  if (hi - 0x3a000000u < 0x0c000000u) {  // 2^-95 <= d2 < 2^97
-    const float s = __uint_as_float(((hi - 0x38000000u) << 3) | ((uint32_t)__double2loint(d2) >> 29));
-    const double y0 = widen(rsqrtf(s));
-    const double e = fma(-(d2 * y0), y0, 1.0);
-    y = fma(y0 * e, fma(e, 0.375, 0.5), y0);
-    double r = d2 * y;
-    r = fma(fma(-r, r, d2), 0.5 * y, r);
-    if (INV) y = fma(fma(-r, y, 1.0), y, y);
-    return r;
-  }
-  const double r = sqrt(d2);
-  y = 1.0 / r;
-  return r;
-}
-
-// 1/d2 from an FP32 seed y0: y0 (1 + e + e^2), e = 1 - d2 y0, remainder e^3.
-__device__ __forceinline__ double inverse(double d2) {
-  const uint32_t hi = (uint32_t)__double2hiint(d2);
-  if (hi - 0x3a000000u < 0x0c000000u) {
-    const float s = __uint_as_float(((hi - 0x38000000u) << 3) | ((uint32_t)__double2loint(d2) >> 29));
-    const double y0 = widen(__frcp_rn(s));
-    const double e = fma(-d2, y0, 1.0);
-    return fma(y0, fma(e, e, e), y0);
-  }
-  return 1.0 / d2;
-}
-
-// Knot m = floor(t), capped at nr - 1, and p = t - m, capped at 1: the integer
-// part of t in [1, 2^20) by shifts, the fraction by one subtraction.
-__device__ __forceinline__ int r_knot_d(double t, int nr, double& p) {
-  const long long b = __double_as_longlong(t);
-  const int ex = (int)(b >> 52) - 1023;
-  if ((unsigned)ex < 20u) {
-    const long long mant = b & 0xfffffffffffffll;
-    const int m = (int)((mant | 0x10000000000000ll) >> (52 - ex));
-    if (m < nr) {
-      p = __longlong_as_double(((mant << ex) & 0xfffffffffffffll) | 0x3ff0000000000000ll) - 1.0;
-      return m;
-    }
-  }
-  const int m = min((int)t, nr - 1);
-  p = fmin(t - m, 1.0);
-  return m;
-}
 
 // Where atom i's pairs start from: its positions and its cell.
 struct PairHome {

@@ -242,6 +242,7 @@ __global__ void __launch_bounds__(256) k_eam_rho(PairArgs A, EamDev E, double* _
   if (T > 1) {
     __shared__ double sum[T > 1 ? 256 / T : 1];
     if (threadIdx.x % T == 0) sum[threadIdx.x / T] = rho;
+    __syncwarp();
     __syncthreads();
     if (threadIdx.x >= blockDim.x / T) return;
     rho = sum[threadIdx.x];

@@ -641,6 +641,7 @@ __global__ void __launch_bounds__(256) k_eam_rho_mixed(PairArgs A, EamDev E, flo
     __shared__ float rho[T > 1 ? 256 / T : 1];
     const int nat = (int)blockDim.x / T;
     if (threadIdx.x % T == 0) rho[threadIdx.x / T] = R;
+    __syncwarp();
     __syncthreads();
     if ((int)threadIdx.x >= nat) return;
     R = rho[threadIdx.x];

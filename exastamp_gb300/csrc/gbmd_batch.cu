@@ -78,7 +78,6 @@ struct BatchArgs {
   double rcut, rcut2;
   int S;
   // adjoint
-  int adjoint;
   const double *Ftx, *Fty, *Ftz, *Et;
   double wF, wE;
   const float4* dtab;    // [knot][ktab]: derivative tables of z2r (nz2), then of rho (nrh), zero-padded
@@ -1339,7 +1338,6 @@ static int batch_launch(gbmd_batch* b, int adjoint, int per_replica) {
   A.queue = b->queue;
   A.err = b->d_err;
   A.S = b->S;
-  A.adjoint = adjoint;
   A.Ftx = b->Ftx; A.Fty = b->Fty; A.Ftz = b->Ftz; A.Et = b->Et;
   if (per_replica) {
     for (int r = 0; r < b->nrep; ++r) {

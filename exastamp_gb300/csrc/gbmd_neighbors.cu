@@ -432,8 +432,8 @@ struct BuildSmem {
 };
 
 __host__ __device__ inline int build_rowlen(int maxnb) { return (maxnb + BUILD_SLACK) | 1; }  // odd: rows start in different banks
-__host__ __device__ inline size_t build_smem(int maxnb) {
-  return sizeof(BuildSmem) + (size_t)(BUILD_G * build_rowlen(maxnb)) * sizeof(uint32_t);
+__host__ __device__ inline size_t build_smem(int maxnb, int homes) {
+  return sizeof(BuildSmem) + (size_t)((homes * build_rowlen(maxnb) + 3) & ~3) * sizeof(uint32_t);
 }
 
 struct BuildArgs {
@@ -445,7 +445,7 @@ struct BuildArgs {
   float R2lo, R2hi;
   uint32_t* nbr;
   int32_t* nnb;
-  int maxnb, W, wsh, tsh, parts;  // parts: warps per cell
+  int maxnb, W, wsh, tsh, homes, parts;  // homes: atoms per group; parts: warps per cell
   int64_t stride;
   int* err;
   int64_t n;
@@ -560,7 +560,7 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32, 6) k_build_list_cells(const 
   const int lane = threadIdx.x & 31, half = lane >> 4, hl = lane & 15;
   const int rowlen = build_rowlen(A.maxnb);
   unsigned char* const mine =
-      reinterpret_cast<unsigned char*>(build_shared) + (threadIdx.x >> 5) * build_smem(A.maxnb);
+      reinterpret_cast<unsigned char*>(build_shared) + (threadIdx.x >> 5) * build_smem(A.maxnb, A.homes);
   BuildSmem& S = *reinterpret_cast<BuildSmem*>(mine);
   uint32_t* const rows = reinterpret_cast<uint32_t*>(mine + sizeof(BuildSmem));
   const int64_t items = A.ncells * A.parts;
@@ -569,7 +569,7 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32, 6) k_build_list_cells(const 
     const int64_t cell = item / A.parts;
     const int part = (int)(item - cell * A.parts);
     const int hb = A.cstart[cell], nh = A.cstart[cell + 1] - hb;
-    if (part * BUILD_G >= nh) continue;
+    if (part * A.homes >= nh) continue;
     const int cx = (int)(cell % g.nc[0]), cy = (int)((cell / g.nc[0]) % g.nc[1]),
               cz = (int)(cell / ((int64_t)g.nc[0] * g.nc[1]));
     // stencil cell of this lane
@@ -611,8 +611,8 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32, 6) k_build_list_cells(const 
     // walk's d2, so no candidate the walk would keep is dropped
     const float R2keep = A.R2hi * (1.0f + 0x1p-10f);
     int warp_max = 0;
-    for (int h0 = part * BUILD_G; h0 < nh; h0 += A.parts * BUILD_G) {
-      const bool hv = h0 + hl < nh;
+    for (int h0 = part * A.homes; h0 < nh; h0 += A.parts * A.homes) {
+      const bool hv = hl < A.homes && h0 + hl < nh;
       const int i = hb + h0 + hl;
       float4 pi = make_float4(FAR, FAR, FAR, 0.f);
       if (hv) pi = A.pf[i];
@@ -852,12 +852,13 @@ static int build_list(gbmd_context* c, const int* gate) {
   A.err = c->d_err;
   A.n = c->n;
   A.cellpack = c->cellpack;
+  A.homes = BUILD_G;  // as a constant in the kernel it costs 2 % (16.6 M-atom mixture: 12.03 -> 12.28 ms)
   if (c->maxnb >= BUILD_LONG) {
     auto kern = c->newton3 ? k_build_list_long<true> : k_build_list_long<false>;
     kern<<<chain_blocks(c, c->n, 4, gate, 8), 128, 0, c->stream>>>(A, c->grid, gate);
     return GBMD_OK;
   }
-  const size_t per_warp = build_smem(c->maxnb);
+  const size_t per_warp = build_smem(c->maxnb, BUILD_G);
   // the widest blocks of which an SM holds several
   int nw = BUILD_WARPS;
   while (nw > 1 && nw * per_warp > 56 * 1024) nw >>= 1;
@@ -868,7 +869,7 @@ static int build_list(gbmd_context* c, const int* gate) {
   const bool loop = gate && !c->full_chain_grids;  // capped grid striding over the cells
   auto kern = loop ? (c->newton3 ? k_build_list_cells<true, true> : k_build_list_cells<true, false>)
                    : (c->newton3 ? k_build_list_cells<false, true> : k_build_list_cells<false, false>);
-  const size_t smem = nw * per_warp, most = 64 * 1024;  // (a warp's rows of BUILD_LONG entries: 60 KB)
+  const size_t smem = nw * per_warp, most = 200 * 1024;
   if (smem > 48 * 1024)
     GBMD_CUDA(c, cudaFuncSetAttribute((const void*)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
   const int per_sm = (int)std::max<size_t>(1, 220 * 1024 / (smem + 1024));

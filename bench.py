@@ -16,9 +16,9 @@ Reported (one JSON line on rank 0):
              host: gbmd_run_nve_host per step (r,v,a copied in from pinned
              memory, one verlet_nve step, r copied out while the force pass
              runs, then v,a)
-  roofline   the final pair kernel (force + fused Verlet halves), algorithmic
-             bytes per launch / its CUDA-event duration, against the measured
-             HBM copy bandwidth
+  roofline   the pair pass (LJ) or the density and force passes together (EAM:
+             they share the pair's work), algorithmic bytes per step / their
+             CUDA-event duration, against the measured HBM copy bandwidth
   fp64       the same steps through the plain-FP64 kernels, and the
              mixed-vs-FP64 force error and energy drift
   cpu_baseline  the FP64 OpenMP oracle on a bounded sample, all host threads
@@ -50,9 +50,8 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 # sigma per component per step (the NVE step 0.002 would move overlapping
 # atoms only 2e-4 sigma per step and leave forces that blow the NVE run up)
 MIN_TOLF = 100.0
-# measured DRAM traffic of the force kernel per atom (see roofline.traffic)
-EAM_FORCE_DRAM_BYTES_PER_ATOM = (273.772288e6 + 51.000832e6) / 864000.0
-# the same for k_lj_mixed on the 864,000-atom LJ mixture (lj_binary_16m --ncell 60)
+# measured DRAM traffic per atom of k_lj_mixed on the 864,000-atom LJ mixture
+# (lj_binary_16m --ncell 60; see roofline.traffic)
 LJ_MULTI_PAIR_DRAM_BYTES_PER_ATOM = (474.028544e6 + 51.887872e6) / 864000.0
 MIN_DT = 0.02
 sys.path.insert(0, ROOT)
@@ -719,15 +718,14 @@ def measure(args, w, ws, dev, stream, torch, *, steps, fp64_steps, e2e_steps, dr
     # EAM: density + force; Newton-3 LJ: half-list pair pass + epilogue
     kernels_per_step = 2 if w["kind"] == "eam" or args.newton3 else 1
     # Launches of the timed gbmd_run_nve call: the pair kernel(s) once per
-    # step; the thermo reduction (2)
-    # at step 0 and every thermo_every steps; the standalone first half at
-    # the start and after every thermo step but the last; the rebuild chain
-    # (wrap/bin, 3 scan kernels, scatter, rank, gather, posf, list build) per
-    # rebuild.  With the trigger the kernels that move the atoms test them, and
-    # a graph step launches the conditional's setter, plus the 13-kernel
-    # rebuild body (2 fills, the chain, copy-back, reference positions) when
-    # the gate opens; the steps after the last whole graph chunk run the 13
-    # gated launches every step.
+    # step; the thermo reduction (2) at step 0 and every thermo_every steps; the
+    # standalone first half at the start and after every thermo step but the
+    # last; the rebuild chain per rebuild: wrap/bin, scan (1 kernel for up to
+    # 16,383 cells, else 3), scatter, rank, gather, list build, reference
+    # positions.  With the trigger the kernels that move the atoms test them,
+    # and a graph step launches the conditional's setter, plus the rebuild body
+    # (the chain and the copy back) when the gate opens; the steps after the
+    # last whole graph chunk run the gated launches every step.
     n_thermo = steps // thermo_every if thermo_every else 0
     last_is_thermo = bool(thermo_every) and steps % thermo_every == 0
     # step 0's forces and energies are recomputed unless the warm-up ended on
@@ -735,19 +733,20 @@ def measure(args, w, ws, dev, stream, torch, *, steps, fp64_steps, e2e_steps, dr
     gpu_launches = kernels_per_step * (steps if energies_reused else steps + 1)
     gpu_launches += 2 * (n_thermo + (1 if thermo_every else 0))
     gpu_launches += 1 + n_thermo - (1 if last_is_thermo else 0)
+    chain = 5 + (1 if int(np.prod(nc)) < 16384 else 3)  # without the reference positions
     # With a list buffer a rebuild is the outer test, the conditional's
-    # setter and the filter (3), plus 13 for an outer build (2 fills, the
-    # chain, copy-back, outer positions); with the trigger all 16 are gated
-    # launches inside its body.
+    # setter, the filter and the reference positions, plus the chain, copy back
+    # and outer positions for an outer build; with the trigger all but the
+    # setter are gated launches inside its body.
     two_level = w.get("list_buffer", 0.0) > 0.0
     if R < 0:
         n_graph = (steps // thermo_every) * thermo_every
-        per = 16 if two_level else 13
+        per = chain + (5 if two_level else 2)
         gpu_launches += n_graph + per * rebuilds + per * (steps - n_graph)
     elif two_level:
-        gpu_launches += 3 * rebuilds + 13 * outer_builds
+        gpu_launches += 4 * rebuilds + (chain + 2) * outer_builds
     else:
-        gpu_launches += 9 * rebuilds
+        gpu_launches += (chain + 1) * rebuilds
 
     out = {"metric": "atom-timesteps/s", "value": value, "unit": "atom-timesteps/s", "n_gpus": ws,
            "steps": steps, "warmup": args.warmup, "ms_per_step": ms / steps,
@@ -786,51 +785,42 @@ def measure(args, w, ws, dev, stream, torch, *, steps, fp64_steps, e2e_steps, dr
     prof = ctx.profile_step(reps=10)
     peak, peak_kind = measured_peaks()
     nbar = npairs / s.n
-    if w["kind"] == "eam":
-        # list 4 B/entry, own posf 16 B + F' 4 B, state r 24+24, v 24+24, a 24, posf 16, posd 32 written
-        per_atom = 4.0 * nbar + 16 + 4 + 48 + 48 + 24 + 16 + 32
-    else:
-        per_atom = 4.0 * nbar + 16 + 48 + 48 + 24 + 16 + 32
-    alg_bytes = per_atom * s.n
-    t_pair = prof["pair"] * 1e-3
-    achieved = alg_bytes / t_pair / 1e9
-    traffic, traffic_src = None, None
+    state = 48 + 48 + 24 + 16 + 32  # r 24+24, v 24+24, a 24, posf 16, posd 32 written
     if w["kind"] == "eam" and args.precision == "mixed":
-        # DRAM bytes per atom of k_eam_force_mixed from one ncu capture of the
-        # same kernel on the 864,000-atom case (60^3 cells), scaled by atoms
-        traffic = EAM_FORCE_DRAM_BYTES_PER_ATOM * s.n
-        traffic_src = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of k_eam_force_mixed<1,4> on the "
-                       "864,000-atom case (273.8 + 51.0 MB), scaled to %d atoms" % s.n)
-    elif w["kind"] == "lj_multi" and args.precision == "mixed":
+        # both passes, which share the pair's work.  Density: list and bond term
+        # 4 + 4 B an entry, posf 16, F' 4, (position, F') 16, f0 16 written; force:
+        # list and bond term again, (position, F') 16, f0 16, F' 4, the state
+        per_atom = 16.0 * nbar + 52 + 36 + state
+        kernels, t_pair = "k_eam_rho_bonds + k_eam_force_bonds", (prof["density"] + prof["pair"]) * 1e-3
+    elif w["kind"] == "eam":
+        per_atom = 8.0 * nbar + 32 + 8 + 32 + 8 + state
+        kernels, t_pair = "k_eam_rho + k_eam_force", (prof["density"] + prof["pair"]) * 1e-3
+    else:
+        per_atom = 4.0 * nbar + 16 + state
+        kernels, t_pair = "k_lj", prof["pair"] * 1e-3
+    alg_bytes = per_atom * s.n
+    achieved = alg_bytes / t_pair / 1e9
+    traffic, traffic_src, binding = None, None, None
+    if w["kind"] == "lj_multi" and args.precision == "mixed":
         traffic = LJ_MULTI_PAIR_DRAM_BYTES_PER_ATOM * s.n
         traffic_src = ("ncu dram__bytes_read.sum + dram__bytes_write.sum of k_lj_mixed<1,4,multi> on the "
                        "864,000-atom mixture (474.0 + 51.9 MB), scaled to %d atoms" % s.n)
-    # the resource that binds the pair kernels (ncu on the 864,000-atom cases)
-    binding = ({"resource": "L1/tex LSU data-pipe wavefronts (neighbour and spline-knot gathers)", "frac": 0.796,
-                "source": "ncu l1tex__data_pipe_lsu_wavefronts.avg.pct_of_peak_sustained_elapsed of "
-                          "k_eam_force_mixed<1,4> (density kernel: 0.858)"}
-               if w["kind"] == "eam" else
-               {"resource": "issue slots + L1/tex (neighbour gathers)", "frac": 0.78,
-                "source": "ncu smsp__issue_active of k_lj_mixed<1,4,multi> (L1/tex throughput 0.75)"}
-               if w["kind"] == "lj_multi" else None)
-    out["roofline"] = {"kernel": "k_eam_force (mixed, fused Verlet halves)" if w["kind"] == "eam" else "k_lj",
-                       "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+        binding = {"resource": "issue slots + L1/tex (neighbour gathers)", "frac": 0.78,
+                   "source": "ncu smsp__issue_active of k_lj_mixed<1,4,multi> (L1/tex throughput 0.75)"}
+    out["roofline"] = {"kernel": kernels, "bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                        "frac": achieved / peak, "peak_source": peak_kind,
                        "algorithmic_bytes_per_launch": alg_bytes, "bytes_per_atom": per_atom,
                        "traffic": traffic, "traffic_source": traffic_src, "binding": binding, "kernel_ms": prof}
     if w["kind"] == "eam" and args.precision == "mixed":
-        # the FP-pipe side of the same kernels: useful flops per unordered
+        # the FP-pipe side of the same passes: useful flops per unordered
         # pair within rc (density 20, force 54, embedding 14 per atom), the
         # FCC Cu lattice's 42 neighbours within rc=5.0 A (21 unordered pairs
         # per atom), against the nominal FP32 rate (no measured FP32 peak)
-        pairs = 21.0 * s.n
+        flop = 74.0 * 21.0 * s.n + 14.0 * s.n
         fp32_peak = 152 * 128 * 2 * (measured_clock_mhz() or 2070.0) * 1e6 / 1e12
-        dens_tf = (20.0 * pairs + 14.0 * s.n) / (prof["density"] * 1e-3) / 1e12
-        force_tf = 54.0 * pairs / (prof["pair"] * 1e-3) / 1e12
         out["roofline"]["fp32"] = {
-            "useful_flop_per_launch": {"density": 20.0 * pairs + 14.0 * s.n, "force": 54.0 * pairs},
-            "achieved_tflops": {"density": dens_tf, "force": force_tf}, "nominal_peak_tflops": fp32_peak,
-            "frac": {"density": dens_tf / fp32_peak, "force": force_tf / fp32_peak},
+            "useful_flop_both_passes": flop, "achieved_tflops": flop / t_pair / 1e12,
+            "nominal_peak_tflops": fp32_peak, "frac": flop / t_pair / 1e12 / fp32_peak,
             "peak_source": "nominal: 152 SMs x 128 FP32 lanes x 2 flop x max SM clock (not measured)",
             "pairs_source": "42 lattice neighbours within rc per atom, counted once per unordered pair"}
 

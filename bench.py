@@ -8,7 +8,7 @@ neighbour rebuild every 10 steps, mixed precision (FP32 pair arithmetic,
 FP64 state).  One step = first half push + (rebuild) + density/embedding +
 force + second half push, for all atoms.
 
-Reported (one JSON line on rank 0):
+Reported (one short JSON line on rank 0; the whole record with --full FILE):
   value      device-resident throughput (state in HBM, K steps timed with
              CUDA events on the library's stream, CUDA graph of 2 rebuild
              intervals, thermo every 20 steps)
@@ -112,6 +112,9 @@ def parse():
                    help="skip the 1,000-step mixed / 200-step FP64 NVE drift section")
     p.add_argument("--no-oracle-check", action="store_true",
                    help="skip the force error against the FP64 oracle at the benchmarked state")
+    p.add_argument("--full", default="",
+                   help="file for the whole record (timelines, tuning, drift, traffic) of which the printed line is "
+                        "the short form")
     a = p.parse_args()
     if a.list_buffer >= 0.0:
         WORKLOADS[a.workload] = dict(WORKLOADS[a.workload], list_buffer=a.list_buffer)
@@ -869,6 +872,41 @@ def measure(args, w, ws, dev, stream, torch, *, steps, fp64_steps, e2e_steps, dr
     return out
 
 
+def brief(out):
+    """The printed line: the contract's fields and one figure of each section,
+    short enough for a reader that keeps the last few thousand characters."""
+    def num(v):
+        return float("%.6g" % v) if isinstance(v, float) else v
+
+    def pick(d, keys):
+        return {k: num(d[k]) for k in keys if isinstance(d, dict) and d.get(k) is not None}
+
+    def short(d, n):
+        return {k: v if not isinstance(v, str) or len(v) <= n else v[:n - 3] + "..." for k, v in d.items()}
+
+    line = {k: num(out[k]) for k in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step",
+                                     "higher_is_better", "scaling", "vs_baseline", "dtype", "data", "gpu_launches")
+            if k in out}
+    line["config"] = short(pick(out["config"], ("workload", "description", "atoms", "precision", "rebuild_every",
+                                                "thermo_every", "lanes_per_atom", "list_entries_per_load", "block",
+                                                "parallelism", "l2", "cuda_graph")), 180)
+    line["clocks"] = pick(out["clocks"], ("sm_mhz", "sm_max_mhz", "reasons"))
+    e2e = ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step", "ms_per_step")
+    for k, keys in (("e2e", e2e), ("roofline", ("kernel", "bound", "achieved", "peak", "unit", "frac")),
+                    ("fp64", ("value", "mixed_over_fp64")), ("accuracy", ("force_rel_rms_error_mixed_vs_oracle", "force_rel_rms_error_fp64_vs_oracle")),
+                    ("cpu_baseline", ("value", "unit", "cores", "kind", "sample")),
+                    ("batched_replicas", ("replicas", "ms_forward_adjoint_persistent_graph")),
+                    ("parameter_adjoint", ("configurations", "ms_per_loss_and_gradient"))):
+        if k in out:
+            line[k] = short(pick(out[k], keys), 120)
+    for k in ("lj_mixture", "lj_fcc_32k"):
+        if k in out:
+            line[k] = pick(out[k], ("value", "ms_per_step"))
+            if "e2e" in out[k]:
+                line[k]["e2e"] = num(out[k]["e2e"]["value"])
+    return line
+
+
 def main():
     args = parse()
     w = WORKLOADS[args.workload]
@@ -929,7 +967,10 @@ def main():
             c1.pop(k, None)
         out["lj_fcc_32k"] = c1
     if rank == 0:
-        print(json.dumps(out), flush=True)
+        if args.full:
+            with open(args.full, "w") as fh:
+                json.dump(out, fh, indent=1)
+        print(json.dumps(brief(out)), flush=True)
     if ws > 1:
         import torch.distributed as dist
         dist.destroy_process_group()

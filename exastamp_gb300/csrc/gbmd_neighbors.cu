@@ -18,6 +18,7 @@
 //                 the FP32 local + FP64 packed gather copies    HBM: ~130 B r/w, 48 B w
 //   k_build_list_cells  warp per home cell over the 27-cell candidates, rows
 //                 in canonical order                            HBM: 4 B per entry
+//   k_build_list_long   the same rows where they are long, a warp per atom
 //
 // Every kernel of the chain takes a `gate` word: when it is non-null and
 // holds 0 the kernel returns at once.  The displacement-triggered step
@@ -747,12 +748,12 @@ __global__ void __launch_bounds__(BUILD_WARPS * 32, 6) k_build_list_cells(const 
 
 // The same list where rows are long: a warp per atom, 32 candidates at a time,
 // the hits straight to the row in global memory.  The walk above holds 16 rows
-// a warp in shared memory: at BUILD_LONG entries an SM has 4 of its warps, from
-// 3,000 entries on a group has fewer atoms, and a row of 51,000 does not fit at
-// all.  Rebuild, us, walk above / this: 256,000 atoms, capacity 560: 1,492 / 2,091;
-// 728: 2,217 / 2,485; 1,000: 3,761 / 3,035; 62,500 atoms, 560: 623 / 623;
-// 1,000: 1,330 / 861; 2,750: 8,400 / 2,270; 8,788 atoms, 6,200: 39,000 / 3,290;
-// 19,600: 6,150,000 / 157,000.
+// a warp in shared memory: at BUILD_LONG entries an SM has 3 of its warps, and
+// longer rows need fewer atoms a warp, up to 51,000 entries where one row does
+// not fit.  Rebuild, us, walk above (fewer atoms a warp from 3,000 entries) / this:
+// 256,000 atoms, capacity 560: 1,492 / 2,091; 728: 2,217 / 2,485; 1,000: 3,761 /
+// 3,035; 62,500 atoms, 560: 623 / 623; 1,000: 1,330 / 861; 2,750: 8,400 / 2,270;
+// 8,788 atoms, 6,200: 39,000 / 3,290; 19,600: 6,150,000 / 157,000.
 template <bool HALF>
 __global__ void __launch_bounds__(128) k_build_list_long(const __grid_constant__ BuildArgs A,
                                                          const __grid_constant__ Grid g,
